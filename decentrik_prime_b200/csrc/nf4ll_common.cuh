@@ -379,6 +379,13 @@ __device__ __forceinline__ uint4 drop8(uint4 raw, uint2 m, float keep_scale) {
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// one whole 32-byte sector (dst 32-byte aligned)
+__device__ __forceinline__ void store_sector(void* dst, const uint4& a, const uint4& b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+               "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // Gated SiLU on 8 packed fp16 values (fp32 math), shared by the stand-alone kernels and the fused
 // gate|up epilogue

@@ -1,36 +1,73 @@
-// Standalone NF4 -> fp16 dequantisation (the bit-exactness probe, and the launcher behind the
-// k_nf4-compatible dequant_layer / dequant_range for callers that still want an fp16 workspace).
+// Standalone NF4 -> fp16 dequantisation: the launcher behind the k_nf4-compatible dequant_layer /
+// dequant_range, and the weight pass in front of the large-batch GEMM (nf4ll_dense.cu).
 // Replaces the reference's nf4_layer_dequant_kernel (solution/k_nf4.py:40-57).
 //
-// Memory-bound: 0.516 B read + 2 B written per weight. One thread decodes half a quantisation
-// block per step: one 128-bit load of 32 codes, coalesced across the warp, and four 128-bit
-// stores. The 16 levels never touch memory: each thread builds the block's 16 fp16 products in
+// Memory-bound: 0.516 B read + 2 B written per weight. One thread decodes half a quantisation block (32 weights)
+// per step: one 128-bit load of codes, coalesced across the warp, and two 256-bit stores, each a whole 32-byte
+// sector (with four 128-bit stores per thread, 64 bytes apart across the warp, every store instruction touched 32
+// half-written sectors). The 16 levels never touch memory: each thread builds the block's 16 fp16 products in
 // registers and looks codes up with byte permutes.
-#include "nf4ll_common.cuh"
+#include "nf4ll_dequant.cuh"
 
 namespace nf4ll {
 
 constexpr int kDequantThreads = 256;
 
+// ALIGNED: `out` starts on a 32-byte boundary. `side`: small jobs done on the way for the GEMM that follows.
+template <bool ALIGNED>
 __global__ void __launch_bounds__(kDequantThreads)
 dequant_kernel(const uint4* __restrict__ nib, const uint8_t* __restrict__ qabs,
                const float* __restrict__ scale2, const float* __restrict__ offset2,
-               const float* __restrict__ code2, int64_t n_half_blocks, uint4* __restrict__ out) {
+               const float* __restrict__ code2, int64_t n_half_blocks, uint4* __restrict__ out, const DequantSide side) {
   __shared__ float s_code2[256];
   s_code2[threadIdx.x] = code2[threadIdx.x];
   __syncthreads();
+  pdl_wait();
+  pdl_launch_dependents();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kDequantThreads;
-  for (int64_t h = static_cast<int64_t>(blockIdx.x) * kDequantThreads + threadIdx.x; h < n_half_blocks; h += stride) {
+  const int64_t first = static_cast<int64_t>(blockIdx.x) * kDequantThreads + threadIdx.x;
+  for (int k = 0; k < side.n_left; ++k) {
+    // the rank-16 left operand of the fused LoRA step, rounded as the in-kernel staging of the other GEMMs rounds it
+    const float4* src = reinterpret_cast<const float4*>(side.left32[k]);
+    uint2* dst = reinterpret_cast<uint2*>(side.left16 + static_cast<int64_t>(k) * side.left_elems);
+    const float s = side.left_scale[k];
+    for (int64_t i = first; i < side.left_elems / 4; i += stride) {
+      const float4 v = src[i];
+      dst[i] = make_uint2(pack_half2_rn(v.x * s, v.y * s), pack_half2_rn(v.z * s, v.w * s));
+    }
+  }
+  for (int64_t h = first; h < n_half_blocks; h += stride) {
     const int64_t qb = h >> 1;
     const uint4 codes = __ldg(nib + h);
     const float absmax = block_absmax(s_code2[__ldg(qabs + qb)], __ldg(scale2 + (qb >> 8)), __ldg(offset2 + (qb >> 8)));
     const BlockTable t = make_block_table(absmax);
     uint4* dst = out + h * 4;
-    dst[0] = decode_word(t, codes.x);
-    dst[1] = decode_word(t, codes.y);
-    dst[2] = decode_word(t, codes.z);
-    dst[3] = decode_word(t, codes.w);
+    if (ALIGNED) {
+      store_sector(dst, decode_word(t, codes.x), decode_word(t, codes.y));
+      store_sector(dst + 2, decode_word(t, codes.z), decode_word(t, codes.w));
+    } else {
+      dst[0] = decode_word(t, codes.x);
+      dst[1] = decode_word(t, codes.y);
+      dst[2] = decode_word(t, codes.z);
+      dst[3] = decode_word(t, codes.w);
+    }
   }
+}
+
+int dequant_launch(const uint8_t* nib, const uint8_t* qabs, const float* scale2, const float* offset2, const float* code2,
+                   int64_t n_qblocks, void* out_f16, const DequantSide& side, cudaStream_t stream) {
+  const int64_t n_half = n_qblocks * 2;
+  int dev = 0, sms = 148;
+  NF4LL_CUDA(cudaGetDevice(&dev));
+  NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int64_t blocks = (n_half + kDequantThreads - 1) / kDequantThreads;
+  const int64_t cap = static_cast<int64_t>(sms) * 8;   // whole waves of 8 resident CTAs per SM
+  if (blocks > cap) blocks = cap;
+  auto kernel = (reinterpret_cast<uintptr_t>(out_f16) & 31) ? dequant_kernel<false> : dequant_kernel<true>;
+  PdlLaunch lc(dim3(static_cast<unsigned>(blocks)), dim3(kDequantThreads), 0, stream);
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, kernel, reinterpret_cast<const uint4*>(nib), qabs, scale2, offset2, code2, n_half,
+                                reinterpret_cast<uint4*>(out_f16), side));
+  return NF4LL_OK;
 }
 
 }  // namespace nf4ll
@@ -53,16 +90,5 @@ extern "C" int nf4ll_dequant(const uint8_t* nib, const uint8_t* qabs, const floa
     return NF4LL_ERR_ALIGN;
   }
   if (int rc = require_sm100()) return rc;
-  const int64_t n_half = n_qblocks * 2;
-  int dev = 0, sms = 148;
-  NF4LL_CUDA(cudaGetDevice(&dev));
-  NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  int64_t blocks = (n_half + kDequantThreads - 1) / kDequantThreads;
-  const int64_t cap = static_cast<int64_t>(sms) * 8;   // whole waves of 8 resident CTAs per SM
-  if (blocks > cap) blocks = cap;
-  count_launch();
-  dequant_kernel<<<static_cast<unsigned>(blocks), kDequantThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      reinterpret_cast<const uint4*>(nib), qabs, scale2, offset2, code2, n_half, reinterpret_cast<uint4*>(out_f16));
-  NF4LL_CUDA(cudaGetLastError());
-  return NF4LL_OK;
+  return dequant_launch(nib, qabs, scale2, offset2, code2, n_qblocks, out_f16, DequantSide{}, static_cast<cudaStream_t>(stream));
 }

@@ -26,6 +26,8 @@
 // one W row (= one quantisation block, 128 bytes), 8 rows per 1024-byte swizzle atom. Forward reads
 // it as a K-major B operand (contraction along the row), backward as an MN-major one (contraction
 // across rows), so the same NF4 bytes serve W and W^T.
+#include "nf4ll_dense.cuh"
+#include "nf4ll_dequant.cuh"
 #include "nf4ll_gemm_shared.cuh"
 
 namespace nf4ll {
@@ -978,20 +980,22 @@ static int get_encode_fn(EncodeTiledFn* out) {
   return NF4LL_OK;
 }
 
-// 2-D map over a row-major matrix [rows, cols] with leading dimension ld (elements): boxes of 128
-// rows x 128 bytes (the swizzle span: 64 fp16 or 32 fp32 columns); loads zero-fill outside the
-// matrix, stores are clipped to it.
-static int make_tile_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, bool f32) {
+// 2-D map over a row-major matrix [rows, cols] with leading dimension ld (elements): boxes of `box_rows`
+// rows x 128 bytes (the swizzle span: 64 fp16 or 32 fp32 columns), or x `box_cols` columns without swizzle;
+// loads zero-fill outside the matrix, stores are clipped to it.
+static int make_tile_map(CUtensorMap* map, const void* base, int64_t rows, int64_t cols, int64_t ld, bool f32,
+                         unsigned box_rows = 128, unsigned box_cols = 0) {
   EncodeTiledFn enc = nullptr;
   if (int rc = get_encode_fn(&enc)) return rc;
   const int esz = f32 ? 4 : 2;
   const cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   const cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * esz};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(128 / esz), 128};
+  const cuuint32_t box[2] = {box_cols ? box_cols : static_cast<cuuint32_t>(128 / esz), box_rows};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2,
                          const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                         CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                         box_cols ? CU_TENSOR_MAP_SWIZZLE_NONE : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_detail("cuTensorMapEncodeTiled failed with CUresult %d (rows=%lld cols=%lld ld=%lld)", static_cast<int>(r),
                static_cast<long long>(rows), static_cast<long long>(cols), static_cast<long long>(ld));
@@ -1235,6 +1239,133 @@ static int64_t small_batch_scratch(int kind, int64_t N, int64_t K, int64_t M, in
   return kind == kStream ? stream_workspace_bytes(N, K, M, sms, force_slices) : swap_workspace_bytes(N, K, M, sms, force_slices);
 }
 
+// ---------------------------------------------------------------------------------------------
+// Large batches: one dequantisation pass into an fp16 scratch, then the dense GEMM (nf4ll_dense.cu)
+// ---------------------------------------------------------------------------------------------
+// Below this many rows decoding inside the GEMM is cheaper than the extra pass over the weight (measured on B200: the
+// 7B-shaped layer of 16384 rows takes 14.3 ms instead of 16.7 ms, at 2048 rows the two are level).
+constexpr int64_t kDenseMinRows = 3072;
+
+// Scratch of a dense call: the rank-16 products the caller does not keep, lora_B transposed (backward), the fp16
+// weight, the rounded rank-16 operands of up to `n_left` branches.
+struct DenseScratch {
+  int64_t left, bt, w16, left16, total;
+};
+static DenseScratch dense_scratch(int64_t M, int64_t N, int64_t K, bool keep_left, bool transpose_b, int n_left) {
+  DenseScratch s{};
+  int64_t at = 0;
+  auto take = [&](int64_t bytes) { const int64_t o = at; at += align256(bytes); return o; };
+  s.left = take(keep_left ? M * 16 * 4 : 0);
+  s.bt = take(transpose_b ? N * 16 * 2 : 0);
+  s.w16 = take(N * K * 2);
+  s.left16 = take(static_cast<int64_t>(n_left) * M * 16 * 2);
+  s.total = at;
+  return s;
+}
+
+// Whether a call runs on the dense path: enough rows that one extra pass over the weights costs less than decoding
+// them once per row block, and a workspace that holds the fp16 weight.
+static bool dense_wanted(int64_t M, const Tune& tune) {
+  return (M >= kDenseMinRows || (tune.flags & 16)) && !tune.any() && !(tune.flags & 8) && g_expire_polls == 0;
+}
+
+struct DenseCall {
+  int mode;
+  const nf4ll_mat* W;
+  const void* act; int64_t ldact;
+  const void* bias;
+  int64_t M;
+  void* out; int64_t ldo;
+  int accumulate;
+  // branches: one (n_seg == 0), or one per stacked segment / per half of gate|up
+  int n_branch;
+  int64_t begin[kMaxSegments], rows[kMaxSegments];
+  const nf4ll_lora* lora[kMaxSegments];
+  void* side[kMaxSegments];        // fp32 [M,16] destination of the branch's product, or null: workspace
+  bool side_ready[kMaxSegments];
+  bool stacked;
+  int64_t gu_inter;
+  void* out_u; int64_t ldu;
+  void* out_h; int64_t ldh;
+};
+
+static int dense_branches(const DenseCall& c) {
+  int n = 0;
+  for (int i = 0; i < c.n_branch; ++i) n += c.lora[i] != nullptr;
+  return n;
+}
+static DensePlan dense_call_plan(const DenseCall& c, int sms) {
+  const int64_t NO = c.mode == kFwd ? c.W->N : c.W->K, KC = c.mode == kFwd ? c.W->K : c.W->N;
+  return dense_plan(c.M, NO, KC, c.gu_inter, sms);
+}
+static DenseScratch dense_call_scratch(const DenseCall& c) {
+  const bool one = c.n_branch == 1 && c.lora[0];
+  return dense_scratch(c.M, c.W->N, c.W->K, one && !c.side[0], c.mode == kBwd && one && !c.lora[0]->Bt, dense_branches(c));
+}
+
+static int run_dense(const DenseCall& c, const DensePlan& d, int sms, const DenseScratch& sc, uint8_t* ws, int32_t* status, cudaStream_t stream) {
+  const nf4ll_mat* W = c.W;
+  const bool fwd = c.mode == kFwd;
+  const int64_t NO = fwd ? W->N : W->K, KC = fwd ? W->K : W->N;
+  DenseMaps maps;
+  DenseParams p{};
+  DequantSide side{};
+  p.M = c.M; p.NO = NO; p.nkb = d.nkb;
+  p.tiles_m = static_cast<int>(d.tiles_m); p.tiles_o = static_cast<int>(d.tiles_o);
+  p.bias = static_cast<const __half*>(c.bias);
+  p.accumulate = c.accumulate;
+  p.n_seg = c.stacked ? c.n_branch : 0;
+  p.gu_inter = c.gu_inter;
+  p.status = status;
+  side.left16 = reinterpret_cast<__half*>(ws + sc.left16);
+  side.left_elems = c.M * 16;
+  for (int i = 0; i < c.n_branch; ++i) {
+    p.seg_begin[i] = c.begin[i]; p.seg_rows[i] = c.rows[i];
+    p.lora_index[i] = -1;
+    const nf4ll_lora* l = c.lora[i];
+    if (!l) continue;
+    float* left = c.side[i] ? static_cast<float*>(c.side[i]) : reinterpret_cast<float*>(ws + sc.left);
+    if (fwd) {
+      if (!c.side_ready[i])
+        if (int rc = lora_down_launch(c.act, c.ldact, l->mask, l->ld_mask, l->keep_scale, l->A, 1.0f, c.M, W->K, left, nullptr, 0, stream)) return rc;
+      if (int rc = make_tile_map(&maps.right[i], l->B, c.rows[i], 16, 16, false, 128, 8)) return rc;
+    } else {
+      const void* bt = l->Bt;
+      if (!bt) {
+        void* tmp = ws + sc.bt;
+        if (int rc = transpose_n16_launch(l->B, tmp, W->N, stream)) return rc;
+        bt = tmp;
+      }
+      if (int rc = lora_down_launch(c.act, c.ldact, nullptr, 0, 1.0f, bt, l->scale, c.M, W->N, left, nullptr, 0, stream)) return rc;
+      if (int rc = make_tile_map(&maps.right[i], l->A, 16, W->K, W->K, false, 16)) return rc;
+      p.mask = l->mask; p.ld_mask = l->ld_mask; p.keep_scale = l->keep_scale;
+    }
+    side.left32[p.n_lora] = left;
+    side.left_scale[p.n_lora] = fwd ? l->scale : 1.0f;
+    p.lora_index[i] = p.n_lora++;
+  }
+  side.n_left = p.n_lora;
+  if (p.n_lora)
+    if (int rc = make_tile_map(&maps.left, side.left16, static_cast<int64_t>(p.n_lora) * c.M, 16, 16, false, 128, 8)) return rc;
+  void* w16 = ws + sc.w16;
+  if (int rc = make_tile_map(&maps.act, c.act, c.M, KC, c.ldact, false)) return rc;
+  if (int rc = make_tile_map(&maps.w, w16, W->N, W->K, W->K, false, fwd ? 128 : 64)) return rc;
+  p.out = static_cast<__half*>(c.out); p.ldo = c.ldo;
+  const int64_t out_cols = c.gu_inter ? c.gu_inter : NO;
+  if (int rc = make_tile_map(&maps.out, c.out, c.M, out_cols, c.ldo, false, 32)) return rc;
+  if (c.gu_inter) {
+    if (int rc = make_tile_map(&maps.out_u, c.out_u, c.M, out_cols, c.ldu, false, 32)) return rc;
+    if (int rc = make_tile_map(&maps.out_h, c.out_h, c.M, out_cols, c.ldh, false, 32)) return rc;
+  }
+  cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
+  g_ev_start = g_ev_stop = nullptr;
+  if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
+  if (int rc = dequant_launch(W->nib, W->qabs, W->scale2, W->offset2, W->code2, W->N * W->K / 64, w16, side, stream)) return rc;
+  const int rc = dense_launch(c.mode, maps, p, d, sms, stream);
+  if (rc == NF4LL_OK && ev1) { if (int rce = record_event(ev1, stream)) return rce; }
+  return rc;
+}
+
 // `segments` (forward only): the weight is several projections stacked along N, each with its own
 // optional LoRA branch; `lora` / `side_out` are then unused.
 static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact, const void* bias,
@@ -1272,6 +1403,25 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     if (at != W->N) { set_detail("%s: segments cover %lld of %lld rows", who, static_cast<long long>(at), static_cast<long long>(W->N)); return NF4LL_ERR_SHAPE; }
   }
   Tune tune = g_tune;
+  if (dense_wanted(M, tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
+    DenseCall c{};
+    c.mode = mode; c.W = W; c.act = act; c.ldact = ldact; c.bias = bias; c.M = M; c.out = out; c.ldo = ldo; c.accumulate = accumulate;
+    c.stacked = segments != nullptr;
+    c.n_branch = segments ? n_segments : 1;
+    if (segments) {
+      int64_t at = 0;
+      for (int i = 0; i < n_segments; ++i) {
+        c.begin[i] = at; c.rows[i] = segments[i].rows; c.lora[i] = segments[i].lora;
+        c.side[i] = segments[i].t_out; c.side_ready[i] = segments[i].t_ready != 0;
+        at += segments[i].rows;
+      }
+    } else {
+      c.rows[0] = NO; c.lora[0] = lora; c.side[0] = side_out;
+    }
+    const DensePlan d = dense_call_plan(c, sms);
+    const DenseScratch sc = dense_call_scratch(c);
+    if (workspace_bytes >= sc.total) return run_dense(c, d, sms, sc, static_cast<uint8_t*>(workspace), status, stream);
+  }
   if (segments && (narrow_tiles || tune.bn == 512)) tune.bn = narrow_tiles ? 128 : 256;
   Plan pl = make_plan(mode, M, NO, KC, lora ? lora->r : 0, sms, tune);
   const int kind = forward_kind(mode, M, W->N, W->K, segments != nullptr, tune);
@@ -1441,6 +1591,18 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     if (int rc = run_gemm(kFwd, &wu, x, ldx, nullptr, lora_up, t_up, M, u, ldu, 0, workspace, workspace_bytes, status, stream_v)) return rc;
     return nf4ll_swiglu_forward(g, ldg, u, ldu, h, ldh, M, I, stream_v);
   }
+  if (dense_wanted(M, g_tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
+    DenseCall c{};
+    c.mode = kFwd; c.W = W; c.act = x; c.ldact = ldx; c.M = M; c.out = g; c.ldo = ldg;
+    c.out_u = u; c.ldu = ldu; c.out_h = h; c.ldh = ldh; c.gu_inter = I; c.n_branch = 2;
+    c.rows[0] = c.rows[1] = I; c.begin[1] = I;
+    c.lora[0] = lora_gate; c.lora[1] = lora_up; c.side[0] = t_gate; c.side[1] = t_up;
+    int sms = 148;
+    if (int rc = device_sms(&sms)) return rc;
+    const DensePlan d = dense_call_plan(c, sms);
+    const DenseScratch sc = dense_call_scratch(c);
+    if (workspace_bytes >= sc.total) return run_dense(c, d, sms, sc, static_cast<uint8_t*>(workspace), status, stream);
+  }
   GemmParams p{};
   p.nib = W->nib; p.qabs = W->qabs; p.scale2 = W->scale2; p.offset2 = W->offset2; p.code2 = W->code2;
   p.N = W->N; p.K = W->K; p.M = M; p.NO = W->N; p.KC = W->K;
@@ -1537,6 +1699,15 @@ extern "C" int64_t nf4ll_workspace_bytes_tuned(int64_t M, int64_t N, int64_t K, 
   const int sms = sms_or_default();
   const int64_t f = forward_need(M, N, K, r, sms, tune), b = make_plan(kBwd, M, K, N, r, sms, tune).total();
   return f > b ? f : b;
+}
+
+extern "C" int64_t nf4ll_workspace_bytes_fast(int64_t M, int64_t N, int64_t K, int32_t r) {
+  using namespace nf4ll;
+  int64_t need = nf4ll_workspace_bytes(M, N, K, r);
+  if (M < kDenseMinRows || N <= 0 || K <= 0) return need;
+  const int64_t n = dense_scratch(M, N, K, r > 0, r > 0, r > 0 ? kMaxSegments : 0).total;
+  if (n > need) need = n;
+  return need;
 }
 
 extern "C" int nf4ll_forward(const nf4ll_mat* W, const void* x, int64_t ldx, const void* bias, const nf4ll_lora* lora,

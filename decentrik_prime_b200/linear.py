@@ -73,7 +73,7 @@ _state = _DeviceState()
 def _workspace_need(M, N, K, r):
     if any(_state.tune):
         return _lib.lib().nf4ll_workspace_bytes_tuned(M, N, K, r, *_state.tune)
-    return _lib.lib().nf4ll_workspace_bytes(M, N, K, r)
+    return _lib.lib().nf4ll_workspace_bytes_fast(M, N, K, r)
 
 
 @contextlib.contextmanager
@@ -222,7 +222,7 @@ def forward_gate_up(w: Nf4Weight, x, lora_gate=None, mask_gate=None, lora_up=Non
     tg = torch.empty(M, RANK, dtype=torch.float32, device=x.device) if lora_gate is not None else None
     tu = torch.empty(M, RANK, dtype=torch.float32, device=x.device) if lora_up is not None else None
     r = RANK if (lora_gate is not None or lora_up is not None) else 0
-    ws = _workspace(x.device, _workspace_need(M, I, w.K, r)) if workspace is None else workspace
+    ws = _workspace(x.device, max(_workspace_need(M, I, w.K, r), _workspace_need(M, w.N, w.K, r))) if workspace is None else workspace
     _lib.check(_lib.lib().nf4ll_forward_gate_up(ctypes.byref(w._c), x.data_ptr(), x.stride(0), rg, ru,
                                                 None if tg is None else tg.data_ptr(), None if tu is None else tu.data_ptr(),
                                                 M, g.data_ptr(), g.stride(0), u.data_ptr(), u.stride(0), h.data_ptr(),

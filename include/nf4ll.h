@@ -89,6 +89,12 @@ int nf4ll_dequant(const uint8_t* nib, const uint8_t* qabs, const float* scale2, 
  * partial sums and tile counters. Always a multiple of 256; the workspace must be 256-byte aligned. */
 int64_t nf4ll_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t r);
 
+/* Scratch with which the calls on W[N,K] run at their best: from several hundred rows on it also holds one fp16 copy of
+ * the weight (2 N K bytes), so that a call dequantises once and multiplies by that. With a smaller workspace (at least
+ * nf4ll_workspace_bytes) the same calls decode the weight inside the GEMM instead. N is the row count of the whole
+ * stacked matrix for nf4ll_forward_multi and nf4ll_forward_gate_up. No counterpart in the reference. */
+int64_t nf4ll_workspace_bytes_fast(int64_t M, int64_t N, int64_t K, int32_t r);
+
 /* The same figure for calls made under nf4ll_tune_override(bm_tiles, bn, splits, ...): a forced split
  * count or tile shape changes the scratch a call needs. nf4ll_workspace_bytes itself never depends on
  * the calling thread's override. Testing hook; no counterpart in the reference. */
@@ -242,7 +248,9 @@ int nf4ll_read_status(const int32_t* status, void* stream);
  * sum to whichever of them finishes last), e.g. under a profiler that replays kernels one at a time.
  * flags bit 1: run a forward of at most 64 rows on the register-level weight-streaming kernel (default: up to
  * 16 rows); flags bit 2: run a forward of at most 64 rows on the swapped-operand tensor-core kernel (default:
- * 9 to 32 rows against weights of at least 2^24 elements, 33 to 64 rows against at least 2^26). With bit 1 or 2, `splits` forces that kernel's
+ * 9 to 32 rows against weights of at least 2^24 elements, 33 to 64 rows against at least 2^26); flags bit 3: never
+ * dequantise into the workspace, whatever its size; flags bit 4: do so for any number of rows if the workspace holds
+ * 2 N K + 192 M + 32 N + 2048 bytes. With bit 1 or 2, `splits` forces that kernel's
  * number of slices of the contraction. Size the workspace of such calls with nf4ll_workspace_bytes_tuned. */
 void nf4ll_tune_override(int32_t bm_tiles, int32_t bn, int32_t splits, int32_t flags);
 

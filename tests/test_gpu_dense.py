@@ -1,0 +1,104 @@
+"""The large-batch path (one dequantisation pass, then the dense tcgen05 GEMM), forced through the tuning hook at the
+sizes where it can go wrong: rows around the 512-row tile and its 128-row quarters, columns around the 256-column tile,
+contractions of one to a few 64-wide steps, tiles cut into 2, 3 and 4 parts of the contraction (clusters), stacked
+segments whose boundaries fall inside a tile, gate|up tiles, accumulation into dx. Against the fp64 oracle at the path's
+tolerance: max-abs-err <= 2e-2 and rel-L2 <= 1e-3."""
+
+import pytest
+import torch
+
+from decentrik_prime_b200 import k_nf4, linear, quantize
+from oracle import nf4_oracle
+from tests.problem import make_problem, oracle_weight, to_device
+
+pytestmark = pytest.mark.gpu
+MAX_ABS, REL_L2 = 2e-2, 1e-3
+DENSE = 16
+
+
+def assert_close(name, got, ref):
+    err, rel = nf4_oracle.errors(got, ref)
+    assert err <= MAX_ABS and rel <= REL_L2, f"{name}: max-abs {err:.3e} rel-L2 {rel:.3e}"
+
+
+def workspace(M, N, K):
+    return torch.empty(2 * N * K + 192 * M + 32 * N + 2048, dtype=torch.uint8, device="cuda")
+
+
+# 256 x 64: one k-block; 1536 x 1536 at 513 rows: 12 tiles, four parts; 4864-wide outputs of 2 row blocks: three parts;
+# 7168 wide: two parts; 192 and 320 columns: ragged tiles
+@pytest.mark.parametrize("N,K,M", [(256, 64, 1), (256, 128, 127), (256, 192, 129), (256, 320, 256), (512, 512, 257), (320, 1024, 511),
+                                   (192, 256, 512), (1536, 1536, 513), (1024, 4864, 600), (768, 7168, 1025), (2048, 768, 700)])
+@pytest.mark.parametrize("lora,dropout,bias", [(True, 0.05, True), (True, 0.0, False), (False, 0.0, True)])
+def test_tile_edges(N, K, M, lora, dropout, bias):
+    pr = make_problem(N, K, M, seed=N + K + M, lora=lora, dropout=dropout, bias=bias)
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, pr.dy, pr.bias, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)
+    d = to_device(pr)
+    ws = workspace(M, N, K)
+    with linear.tune_override(flags=DENSE):
+        y, t = linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, want_t=lora, workspace=ws)
+        dx, u = linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, want_u=lora, workspace=ws)
+        linear.check_status()
+        assert_close("y", y, ref["y"])
+        assert_close("dx", dx, ref["dx"])
+        again, _ = linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, out=dx.clone(), accumulate=True, workspace=ws)
+        y2, _ = linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, workspace=ws)
+        linear.check_status()
+    if not lora:      # (the rank-16 product of a few hundred rows may be summed with atomics)
+        assert torch.equal(y, y2)
+    assert_close("dx + dx", again, 2 * ref["dx"])
+    if lora:
+        assert_close("t", t, ref["t"])
+        assert_close("u", u, ref["u"])
+
+
+@pytest.mark.parametrize("M,H,KV,I", [(300, 512, 128, 1024), (1100, 384, 128, 896)])
+def test_stacked_and_gate_up(M, H, KV, I):
+    """Q|K|V with segment boundaries inside a 256-column tile (LoRA on q and v), and gate|up with one and two branches."""
+    names = k_nf4.LAYER_WEIGHTS
+    shapes = {"q_proj": (H, H), "k_proj": (KV, H), "v_proj": (KV, H), "o_proj": (H, H), "gate_proj": (I, H), "up_proj": (I, H), "down_proj": (H, I)}
+    lin = {n: quantize.random_nf4_weight(*shapes[n], seed=700 + i, device="cuda") for i, n in enumerate(names)}
+    layer, code2 = k_nf4.repack_layer(lin, torch.device("cuda"))
+    gen = torch.Generator().manual_seed(M)
+    x = torch.randn(M, H, generator=gen).half()
+    ks = float(1.0 / torch.tensor(0.95, dtype=torch.float32))
+
+    def branch(n):
+        return ((torch.randn(16, H, generator=gen) * 0.05).half(), (torch.randn(n, 16, generator=gen) * 0.05).half(), 2.0)
+
+    def mask():
+        return (torch.rand(M, H, generator=gen) >= 0.05).to(torch.uint8)
+
+    def dev(l):
+        return None if l is None else (l[0].cuda(), l[1].cuda(), l[2])
+
+    def oracle(name, l, m, bias=None):
+        A, B, s = (None, None, 1.0) if l is None else l
+        return nf4_oracle.lora_linear_o1(nf4_oracle.dequant_weight(layer, name, code2), x, None, bias, A, B, s, m, ks if m is not None else 1.0)
+
+    qkv = ("q_proj", "k_proj", "v_proj")
+    rows = [shapes[n][0] for n in qkv]
+    bias = [(torch.randn(r, generator=gen) * 0.1).half() for r in rows]
+    loras, masks = [branch(rows[0]), None, branch(rows[2])], [mask(), None, mask()]
+    wg = linear.Nf4Weight.from_layer_group(layer, qkv, code2)
+    with linear.tune_override(flags=DENSE):
+        y, ts = linear.forward_multi(wg, x.cuda(), [(r, dev(l), None if m is None else m.cuda(), ks) for r, l, m in zip(rows, loras, masks)],
+                                     bias=torch.cat(bias).cuda(), workspace=workspace(M, wg.N, wg.K))
+        linear.check_status()
+    at = 0
+    for n, r, b, l, m, t in zip(qkv, rows, bias, loras, masks, ts):
+        ref = oracle(n, l, m, b)
+        assert_close(n, y[:, at:at + r], ref["y"])
+        if l is not None:
+            assert_close(n + " t", t, ref["t"])
+        at += r
+    w = linear.Nf4Weight.from_layer_group(layer, ("gate_proj", "up_proj"), code2)
+    for lg, lu in ((branch(I), branch(I)), (None, branch(I)), (None, None)):
+        mg, mu = (mask() if lg else None), (mask() if lu else None)
+        with linear.tune_override(flags=DENSE):
+            g, u, h, tg, tu = linear.forward_gate_up(w, x.cuda(), dev(lg), None if mg is None else mg.cuda(), dev(lu),
+                                                     None if mu is None else mu.cuda(), ks, workspace=workspace(M, w.N, w.K))
+            linear.check_status()
+        assert_close("g", g, oracle("gate_proj", lg, mg)["y"])
+        assert_close("u", u, oracle("up_proj", lu, mu)["y"])
+        assert torch.equal(h, linear.swiglu_forward(g.contiguous(), u.contiguous()))
