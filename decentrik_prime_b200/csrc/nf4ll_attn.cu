@@ -1,0 +1,642 @@
+// Rotary embedding + causal grouped-query attention over packed varlen rows, forward and backward: what lies between the
+// Q|K|V and O projections of a decoder layer (the reference has kernels of its own for it, solution/k_rope.py,
+// k_attn.py). Head dimensions 64 and 128, fp16 in and out, fp32 softmax statistics and accumulation.
+//
+// What bounds it: launches and latency. A data loader's batch is a handful of sequences of tens to a few thousand rows; a
+// 951-row batch at 12 heads is 0.8 GFLOP forward, so one kernel over all sequences and heads instead of a dozen launches
+// per sequence is the whole gain (through PyTorch: 280 launches per layer and step). The contractions use mma.sync:
+// tiles of 64 rows are too small to feed tcgen05, and at a few microseconds per launch there is nothing to win.
+// Sequence boundaries travel in the kernel parameters, so no copy to the device is needed per batch.
+//
+//   rope     q, k rotated once into a buffer (a key row is read by every query tile after it)
+//   forward  one CTA per 64 query rows and head, 4 warps of 16 rows, keys and values in 64-row blocks by cp.async
+//   dK, dV   one CTA per 64 key rows and key-value head, looping over the group's query heads and the later query rows:
+//            sums over heads stay in registers, no atomics
+//   dQ       one CTA per 64 query rows and head, looping over the earlier key rows
+// The backward kernels rotate dQ and dK back in their epilogue (both halves of a rotated pair sit in one thread).
+#include "nf4ll_common.cuh"
+
+namespace nf4ll {
+
+constexpr int kAttnMaxSeqs = 128;            // sequences per launch (longer lists are cut)
+constexpr int kAttnRows = 64;
+constexpr int kAttnThreads = 128;
+
+struct SeqTable {
+  int n;
+  int start[kAttnMaxSeqs + 1];               // first row of each sequence
+  int tile[kAttnMaxSeqs + 1];                // tiles of 64 rows before each sequence
+};
+
+struct AttnParams {
+  const __half* q;      // rotated [rows, ldr]: query heads, then key heads
+  const __half* k;
+  int64_t ldr;
+  const __half* v;      // [rows, ldv]
+  int64_t ldv;
+  const __half* o;      // attention output [rows, ldo] (backward)
+  __half* out;          // forward output
+  int64_t ldo;
+  const __half* dout;   // [rows, lddo]
+  int64_t lddo;
+  __half *dq, *dk, *dv; // [rows, ldd]
+  int64_t ldd;
+  float* lse;           // [heads, rows]: log2-sum-exp2 of the scaled scores
+  float* delta;         // [heads, rows]: sum(dout * o)
+  const float2* trig;   // [positions, hd / 2] (cos, sin)
+  int heads, group;     // query heads, query heads per key-value head
+  int64_t rows;
+  float scale_log2, scale;
+};
+
+__device__ __forceinline__ void attn_cp16(uint32_t dst, const void* src, bool valid) {
+  const int n = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void attn_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void attn_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ void ldsm4t(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
+__device__ __forceinline__ float exp2_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// A tile of ROWS x HD fp16 in shared memory: rows of HD * 2 bytes, 16-byte chunks XOR-swizzled by the row so that the
+// ldmatrix rows of a matrix fall into different banks.
+template <int HD>
+__device__ __forceinline__ uint32_t tile_addr(uint32_t base, int row, int chunk) {
+  return base + row * (HD * 2) + ((chunk ^ (row & 7)) << 4);
+}
+template <int HD, int ROWS>
+__device__ __forceinline__ void load_tile(uint32_t base, const __half* src, int64_t ld, int row0, int end) {
+  constexpr int CH = HD / 8;
+#pragma unroll
+  for (int i = 0; i < ROWS * CH / kAttnThreads; ++i) {
+    const int idx = threadIdx.x + i * kAttnThreads, r = idx / CH, c = idx % CH;
+    const bool v = row0 + r < end;
+    attn_cp16(tile_addr<HD>(base, r, c), v ? src + (row0 + r) * ld + c * 8 : src, v);
+  }
+}
+// A fragment of rows r0 .. r0+15, columns 16 kk ..
+template <int HD>
+__device__ __forceinline__ void frag_a(uint32_t base, int r0, int kk, int lane, uint32_t (&a)[4]) {
+  ldsm4(tile_addr<HD>(base, r0 + (lane & 15), kk * 2 + (lane >> 4)), a);
+}
+// B fragments of two 8-wide n-tiles (rows n0 .. n0+15 of a [n][k] tile), k columns 16 kk ..: b[0..1] first, b[2..3] second
+template <int HD>
+__device__ __forceinline__ void frag_b(uint32_t base, int n0, int kk, int lane, uint32_t (&b)[4]) {
+  ldsm4(tile_addr<HD>(base, n0 + (lane & 7) + ((lane >> 4) << 3), kk * 2 + ((lane >> 3) & 1)), b);
+}
+// B fragments of two 8-wide n-tiles (columns n0 .. n0+15 of a [k][n] tile), k rows k0 .. k0+15
+template <int HD>
+__device__ __forceinline__ void frag_bt(uint32_t base, int k0, int n0, int lane, uint32_t (&b)[4]) {
+  ldsm4t(tile_addr<HD>(base, k0 + (lane & 15), n0 / 8 + (lane >> 4)), b);
+}
+
+__device__ __forceinline__ void find_tile(const SeqTable& t, int tile, int& start, int& len, int& t0) {
+  int lo = 0, hi = t.n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (t.tile[mid] <= tile) lo = mid; else hi = mid - 1;
+  }
+  start = t.start[lo];
+  len = t.start[lo + 1] - start;
+  t0 = (tile - t.tile[lo]) * kAttnRows;
+}
+
+// ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256)
+rope_kernel(const __half* __restrict__ src, int64_t lds, __half* __restrict__ dst, int64_t ldd, const float2* __restrict__ trig, int heads,
+            int hd, const __grid_constant__ SeqTable seqs) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int half = hd / 2, per_row = heads * (half / 8);
+  const int rows = seqs.start[seqs.n] - seqs.start[0];
+  for (int idx = blockIdx.x * 256 + threadIdx.x; idx < rows * per_row; idx += gridDim.x * 256) {
+    const int r = idx / per_row, c = idx - r * per_row;
+    const int head = c / (half / 8), j = (c - head * (half / 8)) * 8;
+    const int row = seqs.start[0] + r;
+    int lo = 0, hi = seqs.n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (seqs.start[mid] <= row) lo = mid; else hi = mid - 1;
+    }
+    const int pos = row - seqs.start[lo];
+    const __half* s = src + row * lds + head * hd + j;
+    float a[8], b[8], x[8], y[8];
+    unpack8(*reinterpret_cast<const uint4*>(s), a);
+    unpack8(*reinterpret_cast<const uint4*>(s + half), b);
+    const float4* tp = reinterpret_cast<const float4*>(trig + static_cast<int64_t>(pos) * half + j);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const float4 t = __ldg(tp + k);
+      x[2 * k] = a[2 * k] * t.x - b[2 * k] * t.y;
+      y[2 * k] = b[2 * k] * t.x + a[2 * k] * t.y;
+      x[2 * k + 1] = a[2 * k + 1] * t.z - b[2 * k + 1] * t.w;
+      y[2 * k + 1] = b[2 * k + 1] * t.z + a[2 * k + 1] * t.w;
+    }
+    __half* d = dst + row * ldd + head * hd + j;
+    *reinterpret_cast<uint4*>(d) = pack8(x);
+    *reinterpret_cast<uint4*>(d + half) = pack8(y);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+template <int HD>
+__global__ void __launch_bounds__(kAttnThreads)
+attn_fwd_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ SeqTable seqs) {
+  pdl_wait();
+  pdl_launch_dependents();
+  extern __shared__ __align__(128) uint8_t a_smem[];
+  constexpr int TILE = kAttnRows * HD * 2, KS = HD / 16, NT = HD / 8;
+  const uint32_t sQ = smem_u32(a_smem), sK = sQ + TILE, sV = sK + 2 * TILE;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  int start, len, q0;
+  find_tile(seqs, seqs.tile[seqs.n] - 1 - blockIdx.x, start, len, q0);      // later (longer) tiles first
+  const int head = blockIdx.y, kvh = head / p.group;
+  const __half* qp = p.q + start * p.ldr + head * HD;
+  const __half* kp = p.k + start * p.ldr + kvh * HD;
+  const __half* vp = p.v + start * p.ldv + kvh * HD;
+  const int n_blocks = q0 / kAttnRows + 1;
+  load_tile<HD, kAttnRows>(sQ, qp, p.ldr, q0, len);
+  load_tile<HD, kAttnRows>(sK, kp, p.ldr, 0, len);
+  load_tile<HD, kAttnRows>(sV, vp, p.ldv, 0, len);
+  attn_commit();
+  float o[NT][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[n][i] = 0.f;
+  const int row_a = q0 + warp * 16 + g;
+  for (int b = 0; b < n_blocks; ++b) {
+    const uint32_t kb = sK + (b & 1) * TILE, vb = sV + (b & 1) * TILE;
+    if (b + 1 < n_blocks) {
+      load_tile<HD, kAttnRows>(sK + ((b + 1) & 1) * TILE, kp, p.ldr, (b + 1) * kAttnRows, len);
+      load_tile<HD, kAttnRows>(sV + ((b + 1) & 1) * TILE, vp, p.ldv, (b + 1) * kAttnRows, len);
+    }
+    attn_commit();
+    attn_wait<1>();
+    __syncthreads();
+    float s[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) {
+      uint32_t a[4];
+      frag_a<HD>(sQ, warp * 16, kk, lane, a);
+#pragma unroll
+      for (int n2 = 0; n2 < 4; ++n2) {
+        uint32_t bf[4];
+        frag_b<HD>(kb, n2 * 16, kk, lane, bf);
+        mma16816(s[2 * n2], a[0], a[1], a[2], a[3], bf[0], bf[1]);
+        mma16816(s[2 * n2 + 1], a[0], a[1], a[2], a[3], bf[2], bf[3]);
+      }
+    }
+    if (b == n_blocks - 1) {                 // the diagonal block (rows past the sequence end are never keys of a live row)
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (b * kAttnRows + n * 8 + 2 * t + (i & 1) > row_a + (i >> 1) * 8) s[n][i] = -INFINITY;
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float mx = -INFINITY;
+#pragma unroll
+      for (int n = 0; n < 8; ++n) mx = fmaxf(mx, fmaxf(s[n][2 * h], s[n][2 * h + 1]));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+      mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+      const float mn = fmaxf(m[h], mx * p.scale_log2);
+      const float corr = exp2_fast(m[h] - mn);
+      m[h] = mn;
+      float sum = 0.f;
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        s[n][2 * h] = exp2_fast(fmaf(s[n][2 * h], p.scale_log2, -mn));
+        s[n][2 * h + 1] = exp2_fast(fmaf(s[n][2 * h + 1], p.scale_log2, -mn));
+        sum += s[n][2 * h] + s[n][2 * h + 1];
+      }
+      l[h] = l[h] * corr + sum;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) { o[n][2 * h] *= corr; o[n][2 * h + 1] *= corr; }
+    }
+#pragma unroll
+    for (int kk = 0; kk < 4; ++kk) {
+      const uint32_t a0 = pack_half2_rn(s[2 * kk][0], s[2 * kk][1]), a1 = pack_half2_rn(s[2 * kk][2], s[2 * kk][3]);
+      const uint32_t a2 = pack_half2_rn(s[2 * kk + 1][0], s[2 * kk + 1][1]), a3 = pack_half2_rn(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+#pragma unroll
+      for (int n2 = 0; n2 < NT / 2; ++n2) {
+        uint32_t bf[4];
+        frag_bt<HD>(vb, kk * 16, n2 * 16, lane, bf);
+        mma16816(o[2 * n2], a0, a1, a2, a3, bf[0], bf[1]);
+        mma16816(o[2 * n2 + 1], a0, a1, a2, a3, bf[2], bf[3]);
+      }
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 1);
+    l[h] += __shfl_xor_sync(0xffffffffu, l[h], 2);
+    const int r = row_a + 8 * h;
+    if (r < len) {
+      const float inv = 1.0f / l[h];
+      __half* dst = p.out + (start + r) * p.ldo + head * HD + 2 * t;
+#pragma unroll
+      for (int n = 0; n < NT; ++n) *reinterpret_cast<uint32_t*>(dst + n * 8) = pack_half2_rn(o[n][2 * h] * inv, o[n][2 * h + 1] * inv);
+      if (t == 0) p.lse[head * p.rows + start + r] = m[h] + log2f(l[h]);
+    }
+  }
+}
+
+// delta[head][row] = sum over the head's columns of dout * out; one warp per (row, head)
+template <int HD>
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __grid_constant__ AttnParams p, int first, int rows) {
+  pdl_wait();
+  pdl_launch_dependents();
+  constexpr int L = HD / 8;                  // lanes per (row, head)
+  const int idx = (blockIdx.x * 256 + threadIdx.x) / L, c = threadIdx.x % L;
+  const bool live = idx < rows * p.heads;
+  const int row = first + (live ? idx / p.heads : 0), head = live ? idx % p.heads : 0;
+  float a[8], b[8], s = 0.f;
+  unpack8(*reinterpret_cast<const uint4*>(p.dout + row * p.lddo + head * HD + c * 8), a);
+  unpack8(*reinterpret_cast<const uint4*>(p.o + row * p.ldo + head * HD + c * 8), b);
+#pragma unroll
+  for (int k = 0; k < 8; ++k) s = fmaf(a[k], b[k], s);
+#pragma unroll
+  for (int x = L / 2; x > 0; x >>= 1) s += __shfl_xor_sync(0xffffffffu, s, x);
+  if (live && c == 0) p.delta[head * p.rows + row] = s;
+}
+
+// Rotate a gradient back (transpose of the rotation) and store it: acc holds rows (g, g + 8) x HD columns of one warp.
+template <int HD>
+__device__ __forceinline__ void store_unrotated(const float (&acc)[HD / 8][4], const AttnParams& p, __half* base, int row_a, int len, int t, float mul) {
+  constexpr int NT = HD / 8;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = row_a + 8 * h;
+    if (r >= len) continue;
+    const float4* tp = reinterpret_cast<const float4*>(p.trig + static_cast<int64_t>(r) * (HD / 2) + 2 * t);
+    __half* dst = base + r * p.ldd + 2 * t;
+#pragma unroll
+    for (int n = 0; n < NT / 2; ++n) {
+      const float4 cs = __ldg(tp + n * 4);   // (cos, sin) of columns 8 n + 2 t, + 1
+      const float x0 = acc[n][2 * h] * mul, x1 = acc[n][2 * h + 1] * mul;
+      const float y0 = acc[n + NT / 2][2 * h] * mul, y1 = acc[n + NT / 2][2 * h + 1] * mul;
+      *reinterpret_cast<uint32_t*>(dst + n * 8) = pack_half2_rn(x0 * cs.x + y0 * cs.y, x1 * cs.z + y1 * cs.w);
+      *reinterpret_cast<uint32_t*>(dst + HD / 2 + n * 8) = pack_half2_rn(y0 * cs.x - x0 * cs.y, y1 * cs.z - x1 * cs.w);
+    }
+  }
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kAttnThreads)
+attn_dq_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ SeqTable seqs) {
+  pdl_wait();
+  pdl_launch_dependents();
+  extern __shared__ __align__(128) uint8_t a_smem[];
+  constexpr int TILE = kAttnRows * HD * 2, KS = HD / 16, NT = HD / 8;
+  const uint32_t sQ = smem_u32(a_smem), sO = sQ + TILE, sK = sO + TILE, sV = sK + 2 * TILE;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  int start, len, q0;
+  find_tile(seqs, seqs.tile[seqs.n] - 1 - blockIdx.x, start, len, q0);
+  const int head = blockIdx.y, kvh = head / p.group;
+  const __half* kp = p.k + start * p.ldr + kvh * HD;
+  const __half* vp = p.v + start * p.ldv + kvh * HD;
+  const int n_blocks = q0 / kAttnRows + 1;
+  load_tile<HD, kAttnRows>(sQ, p.q + start * p.ldr + head * HD, p.ldr, q0, len);
+  load_tile<HD, kAttnRows>(sO, p.dout + start * p.lddo + head * HD, p.lddo, q0, len);
+  load_tile<HD, kAttnRows>(sK, kp, p.ldr, 0, len);
+  load_tile<HD, kAttnRows>(sV, vp, p.ldv, 0, len);
+  attn_commit();
+  const int row_a = q0 + warp * 16 + g;
+  float lse[2], delta[2], dq[NT][4];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const bool live = row_a + 8 * h < len;
+    lse[h] = live ? p.lse[head * p.rows + start + row_a + 8 * h] : 0.f;
+    delta[h] = live ? p.delta[head * p.rows + start + row_a + 8 * h] : 0.f;
+  }
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) dq[n][i] = 0.f;
+  for (int b = 0; b < n_blocks; ++b) {
+    const uint32_t kb = sK + (b & 1) * TILE, vb = sV + (b & 1) * TILE;
+    if (b + 1 < n_blocks) {
+      load_tile<HD, kAttnRows>(sK + ((b + 1) & 1) * TILE, kp, p.ldr, (b + 1) * kAttnRows, len);
+      load_tile<HD, kAttnRows>(sV + ((b + 1) & 1) * TILE, vp, p.ldv, (b + 1) * kAttnRows, len);
+    }
+    attn_commit();
+    attn_wait<1>();
+    __syncthreads();
+#pragma unroll
+    for (int hb = 0; hb < 2; ++hb) {         // 32 keys at a time
+      float s[4][4], dp[4][4];
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { s[n][i] = 0.f; dp[n][i] = 0.f; }
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk) {
+        uint32_t a[4], d[4];
+        frag_a<HD>(sQ, warp * 16, kk, lane, a);
+        frag_a<HD>(sO, warp * 16, kk, lane, d);
+#pragma unroll
+        for (int n2 = 0; n2 < 2; ++n2) {
+          uint32_t bf[4];
+          frag_b<HD>(kb, hb * 32 + n2 * 16, kk, lane, bf);
+          mma16816(s[2 * n2], a[0], a[1], a[2], a[3], bf[0], bf[1]);
+          mma16816(s[2 * n2 + 1], a[0], a[1], a[2], a[3], bf[2], bf[3]);
+          frag_b<HD>(vb, hb * 32 + n2 * 16, kk, lane, bf);
+          mma16816(dp[2 * n2], d[0], d[1], d[2], d[3], bf[0], bf[1]);
+          mma16816(dp[2 * n2 + 1], d[0], d[1], d[2], d[3], bf[2], bf[3]);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int key = b * kAttnRows + hb * 32 + n * 8 + 2 * t + (i & 1);
+          const float pr = key > row_a + (i >> 1) * 8 ? 0.f : exp2_fast(fmaf(s[n][i], p.scale_log2, -lse[i >> 1]));
+          s[n][i] = pr * (dp[n][i] - delta[i >> 1]);
+        }
+#pragma unroll
+      for (int kk = 0; kk < 2; ++kk) {
+        const uint32_t a0 = pack_half2_rn(s[2 * kk][0], s[2 * kk][1]), a1 = pack_half2_rn(s[2 * kk][2], s[2 * kk][3]);
+        const uint32_t a2 = pack_half2_rn(s[2 * kk + 1][0], s[2 * kk + 1][1]), a3 = pack_half2_rn(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+#pragma unroll
+        for (int n2 = 0; n2 < NT / 2; ++n2) {
+          uint32_t bf[4];
+          frag_bt<HD>(kb, hb * 32 + kk * 16, n2 * 16, lane, bf);
+          mma16816(dq[2 * n2], a0, a1, a2, a3, bf[0], bf[1]);
+          mma16816(dq[2 * n2 + 1], a0, a1, a2, a3, bf[2], bf[3]);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  store_unrotated<HD>(dq, p, p.dq + start * p.ldd + head * HD, row_a, len, t, p.scale);
+}
+
+template <int HD>
+__global__ void __launch_bounds__(kAttnThreads)
+attn_dkv_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ SeqTable seqs) {
+  pdl_wait();
+  pdl_launch_dependents();
+  extern __shared__ __align__(128) uint8_t a_smem[];
+  constexpr int QR = 32;                     // query rows per step
+  constexpr int TILE = kAttnRows * HD * 2, QT = QR * HD * 2, KS = HD / 16, NT = HD / 8;
+  const uint32_t sK = smem_u32(a_smem), sV = sK + TILE, sQ = sV + TILE, sO = sQ + 2 * QT;
+  float* sL = reinterpret_cast<float*>(a_smem + 2 * TILE + 4 * QT);      // [2][QR] lse, [2][QR] delta
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  int start, len, k0;
+  find_tile(seqs, blockIdx.x, start, len, k0);                           // earlier key tiles have more query rows: first
+  const int kvh = blockIdx.y;
+  load_tile<HD, kAttnRows>(sK, p.k + start * p.ldr + kvh * HD, p.ldr, k0, len);
+  load_tile<HD, kAttnRows>(sV, p.v + start * p.ldv + kvh * HD, p.ldv, k0, len);
+  const int per_head = (len - k0 + QR - 1) / QR, steps = per_head * p.group;
+  auto issue = [&](int it) {
+    const int head = kvh * p.group + it / per_head, q0 = k0 + (it % per_head) * QR, slot = it & 1;
+    load_tile<HD, QR>(sQ + slot * QT, p.q + start * p.ldr + head * HD, p.ldr, q0, len);
+    load_tile<HD, QR>(sO + slot * QT, p.dout + start * p.lddo + head * HD, p.lddo, q0, len);
+    if (threadIdx.x < QR) {
+      const int r = q0 + threadIdx.x;
+      sL[slot * QR + threadIdx.x] = r < len ? p.lse[head * p.rows + start + r] : 0.f;
+      sL[2 * QR + slot * QR + threadIdx.x] = r < len ? p.delta[head * p.rows + start + r] : 0.f;
+    }
+  };
+  issue(0);
+  attn_commit();
+  float dk[NT][4], dv[NT][4];
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { dk[n][i] = 0.f; dv[n][i] = 0.f; }
+  const int key_a = k0 + warp * 16 + g;
+  for (int it = 0; it < steps; ++it) {
+    if (it + 1 < steps) issue(it + 1);
+    attn_commit();
+    attn_wait<1>();
+    __syncthreads();
+    const int slot = it & 1, q0 = k0 + (it % per_head) * QR;
+    const uint32_t qb = sQ + slot * QT, ob = sO + slot * QT;
+    // transposed scores: 16 keys of this warp x 32 queries
+    float s[4][4], dp[4][4];
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) { s[n][i] = 0.f; dp[n][i] = 0.f; }
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) {
+      uint32_t a[4], d[4];
+      frag_a<HD>(sK, warp * 16, kk, lane, a);
+      frag_a<HD>(sV, warp * 16, kk, lane, d);
+#pragma unroll
+      for (int n2 = 0; n2 < 2; ++n2) {
+        uint32_t bf[4];
+        frag_b<HD>(qb, n2 * 16, kk, lane, bf);
+        mma16816(s[2 * n2], a[0], a[1], a[2], a[3], bf[0], bf[1]);
+        mma16816(s[2 * n2 + 1], a[0], a[1], a[2], a[3], bf[2], bf[3]);
+        frag_b<HD>(ob, n2 * 16, kk, lane, bf);
+        mma16816(dp[2 * n2], d[0], d[1], d[2], d[3], bf[0], bf[1]);
+        mma16816(dp[2 * n2 + 1], d[0], d[1], d[2], d[3], bf[2], bf[3]);
+      }
+    }
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int qi = n * 8 + 2 * t + (i & 1), query = q0 + qi, key = key_a + (i >> 1) * 8;
+        const float pr = (key > query || query >= len) ? 0.f : exp2_fast(fmaf(s[n][i], p.scale_log2, -sL[slot * QR + qi]));
+        s[n][i] = pr;
+        dp[n][i] = pr * (dp[n][i] - sL[2 * QR + slot * QR + qi]);
+      }
+#pragma unroll
+    for (int kk = 0; kk < 2; ++kk) {
+      const uint32_t a0 = pack_half2_rn(s[2 * kk][0], s[2 * kk][1]), a1 = pack_half2_rn(s[2 * kk][2], s[2 * kk][3]);
+      const uint32_t a2 = pack_half2_rn(s[2 * kk + 1][0], s[2 * kk + 1][1]), a3 = pack_half2_rn(s[2 * kk + 1][2], s[2 * kk + 1][3]);
+      const uint32_t e0 = pack_half2_rn(dp[2 * kk][0], dp[2 * kk][1]), e1 = pack_half2_rn(dp[2 * kk][2], dp[2 * kk][3]);
+      const uint32_t e2 = pack_half2_rn(dp[2 * kk + 1][0], dp[2 * kk + 1][1]), e3 = pack_half2_rn(dp[2 * kk + 1][2], dp[2 * kk + 1][3]);
+#pragma unroll
+      for (int n2 = 0; n2 < NT / 2; ++n2) {
+        uint32_t bf[4];
+        frag_bt<HD>(ob, kk * 16, n2 * 16, lane, bf);
+        mma16816(dv[2 * n2], a0, a1, a2, a3, bf[0], bf[1]);
+        mma16816(dv[2 * n2 + 1], a0, a1, a2, a3, bf[2], bf[3]);
+        frag_bt<HD>(qb, kk * 16, n2 * 16, lane, bf);
+        mma16816(dk[2 * n2], e0, e1, e2, e3, bf[0], bf[1]);
+        mma16816(dk[2 * n2 + 1], e0, e1, e2, e3, bf[2], bf[3]);
+      }
+    }
+    __syncthreads();
+  }
+  store_unrotated<HD>(dk, p, p.dk + start * p.ldd + kvh * HD, key_a, len, t, p.scale);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int r = key_a + 8 * h;
+    if (r >= len) continue;
+    __half* dst = p.dv + (start + r) * p.ldd + kvh * HD + 2 * t;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) *reinterpret_cast<uint32_t*>(dst + n * 8) = pack_half2_rn(dv[n][2 * h], dv[n][2 * h + 1]);
+  }
+}
+
+// ---------------------------------------------------------------------------------------------
+struct AttnShape {
+  int heads, kv_heads, hd;
+  int64_t rows;
+};
+
+static int attn_check(const AttnShape& s, const int32_t* lens, int n, const char* who) {
+  if (!lens || n <= 0 || s.heads <= 0 || s.kv_heads <= 0 || s.heads % s.kv_heads || (s.hd != 64 && s.hd != 128)) {
+    set_detail("%s: %d sequences, %d / %d heads of %d (head dimensions 64 and 128)", who, n, s.heads, s.kv_heads, s.hd);
+    return NF4LL_ERR_SHAPE;
+  }
+  int64_t sum = 0;
+  for (int i = 0; i < n; ++i) {
+    if (lens[i] < 0) { set_detail("%s: sequence %d has %d rows", who, i, lens[i]); return NF4LL_ERR_SHAPE; }
+    sum += lens[i];
+  }
+  if (sum != s.rows || s.rows > (int64_t(1) << 30)) {
+    set_detail("%s: the sequences cover %lld of %lld rows", who, static_cast<long long>(sum), static_cast<long long>(s.rows));
+    return NF4LL_ERR_SHAPE;
+  }
+  return NF4LL_OK;
+}
+
+// the next (up to kAttnMaxSeqs) sequences from `at` on; empty ones are skipped
+static int attn_table(SeqTable* t, const int32_t* lens, int n, int at, int64_t* row) {
+  t->n = 0;
+  t->tile[0] = 0;
+  t->start[0] = static_cast<int>(*row);
+  while (at < n && t->n < kAttnMaxSeqs) {
+    const int len = lens[at++];
+    if (len == 0) continue;
+    *row += len;
+    t->start[t->n + 1] = static_cast<int>(*row);
+    t->tile[t->n + 1] = t->tile[t->n] + (len + kAttnRows - 1) / kAttnRows;
+    ++t->n;
+  }
+  return at;
+}
+
+template <int HD>
+static int attn_forward_hd(AttnParams p, const __half* qkv, int64_t ldq, __half* roped, const int32_t* lens, int n, int kv_heads, cudaStream_t stream) {
+  constexpr int smem = 5 * kAttnRows * HD * 2;
+  NF4LL_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  int64_t row = 0;
+  for (int at = 0; at < n;) {
+    SeqTable t;
+    at = attn_table(&t, lens, n, at, &row);
+    if (t.n == 0) continue;
+    const int rows = t.start[t.n] - t.start[0], work = rows * (p.heads + kv_heads) * (HD / 16);
+    PdlLaunch lr(dim3(static_cast<unsigned>((work + 255) / 256 < 1184 ? (work + 255) / 256 : 1184)), dim3(256), 0, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lr.cfg, rope_kernel, qkv, ldq, roped, p.ldr, p.trig, p.heads + kv_heads, HD, t));
+    PdlLaunch lf(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(kAttnThreads), smem, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lf.cfg, attn_fwd_kernel<HD>, p, t));
+  }
+  return NF4LL_OK;
+}
+
+template <int HD>
+static int attn_backward_hd(AttnParams p, const int32_t* lens, int n, int kv_heads, cudaStream_t stream) {
+  constexpr int smem_q = 6 * kAttnRows * HD * 2, smem_kv = 4 * kAttnRows * HD * 2 + 4 * 32 * 4;
+  NF4LL_CUDA(cudaFuncSetAttribute(attn_dq_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q));
+  NF4LL_CUDA(cudaFuncSetAttribute(attn_dkv_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv));
+  int64_t row = 0;
+  for (int at = 0; at < n;) {
+    SeqTable t;
+    at = attn_table(&t, lens, n, at, &row);
+    if (t.n == 0) continue;
+    const int rows = t.start[t.n] - t.start[0];
+    PdlLaunch ld(dim3(static_cast<unsigned>((static_cast<int64_t>(rows) * p.heads * (HD / 8) + 255) / 256)), dim3(256), 0, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&ld.cfg, attn_delta_kernel<HD>, p, t.start[0], rows));
+    PdlLaunch lk(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(kv_heads)), dim3(kAttnThreads), smem_kv, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lk.cfg, attn_dkv_kernel<HD>, p, t));
+    PdlLaunch lq(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(kAttnThreads), smem_q, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lq.cfg, attn_dq_kernel<HD>, p, t));
+  }
+  return NF4LL_OK;
+}
+
+}  // namespace nf4ll
+
+extern "C" int nf4ll_attention_forward(const void* qkv, int64_t ldq, const int32_t* seq_lens, int32_t n_seqs, int64_t rows, int32_t heads,
+                                       int32_t kv_heads, int32_t head_dim, const void* trig, void* roped, int64_t ldr, void* out, int64_t ldo,
+                                       float* lse, void* stream) {
+  using namespace nf4ll;
+  const char* who = "nf4ll_attention_forward";
+  if (rows == 0) return NF4LL_OK;
+  if (!qkv || !trig || !roped || !out || !lse) { set_detail("%s: null pointer", who); return NF4LL_ERR_NULL; }
+  if (int rc = attn_check({heads, kv_heads, head_dim, rows}, seq_lens, n_seqs, who)) return rc;
+  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(trig) | reinterpret_cast<uintptr_t>(roped) | reinterpret_cast<uintptr_t>(out)) & 15 ||
+      (ldq | ldr | ldo) % 8) {
+    set_detail("%s: pointers 16-byte aligned, leading dimensions multiples of 8", who);
+    return NF4LL_ERR_ALIGN;
+  }
+  if (int rc = require_sm100()) return rc;
+  AttnParams p{};
+  p.q = static_cast<const __half*>(roped);
+  p.k = p.q + static_cast<int64_t>(heads) * head_dim;
+  p.ldr = ldr;
+  p.v = static_cast<const __half*>(qkv) + static_cast<int64_t>(heads + kv_heads) * head_dim;
+  p.ldv = ldq;
+  p.out = static_cast<__half*>(out); p.ldo = ldo;
+  p.lse = lse;
+  p.trig = static_cast<const float2*>(trig);
+  p.heads = heads; p.group = heads / kv_heads; p.rows = rows;
+  p.scale = 1.0f / sqrtf(static_cast<float>(head_dim));
+  p.scale_log2 = p.scale * 1.4426950408889634f;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const __half* src = static_cast<const __half*>(qkv);
+  return head_dim == 128 ? attn_forward_hd<128>(p, src, ldq, static_cast<__half*>(roped), seq_lens, n_seqs, kv_heads, st)
+                         : attn_forward_hd<64>(p, src, ldq, static_cast<__half*>(roped), seq_lens, n_seqs, kv_heads, st);
+}
+
+extern "C" int nf4ll_attention_backward(const void* qkv, int64_t ldq, const int32_t* seq_lens, int32_t n_seqs, int64_t rows, int32_t heads,
+                                        int32_t kv_heads, int32_t head_dim, const void* trig, const void* roped, int64_t ldr, const void* out,
+                                        int64_t ldo, const float* lse, const void* dout, int64_t lddo, float* delta, void* dqkv, int64_t ldd,
+                                        void* stream) {
+  using namespace nf4ll;
+  const char* who = "nf4ll_attention_backward";
+  if (rows == 0) return NF4LL_OK;
+  if (!qkv || !trig || !roped || !out || !lse || !dout || !delta || !dqkv) { set_detail("%s: null pointer", who); return NF4LL_ERR_NULL; }
+  if (int rc = attn_check({heads, kv_heads, head_dim, rows}, seq_lens, n_seqs, who)) return rc;
+  if ((reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(trig) | reinterpret_cast<uintptr_t>(roped) | reinterpret_cast<uintptr_t>(out) |
+       reinterpret_cast<uintptr_t>(dout) | reinterpret_cast<uintptr_t>(dqkv)) & 15 || (ldq | ldr | ldo | lddo | ldd) % 8) {
+    set_detail("%s: pointers 16-byte aligned, leading dimensions multiples of 8", who);
+    return NF4LL_ERR_ALIGN;
+  }
+  if (int rc = require_sm100()) return rc;
+  AttnParams p{};
+  p.q = static_cast<const __half*>(roped);
+  p.k = p.q + static_cast<int64_t>(heads) * head_dim;
+  p.ldr = ldr;
+  p.v = static_cast<const __half*>(qkv) + static_cast<int64_t>(heads + kv_heads) * head_dim;
+  p.ldv = ldq;
+  p.o = static_cast<const __half*>(out); p.ldo = ldo;
+  p.dout = static_cast<const __half*>(dout); p.lddo = lddo;
+  p.dq = static_cast<__half*>(dqkv);
+  p.dk = p.dq + static_cast<int64_t>(heads) * head_dim;
+  p.dv = p.dk + static_cast<int64_t>(kv_heads) * head_dim;
+  p.ldd = ldd;
+  p.lse = const_cast<float*>(lse);
+  p.delta = delta;
+  p.trig = static_cast<const float2*>(trig);
+  p.heads = heads; p.group = heads / kv_heads; p.rows = rows;
+  p.scale = 1.0f / sqrtf(static_cast<float>(head_dim));
+  p.scale_log2 = p.scale * 1.4426950408889634f;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  return head_dim == 128 ? attn_backward_hd<128>(p, seq_lens, n_seqs, kv_heads, st) : attn_backward_hd<64>(p, seq_lens, n_seqs, kv_heads, st);
+}
