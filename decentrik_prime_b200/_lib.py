@@ -1,7 +1,9 @@
-"""ctypes binding of the C-ABI library (include/nf4ll.h) and the nvcc recipe that builds it.
+"""ctypes binding of the C-ABI library (include/nf4ll.h), the recipe that builds it, and the loader of the host
+extension (csrc/torch_host.cpp) through which the tensor-level modules call it.
 
-The library is built in-tree (decentrik_prime_b200/libnf4ll.so) for sm_100a only. There is no
-fallback: if it is missing, or a call returns an error code, the caller gets an exception.
+The library is built in-tree (decentrik_prime_b200/libnf4ll.so) for sm_100a only, the extension beside it
+(decentrik_prime_b200/_host.so). There is no fallback: if one is missing, or a call returns an error code, the caller gets
+an exception.
 """
 
 import ctypes
@@ -16,7 +18,9 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libnf4ll.so")
-SOURCES = ("nf4ll_api.cu", "nf4ll_dequant.cu", "nf4ll_dense.cu", "nf4ll_gemm.cu", "nf4ll_gemm2.cu", "nf4ll_lora.cu", "nf4ll_swiglu.cu", "nf4ll_stream.cu", "nf4ll_swap.cu", "nf4ll_norm.cu")
+HOST_PATH = os.path.join(HERE, "_host.so")
+HOST_SOURCE = os.path.join(CSRC, "torch_host.cpp")
+SOURCES = ("nf4ll_api.cu", "nf4ll_dequant.cu", "nf4ll_dense.cu", "nf4ll_gemm.cu", "nf4ll_gemm2.cu", "nf4ll_lora.cu", "nf4ll_swiglu.cu", "nf4ll_stream.cu", "nf4ll_swap.cu", "nf4ll_norm.cu", "nf4ll_attn.cu")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "--fmad=true", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall", "-shared"]
@@ -33,12 +37,40 @@ def sources():
     return [os.path.join(CSRC, s) for s in SOURCES if os.path.exists(os.path.join(CSRC, s))]
 
 
-def needs_build():
+def _library_needs_build():
     if not os.path.exists(LIB_PATH):
         return True
     built = os.path.getmtime(LIB_PATH)
     deps = sources() + _headers()
     return any(os.path.getmtime(d) > built for d in deps)
+
+
+def _host_needs_build():
+    if not os.path.exists(HOST_PATH):
+        return True
+    built = os.path.getmtime(HOST_PATH)
+    return any(os.path.getmtime(d) > built for d in (HOST_SOURCE, os.path.join(INCLUDE, "nf4ll.h")))
+
+
+def needs_build():
+    return _library_needs_build() or _host_needs_build()
+
+
+def _build_host():
+    """Compile csrc/torch_host.cpp against PyTorch's C++ headers into _host.so, linked to libnf4ll.so beside it."""
+    import sysconfig
+    root = os.path.dirname(torch.__file__)
+    libs = os.path.join(root, "lib")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-I", INCLUDE, "-isystem", os.path.join(root, "include"),
+           "-isystem", os.path.join(root, "include", "torch", "csrc", "api", "include"), "-isystem", os.path.join(cuda, "include"),
+           "-isystem", sysconfig.get_paths()["include"], "-o", HOST_PATH + ".tmp", HOST_SOURCE, "-L", HERE, "-l:libnf4ll.so",
+           "-L", libs, "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-lc10", "-lc10_cuda", "-Wl,-rpath,$ORIGIN"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
+    os.replace(HOST_PATH + ".tmp", HOST_PATH)
 
 
 def _headers():
@@ -47,11 +79,17 @@ def _headers():
 
 
 def build(force=False, verbose=False):
-    """Compile csrc/*.cu into libnf4ll.so with nvcc for sm_100a (cross-compiles without a GPU).
-    Every source becomes an object file under decentrik_prime_b200/build/ (compiled in parallel, only
+    """Compile csrc/*.cu into libnf4ll.so with nvcc for sm_100a (cross-compiles without a GPU) and the host extension.
+    Every CUDA source becomes an object file under decentrik_prime_b200/build/ (compiled in parallel, only
     when it or a header is newer than its object), then the objects are linked into the library."""
-    if not force and not needs_build():
-        return LIB_PATH
+    if force or _library_needs_build():
+        _build_library(force, verbose)
+    if force or _host_needs_build():
+        _build_host()
+    return LIB_PATH
+
+
+def _build_library(force, verbose):
     from concurrent.futures import ThreadPoolExecutor
     objdir = os.path.join(HERE, "build")
     os.makedirs(objdir, exist_ok=True)
@@ -80,7 +118,6 @@ def build(force=False, verbose=False):
     os.replace(LIB_PATH + ".tmp", LIB_PATH)
     if verbose:
         print("".join(log for _, log in results))
-    return LIB_PATH
 
 
 class Nf4Mat(ctypes.Structure):
@@ -133,6 +170,11 @@ SIGNATURES = {
     "nf4ll_rms_backward": (_i32, [_vp, _i64, _f32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _LORA, _vp, _LORA, _vp, _vp]),
     "nf4ll_swiglu_forward": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _vp]),
     "nf4ll_swiglu_backward": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _vp]),
+    "nf4ll_lora_project": (_i32, [_vp, _i64, _vp, _i64, _f32, _vp, _f32, _i64, _i64, _vp, _vp]),
+    "nf4ll_lora_shadow": (_i32, [_vp, _vp, _i64, _i64, _vp, _vp, _vp, _vp]),
+    "nf4ll_attention_forward": (_i32, [_vp, _i64, _vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _i64, _vp, _i64, _vp, _vp]),
+    "nf4ll_attention_backward": (_i32, [_vp, _i64, _vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _i64, _vp, _i64, _vp, _vp, _i64, _vp, _vp, _i64,
+                                        _vp]),
     "nf4ll_read_status": (_i32, [_vp, _vp]),
 }
 
@@ -157,6 +199,30 @@ def lib():
                 fn.restype, fn.argtypes = res, args
             _handle = h
     return _handle
+
+
+_host_module = None
+
+
+def host():
+    """The host extension: the same calls on tensors, without ctypes in between."""
+    global _host_module
+    if _host_module is not None:
+        return _host_module
+    lib()                                  # loads libnf4ll.so, or says that it is missing
+    with _lock:
+        if _host_module is None:
+            if not os.path.exists(HOST_PATH):
+                raise RuntimeError(f"{HOST_PATH} is missing: build it with decentrik_prime_b200._lib.build()")
+            import importlib.machinery
+            import importlib.util
+            loader = importlib.machinery.ExtensionFileLoader("decentrik_prime_b200._host", HOST_PATH)
+            mod = importlib.util.module_from_spec(importlib.util.spec_from_loader(loader.name, loader))
+            loader.exec_module(mod)
+            from . import linear
+            mod.setup(check, lambda index: linear.status_word(torch.device("cuda", index)), torch.OutOfMemoryError)
+            _host_module = mod
+    return _host_module
 
 
 class Nf4llError(RuntimeError):

@@ -113,12 +113,7 @@ class Projection:
                                        accumulate=accumulate, want_u=self.has_lora)
         elif self.has_lora:
             # layer 0 of the reference needs no d(input), only LoRA gradients (fast_qwen.py:1363-1364)
-            u = torch.empty(dy.shape[0], linear.RANK, dtype=torch.float32, device=dy.device)
-            from . import _lib
-            _lib.check(_lib.lib().nf4ll_lora_down(dy.data_ptr(), dy.stride(0), None, 0, 1.0, self.B16t.data_ptr(),
-                                                  1.0, linear.RANK, dy.shape[0], self.w.N, u.data_ptr(), None,
-                                                  _lib.current_stream(dy.device)))
-            u.mul_(self.scale)
+            u = linear.lora_u(dy, self.B16t, self.scale)
         if self.has_lora:
             if grad_stream is None:
                 linear.lora_grads(dy, x, t, u, self.scale, mask=mask, keep_scale=keep_scale, dA=self.dA, dB=self.dB,

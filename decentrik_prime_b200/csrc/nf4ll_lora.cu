@@ -176,6 +176,27 @@ __global__ void transpose_n16_kernel(const __half* __restrict__ B, __half* __res
   }
 }
 
+// fp16 shadows of fp32 masters: A [16,K] and B [N,16] rounded, B also transposed to [16,N]
+__global__ void __launch_bounds__(256)
+lora_shadow_kernel(const float* __restrict__ A, const float* __restrict__ B, int64_t K, int64_t N, __half* __restrict__ A16, __half* __restrict__ B16,
+                   __half* __restrict__ Bt16) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x, first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (int64_t i = first; i < K * 16; i += stride) A16[i] = __float2half_rn(A[i]);
+  for (int64_t n = first; n < N; n += stride) {
+    const float4* src = reinterpret_cast<const float4*>(B + n * 16);
+    float v[16];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) { const float4 f = src[j]; v[4 * j] = f.x; v[4 * j + 1] = f.y; v[4 * j + 2] = f.z; v[4 * j + 3] = f.w; }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) Bt16[j * N + n] = __float2half_rn(v[j]);
+    uint4* dst = reinterpret_cast<uint4*>(B16 + n * 16);
+    dst[0] = make_uint4(pack_half2_rn(v[0], v[1]), pack_half2_rn(v[2], v[3]), pack_half2_rn(v[4], v[5]), pack_half2_rn(v[6], v[7]));
+    dst[1] = make_uint4(pack_half2_rn(v[8], v[9]), pack_half2_rn(v[10], v[11]), pack_half2_rn(v[12], v[13]), pack_half2_rn(v[14], v[15]));
+  }
+}
+
 int transpose_n16_launch(const void* B, void* Bt, int64_t N, cudaStream_t stream) {
   const int64_t total = N * 16;
   count_launch();
@@ -532,9 +553,40 @@ extern "C" int nf4ll_lora_grads(const void* dy, int64_t lddy, const void* x, int
     return NF4LL_ERR_ALIGN;
   }
   if (int rc = require_sm100()) return rc;
-  if (dA && !accumulate) NF4LL_CUDA(cudaMemsetAsync(dA, 0, sizeof(float) * 16 * K, stream));
-  if (dB && !accumulate) NF4LL_CUDA(cudaMemsetAsync(dB, 0, sizeof(float) * 16 * N, stream));
+  if (!accumulate) {
+    // gradients that lie back to back are cleared by one fill
+    const bool joined = dA && dB && static_cast<float*>(dB) == static_cast<float*>(dA) + 16 * K;
+    if (dA) NF4LL_CUDA(cudaMemsetAsync(dA, 0, sizeof(float) * 16 * (joined ? K + N : K), stream));
+    if (dB && !joined) NF4LL_CUDA(cudaMemsetAsync(dB, 0, sizeof(float) * 16 * N, stream));
+  }
   if (M > 0 && (dA || dB))
     if (int rc = lora_grads_launch(dy, lddy, x, ldx, mask, ld_mask, keep_scale, t32, u32, scale, M, N, K, dA, dB, stream)) return rc;
+  return NF4LL_OK;
+}
+
+extern "C" int nf4ll_lora_project(const void* x, int64_t ldx, const uint8_t* mask, int64_t ld_mask, float keep_scale, const void* A, float scale,
+                                  int64_t M, int64_t K, void* t32, void* stream) {
+  using namespace nf4ll;
+  if (!x || !A || !t32) { set_detail("nf4ll_lora_project: null pointer"); return NF4LL_ERR_NULL; }
+  if (M < 0 || K <= 0 || K % 8) { set_detail("nf4ll_lora_project: M=%lld K=%lld", (long long)M, (long long)K); return NF4LL_ERR_SHAPE; }
+  if ((reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(A) & 15) || ldx % 8 ||
+      (mask && ((reinterpret_cast<uintptr_t>(mask) & 15) || ld_mask % 16))) {
+    set_detail("nf4ll_lora_project: x/A 16-byte aligned, ldx multiple of 8, mask 16-byte aligned with ld_mask multiple of 16");
+    return NF4LL_ERR_ALIGN;
+  }
+  if (int rc = require_sm100()) return rc;
+  return lora_down_launch(x, ldx, mask, ld_mask, keep_scale, A, scale, M, K, t32, nullptr, 0, static_cast<cudaStream_t>(stream));
+}
+
+extern "C" int nf4ll_lora_shadow(const float* A, const float* B, int64_t K, int64_t N, void* A16, void* B16, void* Bt16, void* stream) {
+  using namespace nf4ll;
+  if (!A || !B || !A16 || !B16 || !Bt16) { set_detail("nf4ll_lora_shadow: null pointer"); return NF4LL_ERR_NULL; }
+  if (K <= 0 || N <= 0) { set_detail("nf4ll_lora_shadow: K=%lld N=%lld", (long long)K, (long long)N); return NF4LL_ERR_SHAPE; }
+  if ((reinterpret_cast<uintptr_t>(B) | reinterpret_cast<uintptr_t>(B16)) & 15) { set_detail("nf4ll_lora_shadow: B and B16 must be 16-byte aligned"); return NF4LL_ERR_ALIGN; }
+  if (int rc = require_sm100()) return rc;
+  const int64_t work = K * 16 > N ? K * 16 : N;
+  const int64_t blocks = (work + 255) / 256 < 296 ? (work + 255) / 256 : 296;
+  PdlLaunch lc(dim3(static_cast<unsigned>(blocks)), dim3(256), 0, static_cast<cudaStream_t>(stream));
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_shadow_kernel, A, B, K, N, static_cast<__half*>(A16), static_cast<__half*>(B16), static_cast<__half*>(Bt16)));
   return NF4LL_OK;
 }

@@ -191,14 +191,7 @@ def dequant_tensors(packed, qabs, scale2, offset2, n_qblocks, code2, nf4, out):
     if key not in _NF4_OK:
         _check_nf4_table(nf4)
         _NF4_OK.add(key)
-    if out.dtype != torch.float16 or out.numel() < n_qblocks * QBLOCK:
-        raise ValueError("dequant output must be fp16 with room for every block")
-    for t in (packed, qabs, scale2, offset2, code2, out):
-        if not t.is_cuda:
-            raise ValueError("dequant operands must live on the GPU")
-    _lib.check(_lib.lib().nf4ll_dequant(
-        packed.data_ptr(), qabs.data_ptr(), scale2.data_ptr(), offset2.data_ptr(),
-        code2.data_ptr(), int(n_qblocks), out.data_ptr(), _lib.current_stream(out.device)))
+    _lib.host().dequant(packed, qabs, scale2, offset2, code2, int(n_qblocks), out)
     return out
 
 

@@ -24,7 +24,7 @@ projections never need the sequence boundaries.
 
 import torch
 
-from . import blocks, k_nf4, linear, quantize
+from . import _lib, blocks, k_nf4, linear, quantize
 
 
 def pack_lengths(batch, lo, hi, seed):
@@ -255,15 +255,28 @@ class ProjectionStack:
 
 
 class PackedAttention:
-    """Rotary embedding + causal grouped-query attention over packed varlen rows, forward and backward, through
-    PyTorch's own kernels (scaled_dot_product_attention per sequence, autograd for the backward). Attention is not
-    on this library's path (the reference has kernels of its own for it, solution/k_rope.py, k_attn.py); this is
-    the glue that makes the layer runner a real Qwen2 decoder layer. Rotary embedding as in Qwen2: the two halves
-    of a head rotate against each other, positions restart at every sequence."""
+    """Rotary embedding + causal grouped-query attention over packed varlen rows, forward and backward: one kernel each way
+    over all sequences and heads (the library's nf4ll_attention_*; reference solution/k_rope.py, k_attn.py) for head
+    dimensions 64 and 128, PyTorch's kernels per sequence (scaled_dot_product_attention, autograd for the backward) for
+    others. Rotary embedding as in Qwen2: the two halves of a head rotate against each other, positions restart at every
+    sequence."""
 
     def __init__(self, n_heads, n_kv_heads, head_dim, theta=1.0e6):
         self.nh, self.nkv, self.hd, self.theta = n_heads, n_kv_heads, head_dim, theta
         self._tables = {}
+        self._trig = {}
+
+    def _trig_table(self, n, device):
+        """fp32 [positions, hd] pairs (cos, sin) per frequency, grown by doubling; it does not depend on the batch."""
+        t = self._trig.get(device)
+        if t is None or t.shape[0] < n:
+            rows = max(1024, 1 << (n - 1).bit_length())
+            pos = torch.arange(rows, dtype=torch.float32, device=device)
+            inv = self.theta ** (-torch.arange(0, self.hd, 2, dtype=torch.float32, device=device) / self.hd)
+            ang = pos[:, None] * inv[None, :]
+            t = torch.stack([ang.cos(), ang.sin()], dim=-1).reshape(rows, self.hd).contiguous()
+            self._trig[device] = t
+        return t
 
     def _cos_sin(self, seq_lens, device):
         key = (tuple(seq_lens), str(device))
@@ -283,10 +296,17 @@ class PackedAttention:
 
     def forward(self, qkv, seq_lens):
         """qkv fp16 [M, (nh + 2 nkv) hd] -> (a fp16 [M, nh hd], state for backward)."""
-        import torch.nn.functional as F
-        H, KV = self.nh * self.hd, self.nkv * self.hd
         if sum(seq_lens) != qkv.shape[0]:
             raise ValueError(f"sequence lengths {seq_lens} do not add up to {qkv.shape[0]} rows")
+        if self.hd in (64, 128):
+            trig = self._trig_table(max(seq_lens), qkv.device)
+            a, roped, lse = _lib.host().attention_forward(qkv, seq_lens, self.nh, self.nkv, self.hd, trig)
+            return a, (self, qkv, tuple(seq_lens), trig, roped, a, lse)
+        return self._forward_torch(qkv, seq_lens)
+
+    def _forward_torch(self, qkv, seq_lens):
+        import torch.nn.functional as F
+        H, KV = self.nh * self.hd, self.nkv * self.hd
         leaf = qkv.detach().requires_grad_(True)
         cos, sin = self._cos_sin(seq_lens, qkv.device)
         with torch.enable_grad():
@@ -305,9 +325,12 @@ class PackedAttention:
 
     @staticmethod
     def backward(state, da):
-        leaf, a = state
-        (dqkv,) = torch.autograd.grad(a, leaf, da)
-        return dqkv
+        if len(state) == 2:
+            leaf, a = state
+            (dqkv,) = torch.autograd.grad(a, leaf, da)
+            return dqkv
+        att, qkv, seq_lens, trig, roped, a, lse = state
+        return _lib.host().attention_backward(qkv, seq_lens, att.nh, att.nkv, att.hd, trig, roped, a, lse, da)
 
 
 class NormedDecoderLayer:
@@ -316,8 +339,8 @@ class NormedDecoderLayer:
     stream, each norm adding the fp16 output of the GEMM before it (`delta`), norm 1 producing y16 AND the rank-16
     LoRA products of q and v, one stacked launch for Q|K|V forward and ONE for its backward (the LoRA input
     gradients are folded into norm 1's backward, as in solution/k_norm.py:64-71), one for gate|up each way.
-    Attention itself (RoPE, softmax) is not on this path: with `attention` (a PackedAttention) and the batch's
-    sequence lengths it runs through PyTorch's kernels, otherwise the stand-in of DecoderLayerProjections is used.
+    Attention (RoPE, softmax) runs with `attention` (a PackedAttention) and the batch's sequence lengths; otherwise the
+    stand-in of DecoderLayerProjections is used.
 
         forward(x32, delta16)  -> (x32', delta16')     with x_next = x32' + delta16'
         backward(dres32, d16)  -> (dres32', d16')      gradients w.r.t. x_next in, w.r.t. this layer's input out

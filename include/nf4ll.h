@@ -189,6 +189,15 @@ int nf4ll_lora_down(const void* x, int64_t ldx, const uint8_t* mask, int64_t ld_
                     float keep_scale, const void* A, float scale, int32_t r,
                     int64_t M, int64_t K, void* t32, void* t16, void* stream);
 
+/* The same projection with the scale folded into the fp32 result:  t32[M,16] = scale * (drop(x) . A^T). With A =
+ * lora_B transposed and scale = alpha / r this is `daq` / `dav` of solution/fast_qwen.py:1370, 1373. */
+int nf4ll_lora_project(const void* x, int64_t ldx, const uint8_t* mask, int64_t ld_mask, float keep_scale, const void* A,
+                       float scale, int64_t M, int64_t K, void* t32, void* stream);
+
+/* fp16 shadows of fp32 LoRA masters A [16,K], B [N,16] (and B transposed, [16,N]) in one launch; replaces the casts of
+ * solution/fast_qwen.py:686-692 (_refresh_lora16). B and B16 16-byte aligned. */
+int nf4ll_lora_shadow(const float* A, const float* B, int64_t K, int64_t N, void* A16, void* B16, void* Bt16, void* stream);
+
 /* LoRA gradients, fp32:  dA[r,K] (+)= u^T . drop(x),   dB[N,r] (+)= scale * dy^T . t
  * with t, u the fp32 [M,r] outputs of nf4ll_forward / nf4ll_backward_dx. fp32 t/u and fp32
  * accumulation keep dA/dB within 2e-2 of an fp32 reference, which the reference's fp16 GEMM outputs
@@ -236,6 +245,25 @@ int nf4ll_swiglu_forward(const void* g, int64_t ldg, const void* u, int64_t ldu,
 int nf4ll_swiglu_backward(const void* g, int64_t ldg, const void* u, int64_t ldu, const void* dh,
                           int64_t lddh, void* dg, int64_t lddg, void* du, int64_t lddu, int64_t M,
                           int64_t I, void* stream);
+
+/* Rotary embedding + causal grouped-query attention over packed varlen rows (the step between the Q|K|V and the O
+ * projection; the reference's own kernels are solution/k_rope.py and solution/k_attn.py).
+ * qkv fp16 [rows, ldq]: `heads` query heads, `kv_heads` key heads, `kv_heads` value heads of head_dim (64 or 128) columns.
+ * seq_lens: HOST array of n_seqs row counts that add up to `rows`; read before the call returns. trig: fp32
+ * [positions, head_dim/2] pairs (cos, sin), at least as many positions as the longest sequence; the two halves of a head
+ * rotate against each other and positions restart at every sequence. roped: fp16 [rows, ldr >= (heads + kv_heads) *
+ * head_dim], written (the rotated q and k; the backward reads it). out fp16 [rows, ldo]; lse fp32 [heads, rows], written.
+ * Pointers 16-byte aligned, leading dimensions multiples of 8. */
+int nf4ll_attention_forward(const void* qkv, int64_t ldq, const int32_t* seq_lens, int32_t n_seqs, int64_t rows,
+                            int32_t heads, int32_t kv_heads, int32_t head_dim, const void* trig, void* roped, int64_t ldr,
+                            void* out, int64_t ldo, float* lse, void* stream);
+
+/* Its backward: dqkv fp16 [rows, ldd] (same column layout as qkv) from dout fp16 [rows, lddo] and what the forward wrote.
+ * delta: fp32 [heads, rows] scratch. Sums over query heads and rows stay in registers: bit-reproducible. */
+int nf4ll_attention_backward(const void* qkv, int64_t ldq, const int32_t* seq_lens, int32_t n_seqs, int64_t rows,
+                             int32_t heads, int32_t kv_heads, int32_t head_dim, const void* trig, const void* roped,
+                             int64_t ldr, const void* out, int64_t ldo, const float* lse, const void* dout, int64_t lddo,
+                             float* delta, void* dqkv, int64_t ldd, void* stream);
 
 /* Synchronise `stream`, copy the device status word to the host and return NF4LL_OK or
  * NF4LL_ERR_DEVICE_WAIT (detail string carries the raw word). */

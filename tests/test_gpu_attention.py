@@ -1,0 +1,61 @@
+"""Rotary embedding + causal grouped-query attention over packed rows against a plain PyTorch fp64 statement of it, forward
+and backward, at the edges of the 64-row tiles, with empty and single-row sequences, both head dimensions, grouped and
+ungrouped heads, and more sequences than one launch takes. fp16 results of fp32 sums over fp16 probabilities: the rounding
+of P, dS (2^-11 each, relative) and of the rotated q, k and the result give a few 2^-11 in the 2-norm; 3e-3 bounds it."""
+
+import pytest
+import torch
+
+from decentrik_prime_b200 import stack
+
+pytestmark = pytest.mark.gpu
+REL = 3e-3
+
+
+def reference(qkv, lens, nh, nkv, hd, theta, da):
+    x = qkv.double().cpu().requires_grad_(True)
+    H, KV = nh * hd, nkv * hd
+    outs, at = [], 0
+    inv = theta ** (-torch.arange(0, hd, 2, dtype=torch.float64) / hd)
+    for n in lens:
+        ang = torch.arange(n, dtype=torch.float64)[:, None] * inv[None, :]
+        cos, sin = torch.cat([ang, ang], 1).cos()[:, None], torch.cat([ang, ang], 1).sin()[:, None]
+
+        def rot(t):
+            return t * cos + torch.cat([-t[..., hd // 2:], t[..., :hd // 2]], -1) * sin
+
+        rows = x[at:at + n]
+        q, k = rot(rows[:, :H].view(n, nh, hd)), rot(rows[:, H:H + KV].view(n, nkv, hd)).repeat_interleave(nh // nkv, 1)
+        v = rows[:, H + KV:].view(n, nkv, hd).repeat_interleave(nh // nkv, 1)
+        s = torch.einsum("ihd,jhd->hij", q, k) / hd ** 0.5
+        s = s.masked_fill(torch.triu(torch.ones(n, n, dtype=torch.bool), 1), float("-inf"))
+        outs.append(torch.einsum("hij,jhd->ihd", s.softmax(-1), v).reshape(n, H))
+        at += n
+    out = torch.cat(outs)
+    (dx,) = torch.autograd.grad(out, x, da.double().cpu())
+    return out.detach(), dx
+
+
+def rel(got, ref):
+    return float((got.double().cpu() - ref).norm() / ref.norm())
+
+
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 64), (3, 1, 128), (2, 2, 128)])
+@pytest.mark.parametrize("lens", [[1], [63, 64, 65], [128, 0, 1, 200], [5] * 131 + [70], [331]])
+def test_attention_against_fp64(nh, nkv, hd, lens):
+    gen = torch.Generator().manual_seed(sum(lens) + nh)
+    M = sum(lens)
+    qkv = torch.randn(M, (nh + 2 * nkv) * hd, generator=gen).half().cuda()
+    da = torch.randn(M, nh * hd, generator=gen).half().cuda()
+    att = stack.PackedAttention(nh, nkv, hd, theta=1.0e4)
+    a, state = att.forward(qkv, lens)
+    dqkv = stack.PackedAttention.backward(state, da)
+    ref, dref = reference(qkv, [n for n in lens if n], nh, nkv, hd, 1.0e4, da)
+    assert rel(a, ref) <= REL
+    H, KV = nh * hd, nkv * hd
+    if M > 1:                      # a single row attends to itself: d(q) = d(k) = 0
+        assert rel(dqkv[:, :H], dref[:, :H]) <= REL
+        assert rel(dqkv[:, H:H + KV], dref[:, H:H + KV]) <= REL
+    assert rel(dqkv[:, H + KV:], dref[:, H + KV:]) <= REL
+    a2, _ = att.forward(qkv, lens)
+    assert torch.equal(a, a2) and torch.equal(dqkv, stack.PackedAttention.backward(state, da))
