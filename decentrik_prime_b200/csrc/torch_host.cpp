@@ -5,6 +5,7 @@
 //
 // No kernel lives here and nothing is decided here: every function checks its tensors, allocates what it returns and makes
 // one call into libnf4ll.so. Errors of the library are raised by the Python side (_lib.check).
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/custom_function.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/torch.h>
@@ -26,14 +27,15 @@ PyObject* g_memory_error = nullptr;      // torch.OutOfMemoryError
 
 struct PyRaised {};                // a Python exception is set
 
+// A C++ exception rather than a Python one: the backward runs these checks on autograd's thread, without the interpreter lock
 [[noreturn]] void value_error(const char* fmt, ...) {
   char buf[256];
   va_list ap;
   va_start(ap, fmt);
   vsnprintf(buf, sizeof(buf), fmt, ap);
   va_end(ap);
-  PyErr_SetString(PyExc_ValueError, buf);
-  throw PyRaised();
+  TORCH_CHECK_VALUE(false, buf);
+  __builtin_unreachable();
 }
 
 void check(int rc) {
@@ -55,7 +57,15 @@ double number(PyObject* o) {
   return v;
 }
 int64_t integer(PyObject* o) {
-  const int64_t v = PyLong_AsLongLong(o);
+  int64_t v;
+  if (PyLong_Check(o)) {
+    v = PyLong_AsLongLong(o);
+  } else {                                 // whatever int() takes
+    PyObject* n = PyNumber_Long(o);
+    if (!n) throw PyRaised();
+    v = PyLong_AsLongLong(n);
+    Py_DECREF(n);
+  }
   if (v == -1 && PyErr_Occurred()) throw PyRaised();
   return v;
 }
@@ -160,9 +170,10 @@ struct Lora {
     c.keep_scale = static_cast<float>(keep_scale);
     set_mask(mask);
   }
-  void set_mask(const at::Tensor* mask) {
+  void set_mask(const at::Tensor* mask, bool any_byte = false) {
     if (!mask) return;
-    if ((mask->scalar_type() != at::kByte && mask->scalar_type() != at::kBool) || mask->dim() < 1 || mask->stride(-1) != 1)
+    const bool type = mask->scalar_type() == at::kByte || mask->scalar_type() == at::kBool || (any_byte && mask->element_size() == 1);
+    if (!type || mask->dim() < 1 || mask->stride(-1) != 1)
       value_error("mask must be uint8/bool with unit inner stride");
     c.mask = static_cast<const uint8_t*>(mask->data_ptr());
     c.ld_mask = mask->dim() > 1 ? (mask->size(0) == 1 && mask->stride(0) < mask->size(1) ? mask->size(1) : mask->stride(0)) : mask->size(0);
@@ -202,6 +213,12 @@ PyObject* guarded(F&& f) {
   try {
     return f();
   } catch (const PyRaised&) {
+    return nullptr;
+  } catch (python_error& e) {
+    e.restore();
+    return nullptr;
+  } catch (const c10::ValueError& e) {
+    PyErr_SetString(PyExc_ValueError, e.what_without_backtrace());
     return nullptr;
   } catch (const c10::Error& e) {
     const bool memory = dynamic_cast<const c10::OutOfMemoryError*>(&e) != nullptr && g_memory_error;
@@ -371,7 +388,7 @@ PyObject* py_lora_grads(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     check_act(x, K, "x");
     check_act(dy, N, "dy");
     Lora m;
-    m.set_mask(optional(a[5], "mask"));
+    m.set_mask(optional(a[5], "mask"), true);
     const bool accumulate = PyObject_IsTrue(a[9]);
     at::Tensor dA = a[7] == Py_None ? empty({kRank, K}, at::kFloat, x) : tensor(a[7], "dA");
     at::Tensor dB = a[8] == Py_None ? empty({N, kRank}, at::kFloat, x) : tensor(a[8], "dB");
@@ -562,8 +579,9 @@ PyObject* py_attention_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) 
   return guarded([&]() -> PyObject* {
     const at::Tensor &qkv = tensor(a[0], "qkv"), &trig = tensor(a[5], "trig");
     const auto lens = lengths(a[1]);
-    const int64_t nh = integer(a[2]), nkv = integer(a[3]), hd = integer(a[4]), M = qkv.size(0);
+    const int64_t nh = integer(a[2]), nkv = integer(a[3]), hd = integer(a[4]);
     check_act(qkv, (nh + 2 * nkv) * hd, "qkv");
+    const int64_t M = qkv.size(0);
     check_f32(trig, {trig.size(0), hd}, "trig");
     for (const int32_t n : lens)
       if (n > trig.size(0)) value_error("the rotary table is shorter than a sequence");
@@ -587,6 +605,7 @@ PyObject* py_attention_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs)
     const auto lens = lengths(a[1]);
     const int64_t nh = integer(a[2]), nkv = integer(a[3]), hd = integer(a[4]), M = qkv.size(0);
     check_act(da, nh * hd, "da");
+    if (da.size(0) != M) value_error("da has %lld rows, the forward had %lld", static_cast<long long>(da.size(0)), static_cast<long long>(M));
     at::Tensor dqkv = empty({M, (nh + 2 * nkv) * hd}, at::kHalf, qkv), delta = empty({nh, M}, at::kFloat, qkv);
     check(nf4ll_attention_backward(qkv.data_ptr(), ld(qkv), lens.data(), static_cast<int32_t>(lens.size()), M, nh, nkv, hd, trig.data_ptr(), roped.data_ptr(),
                                    ld(roped), out.data_ptr(), ld(out), lse.data_ptr<float>(), da.data_ptr(), ld(da), delta.data_ptr<float>(), dqkv.data_ptr(),
@@ -610,18 +629,29 @@ struct WeightRef : torch::CustomClassHolder {      // the Python weight object, 
   }
 };
 
+// f() under the interpreter lock, from a thread that may not hold it; a Python exception travels on as a C++ one
+template <typename F>
+auto locked(F&& f) {
+  struct Gil {
+    PyGILState_STATE s = PyGILState_Ensure();
+    ~Gil() { PyGILState_Release(s); }
+  } gil;
+  try {
+    return f();
+  } catch (const PyRaised&) {
+    python_error e;
+    e.persist();
+    throw e;
+  }
+}
+
 void check_nogil(int rc) {
-  if (rc == 0) return;
-  TORCH_CHECK(false, "nf4ll error ", rc, ": ", nf4ll_error_string(rc), " (", nf4ll_last_error_detail(), ")");
+  if (rc != 0) locked([&] { check(rc); });
 }
 
 int32_t* status_nogil(const Call& c) {
   auto& v = state().status;
-  if (static_cast<int>(v.size()) <= c.device || !v[c.device].defined()) {
-    PyGILState_STATE s = PyGILState_Ensure();
-    struct Release { PyGILState_STATE s; ~Release() { PyGILState_Release(s); } } r{s};
-    return c.status();
-  }
+  if (static_cast<int>(v.size()) <= c.device || !v[c.device].defined()) return locked([&] { return c.status(); });
   return v[c.device].data_ptr<int32_t>();
 }
 
@@ -660,11 +690,12 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
     const Workspace ws(nullptr, c, x2, need(M, m->N, m->K, lora.on ? kRank : 0));
     check(nf4ll_forward(m, x2.data_ptr(), ld(x2), bias ? bias->data_ptr() : nullptr, lora.get(), t.defined() ? t.data_ptr() : nullptr, M, y.data_ptr(), m->N,
                         ws.p, ws.bytes, c.status(), c.stream));
-    // like the raw calls' results these are no autograd inputs or outputs: kept as they are
     ctx->saved_data["w"] = c10::IValue::make_capsule(w);
     ctx->saved_data["s"] = c10::IValue(c10::List<double>({scale, keep_scale}));
     ctx->saved_data["lead"] = x.sizes().vec();
-    ctx->save_for_backward({x2, t, A16, B16, Bt16, m2});
+    // no activations of the graph (saved-tensor hooks do not see them), and the mask may be the caller's reused buffer
+    if (lora.on) ctx->saved_data["lora"] = c10::IValue(std::vector<at::Tensor>{A16, B16, Bt16, m2});
+    ctx->save_for_backward({x2, t});
     if (x.dim() == 2) return y;
     auto shape = x.sizes().vec();
     shape.back() = m->N;
@@ -673,7 +704,12 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
 
   static variable_list backward(AutogradContext* ctx, variable_list grads) {
     const auto saved = ctx->get_saved_variables();
-    const at::Tensor &x2 = saved[0], &t = saved[1], &A16 = saved[2], &B16 = saved[3], &Bt16 = saved[4], &m2 = saved[5];
+    const at::Tensor &x2 = saved[0], &t = saved[1];
+    at::Tensor A16, B16, Bt16, m2;
+    if (const auto it = ctx->saved_data.find("lora"); it != ctx->saved_data.end()) {
+      const auto f = it->second.toTensorVector();
+      A16 = f[0]; B16 = f[1]; Bt16 = f[2]; m2 = f[3];
+    }
     const auto w = c10::static_intrusive_pointer_cast<WeightRef>(ctx->saved_data["w"].toCapsule());
     const auto s = ctx->saved_data["s"].toDoubleVector();
     const nf4ll_mat* m = w->m;

@@ -254,11 +254,17 @@ class ProjectionStack:
         return acts[-1], d
 
 
+def _rows_aligned(t):
+    """t, or a copy of it, with every row on a 16-byte boundary."""
+    ok = t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
+    return t if ok else t.contiguous()
+
+
 class PackedAttention:
     """Rotary embedding + causal grouped-query attention over packed varlen rows, forward and backward: one kernel each way
-    over all sequences and heads (the library's nf4ll_attention_*; reference solution/k_rope.py, k_attn.py) for head
-    dimensions 64 and 128, PyTorch's kernels per sequence (scaled_dot_product_attention, autograd for the backward) for
-    others. Rotary embedding as in Qwen2: the two halves of a head rotate against each other, positions restart at every
+    over all sequences and heads (the library's nf4ll_attention_*; reference solution/k_rope.py, k_attn.py) for fp16 rows on
+    the GPU in heads of 64 or 128, PyTorch's kernels per sequence (scaled_dot_product_attention, autograd for the backward)
+    for others. Rotary embedding as in Qwen2: the two halves of a head rotate against each other, positions restart at every
     sequence."""
 
     def __init__(self, n_heads, n_kv_heads, head_dim, theta=1.0e6):
@@ -267,15 +273,19 @@ class PackedAttention:
         self._trig = {}
 
     def _trig_table(self, n, device):
-        """fp32 [positions, hd] pairs (cos, sin) per frequency, grown by doubling; it does not depend on the batch."""
-        t = self._trig.get(device)
-        if t is None or t.shape[0] < n:
-            rows = max(1024, 1 << (n - 1).bit_length())
+        """fp32 [positions, hd] pairs (cos, sin) per frequency; it does not depend on the batch. One per stream, so that it is
+        written before it is read, in sizes of powers of two that are all kept (a captured graph may read a smaller one);
+        under capture a missing table is the graph's own (it holds values only once the graph has run)."""
+        rows = max(1024, 1 << max(n - 1, 0).bit_length())
+        key = (device, torch.cuda.current_stream(device).cuda_stream, rows)
+        t = self._trig.get(key)
+        if t is None:
             pos = torch.arange(rows, dtype=torch.float32, device=device)
             inv = self.theta ** (-torch.arange(0, self.hd, 2, dtype=torch.float32, device=device) / self.hd)
             ang = pos[:, None] * inv[None, :]
             t = torch.stack([ang.cos(), ang.sin()], dim=-1).reshape(rows, self.hd).contiguous()
-            self._trig[device] = t
+            if not torch.cuda.is_current_stream_capturing():
+                self._trig[key] = t
         return t
 
     def _cos_sin(self, seq_lens, device):
@@ -298,7 +308,8 @@ class PackedAttention:
         """qkv fp16 [M, (nh + 2 nkv) hd] -> (a fp16 [M, nh hd], state for backward)."""
         if sum(seq_lens) != qkv.shape[0]:
             raise ValueError(f"sequence lengths {seq_lens} do not add up to {qkv.shape[0]} rows")
-        if self.hd in (64, 128):
+        if self.hd in (64, 128) and qkv.is_cuda and qkv.dtype == torch.float16:
+            qkv = _rows_aligned(qkv.detach())
             trig = self._trig_table(max(seq_lens), qkv.device)
             a, roped, lse = _lib.host().attention_forward(qkv, seq_lens, self.nh, self.nkv, self.hd, trig)
             return a, (self, qkv, tuple(seq_lens), trig, roped, a, lse)
@@ -330,6 +341,7 @@ class PackedAttention:
             (dqkv,) = torch.autograd.grad(a, leaf, da)
             return dqkv
         att, qkv, seq_lens, trig, roped, a, lse = state
+        da = _rows_aligned(da.to(torch.float16))
         return _lib.host().attention_backward(qkv, seq_lens, att.nh, att.nkv, att.hd, trig, roped, a, lse, da)
 
 

@@ -59,3 +59,19 @@ def test_attention_against_fp64(nh, nkv, hd, lens):
     assert rel(dqkv[:, H + KV:], dref[:, H + KV:]) <= REL
     a2, _ = att.forward(qkv, lens)
     assert torch.equal(a, a2) and torch.equal(dqkv, stack.PackedAttention.backward(state, da))
+
+
+def test_attention_of_unaligned_rows():
+    """Rows that do not start on 16-byte boundaries, and a result gradient of another type, as the PyTorch path takes them."""
+    gen = torch.Generator().manual_seed(3)
+    wide = torch.randn(70, 4 * 64 + 3, generator=gen).half().cuda()
+    da = torch.randn(70, 2 * 64, generator=gen).half().cuda()
+    att = stack.PackedAttention(2, 1, 64)
+    a, state = att.forward(wide[:, 3:], [30, 40])
+    b, state_b = att.forward(wide[:, 3:].contiguous(), [30, 40])
+    assert torch.equal(a, b)
+    odd = torch.empty(70, 2 * 64 + 1, dtype=torch.half, device="cuda")[:, 1:].copy_(da)
+    expected = att.backward(state_b, da)
+    assert torch.equal(att.backward(state, odd), expected) and torch.equal(att.backward(state, da.float()), expected)
+    with pytest.raises(ValueError):
+        att.backward(state, da[:69])
