@@ -672,7 +672,7 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
     if (A.defined()) {
       at::Tensor Ac = A.contiguous(), Bc = B.contiguous();
       if (Ac.scalar_type() == at::kFloat && Bc.scalar_type() == at::kFloat && Ac.dim() == 2 && Bc.dim() == 2 && Ac.size(0) == kRank && Bc.size(1) == kRank &&
-          Ac.is_cuda() && Bc.is_cuda()) {
+          Ac.is_cuda() && Bc.is_cuda() && reinterpret_cast<uintptr_t>(Bc.data_ptr()) % 16 == 0) {
         A16 = empty(Ac.sizes(), at::kHalf, x2);
         B16 = empty(Bc.sizes(), at::kHalf, x2);
         Bt16 = empty({kRank, Bc.size(0)}, at::kHalf, x2);
