@@ -139,8 +139,12 @@ lora_down_kernel(const __half* __restrict__ act, int64_t ldact, const uint8_t* _
       for (int idx = threadIdx.x; idx < ROWS * 16; idx += NW * 32) {
         const int row = idx >> 4, j = idx & 15;
         if (m0 + row < M) {
-          float v = part[0][row][j];
-          for (uint32_t r = 1; r < gridDim.y; ++r) v += down_peer_load(&part[0][row][j], r);
+          float v = part[0][row][j], peer[8];
+#pragma unroll
+          for (uint32_t r = 1; r < 8; ++r) peer[r] = r < gridDim.y ? down_peer_load(&part[0][row][j], r) : 0.f;      // all in flight at once
+#pragma unroll
+          for (uint32_t r = 1; r < 8; ++r)
+            if (r < gridDim.y) v += peer[r];
           t32[(m0 + row) * 16 + j] = v * scale;
         }
       }
@@ -241,19 +245,13 @@ int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_
   ks = (C + c_per_cta - 1) / c_per_cta;
   dim3 grid(static_cast<unsigned>(row_groups), static_cast<unsigned>(ks));
   if (ks == 1) {
-    count_launch();
-    lora_down_kernel<4, kDownDirect, kDownWarps><<<grid, kDownWarps * 32, 0, stream>>>(
-        a, ldact, mask, ld_mask, keep_scale, r, scale, M, C, c_per_cta, t, zero_ptr, zero_words);
+    PdlLaunch lc(grid, dim3(kDownWarps * 32), 0, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<4, kDownDirect, kDownWarps>, a, ldact, mask, ld_mask, keep_scale, r, scale, M, C,
+                                  c_per_cta, t, zero_ptr, zero_words));
   } else if (ks <= 8) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid; cfg.blockDim = dim3(kDownWarps * 32); cfg.dynamicSmemBytes = 0; cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1; attr[0].val.clusterDim.y = static_cast<unsigned>(ks); attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    count_launch();
-    NF4LL_CUDA(cudaLaunchKernelEx(&cfg, lora_down_kernel<4, kDownCluster, kDownWarps>, a, ldact, mask, ld_mask, keep_scale, r,
-                                  scale, M, C, c_per_cta, t, zero_ptr, zero_words));
+    PdlLaunch lc(grid, dim3(kDownWarps * 32), 0, stream, 1, static_cast<unsigned>(ks));
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<4, kDownCluster, kDownWarps>, a, ldact, mask, ld_mask, keep_scale, r, scale, M, C,
+                                  c_per_cta, t, zero_ptr, zero_words));
   } else {
     NF4LL_CUDA(cudaMemsetAsync(t32, 0, sizeof(float) * 16 * M, stream));
     count_launch();
