@@ -29,6 +29,7 @@
 #include "nf4ll_dense.cuh"
 #include "nf4ll_dequant.cuh"
 #include "nf4ll_gemm_shared.cuh"
+#include "nf4ll_stream.cuh"
 
 namespace nf4ll {
 
@@ -1201,42 +1202,37 @@ int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_
 int transpose_n16_launch(const void* B, void* Bt, int64_t N, cudaStream_t stream);
 int launch_pair(int mode, int bm_tiles, const CUtensorMap& map, const CUtensorMap& nib_map, const CUtensorMap& out_map,
                 const GemmParams& p, int64_t tiles_o, int64_t tiles_mp, int splits, int launch_splits, cudaStream_t stream);
-int stream_forward_launch(const nf4ll_mat* W, const void* x, int64_t ldx, const void* bias, const float* t32,
-                          const void* lora_b, float lora_scale, int64_t M, void* y, int64_t ldy, void* scratch,
-                          bool counters_zeroed, int force_slices, cudaStream_t stream);
-int64_t stream_workspace_bytes(int64_t N, int64_t K, int64_t M, int sms, int force_slices);
-int swap_forward_launch(const nf4ll_mat* W, const void* x, int64_t ldx, const void* bias, const float* t32,
-                        const void* lora_b, float lora_scale, int64_t M, void* y, int64_t ldy, void* scratch,
-                        bool counters_zeroed, int force_slices, int32_t* status, cudaStream_t stream);
-int64_t swap_workspace_bytes(int64_t N, int64_t K, int64_t M, int sms, int force_slices);
-constexpr int64_t kStreamMaxRows = 16;     // at or below this many token rows the forward is a weight-streaming pass
-constexpr int64_t kStreamCapRows = 64;     // the streaming kernel's own limit (reachable through the tuning hook)
+constexpr int64_t kStreamMaxRows = 16;     // most token rows of the weight-streaming kernel's own choice
+constexpr int64_t kStreamCapRows = 64;     // its limit (reachable through the tuning hook)
 constexpr int64_t kSwapMaxRows = 64;       // limit of the swapped-operand kernel (weights as the MMA's M operand)
-// measured on B200 against the streaming kernel (two token tiles) and the 128-row tiles: the swapped-operand kernel
-// wins from 9 rows up on weights of at least 2^24 elements, and up to 64 rows on weights of at least 2^26
-constexpr int64_t kSwapMinRows = 9;
+// From 9 to 16 rows the faster of the two by fits of their times: the streaming kernel's depends on how evenly its units go
+// round the SMs (and on the tokens), the swapped-operand kernel cuts the contraction too and pays for that. Measured:
+// 27648 x 5120 at 9 / 16 rows 39 / 44 us against 52 / 54, 5120 x 27648 67 / 78 against 47, 5120 x 5120 13 / 15 against 19,
+// 3584 x 18944 28 / 30 against 29. From 17 rows on the swapped-operand kernel wins over the 128-row tiles on weights of at
+// least 2^24 elements, and up to 64 rows on weights of at least 2^26.
+constexpr int64_t kSwapMinRows = 9;        // below, the streaming kernel keeps its exact fp32 scales
 constexpr int64_t kSwapMidRows = 32;
 constexpr int64_t kSwapMinWeights = int64_t(1) << 24;
 constexpr int64_t kSwapBigWeights = int64_t(1) << 26;
+static double swap_time_us(int64_t N, int64_t K) { return 11.0 + 0.245e-6 * static_cast<double>(N) * static_cast<double>(K); }
 
 // Which kernel computes a forward of M rows: the 256 x 256 / 128-row tile kernels (kTiles), the register-level
 // weight-streaming kernel for decode-sized batches (kStream), or the swapped-operand tensor-core kernel for
 // short batches of 9 to 64 rows against a large weight (kSwap). Bits 1 and 2 of the tuning flags force kStream /
 // kSwap up to that kernel's limit.
 enum : int { kTiles = 0, kStream = 1, kSwap = 2 };
-static int forward_kind(int mode, int64_t M, int64_t N, int64_t K, bool stacked, const Tune& tune) {
-  if (mode != kFwd || stacked) return kTiles;
+static int forward_kind(int mode, int64_t M, int64_t N, int64_t K, bool stacked, int sms, const Tune& tune) {
+  if (mode != kFwd) return kTiles;
+  // stacked projections never took the swapped-operand kernel, whose scales are rounded to fp16: they keep their precision
+  if (stacked) return M <= kStreamMaxRows && !tune.any() && !tune.flags ? kStream : kTiles;
   if (tune.flags & 2) return M <= kStreamCapRows ? kStream : kTiles;
   const bool swap_ok = M <= kSwapMaxRows && N * (K / 64) < (int64_t(1) << 31);      // the kernel indexes quantisation blocks with 32 bits
   if (tune.flags & 4) return swap_ok ? kSwap : kTiles;
   if (tune.any()) return kTiles;
-  if (swap_ok && M >= kSwapMinRows && N * K >= (M <= kSwapMidRows ? kSwapMinWeights : kSwapBigWeights)) return kSwap;
-  if (M <= kStreamMaxRows) return kStream;
-  return kTiles;
-}
-
-static int64_t small_batch_scratch(int kind, int64_t N, int64_t K, int64_t M, int sms, int force_slices) {
-  return kind == kStream ? stream_workspace_bytes(N, K, M, sms, force_slices) : swap_workspace_bytes(N, K, M, sms, force_slices);
+  const bool large = N * K >= (M <= kSwapMidRows ? kSwapMinWeights : kSwapBigWeights);
+  if (M < kSwapMinRows) return kStream;
+  if (M <= kStreamMaxRows) return swap_ok && large && swap_time_us(N, K) < stream_time_us(N, K, M, sms) ? kSwap : kStream;
+  return swap_ok && large ? kSwap : kTiles;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1424,10 +1420,11 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   }
   if (segments && (narrow_tiles || tune.bn == 512)) tune.bn = narrow_tiles ? 128 : 256;
   Plan pl = make_plan(mode, M, NO, KC, lora ? lora->r : 0, sms, tune);
-  const int kind = forward_kind(mode, M, W->N, W->K, segments != nullptr, tune);
+  int kind = forward_kind(mode, M, W->N, W->K, segments != nullptr, sms, g_tune);
+  if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;      // it copies the absmax codes word by word
   const int force_slices = (tune.flags & 6) ? tune.splits : 0;
-  const int64_t need = kind != kTiles ? pl.left_bytes + pl.bt_bytes + small_batch_scratch(kind, W->N, W->K, M, sms, force_slices)
-                                      : pl.total();
+  const int64_t need = kind == kTiles ? pl.total()
+                                      : pl.left_bytes + pl.bt_bytes + (kind == kSwap ? swap_workspace_bytes(W->N, W->K, M, sms, force_slices) : 0);
   if (need > 0) {
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < need) {
       set_detail("%s: needs a 256-byte aligned workspace of %lld bytes (got %lld)", who,
@@ -1460,16 +1457,14 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   }
   int* counters = nullptr;
   int counter_words = 0;
-  if (kind == kStream) {
-    counters = reinterpret_cast<int*>(ws + pl.left_bytes + pl.bt_bytes);      // next-unit counter + one per 16 weight rows
-    counter_words = static_cast<int>(1 + W->N / 16);
-  } else if (kind == kSwap) {
+  if (kind == kSwap) {
     counters = reinterpret_cast<int*>(ws + pl.left_bytes + pl.bt_bytes);      // one per tile of 128 weight rows
     counter_words = static_cast<int>((W->N + 127) / 128);
-  } else if (pl.splits > 1) {
+  } else if (kind == kTiles && pl.splits > 1) {
     counters = reinterpret_cast<int*>(ws + pl.left_bytes + pl.bt_bytes);
     counter_words = static_cast<int>(pl.counter_bytes / sizeof(int));
   }
+  bool projected = false;          // a rank-16 projection is what this call has launched last
   if (segments) {
     int64_t at = 0;
     p.n_seg = n_segments;
@@ -1478,9 +1473,11 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
       p.seg_begin[i] = at;
       if (l) {
         // the rank-16 projection of this segment: computed here unless the producer of x already wrote it
-        if (!segments[i].t_ready)
+        if (!segments[i].t_ready) {
           if (int rc = lora_down_launch(act, ldact, l->mask, l->ld_mask, l->keep_scale, l->A, 1.0f, M, W->K, segments[i].t_out,
                                         nullptr, 0, stream)) return rc;
+          projected = true;
+        }
         p.seg_left[i] = static_cast<const float*>(segments[i].t_out);
         p.seg_right[i] = static_cast<const __half*>(l->B) - at * 16;      // indexed by the fused output column
         p.seg_scale[i] = l->scale;
@@ -1493,6 +1490,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     // it lands in the caller's t_out / u_out when given, else in the workspace. The same kernel
     // resets the split-K tile counters of the GEMM that follows it on the stream.
     float* left = side_out ? static_cast<float*>(side_out) : reinterpret_cast<float*>(ws);
+    projected = true;
     if (mode == kFwd) {
       if (int rc = lora_down_launch(act, ldact, lora->mask, lora->ld_mask, lora->keep_scale, lora->A, 1.0f, M, W->K, left,
                                     counters, counter_words, stream)) return rc;
@@ -1518,14 +1516,19 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   g_ev_start = g_ev_stop = nullptr;
   if (kind != kTiles) {
     if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
-    const float* t32 = lora ? p.lora_left : nullptr;
-    const void* lb = lora ? lora->B : nullptr;
-    const float ls = lora ? lora->scale : 0.f;
-    const int rc = kind == kStream
-                       ? stream_forward_launch(W, act, ldact, bias, t32, lb, ls, M, out, ldo, counters, lora != nullptr,
-                                               force_slices, stream)
-                       : swap_forward_launch(W, act, ldact, bias, t32, lb, ls, M, out, ldo, counters, lora != nullptr,
-                                             force_slices, status, stream);
+    StreamCall c{};
+    c.W = W; c.x = act; c.ldx = ldact; c.M = M; c.bias = bias; c.y = out; c.ldy = ldo;
+    c.n_seg = segments ? n_segments : 1;
+    int64_t at = 0;
+    for (int i = 0; i < c.n_seg; ++i) {
+      at += segments ? segments[i].rows : W->N;
+      c.seg_end[i] = at;
+      c.seg_t[i] = segments ? p.seg_left[i] : (lora ? p.lora_left : nullptr);
+      c.seg_b[i] = segments ? p.seg_right[i] : (lora ? p.lora_right : nullptr);
+      c.seg_scale[i] = segments ? p.seg_scale[i] : (lora ? lora->scale : 0.f);
+    }
+    const int rc = kind == kStream ? stream_forward_launch(c, projected && !ev0, force_slices, stream)
+                                   : swap_forward_launch(c, counters, projected, force_slices, status, stream);
     if (rc == NF4LL_OK && ev1) { if (int rce = record_event(ev1, stream)) return rce; }
     return rc;
   }
@@ -1586,6 +1589,41 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
   if (int rc = require_sm100()) return rc;
   if (M <= 128 || I % 128 || g_tune.any()) {
     // short batches and odd widths: the two projections on their own, then the stand-alone gated product
+    int sms = 148;
+    if (int rc = device_sms(&sms)) return rc;
+    int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, I, W->K, false, sms, g_tune);
+    if (kind != kTiles && M <= kStreamMaxRows && stream_time_us(W->N, W->K, M, sms) < 2 * swap_time_us(I, W->K)) kind = kStream;
+    if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;
+    if (kind == kSwap && (I % 128 || W->N * (W->K / 64) >= (int64_t(1) << 31) || !workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
+                          workspace_bytes < swap_workspace_bytes(W->N, W->K, M, sms, 0))) kind = kTiles;
+    if (kind != kTiles) {
+      // both halves in one pass over the weights
+      StreamCall c{};
+      c.W = W; c.x = x; c.ldx = ldx; c.M = M;
+      c.y = g; c.ldy = ldg; c.y2 = u; c.ldy2 = ldu; c.split = I;
+      c.n_seg = 2;
+      const nf4ll_lora* br[2] = {lora_gate, lora_up};
+      void* tout[2] = {t_gate, t_up};
+      bool projected = false;
+      for (int i = 0; i < 2; ++i) {
+        c.seg_end[i] = (i + 1) * I;
+        if (!br[i]) continue;
+        const bool zero = kind == kSwap && !projected;
+        if (int rc = lora_down_launch(x, ldx, br[i]->mask, br[i]->ld_mask, br[i]->keep_scale, br[i]->A, 1.0f, M, W->K, tout[i],
+                                      zero ? static_cast<int*>(workspace) : nullptr, zero ? static_cast<int>(W->N / 128) : 0, stream)) return rc;
+        projected = true;
+        c.seg_t[i] = static_cast<const float*>(tout[i]);
+        c.seg_b[i] = static_cast<const __half*>(br[i]->B) - i * I * 16;
+        c.seg_scale[i] = br[i]->scale;
+      }
+      cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
+      g_ev_start = g_ev_stop = nullptr;
+      if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
+      if (int rc = kind == kStream ? stream_forward_launch(c, projected && !ev0, 0, stream)
+                                   : swap_forward_launch(c, workspace, projected, 0, status, stream)) return rc;
+      if (ev1) { if (int rce = record_event(ev1, stream)) return rce; }
+      return nf4ll_swiglu_forward(g, ldg, u, ldu, h, ldh, M, I, stream_v);
+    }
     const nf4ll_mat wg = sub_rows(W, 0, I), wu = sub_rows(W, I, I);
     if (int rc = run_gemm(kFwd, &wg, x, ldx, nullptr, lora_gate, t_gate, M, g, ldg, 0, workspace, workspace_bytes, status, stream_v)) return rc;
     if (int rc = run_gemm(kFwd, &wu, x, ldx, nullptr, lora_up, t_up, M, u, ldu, 0, workspace, workspace_bytes, status, stream_v)) return rc;
@@ -1663,13 +1701,9 @@ static int sms_or_default() {
 static int64_t forward_need(int64_t M, int64_t N, int64_t K, int r, int sms, const Tune& tune) {
   const Plan base = make_plan(kFwd, M, N, K, r, sms, tune);
   int64_t need = base.total();
-  // the small-batch kernels keep counters and partial sums in the workspace too; with the kernels forced by
-  // the tuning flags a split count may be forced as well
+  // the swapped-operand kernel keeps counters and partial sums in the workspace too; with it forced by the tuning flags a
+  // split count may be forced as well
   const int fs = tune.splits;
-  if (M <= kStreamCapRows) {
-    const int64_t st = base.left_bytes + base.bt_bytes + stream_workspace_bytes(N, K, M, sms, fs);
-    if (st > need) need = st;
-  }
   if (M <= kSwapMaxRows) {
     const int64_t st = base.left_bytes + base.bt_bytes + swap_workspace_bytes(N, K, M, sms, fs);
     if (st > need) need = st;

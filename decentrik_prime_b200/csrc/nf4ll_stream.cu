@@ -2,26 +2,27 @@
 // of NF4 bytes out of HBM, not by the tensor cores. Replaces, for decode-sized batches, the same
 // reference call sites as the big-tile kernel (solution/fast_qwen.py:947, 1037, 1080-1112).
 //
-// Work is cut into units of 16 weight rows x a slice of the contraction; a warp owns a unit at a time.
-// The first unit of every warp is fixed by its position in the grid (so the weight stream starts before
-// anything else on the stream has to be waited for), later units are handed out through a global counter,
-// which keeps all SMs busy to the end whatever the shape. Per unit and quantisation block a lane loads 8
-// bytes of codes of each of its two rows straight into registers and turns every BYTE (two 4-bit codes)
-// into two fp16 levels with ONE shared-memory load from a 256-entry table of half2 pairs. The table is
-// replicated per lane (entry stride 128 B = 32 lanes x 4 B, lane l reads bank l: no bank conflicts whatever
-// the codes are), so a lookup costs one shift, one logic op and one conflict-free 4-byte LDS for two
-// weights, against 21 integer operations per 8 weights for a byte-permute decode in registers. The levels
-// land directly in the A-operand layout of mma.sync.m16n8k16; the token rows are the B operand with the same
-// column-to-slot assignment. The 64 weights of a block are accumulated on their own and folded into the
-// running sum with that block's fp32 absmax, so the scale is applied once per block:
+// A unit of work is 32 (or 16) weight rows; a team of W warps of one CTA owns it, each warp a part of the contraction, and
+// their partial sums meet in shared memory in a fixed order (results do not depend on timing). Units are dealt out round
+// the SMs. (A split of the contraction over CTAs, with partial sums and arrival counters in global memory, was measured
+// first: the clearing of the counters, the fences and the second pass cost 6 us per call.) A warp fetches for itself:
+// stages of four quantisation blocks by cp.async into a ring of its own (codes, absmax codes, second-level scales), three
+// stages deep and across the ends of units. (Registers as the ring were measured first: a load's scoreboard is shared with
+// the loads issued after it, so every block cost a trip to DRAM.) Every BYTE (two 4-bit codes) becomes two fp16 levels with
+// ONE shared-memory load from a 256-entry table of half2 pairs. The table is replicated per lane (lane l reads word l of an
+// entry: no bank conflicts whatever the codes are) at a stride of 256 B, which makes the byte permute that isolates a code
+// byte the whole address computation; the other 128 B of an entry hold the stages' absmax words. The levels land directly in
+// the A-operand layout of mma.sync.m16n8k16; the token rows are the B operand with the same column-to-slot assignment, loaded
+// once per stage for all of the unit's 16-row tiles. The 64 weights of a block are accumulated on their own and folded into
+// the running sum with that block's fp32 absmax, so the scale is applied once per block:
 //     y[m,n] = sum_blocks absmax[n,b] * sum_{k in b} x[m,k] * fp16(NF4[code[n,k]])
 // This differs from the big-tile kernel's bit-exact fp16 weights by the rounding of NF4[c] * absmax to
 // fp16 (relative 2^-12), inside the 1e-3 tolerance of the path.
 //
-// With the contraction cut into S > 1 slices, a unit writes its 16 x (8 NT) partial sums to a slab in the
-// workspace and bumps its row group's counter; the warp that arrives last adds the S partial sums in slice
-// order (a fixed order: results do not depend on timing), adds bias and the LoRA term and stores fp16.
-#include "nf4ll_common.cuh"
+// 27648 x 5120 (73 MB) at 1 / 8 tokens: 27 / 31 us, of which the fetch alone 19 (with a rank-16 branch at 8 tokens 34, 50
+// for the kernel that handed out units of 16 rows x a slice through a global counter). What is left over the fetch is the
+// table lookups (4 us), the token loads (5 us at 8 tokens) and the MMAs (1 us) that do not hide behind it.
+#include "nf4ll_stream.cuh"
 
 namespace nf4ll {
 
@@ -46,58 +47,134 @@ struct StreamParams {
   __half* y;
   int64_t ldy;
   const __half* bias;
-  const float* t32;        // [M,16] fp32 = drop(x) . A^T, or null (no LoRA)
-  const __half* lora_b;    // [N,16]
-  float lora_scale;
-  int slices;              // S: slices of the contraction
-  int blocks_per_slice;    // quantisation blocks per slice (a multiple of 4, except that the last slice ends with the row)
-  int n_units;             // (N / 16) * S
-  float* slab;             // [N/16][S][8 NT tokens][16 rows] fp32 partial sums (S > 1)
-  int* counters;           // [0]: next unit to hand out (beyond the statically assigned ones); [1 + row group]: arrivals
+  // several projections stacked along N (multiples of 32 rows), each with its own rank-16 branch
+  int n_seg;
+  int64_t seg_end[kMaxSegments];           // first row after the segment
+  const float* seg_t[kMaxSegments];        // [M,16] fp32 = drop(x) . A^T, or null (no LoRA)
+  const __half* seg_b[kMaxSegments];       // lora_B, offset so that it is indexed by the row of W
+  float seg_scale[kMaxSegments];
+  __half* y2;              // rows from `split` on go here (gate|up), null: one output
+  int64_t ldy2, split;
+  int early;               // the kernel before this one is a rank-16 projection of the same call
+  int team;                // W: warps per unit, a divisor of kStreamWarps
 };
 
-constexpr int kStreamWarps = 8;
-constexpr int kTableBytes = 256 * 128;       // 256 byte values x 32 lanes x half2
+constexpr int kStreamWarps = 12;
+constexpr int kStreamRows = 32;              // most weight rows of a unit: one per lane, two 16-row operand tiles
+constexpr int kStep = 4;                     // quantisation blocks per stage
+constexpr int kStreamStages = 3;
+constexpr int kEntryStride = 256;
+constexpr int kTableBytes = 256 * kEntryStride;
+constexpr int kAbsWords = 6;                 // per row and stage: two words of absmax codes, two pairs of scale and offset
+constexpr int kPartBytes = 8 * kStreamRows * 4;              // one warp's sums of 8 tokens x 32 rows
+constexpr int stream_smem(int rt) { return kTableBytes + 1024 + kStreamWarps * (kStreamRows * kStep * 4 + kPartBytes + kStreamStages * kStep * 16 * rt * 32); }
+static_assert(stream_smem(2) <= 227 * 1024, "shared memory budget");
+static_assert(kStreamWarps * kStreamStages * kAbsWords <= 256, "one unused half of a table entry per absmax word of 32 rows");
 
-__device__ __forceinline__ uint32_t lds_u32(uint32_t addr) {
-  uint32_t v;
-  asm("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
-  return v;
-}
-
-// byte offset into the table of the entry of byte `I` of `w` for this lane (lane_off = 4 * lane): entry
-// stride 128 bytes, so bits 7..14 take the byte value and bits 2..6 the lane
+// offset into the table of the entry of byte I of `w` for this lane (lane_off = 4 * lane < 256): one byte permute
 template <int I>
 __device__ __forceinline__ uint32_t entry_offset(uint32_t w, uint32_t lane_off) {
-  const uint32_t shifted = (I == 0) ? (w << 7) : (w >> (8 * I - 7));
-  return (shifted & 0x7F80u) | lane_off;
+  return prmt(w, lane_off, 0x5504u | (I << 4));
 }
 
-// the 8 weights of one 32-bit word of codes as four half2 registers (element order: high nibble first).
-// `table` is the address of a static shared array: a link-time constant that folds into the load's offset.
-__device__ __forceinline__ void decode8(uint32_t w, uint32_t table, uint32_t lane_off, uint32_t (&h)[4]) {
-  h[0] = lds_u32(table + entry_offset<0>(w, lane_off));
-  h[1] = lds_u32(table + entry_offset<1>(w, lane_off));
-  h[2] = lds_u32(table + entry_offset<2>(w, lane_off));
-  h[3] = lds_u32(table + entry_offset<3>(w, lane_off));
+// the 8 weights of one 32-bit word of codes as four half2 registers (element order: high nibble first)
+__device__ __forceinline__ void decode8(const uint8_t* table, uint32_t w, uint32_t lane_off, uint32_t (&h)[4]) {
+  h[0] = *reinterpret_cast<const uint32_t*>(table + entry_offset<0>(w, lane_off));
+  h[1] = *reinterpret_cast<const uint32_t*>(table + entry_offset<1>(w, lane_off));
+  h[2] = *reinterpret_cast<const uint32_t*>(table + entry_offset<2>(w, lane_off));
+  h[3] = *reinterpret_cast<const uint32_t*>(table + entry_offset<3>(w, lane_off));
 }
 
-// NT = number of 8-token tiles (M <= 8 NT).
-template <int NT>
-__global__ void __launch_bounds__(kStreamWarps * 32, NT == 1 ? 3 : (NT == 2 ? 3 : (NT == 4 ? 2 : 1)))
-nf4_stream_kernel(const StreamParams p) {
-  // Launched as a programmatic dependent of the kernel before it (the rank-16 projection T = x . A^T when
-  // there is a LoRA branch, which also clears this launch's counters): the table build and the first unit's
-  // weight stream overlap that kernel; the first write to the workspace waits for it.
+__device__ __forceinline__ void mma16816_first(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
+}
+__device__ __forceinline__ void stream_cp16(uint32_t dst, const void* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void stream_cp4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// NT = number of 8-token tiles (M <= 8 NT), RT = number of 16-row tiles of a unit.
+template <int NT, int RT>
+__global__ void __launch_bounds__(kStreamWarps * 32, 1)
+nf4_stream_kernel(const __grid_constant__ StreamParams p) {
+  // Launched as a programmatic dependent of the kernel before it (the rank-16 projection T = x . A^T when there is a LoRA
+  // branch): the table build and the first units' weight stream overlap that kernel; T is read and the first output
+  // written after it.
   pdl_launch_dependents();
-  __shared__ __align__(128) uint32_t s_tbl[kTableBytes / 4];
-  __shared__ float s_code2[256];
-  __shared__ uint32_t s_lv[16];
+  extern __shared__ __align__(256) uint8_t st_smem[];
+  constexpr int kRows = 16 * RT, kStepBytes = kStep * kRows * 32;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const float code2_mine = threadIdx.x < 256 ? p.code2[threadIdx.x] : 0.f;     // in flight while the table is built
+  float* s_code2 = reinterpret_cast<float*>(st_smem + kTableBytes);
+  float* s_abs = reinterpret_cast<float*>(st_smem + kTableBytes + 1024) + warp * kStreamRows * kStep;      // this warp's [32 rows][4 blocks]
+  float* s_part = reinterpret_cast<float*>(st_smem + kTableBytes + 1024 + kStreamWarps * kStreamRows * kStep * 4);      // [warp][8 tokens][32 rows]
+  uint8_t* ring = reinterpret_cast<uint8_t*>(s_part) + kStreamWarps * kPartBytes + warp * kStreamStages * kStepBytes;
+  uint8_t* words = st_smem + warp * kStreamStages * kAbsWords * kEntryStride + 128 + lane * 4;             // this lane's absmax words
+  const int n_units = static_cast<int>(p.N / kRows);
+  const int bpr = static_cast<int>(p.K / 64);       // quantisation blocks per weight row
+  const bool aligned = (bpr & 3) == 0;
+  const int team = warp / p.team, part = warp - team * p.team;
+  const int first_unit = team * gridDim.x + blockIdx.x, unit_step = kStreamWarps / p.team * gridDim.x;
+  const int steps = (bpr + kStep - 1) / kStep;      // this warp's part of every row, whole stages
+  const int b_begin = steps * part / p.team * kStep;
+  const int b_end = steps * (part + 1) / p.team * kStep < bpr ? steps * (part + 1) / p.team * kStep : bpr;
+  // The fetching side's position: four blocks of unit `fu` from block `fb` on.
+  int fu = b_begin < b_end ? first_unit : n_units, fb = b_begin;
+  // lane l copies half (l & 1) of row l >> 1 (and of that row + 16) of every block, and the absmax words of row l mod kRows
+  const uint8_t* fsrc = p.nib + (static_cast<int64_t>(fu) * kRows + (lane >> 1)) * (p.K / 2) + fb * 32 + (lane & 1) * 16;
+  int64_t fq = (static_cast<int64_t>(fu) * kRows + lane % kRows) * bpr + fb;      // quantisation block of this lane's row
+  const int64_t last_word = p.N * p.K / 64 - 4;     // of the absmax codes (their count is a multiple of 256)
+  auto fetch = [&](int slot) {
+    if (fu < n_units) {
+      const int nb = b_end - fb < kStep ? b_end - fb : kStep;
+      const uint32_t dst = smem_u32(ring + slot * kStepBytes) + lane * 16;
+#pragma unroll
+      for (int u = 0; u < kStep; ++u) {
+        if (u < nb) {
+          stream_cp16(dst + u * (kRows * 32), fsrc + u * 32);
+          if (RT == 2) stream_cp16(dst + u * (kRows * 32) + 512, fsrc + 8 * p.K + u * 32);
+        }
+      }
+      // absmax codes fq .. fq + nb - 1: one aligned word in one second-level group when rows are whole groups of four
+      // blocks long, else two words and the groups of the first and of the last block
+      const uint32_t wd = smem_u32(words) + slot * kAbsWords * kEntryStride;
+      const int64_t w0 = fq & ~int64_t(3), g0 = fq >> 8;
+      stream_cp4(wd, p.qabs + w0);
+      stream_cp4(wd + 2 * kEntryStride, p.scale2 + g0);
+      stream_cp4(wd + 3 * kEntryStride, p.offset2 + g0);
+      if (!aligned) {
+        const int64_t g1 = (fq + nb - 1) >> 8;
+        stream_cp4(wd + kEntryStride, p.qabs + (w0 + 4 < last_word ? w0 + 4 : last_word));
+        stream_cp4(wd + 4 * kEntryStride, p.scale2 + g1);
+        stream_cp4(wd + 5 * kEntryStride, p.offset2 + g1);
+      }
+      fb += kStep;
+      fsrc += kStep * 32;
+      fq += kStep;
+      if (fb >= b_end) {
+        fu += unit_step;
+        fb = b_begin;
+        fsrc = p.nib + (static_cast<int64_t>(fu) * kRows + (lane >> 1)) * (p.K / 2) + fb * 32 + (lane & 1) * 16;
+        fq = (static_cast<int64_t>(fu) * kRows + lane % kRows) * bpr + fb;
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // Behind a rank-16 projection of the same call the weights (and x) may be read at once: that kernel itself went on only
+  // after all earlier work on the stream had finished. Behind anything else only the table build overlaps it.
+  bool waited = false;
+  if (p.early) {
+#pragma unroll
+    for (int s = 0; s < kStreamStages; ++s) fetch(s);
+  }
   {
     constexpr float lv[16] = {NF4LL_LEVELS};
+    uint16_t* s_lv = reinterpret_cast<uint16_t*>(s_code2);      // until code2 takes its place
     if (threadIdx.x < 16) {
       float v = 0.f;
 #pragma unroll
@@ -108,253 +185,243 @@ nf4_stream_kernel(const StreamParams p) {
     // four lanes' copies of an entry per 16-byte store
     for (int idx = threadIdx.x; idx < 256 * 8; idx += kStreamWarps * 32) {
       const int v = idx >> 3;                       // byte value: even element in the high nibble
-      const uint32_t e = s_lv[v >> 4] | (s_lv[v & 15] << 16);
-      reinterpret_cast<uint4*>(s_tbl)[idx] = make_uint4(e, e, e, e);
+      const uint32_t e = s_lv[v >> 4] | (static_cast<uint32_t>(s_lv[v & 15]) << 16);
+      *reinterpret_cast<uint4*>(st_smem + v * kEntryStride + (idx & 7) * 16) = make_uint4(e, e, e, e);
     }
+    if (!p.early) {
+      pdl_wait();
+      waited = true;
+#pragma unroll
+      for (int s = 0; s < kStreamStages; ++s) fetch(s);
+    }
+    const float code2_mine = threadIdx.x < 256 ? p.code2[threadIdx.x] : 0.f;
+    __syncthreads();
+    if (threadIdx.x < 256) s_code2[threadIdx.x] = code2_mine;
+    __syncthreads();
   }
-  // x, the weights and code2 may be read at once: what precedes this kernel on the stream is either the
-  // rank-16 projection kernel, itself started only after all earlier work had finished, or the memset of the
-  // counters, which orders this kernel after everything before it
-  bool waited = false;
-  if (threadIdx.x < 256) s_code2[threadIdx.x] = code2_mine;
-  __syncthreads();
+  const uint32_t lane_off = lane * 4;
+  int slot = 0;
 
-  const uint32_t table = smem_u32(s_tbl), lane_off = lane * 4;
-  const int n_rg = static_cast<int>(p.N / 16);
-  const int bpr = static_cast<int>(p.K / 64);       // quantisation blocks per weight row
-  const int total_warps = gridDim.x * kStreamWarps;
-  int unit = blockIdx.x * kStreamWarps + warp;
-
-  while (unit < p.n_units) {
-    // slice-major order: the warps resident at any time work on one slice of the contraction, i.e. on the
-    // same few columns of x, which then stay in L1
-    const int sl = unit / n_rg, rg = unit - sl * n_rg;
-    const int64_t n0 = static_cast<int64_t>(rg) * 16;
-    const int64_t row0 = n0 + g, row1 = n0 + g + 8;
-    const int b_begin = sl * p.blocks_per_slice;
-    int b_end = b_begin + p.blocks_per_slice;
-    if (b_end > bpr) b_end = bpr;
-
-    // running pointers of this lane: 8 bytes of codes per block and row, the absmax code of block b + t,
-    // 32 bytes of each token row per block. Token rows past M read row 0: their sums are never stored.
-    const uint8_t* w0 = p.nib + (row0 * p.K) / 2 + t * 8 + static_cast<int64_t>(b_begin) * 32;
-    const uint8_t* w1 = p.nib + (row1 * p.K) / 2 + t * 8 + static_cast<int64_t>(b_begin) * 32;
-    int64_t qa = (row0 * p.K) / 64 + b_begin + t, qb = (row1 * p.K) / 64 + b_begin + t;
-    const __half* xr[NT];
+  // The token rows of four blocks (with more than 16 tokens: of one), 32 bytes of each row and block, rows past M zeros. A
+  // block's registers are refilled for the next stage as soon as it has been multiplied: x comes out of L2, and is the same
+  // part of the contraction for every unit of a warp.
+  constexpr int kX = NT <= 2 ? kStep : 1;
+  uint4 x[kX][NT][2];
+  auto load_x = [&](int b, uint4 (&dst)[NT][2]) {
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
-      const int64_t tok = g + 8 * i;
-      xr[i] = p.x + (tok < p.M ? tok : 0) * p.ldx + t * 16 + static_cast<int64_t>(b_begin) * 64;
+      dst[i][0] = dst[i][1] = make_uint4(0, 0, 0, 0);
+      if (b < b_end && g + 8 * i < p.M) {
+        const __half* src = p.x + (g + 8 * i) * p.ldx + t * 16 + static_cast<int64_t>(b) * 64;
+        dst[i][0] = __ldg(reinterpret_cast<const uint4*>(src));
+        dst[i][1] = __ldg(reinterpret_cast<const uint4*>(src + 8));
+      }
     }
-    float acc[NT][4];
+  };
+  if (NT <= 2 && first_unit < n_units) {
 #pragma unroll
-    for (int i = 0; i < NT; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
+    for (int u = 0; u < kX; ++u) load_x(b_begin + u, x[u]);
+  }
 
-    // Four blocks at a time: each lane recovers the absmax of one of them (block b + t) for both of its rows
-    // and the quad shares them by shuffle.
-    for (int b = b_begin; b < b_end; b += 4) {
-      const int nb = (b_end - b < 4) ? b_end - b : 4;
-      uint2 c0[4], c1[4];
+  for (int unit = first_unit; unit < n_units; unit += unit_step) {
+    const int64_t n0 = static_cast<int64_t>(unit) * kRows;
+    float acc[RT][NT][4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (u < nb) {
-          c0[u] = __ldcs(reinterpret_cast<const uint2*>(w0 + u * 32));
-          c1[u] = __ldcs(reinterpret_cast<const uint2*>(w1 + u * 32));
-        } else {
-          c0[u] = make_uint2(0, 0); c1[u] = make_uint2(0, 0);
+    for (int r = 0; r < RT; ++r)
+#pragma unroll
+      for (int i = 0; i < NT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[r][i][j] = 0.f;
+    int64_t q = (n0 + lane % kRows) * bpr + b_begin;        // quantisation block of this lane's row
+
+    for (int b = b_begin; b < b_end; b += kStep, q += kStep) {
+      const int nb = b_end - b < kStep ? b_end - b : kStep;
+      const int b_next = b + kStep < b_end ? b + kStep : b_begin;
+      asm volatile("cp.async.wait_group %0;" ::"n"(kStreamStages - 1) : "memory");
+      __syncwarp();
+      // absmax of this lane's row: codes -> fp32, shared by the warp
+      {
+        const uint8_t* wd = words + slot * kAbsWords * kEntryStride;
+        uint32_t codes = *reinterpret_cast<const uint32_t*>(wd);
+        const float s0 = *reinterpret_cast<const float*>(wd + 2 * kEntryStride), o0 = *reinterpret_cast<const float*>(wd + 3 * kEntryStride);
+        float s1 = s0, o1 = o0;
+        int turn = 4;                               // blocks of the first second-level group
+        if (!aligned) {
+          codes = __funnelshift_r(codes, *reinterpret_cast<const uint32_t*>(wd + kEntryStride), 8 * static_cast<int>(q & 3));
+          s1 = *reinterpret_cast<const float*>(wd + 4 * kEntryStride);
+          o1 = *reinterpret_cast<const float*>(wd + 5 * kEntryStride);
+          const int left = 256 - static_cast<int>(q & 255);
+          turn = left < 4 ? left : 4;
         }
-      }
-      float am0 = 0.f, am1 = 0.f;
-      if (t < nb) {
-        am0 = block_absmax(s_code2[__ldg(p.qabs + qa)], __ldg(p.scale2 + (qa >> 8)), __ldg(p.offset2 + (qa >> 8)));
-        am1 = block_absmax(s_code2[__ldg(p.qabs + qb)], __ldg(p.scale2 + (qb >> 8)), __ldg(p.offset2 + (qb >> 8)));
-      }
+        float v[4];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const float a0 = __shfl_sync(0xffffffffu, am0, (lane & ~3) | u);
-        const float a1 = __shfl_sync(0xffffffffu, am1, (lane & ~3) | u);
+        for (int j = 0; j < 4; ++j)
+          v[j] = block_absmax(s_code2[(codes >> (8 * j)) & 255u], j < turn ? s0 : s1, j < turn ? o0 : o1);
+        *reinterpret_cast<float4*>(s_abs + lane * 4) = make_float4(v[0], v[1], v[2], v[3]);
+        __syncwarp();
+      }
+      float am[2 * RT][4];                          // rows g, g + 8, ...; blocks
+#pragma unroll
+      for (int r = 0; r < 2 * RT; ++r) {
+        const float4 f = *reinterpret_cast<const float4*>(s_abs + (g + 8 * r) * 4);
+        am[r][0] = f.x; am[r][1] = f.y; am[r][2] = f.z; am[r][3] = f.w;
+      }
+      const uint8_t* codes = ring + slot * kStepBytes + g * 32 + t * 8;
+#pragma unroll
+      for (int u = 0; u < kStep; ++u) {
         if (u < nb) {
-          uint32_t lo0[4], hi0[4], lo1[4], hi1[4];
-          decode8(c0[u].x, table, lane_off, lo0); decode8(c0[u].y, table, lane_off, hi0);     // row g:   k 16t..16t+7, +8..+15
-          decode8(c1[u].x, table, lane_off, lo1); decode8(c1[u].y, table, lane_off, hi1);     // row g+8
+          if (NT > 2) load_x(b + u, x[0]);
 #pragma unroll
-          for (int i = 0; i < NT; ++i) {
-            const uint4 xa = __ldg(reinterpret_cast<const uint4*>(xr[i] + u * 64));
-            const uint4 xb = __ldg(reinterpret_cast<const uint4*>(xr[i] + u * 64 + 8));
-            float blk[4] = {0.f, 0.f, 0.f, 0.f};
-            mma16816_acc(blk, lo0[0], lo1[0], lo0[1], lo1[1], xa.x, xa.y);
-            mma16816_acc(blk, lo0[2], lo1[2], lo0[3], lo1[3], xa.z, xa.w);
-            mma16816_acc(blk, hi0[0], hi1[0], hi0[1], hi1[1], xb.x, xb.y);
-            mma16816_acc(blk, hi0[2], hi1[2], hi0[3], hi1[3], xb.z, xb.w);
-            acc[i][0] = fmaf(blk[0], a0, acc[i][0]);
-            acc[i][1] = fmaf(blk[1], a0, acc[i][1]);
-            acc[i][2] = fmaf(blk[2], a1, acc[i][2]);
-            acc[i][3] = fmaf(blk[3], a1, acc[i][3]);
+          for (int r = 0; r < RT; ++r) {
+            const uint2 c0 = *reinterpret_cast<const uint2*>(codes + u * (kRows * 32) + r * 512);
+            const uint2 c1 = *reinterpret_cast<const uint2*>(codes + u * (kRows * 32) + r * 512 + 256);
+            uint32_t lo0[4], hi0[4], lo1[4], hi1[4];
+            decode8(st_smem, c0.x, lane_off, lo0); decode8(st_smem, c0.y, lane_off, hi0);     // row g:   k 16t..16t+7, +8..+15
+            decode8(st_smem, c1.x, lane_off, lo1); decode8(st_smem, c1.y, lane_off, hi1);     // row g+8
+#pragma unroll
+            for (int i = 0; i < NT; ++i) {
+              const uint4 xa = x[u % kX][i][0], xb = x[u % kX][i][1];
+              float blk[4];
+              mma16816_first(blk, lo0[0], lo1[0], lo0[1], lo1[1], xa.x, xa.y);
+              mma16816_acc(blk, lo0[2], lo1[2], lo0[3], lo1[3], xa.z, xa.w);
+              mma16816_acc(blk, hi0[0], hi1[0], hi0[1], hi1[1], xb.x, xb.y);
+              mma16816_acc(blk, hi0[2], hi1[2], hi0[3], hi1[3], xb.z, xb.w);
+              acc[r][i][0] = fmaf(blk[0], am[2 * r][u], acc[r][i][0]);
+              acc[r][i][1] = fmaf(blk[1], am[2 * r][u], acc[r][i][1]);
+              acc[r][i][2] = fmaf(blk[2], am[2 * r + 1][u], acc[r][i][2]);
+              acc[r][i][3] = fmaf(blk[3], am[2 * r + 1][u], acc[r][i][3]);
+            }
           }
         }
+        if (NT <= 2) load_x(b_next + u, x[u % kX]);
       }
-      w0 += 4 * 32; w1 += 4 * 32;
-      qa += 4; qb += 4;
-#pragma unroll
-      for (int i = 0; i < NT; ++i) xr[i] += 4 * 64;
+      __syncwarp();                                 // everybody has read the stage and the absmax values
+      fetch(slot);
+      slot = slot + 1 == kStreamStages ? 0 : slot + 1;
     }
 
-    // accumulator layout: acc[i][0..1] = (weight row g, tokens 8i + 2t, +1); acc[i][2..3] = row g + 8
+    // accumulator layout: acc[r][i][0..1] = (weight row 16 r + g, tokens 8i + 2t, +1); acc[r][i][2..3] = that row + 8
     if (!waited) {
-      pdl_wait();                 // T, and the zeroed counters, come from the kernel this one was launched behind
+      pdl_wait();                 // T comes from the kernel this one was launched behind
       waited = true;
     }
-    bool finish = true;
-    if (p.slices > 1) {
-      float* mine = p.slab + ((static_cast<int64_t>(rg) * p.slices + sl) * (8 * NT)) * 16;
+    int sg = 0;
+    while (sg + 1 < p.n_seg && n0 >= p.seg_end[sg]) ++sg;
+    const float* t32 = p.seg_t[sg];
+    const int64_t row = n0 + lane % kRows;          // from here on a lane is a weight row
+    __half* y = p.y + row;
+    int64_t ldy = p.ldy;
+    if (p.y2 && n0 >= p.split) { y = p.y2 + (row - p.split); ldy = p.ldy2; }
+    const float bias = p.bias ? __half2float(p.bias[row]) : 0.f;
+    float br[16];
+    if (t32) {
+      const uint4* bp = reinterpret_cast<const uint4*>(p.seg_b[sg] + row * 16);
+      const float lora_scale = p.seg_scale[sg];
+      float tmp[8];
+      unpack8(__ldg(bp), tmp);
 #pragma unroll
-      for (int i = 0; i < NT; ++i) {
-        mine[(8 * i + 2 * t) * 16 + g] = acc[i][0];
-        mine[(8 * i + 2 * t + 1) * 16 + g] = acc[i][1];
-        mine[(8 * i + 2 * t) * 16 + g + 8] = acc[i][2];
-        mine[(8 * i + 2 * t + 1) * 16 + g + 8] = acc[i][3];
-      }
-      __threadfence();
-      __syncwarp();
-      int prev = 0;
-      if (lane == 0) prev = atomicAdd(p.counters + 1 + rg, 1);
-      prev = __shfl_sync(0xffffffffu, prev, 0);
-      finish = (prev == p.slices - 1);
-      if (finish) {
-        __threadfence();
-        const float* all = p.slab + (static_cast<int64_t>(rg) * p.slices * (8 * NT)) * 16;
+      for (int j = 0; j < 8; ++j) br[j] = tmp[j] * lora_scale;
+      unpack8(__ldg(bp + 1), tmp);
 #pragma unroll
-        for (int i = 0; i < NT; ++i)
-#pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-        for (int s2 = 0; s2 < p.slices; ++s2) {
-          const float* part = all + static_cast<int64_t>(s2) * (8 * NT) * 16;
-#pragma unroll
-          for (int i = 0; i < NT; ++i) {
-            acc[i][0] += __ldcg(part + (8 * i + 2 * t) * 16 + g);
-            acc[i][1] += __ldcg(part + (8 * i + 2 * t + 1) * 16 + g);
-            acc[i][2] += __ldcg(part + (8 * i + 2 * t) * 16 + g + 8);
-            acc[i][3] += __ldcg(part + (8 * i + 2 * t + 1) * 16 + g + 8);
-          }
-        }
-      }
+      for (int j = 0; j < 8; ++j) br[8 + j] = tmp[j] * lora_scale;
     }
-    if (finish) {
-      // bias, LoRA term, one rounding to fp16
-      float bias0 = 0.f, bias1 = 0.f;
-      if (p.bias) { bias0 = __half2float(p.bias[row0]); bias1 = __half2float(p.bias[row1]); }
-      float br0[16], br1[16];
-      if (p.t32) {
-        const uint4* b0p = reinterpret_cast<const uint4*>(p.lora_b + row0 * 16);
-        const uint4* b1p = reinterpret_cast<const uint4*>(p.lora_b + row1 * 16);
-        float tmp[8];
-        unpack8(__ldg(b0p), tmp);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) br0[j] = tmp[j] * p.lora_scale;
-        unpack8(__ldg(b0p + 1), tmp);
+    for (int i = 0; i < NT; ++i) {
+      if (8 * i < p.M) {
+        // [token][row], rows XORed with the token so that neither side has bank conflicts
+        float* mine = s_part + warp * (8 * kStreamRows);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) br0[8 + j] = tmp[j] * p.lora_scale;
-        unpack8(__ldg(b1p), tmp);
+        for (int r = 0; r < RT; ++r)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) br1[j] = tmp[j] * p.lora_scale;
-        unpack8(__ldg(b1p + 1), tmp);
+          for (int j = 0; j < 4; ++j) mine[(2 * t + (j & 1)) * kStreamRows + ((16 * r + 8 * (j >> 1) + g) ^ (8 * t))] = acc[r][i][j];
+        named_barrier(1 + team, p.team * 32);
+        // the team's warps (of 16 rows: half warps) share the tokens out
+        for (int k = RT == 2 ? part : 2 * part + (lane >> 4); k < 8; k += (3 - RT) * p.team) {
+          const int64_t tok = 8 * i + k;
+          if (tok >= p.M) break;
+          float v = 0.f;
+          for (int w = 0; w < p.team; ++w) v += s_part[(team * p.team + w) * (8 * kStreamRows) + k * kStreamRows + ((lane % kRows) ^ (8 * (k >> 1)))];
+          v += bias;
+          if (t32) {
+            const float4* tr = reinterpret_cast<const float4*>(t32 + tok * 16);
+            float l = 0.f;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) br1[8 + j] = tmp[j] * p.lora_scale;
-      }
-#pragma unroll
-      for (int i = 0; i < NT; ++i) {
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int64_t tok = 8 * i + 2 * t + e;
-          if (tok < p.M) {
-            float v0 = acc[i][e] + bias0, v1 = acc[i][2 + e] + bias1;
-            if (p.t32) {
-              const float4* tr = reinterpret_cast<const float4*>(p.t32 + tok * 16);
-              float l0 = 0.f, l1 = 0.f;
-#pragma unroll
-              for (int j4 = 0; j4 < 4; ++j4) {
-                const float4 tv = __ldcg(tr + j4);
-                l0 = fmaf(tv.x, br0[4 * j4], l0); l0 = fmaf(tv.y, br0[4 * j4 + 1], l0);
-                l0 = fmaf(tv.z, br0[4 * j4 + 2], l0); l0 = fmaf(tv.w, br0[4 * j4 + 3], l0);
-                l1 = fmaf(tv.x, br1[4 * j4], l1); l1 = fmaf(tv.y, br1[4 * j4 + 1], l1);
-                l1 = fmaf(tv.z, br1[4 * j4 + 2], l1); l1 = fmaf(tv.w, br1[4 * j4 + 3], l1);
-              }
-              v0 += l0; v1 += l1;
+            for (int j4 = 0; j4 < 4; ++j4) {
+              const float4 tv = __ldcg(tr + j4);
+              l = fmaf(tv.x, br[4 * j4], l); l = fmaf(tv.y, br[4 * j4 + 1], l);
+              l = fmaf(tv.z, br[4 * j4 + 2], l); l = fmaf(tv.w, br[4 * j4 + 3], l);
             }
-            p.y[tok * p.ldy + row0] = __float2half_rn(v0);
-            p.y[tok * p.ldy + row1] = __float2half_rn(v1);
+            v += l;
           }
+          y[tok * ldy] = __float2half_rn(v);
         }
+        __syncwarp();
+        named_barrier(1 + team, p.team * 32);       // the sums have been read
       }
     }
-    // next unit from the shared counter (the first `total_warps` units were assigned statically)
-    int next = 0;
-    if (lane == 0) next = total_warps + atomicAdd(p.counters, 1);
-    unit = __shfl_sync(0xffffffffu, next, 0);
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
 }
 
-// Units and slices for W[N,K] at M rows: aim at several units per resident warp so that the dynamic hand-out
-// can balance the SMs, but never cut a row into slices shorter than 8 quantisation blocks.
-void stream_plan(int64_t N, int64_t K, int64_t M, int sms, int force_slices, int* slices, int* blocks_per_slice) {
-  const int bpr = static_cast<int>(K / 64);
-  const int64_t row_groups = N / 16;
-  int s = 1;
-  const int64_t want = static_cast<int64_t>(sms) * 48;            // units to aim for
-  if (row_groups < want) s = static_cast<int>((want + row_groups - 1) / row_groups);
-  int max_s = bpr / 8;
-  if (max_s < 1) max_s = 1;
-  if (s > max_s) s = max_s;
-  if (force_slices > 0) s = force_slices;
-  int per = (bpr + s - 1) / s;
-  per = (per + 3) / 4 * 4;                                        // whole groups of four blocks
-  s = (bpr + per - 1) / per;
-  *slices = s;
-  *blocks_per_slice = per;
+// Rows and warps per unit: the pair with the least work in blocks over the rounds of units that the busiest warp takes, a unit
+// costing its blocks and about three more (filling the pipeline, the exchange). Units of 16 rows cost 0.6 of one of 32
+// (token rows and absmax words are fetched for half the weights); they pay where 32 leave SMs idle in the last round
+// (5120 x 5120 at 1 token: 9.3 us in units of 16, 10.3 in units of 32; 5120 x 27648: 38.6 and 45.4).
+static int64_t stream_plan(int64_t N, int64_t K, int sms, int force, int* row_tiles, int* team) {
+  const int64_t steps = (K / 64 + kStep - 1) / kStep;
+  int64_t best = 0;
+  *row_tiles = 0;
+  for (int rt = 2; rt >= 1; --rt) {
+    const int64_t units = N / (16 * rt);
+    for (int w : {1, 2, 3, 4, 6, 12}) {
+      static_assert(kStreamWarps == 12, "its divisors");
+      const int64_t at_once = static_cast<int64_t>(sms) * (kStreamWarps / w);
+      const int64_t cost = (units + at_once - 1) / at_once * ((steps + w - 1) / w * kStep + 3) * (rt == 2 ? 10 : 6);
+      if (force > 0 ? (rt == 1 + (force & 1) && w <= force) : (*row_tiles == 0 || cost < best || (cost == best && rt == *row_tiles))) {
+        best = cost;
+        *row_tiles = rt;
+        *team = w;
+      }
+    }
+  }
+  return best;
 }
 
-int64_t stream_workspace_bytes(int64_t N, int64_t K, int64_t M, int sms, int force_slices) {
-  int s = 1, per = 0;
-  stream_plan(N, K, M, sms, force_slices, &s, &per);
-  const int nt = M <= 8 ? 1 : (M <= 16 ? 2 : (M <= 32 ? 4 : 8));
-  const int64_t counters = (1 + N / 16) * 4;
-  const int64_t slab = s > 1 ? (N / 16) * s * (8 * nt) * 16 * 4 : 0;
-  return (counters + 255) / 256 * 256 + (slab + 255) / 256 * 256;
+double stream_time_us(int64_t N, int64_t K, int64_t M, int sms) {
+  int rt = 0, team = 0;
+  const int64_t cost = stream_plan(N, K, sms, 0, &rt, &team);      // in tenths of a block of 32 rows
+  return 0.06 * cost * (M > 8 ? 1.3 : 1.0) + 0.0125 * M * cost / (rt == 2 ? 10 : 6);
 }
 
-// `scratch` holds the counters (zeroed here unless `counters_zeroed`: the rank-16 projection kernel launched just
-// before has then done it) followed, 256-byte aligned, by the slab.
-int stream_forward_launch(const nf4ll_mat* W, const void* x, int64_t ldx, const void* bias, const float* t32,
-                          const void* lora_b, float lora_scale, int64_t M, void* y, int64_t ldy, void* scratch,
-                          bool counters_zeroed, int force_slices, cudaStream_t stream) {
+template <int RT>
+static auto stream_kernel(int64_t M) {
+  return M <= 8 ? nf4_stream_kernel<1, RT> : (M <= 16 ? nf4_stream_kernel<2, RT> : (M <= 32 ? nf4_stream_kernel<4, RT> : nf4_stream_kernel<8, RT>));
+}
+
+int stream_forward_launch(const StreamCall& c, bool early, int force_team, cudaStream_t stream) {
   int dev = 0, sms = 148;
   NF4LL_CUDA(cudaGetDevice(&dev));
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const nf4ll_mat* W = c.W;
   StreamParams p{};
   p.nib = W->nib; p.qabs = W->qabs; p.scale2 = W->scale2; p.offset2 = W->offset2; p.code2 = W->code2;
-  p.N = W->N; p.K = W->K; p.M = M;
-  p.x = static_cast<const __half*>(x); p.ldx = ldx;
-  p.y = static_cast<__half*>(y); p.ldy = ldy;
-  p.bias = static_cast<const __half*>(bias);
-  p.t32 = t32; p.lora_b = static_cast<const __half*>(lora_b); p.lora_scale = lora_scale;
-  stream_plan(W->N, W->K, M, sms, force_slices, &p.slices, &p.blocks_per_slice);
-  p.n_units = static_cast<int>(W->N / 16) * p.slices;
-  const int64_t counter_bytes = ((1 + W->N / 16) * 4 + 255) / 256 * 256;
-  p.counters = static_cast<int*>(scratch);
-  p.slab = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + counter_bytes);
-  if (!counters_zeroed) NF4LL_CUDA(cudaMemsetAsync(p.counters, 0, (1 + W->N / 16) * 4, stream));
-  const int nt = M <= 8 ? 1 : (M <= 16 ? 2 : (M <= 32 ? 4 : 8));
-  void (*kernel)(const StreamParams) = nt == 1 ? nf4_stream_kernel<1> : (nt == 2 ? nf4_stream_kernel<2>
-                                       : (nt == 4 ? nf4_stream_kernel<4> : nf4_stream_kernel<8>));
-  const int smem = 0;
-  int per_sm = 0;
-  NF4LL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kStreamWarps * 32, smem));
-  if (per_sm < 1) per_sm = 1;
-  int64_t grid = (p.n_units + kStreamWarps - 1) / kStreamWarps;
-  if (grid > static_cast<int64_t>(sms) * per_sm) grid = static_cast<int64_t>(sms) * per_sm;
-  PdlLaunch lc(dim3(static_cast<unsigned>(grid)), dim3(kStreamWarps * 32), smem, stream);
+  p.N = W->N; p.K = W->K; p.M = c.M;
+  p.x = static_cast<const __half*>(c.x); p.ldx = c.ldx;
+  p.y = static_cast<__half*>(c.y); p.ldy = c.ldy;
+  p.y2 = static_cast<__half*>(c.y2); p.ldy2 = c.ldy2; p.split = c.split;
+  p.bias = static_cast<const __half*>(c.bias);
+  p.n_seg = c.n_seg;
+  for (int i = 0; i < c.n_seg; ++i) {
+    p.seg_end[i] = c.seg_end[i];
+    p.seg_t[i] = c.seg_t[i]; p.seg_b[i] = c.seg_b[i]; p.seg_scale[i] = c.seg_scale[i];
+  }
+  p.early = early ? 1 : 0;
+  int rt = 0;
+  stream_plan(W->N, W->K, sms, force_team, &rt, &p.team);
+  const auto kernel = rt == 2 ? stream_kernel<2>(c.M) : stream_kernel<1>(c.M);
+  NF4LL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, stream_smem(rt)));
+  const int64_t units = W->N / (16 * rt);
+  PdlLaunch lc(dim3(static_cast<unsigned>(units < sms ? units : sms)), dim3(kStreamWarps * 32), stream_smem(rt), stream);
   NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, kernel, p));
   return NF4LL_OK;
 }

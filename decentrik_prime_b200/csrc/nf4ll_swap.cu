@@ -43,7 +43,7 @@
 // Warp roles: 0 producer of codes (TMA) and absmax codes (cp.async), 1 tensor-memory allocation + MMA issue (first
 // half of every group), 2 TMA producer of token tiles, 3..18 decode and then the epilogue, 19 MMA issue (second half). Every wait is bounded and reports through
 // the status word.
-#include "nf4ll_gemm_shared.cuh"
+#include "nf4ll_stream.cuh"
 
 namespace nf4ll {
 
@@ -56,9 +56,14 @@ struct SwapParams {
   __half* y;
   int64_t ldy;
   const __half* bias;
-  const float* t32;        // [M,16] fp32 = drop(x) . A^T, or null (no LoRA)
-  const __half* lora_b;    // [N,16]
-  float lora_scale;
+  __half* y2;              // rows from `split` on go here (gate|up), null: one output
+  int64_t ldy2, split;
+  // projections stacked along N (multiples of 128 rows: a tile lies in one), each with its own rank-16 branch
+  int n_seg;
+  int64_t seg_end[kMaxSegments];           // first row after the segment
+  const float* seg_t[kMaxSegments];        // [M,16] fp32 = drop(x) . A^T, or null (no LoRA)
+  const __half* seg_b[kMaxSegments];       // lora_B, offset so that it is indexed by the row of W
+  float seg_scale[kMaxSegments];
   int slices;              // slices of the contraction
   int groups_per_slice;    // groups of four quantisation blocks per slice
   int n_units;             // tiles * slices
@@ -176,7 +181,7 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 
 template <int NTOK>
 __global__ void __launch_bounds__(kSwapThreads, 1)
-nf4_swap_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_nib, const SwapParams p) {
+nf4_swap_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_nib, const __grid_constant__ SwapParams p) {
   using Cfg = SwapCfg<NTOK>;
   // x, the weights and code2 may be read at once (what precedes this kernel on the stream is the rank-16
   // projection kernel, itself started only after all earlier work had finished, or a memset, which orders this
@@ -491,23 +496,30 @@ nf4_swap_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       if (ok) ok = wait_or_abort(smem_u32(acc_full), ul & 1, ab, 0x0506);
       pdl_wait();                                 // T and the cleared counters come from the kernel before this one
       float bias = 0.f, bs[16];
+      int sg = 0;
+      while (sg + 1 < p.n_seg && static_cast<int64_t>(tile) * 128 >= p.seg_end[sg]) ++sg;
+      const float* t32 = p.seg_t[sg];
+      const bool second = p.y2 && static_cast<int64_t>(tile) * 128 >= p.split;
+      __half* y = second ? p.y2 + (n - p.split) : p.y + n;
+      const int64_t ldy = second ? p.ldy2 : p.ldy;
       auto load_row_terms = [&]() {
         if (p.bias && row_ok) bias = __half2float(p.bias[n]);
-        if (p.t32 && row_ok) {
+        if (t32 && row_ok) {
           float tmp[8];
-          const uint4* bp = reinterpret_cast<const uint4*>(p.lora_b + n * 16);
+          const uint4* bp = reinterpret_cast<const uint4*>(p.seg_b[sg] + n * 16);
+          const float lora_scale = p.seg_scale[sg];
           unpack8(__ldg(bp), tmp);
 #pragma unroll
-          for (int jj = 0; jj < 8; ++jj) bs[jj] = tmp[jj] * p.lora_scale;
+          for (int jj = 0; jj < 8; ++jj) bs[jj] = tmp[jj] * lora_scale;
           unpack8(__ldg(bp + 1), tmp);
 #pragma unroll
-          for (int jj = 0; jj < 8; ++jj) bs[8 + jj] = tmp[jj] * p.lora_scale;
+          for (int jj = 0; jj < 8; ++jj) bs[8 + jj] = tmp[jj] * lora_scale;
         }
       };
       auto finish = [&](int tok, float v) {
         // bias, LoRA term, one rounding; 32 lanes store 32 consecutive output columns of one token row
-        if (p.t32) {
-          const float4* tr = reinterpret_cast<const float4*>(p.t32 + static_cast<int64_t>(tok) * 16);
+        if (t32) {
+          const float4* tr = reinterpret_cast<const float4*>(t32 + static_cast<int64_t>(tok) * 16);
           float l = 0.f;
 #pragma unroll
           for (int j4 = 0; j4 < 4; ++j4) {
@@ -517,7 +529,7 @@ nf4_swap_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
           }
           v += l;
         }
-        p.y[static_cast<int64_t>(tok) * p.ldy + n] = __float2half_rn(v + bias);
+        y[static_cast<int64_t>(tok) * ldy] = __float2half_rn(v + bias);
       };
       const bool has_cols = team * 16 < NTOK;
       if (ok) {
@@ -683,20 +695,34 @@ static int swap_launch_cfg(const CUtensorMap& mx, const CUtensorMap& mn, const S
   return NF4LL_OK;
 }
 
+// Clears the counters of a launch that no rank-16 projection precedes. Launched also where there are none to clear: the
+// kernel after it reads x and the weights at once, which is right only behind a kernel that itself went on after all earlier
+// work. (A kernel and not a memset: the next one can start meanwhile.)
+__global__ void __launch_bounds__(256) swap_zero_kernel(int* counters, int n) {
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int i = threadIdx.x; i < n; i += 256) counters[i] = 0;
+}
+
 // `scratch`: the tile counters (cleared here unless `counters_zeroed`: the rank-16 projection kernel launched
 // just before has then done it) followed, 256-byte aligned, by the slab.
-int swap_forward_launch(const nf4ll_mat* W, const void* x, int64_t ldx, const void* bias, const float* t32,
-                        const void* lora_b, float lora_scale, int64_t M, void* y, int64_t ldy, void* scratch,
-                        bool counters_zeroed, int force_slices, int32_t* status, cudaStream_t stream) {
+int swap_forward_launch(const StreamCall& c, void* scratch, bool counters_zeroed, int force_slices, int32_t* status, cudaStream_t stream) {
   int dev = 0, sms = 148;
   NF4LL_CUDA(cudaGetDevice(&dev));
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const nf4ll_mat* W = c.W;
+  const int64_t M = c.M;
   SwapParams p{};
   p.qabs = W->qabs; p.scale2 = W->scale2; p.offset2 = W->offset2; p.code2 = W->code2;
   p.N = W->N; p.K = W->K; p.M = M;
-  p.y = static_cast<__half*>(y); p.ldy = ldy;
-  p.bias = static_cast<const __half*>(bias);
-  p.t32 = t32; p.lora_b = static_cast<const __half*>(lora_b); p.lora_scale = lora_scale;
+  p.y = static_cast<__half*>(c.y); p.ldy = c.ldy;
+  p.y2 = static_cast<__half*>(c.y2); p.ldy2 = c.ldy2; p.split = c.split;
+  p.bias = static_cast<const __half*>(c.bias);
+  p.n_seg = c.n_seg;
+  for (int i = 0; i < c.n_seg; ++i) {
+    p.seg_end[i] = c.seg_end[i];
+    p.seg_t[i] = c.seg_t[i]; p.seg_b[i] = c.seg_b[i]; p.seg_scale[i] = c.seg_scale[i];
+  }
   p.status = status;
   const int ntok = swap_ntok(M);
   swap_plan(W->N, W->K, ntok, sms, force_slices, &p.slices, &p.groups_per_slice);
@@ -705,10 +731,13 @@ int swap_forward_launch(const nf4ll_mat* W, const void* x, int64_t ldx, const vo
   const int64_t counter_bytes = (tiles * 4 + 255) / 256 * 256;
   p.counters = static_cast<int*>(scratch);
   p.slab = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + counter_bytes);
-  if (p.slices > 1 && !counters_zeroed) NF4LL_CUDA(cudaMemsetAsync(p.counters, 0, tiles * 4, stream));
+  if (!counters_zeroed) {
+    PdlLaunch lz(dim3(1), dim3(256), 0, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lz.cfg, swap_zero_kernel, p.counters, p.slices > 1 ? static_cast<int>(tiles) : 0));
+  }
   CUtensorMap mx, mn;
-  if (int rc = swap_encode(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, x, static_cast<uint64_t>(W->K), static_cast<uint64_t>(M),
-                           static_cast<uint64_t>(ldx) * 2, 64, static_cast<uint32_t>(ntok), "token tile")) return rc;
+  if (int rc = swap_encode(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, c.x, static_cast<uint64_t>(W->K), static_cast<uint64_t>(M),
+                           static_cast<uint64_t>(c.ldx) * 2, 64, static_cast<uint32_t>(ntok), "token tile")) return rc;
   if (int rc = swap_encode(&mn, CU_TENSOR_MAP_DATA_TYPE_UINT8, W->nib, static_cast<uint64_t>(W->K / 2), static_cast<uint64_t>(W->N),
                            static_cast<uint64_t>(W->K / 2), 128, 128, "codes")) return rc;
   int64_t ctas = sms;
