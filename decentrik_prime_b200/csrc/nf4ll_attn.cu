@@ -10,11 +10,12 @@
 //
 //   rope     q, k rotated once into a buffer (a key row is read by every query tile after it)
 //   forward  one CTA per 64 query rows and head, 4 warps of 16 rows, keys and values in 64-row blocks by cp.async
-//   dK, dV   one CTA per 64 key rows and key-value head, looping over the group's query heads and the later query rows:
-//            sums over heads stay in registers, no atomics
+//   dK, dV   a cluster of up to 8 CTAs per 64 key rows and key-value head, the group's query heads dealt out among them,
+//            each looping over the later query rows; their sums meet through distributed shared memory in a fixed order. One
+//            CTA for the whole group left most SMs idle: 951 rows, 12 heads of 128 in groups of 6, 115 us, 28 now
 //   dQ       one CTA per 64 query rows and head, looping over the earlier key rows
 // The backward kernels rotate dQ and dK back in their epilogue (both halves of a rotated pair sit in one thread).
-#include "nf4ll_common.cuh"
+#include "nf4ll_pair.cuh"
 
 namespace nf4ll {
 
@@ -299,6 +300,17 @@ __device__ __forceinline__ void store_unrotated(const float (&acc)[HD / 8][4], c
   }
 }
 
+__device__ __forceinline__ float4 attn_peer128(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+// 4 bytes global -> shared, zeros when `valid` is false
+__device__ __forceinline__ void attn_cp4(uint32_t dst, const void* src, bool valid) {
+  const int n = valid ? 4 : 0;
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
 template <int HD>
 __global__ void __launch_bounds__(kAttnThreads)
 attn_dq_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ SeqTable seqs) {
@@ -401,19 +413,22 @@ attn_dkv_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Se
   float* sL = reinterpret_cast<float*>(a_smem + 2 * TILE + 4 * QT);      // [2][QR] lse, [2][QR] delta
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   int start, len, k0;
-  find_tile(seqs, blockIdx.x, start, len, k0);                           // earlier key tiles have more query rows: first
+  // cluster of C CTAs: rank r takes the group's heads r, r + C, ...
+  const int C = static_cast<int>(gridDim.x) / seqs.tile[seqs.n], rank = static_cast<int>(blockIdx.x) % C;
+  find_tile(seqs, blockIdx.x / C, start, len, k0);                       // earlier key tiles have more query rows: first
   const int kvh = blockIdx.y;
   load_tile<HD, kAttnRows>(sK, p.k + start * p.ldr + kvh * HD, p.ldr, k0, len);
   load_tile<HD, kAttnRows>(sV, p.v + start * p.ldv + kvh * HD, p.ldv, k0, len);
-  const int per_head = (len - k0 + QR - 1) / QR, steps = per_head * p.group;
+  const int per_head = (len - k0 + QR - 1) / QR, steps = per_head * ((p.group - rank + C - 1) / C);
   auto issue = [&](int it) {
-    const int head = kvh * p.group + it / per_head, q0 = k0 + (it % per_head) * QR, slot = it & 1;
+    const int head = kvh * p.group + rank + it / per_head * C, q0 = k0 + (it % per_head) * QR, slot = it & 1;
     load_tile<HD, QR>(sQ + slot * QT, p.q + start * p.ldr + head * HD, p.ldr, q0, len);
     load_tile<HD, QR>(sO + slot * QT, p.dout + start * p.lddo + head * HD, p.lddo, q0, len);
     if (threadIdx.x < QR) {
       const int r = q0 + threadIdx.x;
-      sL[slot * QR + threadIdx.x] = r < len ? p.lse[head * p.rows + start + r] : 0.f;
-      sL[2 * QR + slot * QR + threadIdx.x] = r < len ? p.delta[head * p.rows + start + r] : 0.f;
+      const int64_t at = head * p.rows + start + (r < len ? r : 0);
+      attn_cp4(smem_u32(sL + slot * QR + threadIdx.x), p.lse + at, r < len);
+      attn_cp4(smem_u32(sL + 2 * QR + slot * QR + threadIdx.x), p.delta + at, r < len);
     }
   };
   issue(0);
@@ -480,6 +495,48 @@ attn_dkv_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Se
       }
     }
     __syncthreads();
+  }
+  if (C > 1) {
+    // every CTA leaves its sums where the tiles were ([dk, dv][n][thread], 16 bytes each); rank r adds up the column groups
+    // n = r, r + C, ... below the half and their partners of the rotation, over the ranks in order
+    const uint32_t mine = smem_u32(a_smem) + threadIdx.x * 16;
+#pragma unroll
+    for (int n = 0; n < NT; ++n) {
+      *reinterpret_cast<float4*>(a_smem + (n * kAttnThreads + threadIdx.x) * 16) = make_float4(dk[n][0], dk[n][1], dk[n][2], dk[n][3]);
+      *reinterpret_cast<float4*>(a_smem + ((NT + n) * kAttnThreads + threadIdx.x) * 16) = make_float4(dv[n][0], dv[n][1], dv[n][2], dv[n][3]);
+    }
+    cluster_sync_all();
+#pragma unroll 1
+    for (int n = rank; n < NT / 2; n += C) {
+      float sum[4][4];                       // dk of n and its partner, dv of both
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const uint32_t at = mine + ((k >> 1) * NT + n + (k & 1) * (NT / 2)) * (kAttnThreads * 16);
+        float4 v[8];
+#pragma unroll
+        for (int r = 0; r < 8; ++r) v[r] = r < C ? attn_peer128(map_to_cta(at, r)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 w = v[0];
+#pragma unroll
+        for (int r = 1; r < 8; ++r)
+          if (r < C) { w.x += v[r].x; w.y += v[r].y; w.z += v[r].z; w.w += v[r].w; }
+        sum[k][0] = w.x; sum[k][1] = w.y; sum[k][2] = w.z; sum[k][3] = w.w;
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int r = key_a + 8 * h;
+        if (r >= len) continue;
+        const float4 cs = __ldg(reinterpret_cast<const float4*>(p.trig + static_cast<int64_t>(r) * (HD / 2) + n * 8 + 2 * t));
+        const int64_t at = (start + r) * p.ldd + kvh * HD + n * 8 + 2 * t;
+        const float x0 = sum[0][2 * h] * p.scale, x1 = sum[0][2 * h + 1] * p.scale, y0 = sum[1][2 * h] * p.scale, y1 = sum[1][2 * h + 1] * p.scale;
+        *reinterpret_cast<uint32_t*>(p.dk + at) = pack_half2_rn(x0 * cs.x + y0 * cs.y, x1 * cs.z + y1 * cs.w);
+        *reinterpret_cast<uint32_t*>(p.dk + at + HD / 2) = pack_half2_rn(y0 * cs.x - x0 * cs.y, y1 * cs.z - x1 * cs.w);
+        *reinterpret_cast<uint32_t*>(p.dv + at) = pack_half2_rn(sum[2][2 * h], sum[2][2 * h + 1]);
+        *reinterpret_cast<uint32_t*>(p.dv + at + HD / 2) = pack_half2_rn(sum[3][2 * h], sum[3][2 * h + 1]);
+      }
+    }
+    __syncwarp();
+    cluster_sync_all();                      // peers keep their sums until everybody has read them
+    return;
   }
   store_unrotated<HD>(dk, p, p.dk + start * p.ldd + kvh * HD, key_a, len, t, p.scale);
 #pragma unroll
@@ -562,7 +619,8 @@ static int attn_backward_hd(AttnParams p, const int32_t* lens, int n, int kv_hea
     const int rows = t.start[t.n] - t.start[0];
     PdlLaunch ld(dim3(static_cast<unsigned>((static_cast<int64_t>(rows) * p.heads * (HD / 8) + 255) / 256)), dim3(256), 0, stream);
     NF4LL_CUDA(cudaLaunchKernelEx(&ld.cfg, attn_delta_kernel<HD>, p, t.start[0], rows));
-    PdlLaunch lk(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(kv_heads)), dim3(kAttnThreads), smem_kv, stream);
+    const unsigned parts = static_cast<unsigned>(p.group < 8 ? p.group : 8);
+    PdlLaunch lk(dim3(static_cast<unsigned>(t.tile[t.n]) * parts, static_cast<unsigned>(kv_heads)), dim3(kAttnThreads), smem_kv, stream, parts, 1);
     NF4LL_CUDA(cudaLaunchKernelEx(&lk.cfg, attn_dkv_kernel<HD>, p, t));
     PdlLaunch lq(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(kAttnThreads), smem_q, stream);
     NF4LL_CUDA(cudaLaunchKernelEx(&lq.cfg, attn_dq_kernel<HD>, p, t));

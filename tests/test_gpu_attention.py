@@ -40,7 +40,7 @@ def rel(got, ref):
     return float((got.double().cpu() - ref).norm() / ref.norm())
 
 
-@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 64), (3, 1, 128), (2, 2, 128)])
+@pytest.mark.parametrize("nh,nkv,hd", [(4, 2, 64), (3, 1, 128), (2, 2, 128), (11, 1, 64), (7, 1, 128)])
 @pytest.mark.parametrize("lens", [[1], [63, 64, 65], [128, 0, 1, 200], [5] * 131 + [70], [331]])
 def test_attention_against_fp64(nh, nkv, hd, lens):
     gen = torch.Generator().manual_seed(sum(lens) + nh)
