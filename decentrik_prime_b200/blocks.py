@@ -10,7 +10,7 @@ import math
 import torch
 import torch.nn.functional as F
 
-from . import k_nf4, linear, quantize
+from . import _lib, k_nf4, linear, quantize
 
 
 class GradBucket:
@@ -77,6 +77,9 @@ class Projection:
         self._saved = None
 
     def refresh16(self):
+        if self.A.is_cuda and self.A.is_contiguous() and self.B.is_contiguous() and self.B.data_ptr() % 16 == 0:
+            _lib.host().lora_shadow(self.A, self.B, self.A16, self.B16, self.B16t)      # one launch for the three
+            return
         self.A16.copy_(self.A)
         self.B16.copy_(self.B)
         self.B16t.copy_(self.B.t())

@@ -426,6 +426,22 @@ PyObject* py_lora_u(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   });
 }
 
+// lora_shadow(A, B, A16, B16, B16t): fp16 copies of the fp32 masters, lora_B also transposed
+PyObject* py_lora_shadow(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  ARGS(5);
+  return guarded([&]() -> PyObject* {
+    const at::Tensor &A = tensor(a[0], "A"), &B = tensor(a[1], "B"), &A16 = tensor(a[2], "A16"), &B16 = tensor(a[3], "B16"), &Bt = tensor(a[4], "B16t");
+    if (A.dim() != 2 || B.dim() != 2 || A.size(0) != kRank || B.size(1) != kRank || Bt.dim() != 2 || Bt.size(0) != kRank || Bt.size(1) != B.size(0) ||
+        A16.sizes() != A.sizes() || B16.sizes() != B.sizes())
+      value_error("lora_A [16, K], lora_B [N, 16] and their shadows do not fit each other");
+    for (const auto* t : {&A, &B, &A16, &B16, &Bt})
+      if (!t->is_cuda() || !t->is_contiguous() || t->scalar_type() != (t == &A || t == &B ? at::kFloat : at::kHalf))
+        value_error("LoRA masters must be contiguous CUDA fp32 and their shadows contiguous CUDA fp16");
+    check(nf4ll_lora_shadow(A.data_ptr<float>(), B.data_ptr<float>(), A.size(1), B.size(0), A16.data_ptr(), B16.data_ptr(), Bt.data_ptr(), Call(A).stream));
+    Py_RETURN_NONE;
+  });
+}
+
 // swiglu_forward(g, u, out) -> h
 PyObject* py_swiglu_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   ARGS(3);
@@ -774,7 +790,7 @@ PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 }
 
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
-PyMethodDef methods[] = {METHOD(forward), METHOD(forward_multi), METHOD(forward_gate_up), METHOD(backward_dx), METHOD(lora_grads), METHOD(lora_u),
+PyMethodDef methods[] = {METHOD(forward), METHOD(forward_multi), METHOD(forward_gate_up), METHOD(backward_dx), METHOD(lora_grads), METHOD(lora_u), METHOD(lora_shadow),
                          METHOD(swiglu_forward), METHOD(swiglu_backward), METHOD(rms_forward), METHOD(rms_backward), METHOD(dequant),
                          METHOD(attention_forward), METHOD(attention_backward), METHOD(linear), METHOD(set_tune), METHOD(setup), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "host path between PyTorch tensors and libnf4ll.so", -1, methods, nullptr, nullptr, nullptr, nullptr};
