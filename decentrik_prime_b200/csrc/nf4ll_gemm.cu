@@ -1535,7 +1535,8 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   if (pl.splits > 1) {
     p.counters = counters;
     p.partial = reinterpret_cast<float*>(ws + pl.left_bytes + pl.bt_bytes + pl.counter_bytes);
-    if (!lora) NF4LL_CUDA(cudaMemsetAsync(p.counters, 0, pl.counter_bytes, stream));
+    if (!lora)
+      if (int rc = zero_words_launch(p.counters, static_cast<int>(pl.counter_bytes / sizeof(int)), stream)) return rc;
   }
   CUtensorMap map;
   if (int rc = make_tile_map(&map, act, M, KC, ldact, false)) return rc;

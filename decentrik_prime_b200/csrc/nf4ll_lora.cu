@@ -210,6 +210,21 @@ int transpose_n16_launch(const void* B, void* Bt, int64_t N, cudaStream_t stream
   return NF4LL_OK;
 }
 
+// Clears 32-bit words that the next kernel counts in. A kernel and not a memset: it is launched while the kernel before it
+// drains and the one after it while it runs (a split-K GEMM of 951 rows starts 3 us earlier).
+__global__ void __launch_bounds__(256) zero_words_kernel(int* words, int n) {
+  pdl_wait();
+  pdl_launch_dependents();
+  for (int i = blockIdx.x * 256 + threadIdx.x; i < n; i += gridDim.x * 256) words[i] = 0;
+}
+
+int zero_words_launch(int* words, int n, cudaStream_t stream) {
+  const int blocks = (n + 1023) / 1024;
+  PdlLaunch lc(dim3(static_cast<unsigned>(blocks < 1 ? 1 : (blocks > 148 ? 148 : blocks))), dim3(256), 0, stream);
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, zero_words_kernel, words, n));
+  return NF4LL_OK;
+}
+
 // R is [16,C] row-major. t32 (fp32 [M,16], required) = scale * (drop(act) . R^T). `zero_ptr` / `zero_words`:
 // optional 32-bit words the kernel clears on the way (see the kernel).
 int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_t ld_mask, float keep_scale,

@@ -27,6 +27,8 @@ double stream_time_us(int64_t N, int64_t K, int64_t M, int sms);
 // `early`: the kernel launched right before on the stream is a rank-16 projection of the same call
 int stream_forward_launch(const StreamCall& c, bool early, int force_team, cudaStream_t stream);
 
+int zero_words_launch(int* words, int n, cudaStream_t stream);      // nf4ll_lora.cu
+
 int64_t swap_workspace_bytes(int64_t N, int64_t K, int64_t M, int sms, int force_slices);
 int swap_forward_launch(const StreamCall& c, void* scratch, bool counters_zeroed, int force_slices, int32_t* status, cudaStream_t stream);
 

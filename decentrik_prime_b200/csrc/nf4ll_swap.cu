@@ -695,15 +695,6 @@ static int swap_launch_cfg(const CUtensorMap& mx, const CUtensorMap& mn, const S
   return NF4LL_OK;
 }
 
-// Clears the counters of a launch that no rank-16 projection precedes. Launched also where there are none to clear: the
-// kernel after it reads x and the weights at once, which is right only behind a kernel that itself went on after all earlier
-// work. (A kernel and not a memset: the next one can start meanwhile.)
-__global__ void __launch_bounds__(256) swap_zero_kernel(int* counters, int n) {
-  pdl_wait();
-  pdl_launch_dependents();
-  for (int i = threadIdx.x; i < n; i += 256) counters[i] = 0;
-}
-
 // `scratch`: the tile counters (cleared here unless `counters_zeroed`: the rank-16 projection kernel launched
 // just before has then done it) followed, 256-byte aligned, by the slab.
 int swap_forward_launch(const StreamCall& c, void* scratch, bool counters_zeroed, int force_slices, int32_t* status, cudaStream_t stream) {
@@ -731,10 +722,10 @@ int swap_forward_launch(const StreamCall& c, void* scratch, bool counters_zeroed
   const int64_t counter_bytes = (tiles * 4 + 255) / 256 * 256;
   p.counters = static_cast<int*>(scratch);
   p.slab = reinterpret_cast<float*>(static_cast<uint8_t*>(scratch) + counter_bytes);
-  if (!counters_zeroed) {
-    PdlLaunch lz(dim3(1), dim3(256), 0, stream);
-    NF4LL_CUDA(cudaLaunchKernelEx(&lz.cfg, swap_zero_kernel, p.counters, p.slices > 1 ? static_cast<int>(tiles) : 0));
-  }
+  // launched also where there are no counters: this kernel reads x and the weights at once, which is right only behind a
+  // kernel that itself went on after all earlier work
+  if (!counters_zeroed)
+    if (int rc = zero_words_launch(p.counters, p.slices > 1 ? static_cast<int>(tiles) : 0, stream)) return rc;
   CUtensorMap mx, mn;
   if (int rc = swap_encode(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, c.x, static_cast<uint64_t>(W->K), static_cast<uint64_t>(M),
                            static_cast<uint64_t>(c.ldx) * 2, 64, static_cast<uint32_t>(ntok), "token tile")) return rc;
