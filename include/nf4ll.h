@@ -89,7 +89,7 @@ int nf4ll_dequant(const uint8_t* nib, const uint8_t* qabs, const float* scale2, 
  * partial sums and tile counters. Always a multiple of 256; the workspace must be 256-byte aligned. */
 int64_t nf4ll_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t r);
 
-/* Scratch with which the calls on W[N,K] run at their best: from several hundred rows on it also holds one fp16 copy of
+/* Scratch with which the calls on W[N,K] run at their best: where that is faster (above 128 rows) it also holds one fp16 copy of
  * the weight (2 N K bytes), so that a call dequantises once and multiplies by that. With a smaller workspace (at least
  * nf4ll_workspace_bytes) the same calls decode the weight inside the GEMM instead. N is the row count of the whole
  * stacked matrix for nf4ll_forward_multi and nf4ll_forward_gate_up. No counterpart in the reference. */
