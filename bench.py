@@ -771,7 +771,7 @@ def decoder_stack_numbers(dev, args):
            "tokens_per_s": M * steps / (ms * 1e-3), "projection_tflops": float(ns.flops(M)) * steps / (ms * 1e-3) / 1e12,
            "ms_per_step": ms / steps, "steps": steps, "warmup": warmup,
            "launch": ("cuda graph of the whole step, replayed" if graph is not None else "eager") +
-                     "; attention through torch.nn.functional.scaled_dot_product_attention per sequence"}
+                     "; rotary embedding and attention in the library's own kernels"}
     del ns, graph
     torch.cuda.empty_cache()
     return res
