@@ -1207,8 +1207,8 @@ constexpr int64_t kStreamCapRows = 64;     // its limit (reachable through the t
 constexpr int64_t kSwapMaxRows = 64;       // limit of the swapped-operand kernel (weights as the MMA's M operand)
 // From 9 to 16 rows the faster of the two by fits of their times: the streaming kernel's depends on how evenly its units go
 // round the SMs (and on the tokens), the swapped-operand kernel cuts the contraction too and pays for that. Measured:
-// 27648 x 5120 at 9 / 16 rows 39 / 44 us against 52 / 54, 5120 x 27648 67 / 78 against 47, 5120 x 5120 13 / 15 against 19,
-// 3584 x 18944 28 / 30 against 29. From 17 rows on the swapped-operand kernel wins over the 128-row tiles on weights of at
+// 27648 x 5120 at 9 / 16 rows 38 / 40 us against 52 / 54, 5120 x 27648 55 / 62 against 45, 5120 x 5120 14 / 15 against 19,
+// 3584 x 18944 27 / 29 against 26 / 27. From 17 rows on the swapped-operand kernel wins over the 128-row tiles on weights of at
 // least 2^24 elements, and up to 64 rows on weights of at least 2^26.
 constexpr int64_t kSwapMinRows = 9;        // below, the streaming kernel keeps its exact fp32 scales
 constexpr int64_t kSwapMidRows = 32;

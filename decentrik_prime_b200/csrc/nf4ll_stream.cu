@@ -19,9 +19,9 @@
 // This differs from the big-tile kernel's bit-exact fp16 weights by the rounding of NF4[c] * absmax to
 // fp16 (relative 2^-12), inside the 1e-3 tolerance of the path.
 //
-// 27648 x 5120 (73 MB) at 1 / 8 tokens: 27 / 31 us, of which the fetch alone 19 (with a rank-16 branch at 8 tokens 34, 50
-// for the kernel that handed out units of 16 rows x a slice through a global counter). What is left over the fetch is the
-// table lookups (4 us), the token loads (5 us at 8 tokens) and the MMAs (1 us) that do not hide behind it.
+// 27648 x 5120 (73 MB) at 1 / 8 tokens: 26.7 / 29.4 us (2.7 / 2.5 TB/s), of which the fetch alone 19; 42 / 46 for the kernel that
+// handed out units of 16 rows x a slice through a global counter. What is left over the fetch is the table lookups (4 us), the
+// token loads (3 us at 8 tokens) and the MMAs (1 us) that do not hide behind it.
 #include "nf4ll_stream.cuh"
 
 namespace nf4ll {
