@@ -20,10 +20,10 @@ dequant_kernel(const uint4* __restrict__ nib, const uint8_t* __restrict__ qabs,
                const float* __restrict__ scale2, const float* __restrict__ offset2,
                const float* __restrict__ code2, int64_t n_half_blocks, uint4* __restrict__ out, const DequantSide side) {
   __shared__ float s_code2[256];
+  pdl_wait();                  // before code2 too: whatever ran before this kernel may have written it
+  pdl_launch_dependents();
   s_code2[threadIdx.x] = code2[threadIdx.x];
   __syncthreads();
-  pdl_wait();
-  pdl_launch_dependents();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * kDequantThreads;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * kDequantThreads + threadIdx.x;
   for (int k = 0; k < side.n_left; ++k) {
