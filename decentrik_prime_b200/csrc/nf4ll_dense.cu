@@ -80,17 +80,17 @@ __device__ __forceinline__ void dense_tile_pos(const DenseParams& p, int tile, i
   tm = g * 8 + (r - to * gm);
 }
 
-// The rank-16 steps of a tile: one when both 128-column halves belong to the same branch, else one per branch
-// (the other half then multiplies a block of zeros, which TMA supplies by reading outside the factor).
+// The rank-16 steps of a tile: one over all 256 columns when both 128-column halves belong to the same branch, else one
+// per half, of 128 columns: a branch whose product is infinite or NaN must not reach the other half's columns (times
+// zeros it would). A half without a branch gets zeros on both sides, which TMA supplies by reading outside the factors.
 struct DenseLora {
-  int n;
-  int seg[2];
-  int halves[2];      // bit h: half h of the columns takes part
+  int n;              // steps: 0, 1 (whole tile) or 2 (halves)
+  int seg[2];         // -1: no branch
 };
 template <int MODE>
 __device__ __forceinline__ DenseLora dense_lora(const DenseParams& p, int64_t o0) {
   DenseLora l;
-  l.n = 0; l.seg[0] = l.seg[1] = 0; l.halves[0] = l.halves[1] = 3;
+  l.n = 0; l.seg[0] = l.seg[1] = 0;
   if (p.n_lora == 0) return l;
   if (MODE == kBwd || (p.n_seg == 0 && p.gu_inter == 0)) { l.n = 1; return l; }
   int s0 = 0, s1 = 1;
@@ -101,12 +101,10 @@ __device__ __forceinline__ DenseLora dense_lora(const DenseParams& p, int64_t o0
       if (o0 + 128 >= p.seg_begin[i] && p.seg_begin[i] < p.NO) s1 = i;
     }
   }
-  if (s0 == s1) {
-    if (p.lora_index[s0] >= 0) { l.n = 1; l.seg[0] = s0; }
-    return l;
-  }
-  if (p.lora_index[s0] >= 0) { l.seg[l.n] = s0; l.halves[l.n] = 1; ++l.n; }
-  if (p.lora_index[s1] >= 0) { l.seg[l.n] = s1; l.halves[l.n] = 2; ++l.n; }
+  l.seg[0] = p.lora_index[s0] >= 0 ? s0 : -1;
+  l.seg[1] = p.lora_index[s1] >= 0 ? s1 : -1;
+  if (s0 == s1) l.n = l.seg[0] >= 0 ? 1 : 0;
+  else l.n = (l.seg[0] >= 0 || l.seg[1] >= 0) ? 2 : 0;
   return l;
 }
 
@@ -189,17 +187,20 @@ dense_gemm_kernel(const __grid_constant__ DenseMaps maps, const __grid_constant_
         const uint32_t base = smem_u32(smem) + (n % S) * kDnStageBytes;
         const int m0 = tm * 512 + static_cast<int>(rank) * 128;
         for (int k = 0; k < l.n; ++k) {
-          const int sg = l.seg[k];
+          const bool none = l.seg[k] < 0;
+          const int sg = none ? l.seg[1 - k] : l.seg[k];
           const uint32_t kb = base + k * 3 * kDnLoraStep;
 #pragma unroll 1
           for (int h = 0; h < 4; ++h) {
-            const int row = static_cast<int>(p.lora_index[sg] * p.M) + m0 + (h >> 1) * 256;
+            const int row = static_cast<int>((none ? p.n_lora : p.lora_index[sg]) * p.M) + m0 + (h >> 1) * 256;      // past all branches: zeros
             tma_load_2d_pair(kb + h * 2048, &maps.left, (h & 1) * 8, row, bar);
           }
           const uint32_t rb = kb + 2 * kDnLoraStep;
           if (MODE == kFwd) {
-            int y = static_cast<int>(p.gu_inter ? o0 : o0 + rank * 128 - p.seg_begin[sg]);
-            if (!((l.halves[k] >> rank) & 1)) y = static_cast<int>(p.seg_rows[sg]);     // outside: zeros
+            // this CTA's half of the step's columns: 128 of 256, or 64 of 128 (the box brings 64 more, which are not used)
+            int y = static_cast<int>(l.n == 1 ? o0 + rank * 128 - p.seg_begin[sg]
+                                              : (p.gu_inter ? o0 : o0 + k * 128 - p.seg_begin[sg]) + rank * 64);
+            if (none) y = static_cast<int>(p.seg_rows[sg]);     // outside: zeros
             tma_load_2d_pair(rb, &maps.right[sg], 0, y, bar);
             tma_load_2d_pair(rb + 2048, &maps.right[sg], 8, y, bar);
           } else {
@@ -264,7 +265,7 @@ dense_gemm_kernel(const __grid_constant__ DenseMaps maps, const __grid_constant_
   } else if (warp == 1) {
     // ----------------------------------------------------------------------------- MMA issuer
     if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc = make_idesc_f16(256, 256, 0, MODE == kBwd ? 1 : 0);
+      constexpr uint32_t idesc = make_idesc_f16(256, 256, 0, MODE == kBwd ? 1 : 0), idesc_half = make_idesc_f16(256, 128, 0, 0);
       const int G = premask ? 3 : 2;             // k-blocks the accumulators run apart at the ends of a tile
       const int cnt = kb1 - kb0;
       int n = 0, i = 0;                          // stages consumed by accumulator 0, tiles started
@@ -291,12 +292,13 @@ dense_gemm_kernel(const __grid_constant__ DenseMaps maps, const __grid_constant_
       };
       // the rank-16 steps as the first products of accumulator mt
       auto mma_lora = [&](int mt) {
+        const bool halves = lora.n == 2;
 #pragma unroll 1
         for (int k = 0; k < lora.n; ++k) {
           const uint32_t kb = stage_base(lora_at) + k * 3 * kDnLoraStep, rb = kb + 2 * kDnLoraStep;
           const uint64_t ad = make_smem_desc(kb + mt * kDnLoraStep, 2048, 128, kSwizzleNone);
           const uint64_t bd = (MODE == kFwd) ? make_smem_desc(rb, 2048, 128, kSwizzleNone) : make_smem_desc(rb, 2048, 1024, kSwizzle128B);
-          tc_mma2_f16(tmem_base + mt * 256, ad, bd, idesc, k > 0 ? 1u : 0u);
+          tc_mma2_f16(tmem_base + mt * 256 + (halves ? k * 128 : 0), ad, bd, halves ? idesc_half : idesc, 0u);
         }
       };
       auto b_desc = [&](uint32_t b_base, int kk) {

@@ -102,3 +102,47 @@ def test_stacked_and_gate_up(M, H, KV, I):
         assert_close("g", g, oracle("gate_proj", lg, mg)["y"])
         assert_close("u", u, oracle("up_proj", lu, mu)["y"])
         assert torch.equal(h, linear.swiglu_forward(g.contiguous(), u.contiguous()))
+
+
+@pytest.mark.parametrize("bad", [float("inf"), float("nan"), 3.0e4])      # 3e4: the product overflows where it is rounded to fp16
+def test_branches_do_not_mix(bad):
+    """Two branches in one 256-column tile: a product that is not finite stays in its own branch's columns."""
+    M, H, KV, I = 200, 384, 128, 384
+    shapes = {"q_proj": (H, H), "k_proj": (KV, H), "v_proj": (KV, H), "gate_proj": (I, H), "up_proj": (I, H)}
+    lin = {n: quantize.random_nf4_weight(*s, seed=40 + i, device="cuda") for i, (n, s) in enumerate(shapes.items())}
+    layer, code2 = k_nf4.repack_layer(lin, torch.device("cuda"), names=tuple(shapes))
+    gen = torch.Generator().manual_seed(5)
+    x = torch.randn(M, H, generator=gen).half().cuda()
+
+    def branch(n, ill=False):
+        A = torch.randn(16, H, generator=gen) * 0.05
+        if ill:
+            A[3] = bad
+        return A.half().cuda(), (torch.randn(n, 16, generator=gen) * 0.05).half().cuda(), 2.0
+
+    wq = linear.Nf4Weight.from_layer_group(layer, ("q_proj", "k_proj", "v_proj"), code2)
+    wg = linear.Nf4Weight.from_layer_group(layer, ("gate_proj", "up_proj"), code2)
+    ws = workspace(M, wg.N, wg.K)
+    for ill, well, multi in (((0,), (1, 2), (True, False, True)), ((2,), (0, 1), (True, False, True)), ((0,), (1, 2), (True, True, True)),
+                             ((2,), (0, 1), (False, False, True))):
+        loras = [branch(n, i in ill) if has else None for i, (n, has) in enumerate(zip((H, KV, KV), multi))]
+        with linear.tune_override(flags=DENSE):
+            y, _ = linear.forward_multi(wq, x, [(n, l, None, 1.0) for n, l in zip((H, KV, KV), loras)], workspace=ws)
+        linear.check_status()
+        parts = y.split((H, KV, KV), dim=1)
+        for i in well:
+            A, B, s = (None, None, 1.0) if loras[i] is None else (loras[i][0].cpu(), loras[i][1].cpu(), loras[i][2])
+            ref = nf4_oracle.lora_linear_o1(nf4_oracle.dequant_weight(layer, ("q_proj", "k_proj", "v_proj")[i], code2), x.cpu(), None, None, A, B, s, None, 1.0)
+            assert_close(f"segment {i}", parts[i], ref["y"])
+        assert not all(bool(torch.isfinite(parts[i]).all()) for i in ill)
+    for ill in (0, 1):
+        for other in (True, False):
+            loras = [branch(I, True), branch(I) if other else None][::1 if ill == 0 else -1]
+            with linear.tune_override(flags=DENSE):
+                g, u, h, _, _ = linear.forward_gate_up(wg, x, loras[0], None, loras[1], None, 1.0, workspace=ws)
+            linear.check_status()
+            l = loras[1 - ill]
+            A, B, s = (None, None, 1.0) if l is None else (l[0].cpu(), l[1].cpu(), l[2])
+            ref = nf4_oracle.lora_linear_o1(nf4_oracle.dequant_weight(layer, ("up_proj", "gate_proj")[ill], code2), x.cpu(), None, None, A, B, s, None, 1.0)
+            assert_close("other half", (u, g)[ill], ref["y"])
+            assert not torch.isfinite((g, u)[ill]).all()
