@@ -306,13 +306,14 @@ class PackedAttention:
 
     def forward(self, qkv, seq_lens):
         """qkv fp16 [M, (nh + 2 nkv) hd] -> (a fp16 [M, nh hd], state for backward)."""
+        seq_lens = [int(n) for n in seq_lens]                  # numpy integers and tensors too
         if sum(seq_lens) != qkv.shape[0]:
             raise ValueError(f"sequence lengths {seq_lens} do not add up to {qkv.shape[0]} rows")
         if self.hd in (64, 128) and qkv.is_cuda and qkv.dtype == torch.float16:
             qkv = _rows_aligned(qkv.detach())
             trig = self._trig_table(max(seq_lens), qkv.device)
             a, roped, lse = _lib.host().attention_forward(qkv, seq_lens, self.nh, self.nkv, self.hd, trig)
-            return a, (self, qkv, tuple(seq_lens), trig, roped, a, lse)
+            return a, (self, qkv, seq_lens, trig, roped, a, lse)
         return self._forward_torch(qkv, seq_lens)
 
     def _forward_torch(self, qkv, seq_lens):

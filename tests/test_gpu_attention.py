@@ -3,6 +3,7 @@ and backward, at the edges of the 64-row tiles, with empty and single-row sequen
 ungrouped heads, and more sequences than one launch takes. fp16 results of fp32 sums over fp16 probabilities: the rounding
 of P, dS (2^-11 each, relative) and of the rotated q, k and the result give a few 2^-11 in the 2-norm; 3e-3 bounds it."""
 
+import numpy as np
 import pytest
 import torch
 
@@ -75,3 +76,13 @@ def test_attention_of_unaligned_rows():
     assert torch.equal(att.backward(state, odd), expected) and torch.equal(att.backward(state, da.float()), expected)
     with pytest.raises(ValueError):
         att.backward(state, da[:69])
+
+
+@pytest.mark.parametrize("lens", [np.diff(np.array([0, 30, 31, 70])), torch.tensor([30, 1, 39]), (30, 1, 39)], ids=["numpy", "tensor", "tuple"])
+def test_sequence_lengths_of_other_types(lens):
+    gen = torch.Generator().manual_seed(4)
+    qkv = torch.randn(70, 4 * 64, generator=gen).half().cuda()
+    att = stack.PackedAttention(2, 1, 64)
+    a, state = att.forward(qkv, lens)
+    b, state_b = att.forward(qkv, [30, 1, 39])
+    assert torch.equal(a, b) and torch.equal(att.backward(state, a), att.backward(state_b, b))
