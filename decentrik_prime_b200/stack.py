@@ -257,7 +257,7 @@ class ProjectionStack:
 def _rows_aligned(t):
     """t, or a copy of it, with every row on a 16-byte boundary."""
     ok = t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0
-    return t if ok else t.contiguous()
+    return t if ok else t.clone(memory_format=torch.contiguous_format)      # contiguous() would hand back a packed view as it is
 
 
 class PackedAttention:

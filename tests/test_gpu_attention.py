@@ -86,3 +86,16 @@ def test_sequence_lengths_of_other_types(lens):
     a, state = att.forward(qkv, lens)
     b, state_b = att.forward(qkv, [30, 1, 39])
     assert torch.equal(a, b) and torch.equal(att.backward(state, a), att.backward(state_b, b))
+
+
+def test_attention_of_a_packed_view_at_an_odd_offset():
+    """Contiguous, but off a 16-byte boundary."""
+    gen = torch.Generator().manual_seed(6)
+    flat = torch.randn(70 * 4 * 64 + 1, generator=gen).half().cuda()
+    odd = flat[1:].view(70, 4 * 64)
+    assert odd.is_contiguous() and odd.data_ptr() % 16
+    da_odd = torch.randn(70 * 2 * 64 + 3, generator=gen).half().cuda()[3:].view(70, 2 * 64)
+    att = stack.PackedAttention(2, 1, 64)
+    a, state = att.forward(odd, [30, 40])
+    b, state_b = att.forward(odd.clone(), [30, 40])
+    assert torch.equal(a, b) and torch.equal(att.backward(state, da_odd), att.backward(state_b, da_odd.clone()))
