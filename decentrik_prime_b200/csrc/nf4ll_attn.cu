@@ -119,9 +119,10 @@ rope_kernel(const __half* __restrict__ src, int64_t lds, __half* __restrict__ ds
   pdl_wait();
   pdl_launch_dependents();
   const int half = hd / 2, per_row = heads * (half / 8);
-  const int rows = seqs.start[seqs.n] - seqs.start[0];
-  for (int idx = blockIdx.x * 256 + threadIdx.x; idx < rows * per_row; idx += gridDim.x * 256) {
-    const int r = idx / per_row, c = idx - r * per_row;
+  const int64_t work = static_cast<int64_t>(seqs.start[seqs.n] - seqs.start[0]) * per_row;      // may exceed 32 bits
+  for (int64_t idx = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x; idx < work; idx += gridDim.x * 256) {
+    const int r = static_cast<int>(work >> 32 ? idx / per_row : static_cast<uint32_t>(idx) / static_cast<uint32_t>(per_row));
+    const int c = static_cast<int>(idx - static_cast<int64_t>(r) * per_row);
     const int head = c / (half / 8), j = (c - head * (half / 8)) * 8;
     const int row = seqs.start[0] + r;
     int lo = 0, hi = seqs.n - 1;
@@ -266,9 +267,11 @@ attn_delta_kernel(const __grid_constant__ AttnParams p, int first, int rows) {
   pdl_wait();
   pdl_launch_dependents();
   constexpr int L = HD / 8;                  // lanes per (row, head)
-  const int idx = (blockIdx.x * 256 + threadIdx.x) / L, c = threadIdx.x % L;
-  const bool live = idx < rows * p.heads;
-  const int row = first + (live ? idx / p.heads : 0), head = live ? idx % p.heads : 0;
+  const int64_t idx = (static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x) / L;
+  const int c = threadIdx.x % L;
+  const bool live = idx < static_cast<int64_t>(rows) * p.heads;
+  const uint32_t i = live ? static_cast<uint32_t>(idx) : 0;      // rows x heads fits: each holds 128 bytes of dout at least
+  const int row = first + static_cast<int>(i / static_cast<uint32_t>(p.heads)), head = static_cast<int>(i % static_cast<uint32_t>(p.heads));
   float a[8], b[8], s = 0.f;
   unpack8(*reinterpret_cast<const uint4*>(p.dout + row * p.lddo + head * HD + c * 8), a);
   unpack8(*reinterpret_cast<const uint4*>(p.o + row * p.ldo + head * HD + c * 8), b);
@@ -597,7 +600,7 @@ static int attn_forward_hd(AttnParams p, const __half* qkv, int64_t ldq, __half*
     SeqTable t;
     at = attn_table(&t, lens, n, at, &row);
     if (t.n == 0) continue;
-    const int rows = t.start[t.n] - t.start[0], work = rows * (p.heads + kv_heads) * (HD / 16);
+    const int64_t work = static_cast<int64_t>(t.start[t.n] - t.start[0]) * (p.heads + kv_heads) * (HD / 16);
     PdlLaunch lr(dim3(static_cast<unsigned>((work + 255) / 256 < 1184 ? (work + 255) / 256 : 1184)), dim3(256), 0, stream);
     NF4LL_CUDA(cudaLaunchKernelEx(&lr.cfg, rope_kernel, qkv, ldq, roped, p.ldr, p.trig, p.heads + kv_heads, HD, t));
     PdlLaunch lf(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(kAttnThreads), smem, stream);
