@@ -77,7 +77,10 @@ class Projection:
         self._saved = None
 
     def refresh16(self):
-        if self.A.is_cuda and self.A.is_contiguous() and self.B.is_contiguous() and self.B.data_ptr() % 16 == 0:
+        masters, shadows = (self.A, self.B), (self.A16, self.B16, self.B16t)
+        if (all(t.is_cuda and t.is_contiguous() and t.dtype == torch.float32 for t in masters)
+                and all(t.is_cuda and t.is_contiguous() and t.dtype == torch.float16 for t in shadows)
+                and (self.B.data_ptr() | self.B16.data_ptr()) % 16 == 0):
             _lib.host().lora_shadow(self.A, self.B, self.A16, self.B16, self.B16t)      # one launch for the three
             return
         self.A16.copy_(self.A)

@@ -365,3 +365,17 @@ def test_split_contraction_is_stable_under_back_to_back_launches():
     linear.check_status()
     assert all(torch.equal(o, outs[0]) for o in outs), "forward with LoRA differs between launches"
     assert all(torch.equal(o, dxs[0]) for o in dxs), "backward-dX with LoRA differs between launches"
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float16, torch.bfloat16, torch.float32])
+def test_shadows_follow_masters_of_any_type(dtype):
+    from decentrik_prime_b200 import blocks
+    d = to_device(make_problem(256, 128, 4, seed=9, lora=False))
+    p = blocks.Projection(d.w, lora=True)
+    gen = torch.Generator().manual_seed(1)
+    p.A, p.B = torch.randn(16, 128, generator=gen).cuda().to(dtype), torch.randn(256, 16, generator=gen).cuda().to(dtype)
+    p.refresh16()
+    assert torch.equal(p.A16, p.A.half()) and torch.equal(p.B16, p.B.half()) and torch.equal(p.B16t, p.B.half().t())
+    p.B = torch.randn(256 * 16 + 1, generator=gen).cuda()[1:].view(256, 16)      # off a 16-byte boundary
+    p.refresh16()
+    assert torch.equal(p.B16, p.B.half()) and torch.equal(p.B16t, p.B.half().t())
