@@ -379,3 +379,24 @@ def test_shadows_follow_masters_of_any_type(dtype):
     p.B = torch.randn(256 * 16 + 1, generator=gen).cuda()[1:].view(256, 16)      # off a 16-byte boundary
     p.refresh16()
     assert torch.equal(p.B16, p.B.half()) and torch.equal(p.B16t, p.B.half().t())
+
+
+def test_autograd_linear_takes_factors_off_16_byte_boundaries():
+    """lora_A and lora_B as views at odd offsets of a flat parameter buffer."""
+    pr = make_problem(256, 128, 70, seed=10, lora=True, dropout=0.05)
+    d = to_device(pr)
+    n = 16 * 128
+    flat = torch.zeros(1 + n + 256 * 16, device="cuda")
+    flat[1:1 + n] = pr.A.reshape(-1).cuda()
+    flat[1 + n:] = pr.B.reshape(-1).cuda()
+    got = []
+    for A, B in ((pr.A.cuda(), pr.B.cuda()), (flat[1:1 + n].view(16, 128), flat[1 + n:].view(256, 16))):
+        x, A, B = d.x.detach().requires_grad_(True), A.requires_grad_(True), B.requires_grad_(True)
+        y = linear.nf4_lora_linear(x, d.w, lora=(A, B, pr.scale), mask=d.mask, keep_scale=d.keep_scale)
+        got.append((y.detach(), *torch.autograd.grad(y, (x, A, B), d.dy)))
+    assert B.data_ptr() % 16
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, pr.dy, None, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)
+    for tensors in got:
+        for name, t in zip(("y", "dx", "dA", "dB"), tensors):
+            err, rel = nf4_oracle.errors(t, ref[name])
+            assert err <= 2e-2 and rel <= 1e-3, (name, err, rel)
