@@ -12,6 +12,7 @@
 
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
 
 #include <vector>
@@ -86,8 +87,8 @@ at::Tensor empty(at::IntArrayRef size, at::ScalarType type, const at::Tensor& li
   return at::detail::empty_cuda(size, type, like.device(), std::nullopt);
 }
 
-// Per-thread scratch: one workspace per (device, stream), grown on demand, and the device's status word. Both end with
-// the thread.
+// Per-thread scratch of eager calls: one workspace per (device, stream), grown on demand, and the device's status word. Both
+// end with the thread.
 struct Scratch {
   int device;
   cudaStream_t stream;
@@ -126,13 +127,22 @@ int64_t need(int64_t M, int64_t N, int64_t K, int32_t r) {
   return nf4ll_workspace_bytes_fast(M, N, K, r);
 }
 
+// A captured call has scratch of its own from the graph's memory pool, which lives as long as the graph: the thread's buffer
+// is released when it grows, and eager calls write to it while a replay runs.
 struct Workspace {
   void* p;
   int64_t bytes;
+  at::Tensor own;
   Workspace(const at::Tensor* given, const Call& c, const at::Tensor& like, int64_t bytes_needed) {
     if (given) {
       p = given->data_ptr();
       bytes = given->numel();
+      return;
+    }
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+      own = empty({bytes_needed > 0 ? bytes_needed : 1}, at::kByte, like);
+      p = own.data_ptr();
+      bytes = own.numel();
       return;
     }
     auto& v = state().ws;

@@ -102,7 +102,8 @@ def check_status(device=None):
 
 # Each function below is one call into the host extension (csrc/torch_host.cpp), which checks the tensors, allocates the
 # results and finds the calling thread's workspace for the current device and stream (grown on demand; calls on different
-# streams of one thread use different ones, `workspace=` replaces it).
+# streams of one thread use different ones, `workspace=` replaces it). A call captured by torch.cuda.graph takes its scratch
+# from the graph's own memory.
 def forward(w: Nf4Weight, x, bias=None, lora=None, mask=None, keep_scale=1.0, out=None, want_t=False,
             workspace=None):
     """y = x . W^T (+ bias) + scale * (drop(x) . A^T) . B^T. `lora` = (A16 [16,K], B16 [N,16], scale) or
