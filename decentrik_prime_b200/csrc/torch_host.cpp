@@ -93,6 +93,8 @@ struct Scratch {
   int device;
   cudaStream_t stream;
   at::Tensor ws;
+  int64_t refused = 0;                   // bytes that the allocator did not have
+  int again = 0;                         // calls until it is asked for them again
 };
 struct ThreadState {
   std::vector<Scratch> ws;
@@ -121,28 +123,45 @@ struct Call {
   }
 };
 
-int64_t need(int64_t M, int64_t N, int64_t K, int32_t r) {
-  const int* t = state().tune;
-  if (t[0] || t[1] || t[2]) return nf4ll_workspace_bytes_tuned(M, N, K, r, t[0], t[1], t[2]);
-  return nf4ll_workspace_bytes_fast(M, N, K, r);
-}
+// Scratch of a call: fast() is what it runs best with (it may hold an fp16 copy of the weight), least() what it runs with.
+struct Need {
+  int64_t M, N, K;
+  int32_t r;
+  int64_t fast() const {
+    const int* t = state().tune;
+    return t[0] || t[1] || t[2] ? tuned(t) : nf4ll_workspace_bytes_fast(M, N, K, r);
+  }
+  int64_t least() const {
+    const int* t = state().tune;
+    return t[0] || t[1] || t[2] ? tuned(t) : nf4ll_workspace_bytes(M, N, K, r);
+  }
+  int64_t tuned(const int* t) const { return nf4ll_workspace_bytes_tuned(M, N, K, r, t[0], t[1], t[2]); }
+};
+constexpr int kAskAgain = 256;           // calls on the smaller route after an allocation has failed: every failure empties the allocator's cache
 
+// Where the allocator does not have the memory for a call's fast route, the call takes the route that needs less.
 // A captured call has scratch of its own from the graph's memory pool, which lives as long as the graph: the thread's buffer
 // is released when it grows, and eager calls write to it while a replay runs.
 struct Workspace {
   void* p;
   int64_t bytes;
   at::Tensor own;
-  Workspace(const at::Tensor* given, const Call& c, const at::Tensor& like, int64_t bytes_needed) {
+  Workspace(const at::Tensor* given, const Call& c, const at::Tensor& like, std::initializer_list<Need> needs) {
     if (given) {
       p = given->data_ptr();
       bytes = given->numel();
       return;
     }
+    int64_t fast = 0;
+    for (const Need& n : needs) fast = std::max(fast, n.fast());
+    auto least = [&] {
+      int64_t b = 0;
+      for (const Need& n : needs) b = std::max(b, n.least());
+      return b;
+    };
     if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
-      own = empty({bytes_needed > 0 ? bytes_needed : 1}, at::kByte, like);
-      p = own.data_ptr();
-      bytes = own.numel();
+      own = allocate(fast, least, like);
+      use(own);
       return;
     }
     auto& v = state().ws;
@@ -153,12 +172,37 @@ struct Workspace {
       v.push_back({c.device, c.stream, at::Tensor()});
       s = &v.back();
     }
-    if (!s->ws.defined() || s->ws.numel() < bytes_needed) {
-      s->ws = at::Tensor();
-      s->ws = empty({bytes_needed > (1 << 20) ? bytes_needed : (1 << 20)}, at::kByte, like);
+    const int64_t have = s->ws.defined() ? s->ws.numel() : 0;
+    if (have < fast) {
+      const bool ask = s->refused == 0 || fast < s->refused || --s->again < 0;
+      const int64_t want = ask ? fast : least();
+      if (have < want) {
+        s->ws = at::Tensor();
+        s->ws = allocate(std::max<int64_t>(want, 1 << 20), least, like);
+        if (ask) {
+          const bool got = s->ws.numel() >= want;
+          s->refused = got ? 0 : want;
+          s->again = kAskAgain;
+        }
+      }
     }
-    p = s->ws.data_ptr();
-    bytes = s->ws.numel();
+    use(s->ws);
+  }
+
+ private:
+  void use(const at::Tensor& t) {
+    p = t.data_ptr();
+    bytes = t.numel();
+  }
+  template <typename F>
+  static at::Tensor allocate(int64_t want, F&& least, const at::Tensor& like) {
+    try {
+      return empty({std::max<int64_t>(want, 1)}, at::kByte, like);
+    } catch (const c10::OutOfMemoryError&) {
+      const int64_t b = std::max<int64_t>(least(), 1);
+      if (b >= want) throw;
+      return empty({b}, at::kByte, like);
+    }
   }
 };
 
@@ -263,7 +307,7 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     at::Tensor t;
     if (lora.on && PyObject_IsTrue(a[7])) t = empty({M, kRank}, at::kFloat, x);
     const Call c(x);
-    const Workspace ws(optional(a[8], "workspace"), c, x, a[8] == Py_None ? need(M, w->N, w->K, lora.on ? kRank : 0) : 0);
+    const Workspace ws(optional(a[8], "workspace"), c, x, {Need{M, w->N, w->K, lora.on ? kRank : 0}});
     check(nf4ll_forward(w, x.data_ptr(), ld(x), ptr(bias), lora.get(), t.defined() ? t.data_ptr() : nullptr, M, y.data_ptr(), ld(y), ws.p, ws.bytes,
                         c.status(), c.stream));
     return pair(a[6] == Py_None ? wrap(y) : again(a[6]), wrap(&t));
@@ -319,7 +363,7 @@ PyObject* py_forward_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       PyList_SET_ITEM(ts.o, i, out);
     }
     const Call c(x);
-    const Workspace ws(optional(a[5], "workspace"), c, x, a[5] == Py_None ? need(M, w->N, w->K, kRank) : 0);
+    const Workspace ws(optional(a[5], "workspace"), c, x, {Need{M, w->N, w->K, kRank}});
     check(nf4ll_forward_multi(w, x.data_ptr(), ld(x), ptr(optional(a[3], "bias")), arr.data(), static_cast<int32_t>(n), M, y.data_ptr(), ld(y), ws.p,
                               ws.bytes, c.status(), c.stream));
     return pair(a[4] == Py_None ? wrap(y) : again(a[4]), again(ts.o));
@@ -342,12 +386,8 @@ PyObject* py_forward_gate_up(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (lg.on) tg = empty({M, kRank}, at::kFloat, x);
     if (lu.on) tu = empty({M, kRank}, at::kFloat, x);
     const Call c(x);
-    int64_t bytes = 0;
-    if (a[7] == Py_None) {
-      const int r = (lg.on || lu.on) ? kRank : 0;
-      bytes = std::max(need(M, I, w->K, r), need(M, w->N, w->K, r));
-    }
-    const Workspace ws(optional(a[7], "workspace"), c, x, bytes);
+    const int32_t rank = (lg.on || lu.on) ? kRank : 0;
+    const Workspace ws(optional(a[7], "workspace"), c, x, {Need{M, I, w->K, rank}, Need{M, w->N, w->K, rank}});
     check(nf4ll_forward_gate_up(w, x.data_ptr(), ld(x), lg.get(), lu.get(), tg.defined() ? tg.data_ptr() : nullptr, tu.defined() ? tu.data_ptr() : nullptr,
                                 M, g.data_ptr(), 2 * I, u.data_ptr(), 2 * I, h.data_ptr(), I, ws.p, ws.bytes, c.status(), c.stream));
     PyObject* r = PyTuple_New(5);
@@ -377,7 +417,7 @@ PyObject* py_backward_dx(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     at::Tensor u;
     if (lora.on && PyObject_IsTrue(a[7])) u = empty({M, kRank}, at::kFloat, dy);
     const Call c(dy);
-    const Workspace ws(optional(a[8], "workspace"), c, dy, a[8] == Py_None ? need(M, w->N, w->K, lora.on ? kRank : 0) : 0);
+    const Workspace ws(optional(a[8], "workspace"), c, dy, {Need{M, w->N, w->K, lora.on ? kRank : 0}});
     check(nf4ll_backward_dx(w, dy.data_ptr(), ld(dy), lora.get(), u.defined() ? u.data_ptr() : nullptr, M, dx.data_ptr(), ld(dx), accumulate, ws.p, ws.bytes,
                             c.status(), c.stream));
     return pair(a[5] == Py_None ? wrap(dx) : again(a[5]), wrap(&u));
@@ -713,7 +753,7 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
       value_error("a dropout mask without a LoRA branch has no meaning");
     }
     at::Tensor y = empty({M, m->N}, at::kHalf, x2);
-    const Workspace ws(nullptr, c, x2, need(M, m->N, m->K, lora.on ? kRank : 0));
+    const Workspace ws(nullptr, c, x2, {Need{M, m->N, m->K, lora.on ? kRank : 0}});
     check(nf4ll_forward(m, x2.data_ptr(), ld(x2), bias ? bias->data_ptr() : nullptr, lora.get(), t.defined() ? t.data_ptr() : nullptr, M, y.data_ptr(), m->N,
                         ws.p, ws.bytes, c.status(), c.stream));
     ctx->saved_data["w"] = c10::IValue::make_capsule(w);
@@ -752,7 +792,7 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
       lora.set(A16, B16, s[0], Bt16.defined() ? &Bt16 : nullptr, m2.defined() ? &m2 : nullptr, s[1]);
       u = empty({M, kRank}, at::kFloat, dy2);
     }
-    const Workspace ws(nullptr, c, dy2, need(M, m->N, m->K, lora.on ? kRank : 0));
+    const Workspace ws(nullptr, c, dy2, {Need{M, m->N, m->K, lora.on ? kRank : 0}});
     check_nogil(nf4ll_backward_dx(m, dy2.data_ptr(), ld(dy2), lora.get(), u.defined() ? u.data_ptr() : nullptr, M, dx.data_ptr(), m->K, 0, ws.p, ws.bytes,
                                   status_nogil(c), c.stream));
     if (lora.on) {
