@@ -725,7 +725,9 @@ using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
 struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
-  static at::Tensor forward(AutogradContext* ctx, const at::Tensor& x, const at::Tensor& A, const at::Tensor& B, const c10::intrusive_ptr<WeightRef>& w,
+  // the factors are optional and not undefined tensors, which the autograd machinery does not take for inputs
+  static at::Tensor forward(AutogradContext* ctx, const at::Tensor& x, const std::optional<at::Tensor>& A, const std::optional<at::Tensor>& B,
+                            const c10::intrusive_ptr<WeightRef>& w,
                             const std::optional<at::Tensor>& bias, double scale, const std::optional<at::Tensor>& mask, double keep_scale) {
     const nf4ll_mat* m = w->m;
     at::Tensor x2 = x.dim() == 2 ? x : x.reshape({-1, x.size(-1)});
@@ -735,8 +737,8 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
     at::Tensor A16, B16, Bt16, t;
     Lora lora;
     const Call c(x2);
-    if (A.defined()) {
-      at::Tensor Ac = A.contiguous(), Bc = B.contiguous();
+    if (A) {
+      at::Tensor Ac = A->contiguous(), Bc = B->contiguous();
       if (Ac.scalar_type() == at::kFloat && Bc.scalar_type() == at::kFloat && Ac.dim() == 2 && Bc.dim() == 2 && Ac.size(0) == kRank && Bc.size(1) == kRank &&
           Ac.is_cuda() && Bc.is_cuda() && reinterpret_cast<uintptr_t>(Bc.data_ptr()) % 16 == 0) {
         A16 = empty(Ac.sizes(), at::kHalf, x2);
@@ -816,8 +818,9 @@ PyObject* py_linear(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const at::Tensor *A = optional(a[1], "A"), *B = optional(a[2], "B"), *bias = optional(a[5], "bias"), *mask = optional(a[7], "mask");
     if (x.dim() < 1) value_error("x must have a last dimension");
     auto w = c10::make_intrusive<WeightRef>(a[3], mat(a[4]));
-    return wrap(Nf4Linear::apply(x, A ? *A : at::Tensor(), B ? *B : at::Tensor(), w, bias ? std::optional<at::Tensor>(*bias) : std::nullopt, number(a[6]),
-                                 mask ? std::optional<at::Tensor>(*mask) : std::nullopt, number(a[8])));
+    if (!A != !B) value_error("a LoRA branch needs both of its factors");
+    auto given = [](const at::Tensor* t) { return t ? std::optional<at::Tensor>(*t) : std::nullopt; };
+    return wrap(Nf4Linear::apply(x, given(A), given(B), w, given(bias), number(a[6]), given(mask), number(a[8])));
   });
 }
 

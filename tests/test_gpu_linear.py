@@ -400,3 +400,21 @@ def test_autograd_linear_takes_factors_off_16_byte_boundaries():
         for name, t in zip(("y", "dx", "dA", "dB"), tensors):
             err, rel = nf4_oracle.errors(t, ref[name])
             assert err <= 2e-2 and rel <= 1e-3, (name, err, rel)
+
+
+@pytest.mark.parametrize("bias", [True, False])
+@pytest.mark.parametrize("lead", [(70,), (7, 10), (2, 5, 7)])
+def test_autograd_linear_without_lora(bias, lead):
+    pr = make_problem(256, 128, 70, seed=11, lora=False, bias=bias)
+    d = to_device(pr)
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, pr.dy, pr.bias)
+    x = d.x.detach().view(*lead, 128).requires_grad_(True)
+    y = linear.nf4_lora_linear(x, d.w, bias=d.bias)
+    (dx,) = torch.autograd.grad(y, x, d.dy.view(*lead, 256))
+    assert y.shape == (*lead, 256) and dx.shape == x.shape
+    assert_close("y", y.detach().reshape(70, 256), ref["y"])
+    assert_close("dx", dx.reshape(70, 128), ref["dx"])
+    with torch.no_grad():
+        assert torch.equal(linear.nf4_lora_linear(x, d.w, bias=d.bias), y)
+    with pytest.raises(ValueError):
+        linear.nf4_lora_linear(x, d.w, mask=torch.ones(*lead, 128, dtype=torch.uint8, device="cuda"))
