@@ -77,9 +77,20 @@ const nf4ll_mat* mat(PyObject* o) {
 }
 void* ptr(const at::Tensor* t) { return t ? t->data_ptr() : nullptr; }
 
-void check_act(const at::Tensor& t, int64_t cols, const char* what) {
+// `rows`: how many the call reads or writes (it may have more)
+void check_act(const at::Tensor& t, int64_t cols, const char* what, int64_t rows = 0) {
   if (t.scalar_type() != at::kHalf || t.dim() != 2 || t.size(1) != cols || t.stride(1) != 1 || !t.is_cuda())
     value_error("%s must be a CUDA fp16 matrix [M, %lld] with unit inner stride", what, static_cast<long long>(cols));
+  if (t.size(0) < rows) value_error("%s has %lld rows, the call has %lld", what, static_cast<long long>(t.size(0)), static_cast<long long>(rows));
+}
+// a packed fp32 side array of at least `n` elements
+void check_side(const at::Tensor& t, int64_t n, const char* what) {
+  if (t.scalar_type() != at::kFloat || !t.is_contiguous() || !t.is_cuda() || t.numel() < n)
+    value_error("%s must be contiguous CUDA fp32 with at least %lld elements", what, static_cast<long long>(n));
+}
+void check_bias(const at::Tensor* b, int64_t N) {
+  if (b && (b->scalar_type() != at::kHalf || !b->is_contiguous() || !b->is_cuda() || b->numel() < N))
+    value_error("bias must be contiguous CUDA fp16 with %lld elements", static_cast<long long>(N));
 }
 int64_t ld(const at::Tensor& t) { return t.size(0) == 1 && t.stride(0) < t.size(1) ? t.size(1) : t.stride(0); }
 
@@ -148,6 +159,7 @@ struct Workspace {
   at::Tensor own;
   Workspace(const at::Tensor* given, const Call& c, const at::Tensor& like, std::initializer_list<Need> needs) {
     if (given) {
+      if (!given->is_cuda()) value_error("workspace must be a CUDA tensor");
       p = given->data_ptr();
       bytes = given->numel();
       return;
@@ -232,7 +244,7 @@ struct Lora {
     c.mask = static_cast<const uint8_t*>(mask->data_ptr());
     c.ld_mask = mask->dim() > 1 ? (mask->size(0) == 1 && mask->stride(0) < mask->size(1) ? mask->size(1) : mask->stride(0)) : mask->size(0);
   }
-  void parse(PyObject* lora, PyObject* mask, double keep_scale) {
+  void parse(PyObject* lora, PyObject* mask, double keep_scale, int64_t M, int64_t N, int64_t K) {
     if (lora == Py_None) return;
     PyObject* seq = PySequence_Fast(lora, "a LoRA branch is (A16, B16, scale) or (A16, B16, scale, B16t)");
     if (!seq) throw PyRaised();
@@ -240,7 +252,23 @@ struct Lora {
     PyObject** it = PySequence_Fast_ITEMS(seq);
     struct Drop { PyObject* o; ~Drop() { Py_DECREF(o); } } drop{seq};
     if (n < 3) value_error("a LoRA branch is (A16, B16, scale) or (A16, B16, scale, B16t)");
-    set(tensor(it[0], "lora_A"), tensor(it[1], "lora_B"), number(it[2]), n > 3 ? optional(it[3], "B16t") : nullptr, optional(mask, "mask"), keep_scale);
+    const at::Tensor &A = tensor(it[0], "lora_A"), &B = tensor(it[1], "lora_B");
+    const at::Tensor *Bt = n > 3 ? optional(it[3], "B16t") : nullptr, *m = optional(mask, "mask");
+    set(A, B, number(it[2]), Bt, m, keep_scale);
+    fit(A, B, Bt, m, M, N, K);
+  }
+  // the factors and the mask cover a call of M rows on W[N, K]
+  void fit(const at::Tensor& A, const at::Tensor& B, const at::Tensor* Bt, const at::Tensor* mask, int64_t M, int64_t N, int64_t K) const {
+    if (!A.is_cuda() || !B.is_cuda() || (Bt && !Bt->is_cuda())) value_error("LoRA factors must be CUDA tensors");
+    if (A.numel() < c.r * K || B.numel() < N * c.r || (Bt && Bt->numel() < N * c.r))
+      value_error("LoRA factors of %lld and %lld elements do not fit W[%lld, %lld]", static_cast<long long>(A.numel()), static_cast<long long>(B.numel()),
+                  static_cast<long long>(N), static_cast<long long>(K));
+    fit_mask(mask, M, K);
+  }
+  static void fit_mask(const at::Tensor* mask, int64_t M, int64_t K) {
+    if (!mask) return;
+    if (!mask->is_cuda() || mask->size(-1) < K || (mask->dim() == 1 ? 1 : mask->size(0)) < M)
+      value_error("mask must be a CUDA tensor of at least %lld rows of %lld", static_cast<long long>(M), static_cast<long long>(K));
   }
   const nf4ll_lora* get() const { return on ? &c : nullptr; }
 };
@@ -299,11 +327,12 @@ PyObject* py_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     check_act(x, w->K, "x");
     const at::Tensor* bias = optional(a[2], "bias");
     if (a[4] != Py_None && a[3] == Py_None) value_error("a dropout mask without a LoRA branch has no meaning");
-    Lora lora;
-    lora.parse(a[3], a[4], number(a[5]));
     const int64_t M = x.size(0);
+    check_bias(bias, w->N);
+    Lora lora;
+    lora.parse(a[3], a[4], number(a[5]), M, w->N, w->K);
     at::Tensor y = a[6] == Py_None ? empty({M, w->N}, at::kHalf, x) : tensor(a[6], "out");
-    check_act(y, w->N, "out");
+    check_act(y, w->N, "out", M);
     at::Tensor t;
     if (lora.on && PyObject_IsTrue(a[7])) t = empty({M, kRank}, at::kFloat, x);
     const Call c(x);
@@ -323,7 +352,9 @@ PyObject* py_forward_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     check_act(x, w->K, "x");
     const int64_t M = x.size(0);
     at::Tensor y = a[4] == Py_None ? empty({M, w->N}, at::kHalf, x) : tensor(a[4], "out");
-    check_act(y, w->N, "out");
+    check_act(y, w->N, "out", M);
+    const at::Tensor* bias = optional(a[3], "bias");
+    check_bias(bias, w->N);
     PyObject* segs = PySequence_Fast(a[2], "segments must be a sequence");
     if (!segs) throw PyRaised();
     struct Drop { PyObject* o; ~Drop() { Py_XDECREF(o); } } drop{segs};
@@ -340,8 +371,8 @@ PyObject* py_forward_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       PyObject** it = PySequence_Fast_ITEMS(seg.o);
       if (k < 4) value_error("a segment is (rows, lora, mask, keep_scale[, t])");
       if (it[2] != Py_None && it[1] == Py_None) value_error("a dropout mask without a LoRA branch has no meaning");
-      loras[i].parse(it[1], it[2], number(it[3]));
       arr[i].rows = integer(it[0]);
+      loras[i].parse(it[1], it[2], number(it[3]), M, arr[i].rows, w->K);
       arr[i].lora = loras[i].get();
       arr[i].t_out = nullptr;
       arr[i].t_ready = 0;
@@ -364,7 +395,7 @@ PyObject* py_forward_multi(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     }
     const Call c(x);
     const Workspace ws(optional(a[5], "workspace"), c, x, {Need{M, w->N, w->K, kRank}});
-    check(nf4ll_forward_multi(w, x.data_ptr(), ld(x), ptr(optional(a[3], "bias")), arr.data(), static_cast<int32_t>(n), M, y.data_ptr(), ld(y), ws.p,
+    check(nf4ll_forward_multi(w, x.data_ptr(), ld(x), ptr(bias), arr.data(), static_cast<int32_t>(n), M, y.data_ptr(), ld(y), ws.p,
                               ws.bytes, c.status(), c.stream));
     return pair(a[4] == Py_None ? wrap(y) : again(a[4]), again(ts.o));
   });
@@ -380,8 +411,8 @@ PyObject* py_forward_gate_up(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const int64_t M = x.size(0), I = w->N / 2;
     const double ks = number(a[6]);
     Lora lg, lu;
-    lg.parse(a[2], a[3], ks);
-    lu.parse(a[4], a[5], ks);
+    lg.parse(a[2], a[3], ks, M, I, w->K);
+    lu.parse(a[4], a[5], ks, M, I, w->K);
     at::Tensor gu = empty({M, 2 * I}, at::kHalf, x), g = gu.narrow(1, 0, I), u = gu.narrow(1, I, I), h = empty({M, I}, at::kHalf, x), tg, tu;
     if (lg.on) tg = empty({M, kRank}, at::kFloat, x);
     if (lu.on) tu = empty({M, kRank}, at::kFloat, x);
@@ -411,9 +442,9 @@ PyObject* py_backward_dx(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     const int accumulate = PyObject_IsTrue(a[6]);
     if (a[5] == Py_None && accumulate) value_error("accumulate needs an existing dx");
     at::Tensor dx = a[5] == Py_None ? empty({M, w->K}, at::kHalf, dy) : tensor(a[5], "dx");
-    check_act(dx, w->K, "dx");
+    check_act(dx, w->K, "dx", M);
     Lora lora;
-    lora.parse(a[2], a[3], number(a[4]));
+    lora.parse(a[2], a[3], number(a[4]), M, w->N, w->K);
     at::Tensor u;
     if (lora.on && PyObject_IsTrue(a[7])) u = empty({M, kRank}, at::kFloat, dy);
     const Call c(dy);
@@ -424,10 +455,6 @@ PyObject* py_backward_dx(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   });
 }
 
-void check_grad(const at::Tensor& g) {
-  if (g.scalar_type() != at::kFloat || !g.is_contiguous()) value_error("dA/dB must be contiguous fp32");
-}
-
 // lora_grads(dy, x, t, u, scale, mask, keep_scale, dA, dB, accumulate) -> (dA, dB)
 PyObject* py_lora_grads(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   ARGS(10);
@@ -436,14 +463,17 @@ PyObject* py_lora_grads(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (x.dim() != 2 || dy.dim() != 2) value_error("x and dy must be matrices");
     const int64_t M = x.size(0), K = x.size(1), N = dy.size(1);
     check_act(x, K, "x");
-    check_act(dy, N, "dy");
+    check_act(dy, N, "dy", M);
+    check_side(t, M * kRank, "t");
+    check_side(u, M * kRank, "u");
     Lora m;
     m.set_mask(optional(a[5], "mask"), true);
+    Lora::fit_mask(optional(a[5], "mask"), M, K);
     const bool accumulate = PyObject_IsTrue(a[9]);
     at::Tensor dA = a[7] == Py_None ? empty({kRank, K}, at::kFloat, x) : tensor(a[7], "dA");
     at::Tensor dB = a[8] == Py_None ? empty({N, kRank}, at::kFloat, x) : tensor(a[8], "dB");
-    check_grad(dA);
-    check_grad(dB);
+    check_side(dA, kRank * K, "dA");
+    check_side(dB, kRank * N, "dB");
     const int acc_a = accumulate && a[7] != Py_None, acc_b = accumulate && a[8] != Py_None;
     const Call c(x);
     auto call = [&](void* pa, void* pb, int acc) {
@@ -500,9 +530,9 @@ PyObject* py_swiglu_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (g.dim() != 2) value_error("g must be a matrix");
     const int64_t M = g.size(0), I = g.size(1);
     check_act(g, I, "g");
-    check_act(u, I, "u");
+    check_act(u, I, "u", M);
     at::Tensor h = a[2] == Py_None ? empty({M, I}, at::kHalf, g) : tensor(a[2], "out");
-    check_act(h, I, "h");
+    check_act(h, I, "h", M);
     check(nf4ll_swiglu_forward(g.data_ptr(), ld(g), u.data_ptr(), ld(u), h.data_ptr(), ld(h), M, I, Call(g).stream));
     return a[2] == Py_None ? wrap(h) : again(a[2]);
   });
@@ -516,8 +546,10 @@ PyObject* py_swiglu_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (g.dim() != 2) value_error("g must be a matrix");
     const int64_t M = g.size(0), I = g.size(1);
     check_act(g, I, "g");
-    check_act(u, I, "u");
-    check_act(dh, I, "dh");
+    check_act(u, I, "u", M);
+    check_act(dh, I, "dh", M);
+    check_act(dg, I, "dg", M);
+    check_act(du, I, "du", M);
     check(nf4ll_swiglu_backward(g.data_ptr(), ld(g), u.data_ptr(), ld(u), dh.data_ptr(), ld(dh), dg.data_ptr(), ld(dg), du.data_ptr(), ld(du), M, I,
                                 Call(g).stream));
     Py_RETURN_NONE;
@@ -531,12 +563,14 @@ void check_f32(const at::Tensor& t, at::IntArrayRef shape, const char* what) {
 struct NormBranch {
   nf4ll_lora c{};
   bool on = false;
-  void parse(PyObject* A, PyObject* mask, double keep_scale) {
+  void parse(PyObject* A, PyObject* mask, double keep_scale, int64_t n, int64_t d) {
     if (A == Py_None) return;
     const at::Tensor& t = tensor(A, "lora_A");
-    if (t.scalar_type() != at::kHalf || !t.is_contiguous() || t.dim() != 2 || t.size(0) != kRank) value_error("lora_A shadow must be contiguous fp16 [16, D]");
+    if (t.scalar_type() != at::kHalf || !t.is_contiguous() || !t.is_cuda() || t.dim() != 2 || t.size(0) != kRank || t.numel() < kRank * d)
+      value_error("lora_A shadow must be contiguous CUDA fp16 [16, D]");
     Lora m;
     m.set_mask(optional(mask, "mask"));
+    Lora::fit_mask(optional(mask, "mask"), n, d);
     on = true;
     c.A = t.data_ptr();
     c.r = kRank;
@@ -571,8 +605,8 @@ PyObject* py_rms_forward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     }
     NormBranch q, v;
     const double ks = number(a[13]);
-    q.parse(a[7], a[11], ks);
-    v.parse(a[8], a[12], ks);
+    q.parse(a[7], a[11], ks, n, d);
+    v.parse(a[8], a[12], ks, n, d);
     check(nf4ll_rms_forward(x.data_ptr<float>(), ptr(delta), static_cast<float*>(ptr(xout)), w.data_ptr<float>(), static_cast<float>(number(a[4])), n, d,
                             ptr(y), y ? ld(*y) : 0, rstd.data_ptr<float>(), q.get(), ptr(tq), v.get(), ptr(tv), Call(x).stream));
     Py_RETURN_NONE;
@@ -602,8 +636,8 @@ PyObject* py_rms_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     }
     NormBranch q, v;
     const double ks = number(a[13]);
-    q.parse(a[9], a[11], ks);
-    v.parse(a[10], a[12], ks);
+    q.parse(a[9], a[11], ks, n, d);
+    v.parse(a[10], a[12], ks, n, d);
     check(nf4ll_rms_backward(dy.data_ptr(), ld(dy), static_cast<float>(number(a[1])), x.data_ptr<float>(), ptr(delta), w.data_ptr<float>(),
                              rstd.data_ptr<float>(), dres ? dres->data_ptr<float>() : nullptr, out.data_ptr<float>(), ptr(out16), n, d, q.get(), ptr(uq),
                              v.get(), ptr(uv), Call(x).stream));
@@ -624,6 +658,9 @@ PyObject* py_dequant(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     if (out.scalar_type() != at::kHalf || out.numel() < n * 64) value_error("dequant output must be fp16 with room for every block");
     for (auto* x : t)
       if (!x->is_cuda()) value_error("dequant operands must live on the GPU");
+    const int64_t groups = (n + 255) / 256, bytes[5] = {n * 32, n, groups * 4, groups * 4, 256 * 4};
+    for (int i = 0; i < 5; ++i)
+      if (static_cast<int64_t>(t[i]->nbytes()) < bytes[i]) value_error("dequant operand %d has %lld bytes, the blocks need %lld", i, static_cast<long long>(t[i]->nbytes()), static_cast<long long>(bytes[i]));
     check(nf4ll_dequant(static_cast<const uint8_t*>(t[0]->data_ptr()), static_cast<const uint8_t*>(t[1]->data_ptr()), static_cast<const float*>(t[2]->data_ptr()),
                         static_cast<const float*>(t[3]->data_ptr()), static_cast<const float*>(t[4]->data_ptr()), n, out.data_ptr(), Call(out).stream));
     Py_RETURN_NONE;
@@ -670,6 +707,13 @@ PyObject* py_attention_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs)
                      &da = tensor(a[9], "da");
     const auto lens = lengths(a[1]);
     const int64_t nh = integer(a[2]), nkv = integer(a[3]), hd = integer(a[4]), M = qkv.size(0);
+    check_act(qkv, (nh + 2 * nkv) * hd, "qkv");
+    check_act(roped, (nh + nkv) * hd, "roped", M);
+    check_act(out, nh * hd, "a", M);
+    check_side(lse, nh * M, "lse");
+    check_f32(trig, {trig.size(0), hd}, "trig");
+    for (const int32_t n : lens)
+      if (n > trig.size(0)) value_error("the rotary table is shorter than a sequence");
     check_act(da, nh * hd, "da");
     if (da.size(0) != M) value_error("da has %lld rows, the forward had %lld", static_cast<long long>(da.size(0)), static_cast<long long>(M));
     at::Tensor dqkv = empty({M, (nh + 2 * nkv) * hd}, at::kHalf, qkv), delta = empty({nh, M}, at::kFloat, qkv);
@@ -750,10 +794,12 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
         B16 = Bc.to(at::kHalf);
       }
       lora.set(A16, B16, scale, Bt16.defined() ? &Bt16 : nullptr, m2.defined() ? &m2 : nullptr, keep_scale);
+      lora.fit(A16, B16, Bt16.defined() ? &Bt16 : nullptr, m2.defined() ? &m2 : nullptr, M, m->N, m->K);
       t = empty({M, kRank}, at::kFloat, x2);
     } else if (m2.defined()) {
       value_error("a dropout mask without a LoRA branch has no meaning");
     }
+    if (bias) check_bias(&*bias, m->N);
     at::Tensor y = empty({M, m->N}, at::kHalf, x2);
     const Workspace ws(nullptr, c, x2, {Need{M, m->N, m->K, lora.on ? kRank : 0}});
     check(nf4ll_forward(m, x2.data_ptr(), ld(x2), bias ? bias->data_ptr() : nullptr, lora.get(), t.defined() ? t.data_ptr() : nullptr, M, y.data_ptr(), m->N,
@@ -787,6 +833,7 @@ struct Nf4Linear : torch::autograd::Function<Nf4Linear> {
     if (dy2.stride(1) != 1) dy2 = dy2.contiguous();
     TORCH_CHECK_VALUE(dy2.scalar_type() == at::kHalf && dy2.size(1) == m->N && dy2.is_cuda(), "dy must be a CUDA fp16 matrix [M, N]");
     const int64_t M = dy2.size(0);
+    check_act(x2, m->K, "saved x", M);
     const Call c(dy2);
     at::Tensor dx = empty({M, m->K}, at::kHalf, dy2), u, dA, dB;
     Lora lora;
