@@ -670,14 +670,16 @@ DensePlan dense_plan(int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, int sm
   d.nkb = static_cast<int>(KC / 64);
   d.whole = d.tiles;
   d.parts = 1;
-  // A last wave of at most half the pairs: cut its tiles. Costs in k-blocks of time: the exchange about 5, a second launch
-  // about 8 (measured). gate|up pairs columns of both halves of a tile in its epilogue and is not cut.
+  // A last wave of at most half the pairs: cut its tiles. Costs in k-blocks of time: the exchange 7 and 2 per part, a second
+  // launch 8. Cut / whole in us, forward: 16 k-blocks, 12 tiles in 4 parts 27.6 / 23.6 (not cut); 24, 12 in 4 27.6 / 29.7;
+  // 64, 5 in 4 34 / 54; with whole waves before them 24, 6 in 4 54 / 50 (not cut); 40, 12 in 4 101 / 103; 56, 4 in 4 298 / 310.
+  // gate|up pairs columns of both halves of a tile in its epilogue and is not cut.
   const int64_t rest = d.tiles % pairs;
   if (rest > 0 && rest * 2 <= pairs && !gu_inter) {
     int64_t best = d.nkb;
     for (int s = 2; s <= 4; ++s) {
       if (d.nkb < 4 * s || rest > dense_clusters(s)) continue;
-      const int64_t cost = (d.nkb + s - 1) / s + 5 + (d.tiles > rest ? 8 : 0);
+      const int64_t cost = (d.nkb + s - 1) / s + kDnExchange(s) + (d.tiles > rest ? kDnSecondLaunch : 0);
       if (cost < best) { best = cost; d.parts = s; }
     }
     if (d.parts > 1) d.whole = d.tiles - rest;

@@ -38,6 +38,10 @@ struct DensePlan {
   int64_t tiles, tiles_m, tiles_o, whole;      // whole: tiles of the first launch, the others are cut
 };
 
+// What cutting tiles costs, in k-blocks of time (nf4ll_dense.cu)
+constexpr int kDnExchange(int parts) { return 7 + 2 * parts; }
+constexpr int kDnSecondLaunch = 8;
+
 DensePlan dense_plan(int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, int sms);
 int dense_launch(int mode, const DenseMaps& maps, const DenseParams& p, const DensePlan& d, int sms, cudaStream_t stream);
 

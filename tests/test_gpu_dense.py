@@ -7,7 +7,7 @@ tolerance: max-abs-err <= 2e-2 and rel-L2 <= 1e-3."""
 import pytest
 import torch
 
-from decentrik_prime_b200 import k_nf4, linear, quantize
+from decentrik_prime_b200 import _lib, k_nf4, linear, quantize
 from oracle import nf4_oracle
 from tests.problem import make_problem, oracle_weight, to_device
 
@@ -146,3 +146,34 @@ def test_branches_do_not_mix(bad):
             ref = nf4_oracle.lora_linear_o1(nf4_oracle.dequant_weight(layer, ("up_proj", "gate_proj")[ill], code2), x.cpu(), None, None, A, B, s, None, 1.0)
             assert_close("other half", (u, g)[ill], ref["y"])
             assert not torch.isfinite((g, u)[ill]).all()
+
+
+@pytest.mark.parametrize("N,K,M,rows,dense", [(768, 26496, 5884, None, False),            # 36 tiles of 414 steps
+                                              (3584, 3584, 3100, None, True),
+                                              (1280, 1024, 2604, (1024, 128, 128), False),  # stacked with odd boundaries: 128-wide tiles
+                                              (2176, 1664, 2943, (1664, 256, 256), True)])
+def test_large_batches_take_the_way_that_the_model_puts_ahead(N, K, M, rows, dense):
+    w = to_device(make_problem(N, K, 1, seed=N, lora=False)).w
+    x = torch.randn(M, K, generator=torch.Generator().manual_seed(0)).half().cuda()
+
+    def run(flags):
+        with linear.tune_override(flags=flags):
+            if rows is None:
+                return linear.forward(w, x, workspace=ws)[0]
+            return linear.forward_multi(w, x, [(r, None, None, 1.0) for r in rows], workspace=ws)[0]
+
+    def route(flags):
+        before = _lib.lib().nf4ll_launch_count()
+        y = run(flags)
+        return _lib.lib().nf4ll_launch_count() - before, y
+
+    ws = torch.empty(max(2 * N * K + 192 * M + 32 * N + 2048, _lib.lib().nf4ll_workspace_bytes(M, N, K, 0)), dtype=torch.uint8, device="cuda")
+    decoded, dequantised = route(8), route(DENSE)
+    assert decoded[0] != dequantised[0] or not torch.equal(decoded[1], dequantised[1])      # launches or the order of sums tell them apart
+    taken = dequantised if dense else decoded
+    for workspace_given in (True, False):             # the call's own workspace takes the same way
+        if not workspace_given:
+            ws = None
+        n, y = route(0)
+        assert n == taken[0] and torch.equal(y, taken[1])
+    linear.check_status()
