@@ -260,12 +260,23 @@ def _rows_aligned(t):
     return t if ok else t.clone(memory_format=torch.contiguous_format)      # contiguous() would hand back a packed view as it is
 
 
+# Times in us of attention forward + backward, fitted to five head layouts and eighteen batches of 128 to 8192 rows (within 15 %):
+# (start, per query head and pair of rows, per query head and row, per row of the longest sequence) of the library's kernels,
+# (start, per query head and pair of rows, per element of q, k and v, per sequence) of PyTorch's on the GPU.
+_ATTN_OWN_US = {128: (23, 3.75e-6, 1.25e-3, 0.070), 64: (18, 1.69e-6, 0.57e-3, 0.060)}
+_ATTN_TORCH_US = {128: (48, 0.60e-6, 42.8e-6, 65), 64: (66, 0.73e-6, 24.6e-6, 60)}
+_ATTN_TORCH_HOST_US = (630, 210)        # issuing PyTorch's launches, some 70 a sequence: start, per sequence
+
+
 class PackedAttention:
     """Rotary embedding + causal grouped-query attention over packed varlen rows, forward and backward: one kernel each way
     over all sequences and heads (the library's nf4ll_attention_*; reference solution/k_rope.py, k_attn.py) for fp16 rows on
     the GPU in heads of 64 or 128, PyTorch's kernels per sequence (scaled_dot_product_attention, autograd for the backward)
-    for others. Rotary embedding as in Qwen2: the two halves of a head rotate against each other, positions restart at every
-    sequence."""
+    for others, and for long sequences: the library's use mma.sync on tiles of 64 rows, which is faster where launches and
+    short sequences count (4 sequences of 951 rows in all, 12 heads of 128: 77 us and 1507), and slower once the products do
+    (one of 2048 rows, 28 heads: 655 us, PyTorch's 557 replayed from a graph and 840 called one by one; of 4096 rows 2257 and
+    1342; 8 of 1024 rows 1317 and 2991). Rotary embedding as in Qwen2: the two halves of a head rotate against each other,
+    positions restart at every sequence."""
 
     def __init__(self, n_heads, n_kv_heads, head_dim, theta=1.0e6):
         self.nh, self.nkv, self.hd, self.theta = n_heads, n_kv_heads, head_dim, theta
@@ -288,7 +299,32 @@ class PackedAttention:
                 self._trig[key] = t
         return t
 
+    def _own_kernels(self, seq_lens, capturing):
+        """Whether the library's kernels are the faster ones, forward and backward together (a forward does not know whether a
+        backward follows; on its own the forward would change over at longer sequences still). Under capture PyTorch's
+        launches cost no host time, so a captured call may take them where the same call, issued, does not."""
+        pairs, rows = self.nh * sum(n * n for n in seq_lens), sum(seq_lens)
+        c = _ATTN_OWN_US[self.hd]
+        own = c[0] + c[1] * pairs + c[2] * self.nh * rows + c[3] * max(seq_lens, default=0)
+        c = _ATTN_TORCH_US[self.hd]
+        other = c[0] + c[1] * pairs + c[2] * rows * (self.nh + 2 * self.nkv) * self.hd + c[3] * len(seq_lens)
+        if not capturing:
+            other = max(other, _ATTN_TORCH_HOST_US[0] + _ATTN_TORCH_HOST_US[1] * len(seq_lens))
+        return own <= other
+
     def _cos_sin(self, seq_lens, device):
+        if device.type == "cuda":
+            # from the table that is kept: a graph may be captured of lengths never seen before, and outlives the next batch
+            key = (tuple(seq_lens), device, torch.cuda.current_stream(device).cuda_stream)
+            capturing = torch.cuda.is_current_stream_capturing()
+            if capturing or key not in self._tables:
+                table = self._trig_table(max(seq_lens, default=1), device).view(-1, self.hd // 2, 2)
+                rows = torch.cat([table[:n] for n in seq_lens])
+                pair = tuple(torch.cat([rows[..., i], rows[..., i]], dim=1)[:, None, :] for i in (0, 1))
+                if capturing:
+                    return pair
+                self._tables = {key: pair}
+            return self._tables[key]
         key = (tuple(seq_lens), str(device))
         if key not in self._tables:
             pos = torch.cat([torch.arange(n, dtype=torch.float32) for n in seq_lens]).to(device)
@@ -309,7 +345,8 @@ class PackedAttention:
         seq_lens = [int(n) for n in seq_lens]                  # numpy integers and tensors too
         if sum(seq_lens) != qkv.shape[0]:
             raise ValueError(f"sequence lengths {seq_lens} do not add up to {qkv.shape[0]} rows")
-        if self.hd in (64, 128) and qkv.is_cuda and qkv.dtype == torch.float16:
+        if (self.hd in _ATTN_OWN_US and qkv.is_cuda and qkv.dtype == torch.float16
+                and self._own_kernels(seq_lens, torch.cuda.is_current_stream_capturing())):
             qkv = _rows_aligned(qkv.detach())
             trig = self._trig_table(max(seq_lens), qkv.device)
             a, roped, lse = _lib.host().attention_forward(qkv, seq_lens, self.nh, self.nkv, self.hd, trig)

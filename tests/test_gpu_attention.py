@@ -99,3 +99,37 @@ def test_attention_of_a_packed_view_at_an_odd_offset():
     a, state = att.forward(odd, [30, 40])
     b, state_b = att.forward(odd.clone(), [30, 40])
     assert torch.equal(a, b) and torch.equal(att.backward(state, da_odd), att.backward(state_b, da_odd.clone()))
+
+
+@pytest.mark.parametrize("nh,nkv,hd,lens,graph", [(28, 4, 128, [3100], False), (12, 2, 128, [2300], True), (14, 2, 64, [4100, 70, 0, 1], True)])
+def test_long_sequences(nh, nkv, hd, lens, graph):
+    """PyTorch's kernels where they are the faster ones, also in a graph captured of lengths that no call has had before."""
+    gen = torch.Generator().manual_seed(nh)
+    M = sum(lens)
+    qkv = torch.randn(M, (nh + 2 * nkv) * hd, generator=gen).half().cuda()
+    da = torch.randn(M, nh * hd, generator=gen).half().cuda()
+    att = stack.PackedAttention(nh, nkv, hd)
+    assert not att._own_kernels(lens, graph)
+    own = stack.PackedAttention(nh, nkv, hd)
+    own._own_kernels = lambda lens, capturing: True
+    a_own, state = own.forward(qkv, lens)
+    assert len(state) > 2
+    d_own = own.backward(state, da)
+    if graph:
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(side):
+            att.backward(att.forward(qkv[:70], [70])[1], da[:70])
+            g = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(g, stream=side):
+                a, state = att.forward(qkv, lens)
+                d = att.backward(state, da)
+            assert len(state) == 2
+            att.forward(qkv[:71], [71])
+            g.replay()
+        side.synchronize()
+    else:
+        a, state = att.forward(qkv, lens)
+        assert len(state) == 2
+        d = att.backward(state, da)
+    assert rel(a, a_own.double().cpu()) <= REL and rel(d, d_own.double().cpu()) <= REL
