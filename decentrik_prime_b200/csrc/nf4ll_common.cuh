@@ -11,7 +11,7 @@
 namespace nf4ll {
 
 // Launch configuration with the attributes this library uses: programmatic dependent launch (only
-// for kernels that call pdl_wait() first thing), an optional thread-block cluster, an optional
+// for kernels that keep the rule at pdl_wait() below), an optional thread-block cluster, an optional
 // cooperative launch (whole grid resident at once; not combined with the programmatic attribute).
 void count_launch();   // definition in nf4ll_api.cu: one more kernel launched by the calling thread
 
@@ -143,7 +143,10 @@ __device__ __forceinline__ uint4 decode_word(const BlockTable& t, uint32_t w) {
 // Programmatic dependent launch. A kernel launched through PdlLaunch may be set up on the SMs
 // while the kernel before it on the stream is still finishing; pdl_wait() blocks until that kernel
 // has completed and its writes are visible, and must come before the first access to global
-// memory. pdl_launch_dependents() lets the NEXT kernel's blocks start as soon as every block of this
+// memory. Three kernels read earlier, all of them behind a kernel of the same call that has itself waited before it let
+// them start, so that only what that kernel writes is not there yet: the streaming kernel behind a rank-16 projection and
+// the swapped-operand kernel (x, weights, tables), the dense GEMM behind the dequantisation pass (activations, mask).
+// pdl_launch_dependents() lets the NEXT kernel's blocks start as soon as every block of this
 // one has called it (or exited). Both are no-ops for an ordinary launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

@@ -1209,7 +1209,10 @@ constexpr int64_t kSwapMaxRows = 64;       // limit of the swapped-operand kerne
 // round the SMs (and on the tokens), the swapped-operand kernel cuts the contraction too and pays for that. Measured:
 // 27648 x 5120 at 9 / 16 rows 38 / 40 us against 52 / 54, 5120 x 27648 55 / 62 against 45, 5120 x 5120 14 / 15 against 19,
 // 3584 x 18944 27 / 29 against 26 / 27. From 17 rows on the swapped-operand kernel wins over the 128-row tiles on weights of at
-// least 2^24 elements, and up to 64 rows on weights of at least 2^26.
+// least 2^24 elements, and up to 64 rows on weights of at least 2^26. The streaming kernel is behind it there (27648 x 5120 at
+// 17 / 32 / 64 rows 70 / 74 / 133 us against 56; 5120 x 27648 108 / 117 / 160 against 54 / 56 / 60); on smaller weights, which
+// take the tiles, it would be ahead of them (3584 x 3584 at 17 / 32 / 48 rows 18 / 21 / 25 against 26, 8960 x 1536
+// 16 / 18 / 23 against 26), but is not asked.
 constexpr int64_t kSwapMinRows = 9;        // below, the streaming kernel keeps its exact fp32 scales
 constexpr int64_t kSwapMidRows = 32;
 constexpr int64_t kSwapMinWeights = int64_t(1) << 24;
@@ -1621,7 +1624,10 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     int sms = 148;
     if (int rc = device_sms(&sms)) return rc;
     int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, I, W->K, false, sms, g_tune);
-    if (kind != kTiles && M <= kStreamMaxRows && stream_time_us(W->N, W->K, M, sms) < 2 * swap_time_us(I, W->K)) kind = kStream;
+    // up to 16 rows the streaming kernel, whose scales stay fp32, unless the other one's single launch is far ahead: streaming /
+    // swapped in us, 2 x 18944 x 3584 at 9 / 16 rows 52 / 54 against 50, 2 x 27648 x 5120 85 / 91 against 81 / 83,
+    // 2 x 11008 x 2048 30 / 32 against 36
+    if (kind != kTiles && M <= kStreamMaxRows && stream_time_us(W->N, W->K, M, sms) < swap_time_us(W->N, W->K) + 11) kind = kStream;
     if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;
     if (kind == kSwap && (I % 128 || W->N * (W->K / 64) >= (int64_t(1) << 31) || !workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
                           workspace_bytes < swap_workspace_bytes(W->N, W->K, M, sms, 0))) kind = kTiles;

@@ -183,9 +183,9 @@ template <int NTOK>
 __global__ void __launch_bounds__(kSwapThreads, 1)
 nf4_swap_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_nib, const __grid_constant__ SwapParams p) {
   using Cfg = SwapCfg<NTOK>;
-  // x, the weights and code2 may be read at once (what precedes this kernel on the stream is the rank-16
-  // projection kernel, itself started only after all earlier work had finished, or a memset, which orders this
-  // kernel after everything before it); the first write to global memory waits for the predecessor.
+  // x, the weights and code2 may be read at once: what precedes this kernel on the stream is the rank-16 projection or the
+  // kernel that clears the counters, and neither lets this one start before it has waited for all earlier work itself.
+  // T, the counters and the first write to global memory wait for that predecessor.
   pdl_launch_dependents();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));

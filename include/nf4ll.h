@@ -85,8 +85,9 @@ int nf4ll_dequant(const uint8_t* nib, const uint8_t* qabs, const float* scale2, 
                   const float* code2, int64_t n_qblocks, void* out_f16, void* stream);
 
 /* Bytes of scratch that nf4ll_forward / nf4ll_backward_dx need for M rows against W[N,K] with LoRA
- * rank r (0 = no LoRA). The scratch holds the fp32 rank-r projection feeding the fused LoRA step, split-K
- * partial sums and tile counters. Always a multiple of 256; the workspace must be 256-byte aligned. */
+ * rank r (0 = no LoRA), at the least: from 129 rows on nf4ll_workspace_bytes_fast may be the size to give. The scratch holds
+ * the fp32 rank-r projection feeding the fused LoRA step, split-K partial sums and tile counters. Always a multiple of
+ * 256; the workspace must be 256-byte aligned. */
 int64_t nf4ll_workspace_bytes(int64_t M, int64_t N, int64_t K, int32_t r);
 
 /* Scratch with which the calls on W[N,K] run at their best: where that is faster (above 128 rows) it also holds one fp16 copy of
@@ -102,9 +103,11 @@ int64_t nf4ll_workspace_bytes_tuned(int64_t M, int64_t N, int64_t K, int32_t r, 
                                     int32_t splits);
 
 /* Forward:  y[M,N] = x[M,K] . W^T (+ bias) + scale * (drop(x) . A^T) . B^T,  drop(x) = fp16(x * mask * keep_scale)
- * in ONE pass over the NF4 bytes: tiles of W are dequantised into shared memory and fed to
- * tcgen05 MMAs (fp32 accumulation in tensor memory); bias and the LoRA term are added to the fp32
- * accumulator before the single rounding to fp16.
+ * in one pass over the NF4 bytes: tiles of W are dequantised into shared memory and fed to
+ * tcgen05 MMAs (fp32 accumulation in tensor memory), or, with a workspace of nf4ll_workspace_bytes_fast
+ * and where that is faster, once into that workspace and from there; decode-sized batches stream the
+ * codes through registers. bias and the LoRA term are added to the fp32 accumulator before the single
+ * rounding to fp16.
  * Replaces, per projection, the reference's dequant into the fp16 workspace + cuBLAS GEMM + LoRA
  * GEMMs + LoRA add: solution/fast_qwen.py:716-750 (_ws_load/_ws_use), 943-947, 1037, 1080-1098,
  * 1112 and solution/k_rope.py:39-45, 56-58.
@@ -126,7 +129,8 @@ int nf4ll_forward(const nf4ll_mat* W, const void* x, int64_t ldx, const void* bi
  *   y[:, segment i] = x . W_i^T (+ bias over all N columns) + scale_i * (drop_i(x) . A_i^T) . B_i^T
  * W describes the stacked matrix (N = sum of the segments' rows); every segment's row count is a
  * multiple of 128; a segment with a LoRA branch must give t_out (fp32 [M,r], written by the call: the
- * backward needs it anyway). At most 4 segments. Workspace: nf4ll_workspace_bytes(M, N, K, 0).
+ * backward needs it anyway). At most 4 segments. Workspace: at least nf4ll_workspace_bytes(M, N, K, 0),
+ * at best nf4ll_workspace_bytes_fast(M, N, K, r).
  * The backward of such a group needs no entry point of its own: dX = [dY_1 | dY_2 | ...] . W is one
  * nf4ll_backward_dx on the stacked matrix for the base term (LoRA terms per projection). */
 typedef struct {
@@ -149,8 +153,10 @@ int nf4ll_forward_multi(const nf4ll_mat* W, const void* x, int64_t ldx, const vo
  * nf4ll_swiglu_forward on the stored g, u). Replaces the two GEMMs and the gated_silu kernel of
  * solution/fast_qwen.py:1080-1108 (k_mlp.py:21-29). g and u are still written: the backward needs them.
  * A LoRA branch needs its t_out (fp32 [M,r]). I must be a multiple of 8 (of 128 for the fused path;
- * other widths, batches of at most 128 rows and calls under nf4ll_tune_override run the two
- * projections and the stand-alone product instead). Workspace: nf4ll_workspace_bytes(M, I, K, r). */
+ * other widths, batches of at most 128 rows and calls under nf4ll_tune_override run the
+ * projections, in one launch up to 64 rows, and the stand-alone product instead). Workspace: at least
+ * nf4ll_workspace_bytes(M, I, K, r), at best the larger of nf4ll_workspace_bytes(M, 2I, K, r) and
+ * nf4ll_workspace_bytes_fast(M, 2I, K, r). */
 int nf4ll_forward_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4ll_lora* lora_gate,
                           const nf4ll_lora* lora_up, void* t_gate, void* t_up, int64_t M, void* g, int64_t ldg,
                           void* u, int64_t ldu, void* h, int64_t ldh, void* workspace, int64_t workspace_bytes,
@@ -172,7 +178,8 @@ int nf4ll_forward_static(const nf4ll_mat* W, const void* x, int64_t ldx, const v
                          int32_t* status, void* stream);
 
 /* Backward-dX:  dx[M,K] (+)= dy[M,N] . W + keep_scale * mask (.) ((scale * dy . B) . A)
- * reading the same NF4 bytes (the contraction runs over N; no fp16 W and no W^T is materialised).
+ * reading the same NF4 bytes (the contraction runs over N; no W^T is materialised, and an fp16 W only
+ * in a workspace of nf4ll_workspace_bytes_fast).
  * Replaces solution/fast_qwen.py:1310, 1320-1327, 1333-1338, 1350, 1364 (cuBLAS NN GEMMs on the
  * workspace), 1370/1373 (`daq`, `dav`), 1376-1377 (`lqx`, `lvx`) and the masked add in
  * solution/k_norm.py:64-71. accumulate != 0 adds to the existing dx (gate + up, q + k + v).
