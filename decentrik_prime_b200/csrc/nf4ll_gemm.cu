@@ -1824,6 +1824,12 @@ extern "C" void nf4ll_kernel_events(void* start, void* stop) {
 // Failure-detection test hook (no counterpart in the reference). One-shot.
 extern "C" void nf4ll_test_expire_wait(uint32_t polls) { nf4ll::g_expire_polls = polls; }
 
+// Testing hook (no counterpart in the reference)
+extern "C" int32_t nf4ll_test_dense_plan(int64_t M, int64_t NO, int64_t KC) {
+  const nf4ll::DensePlan d = nf4ll::dense_plan(M, NO, KC, 0, nf4ll::sms_or_default());
+  return d.parts + (d.parts > 1 && d.whole > 0 ? 16 : 0);
+}
+
 // ---------------------------------------------------------------------------------------------
 // Forward without a caller-supplied workspace.
 //

@@ -311,6 +311,11 @@ int64_t nf4ll_launch_count(void);
  * ignored by calls that do not split cooperatively. */
 void nf4ll_test_expire_wait(uint32_t polls);
 
+/* Testing hook; no counterpart in the reference. How the large-batch GEMM over a dequantised weight distributes [M, NO] with a
+ * contraction of KC: the parts (1-4) into which the tiles of a last, short wave are cut, plus 16 if whole waves are launched
+ * before them. */
+int32_t nf4ll_test_dense_plan(int64_t M, int64_t NO, int64_t KC);
+
 #ifdef __cplusplus
 }
 #endif

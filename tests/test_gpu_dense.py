@@ -1,7 +1,8 @@
 """The large-batch path (one dequantisation pass, then the dense tcgen05 GEMM), forced through the tuning hook at the
 sizes where it can go wrong: rows around the 512-row tile and its 128-row quarters, columns around the 256-column tile,
-contractions of one to a few 64-wide steps, tiles cut into 2, 3 and 4 parts of the contraction (clusters), stacked
-segments whose boundaries fall inside a tile, gate|up tiles, accumulation into dx. Against the fp64 oracle at the path's
+contractions of one to a few 64-wide steps, tiles cut into 2, 3 and 4 parts of the contraction (clusters), alone and behind
+whole waves, stacked segments whose boundaries fall inside a tile, gate|up tiles, accumulation into dx. Launch counts show
+that the path ran. Against the fp64 oracle at the path's
 tolerance: max-abs-err <= 2e-2 and rel-L2 <= 1e-3."""
 
 import pytest
@@ -25,19 +26,34 @@ def workspace(M, N, K):
     return torch.empty(2 * N * K + 192 * M + 32 * N + 2048, dtype=torch.uint8, device="cuda")
 
 
-# 256 x 64: one k-block; 1536 x 1536 at 513 rows: 12 tiles, four parts; 4864-wide outputs of 2 row blocks: three parts;
-# 7168 wide: two parts; 192 and 320 columns: ragged tiles
-@pytest.mark.parametrize("N,K,M", [(256, 64, 1), (256, 128, 127), (256, 192, 129), (256, 320, 256), (512, 512, 257), (320, 1024, 511),
-                                   (192, 256, 512), (1536, 1536, 513), (1024, 4864, 600), (768, 7168, 1025), (2048, 768, 700)])
+WHOLE, BOTH = 1, 16      # what nf4ll_test_dense_plan says: whole tiles, and whole waves before the cut ones
+
+
+def launches(f):
+    before = _lib.lib().nf4ll_launch_count()
+    r = f()
+    return r, _lib.lib().nf4ll_launch_count() - before
+
+
+# One to five k-blocks; rows around the tile and its quarters; 192 and 320 columns: ragged tiles. Then the plans, forward and
+# backward: short waves cut into 2, 3 and 4 parts, in both directions
+@pytest.mark.parametrize("N,K,M,plans", [(256, 64, 1, (WHOLE, WHOLE)), (256, 128, 127, (WHOLE, WHOLE)), (256, 192, 129, (WHOLE, WHOLE)),
+                                         (256, 320, 256, (WHOLE, WHOLE)), (512, 512, 257, (WHOLE, WHOLE)), (320, 1024, 511, (WHOLE, WHOLE)),
+                                         (192, 256, 512, (WHOLE, WHOLE)), (1536, 1536, 513, (3, 3)), (1024, 4864, 600, (4, WHOLE)),
+                                         (768, 7168, 1025, (4, WHOLE)), (2048, 768, 700, (WHOLE, 4)), (2048, 1536, 1500, (2, 3)),
+                                         (1536, 2048, 1500, (3, 2)), (1600, 2560, 300, (4, 3))])
 @pytest.mark.parametrize("lora,dropout,bias", [(True, 0.05, True), (True, 0.0, False), (False, 0.0, True)])
-def test_tile_edges(N, K, M, lora, dropout, bias):
+def test_tile_edges(N, K, M, plans, lora, dropout, bias):
+    assert (_lib.lib().nf4ll_test_dense_plan(M, N, K), _lib.lib().nf4ll_test_dense_plan(M, K, N)) == plans
     pr = make_problem(N, K, M, seed=N + K + M, lora=lora, dropout=dropout, bias=bias)
     ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, pr.dy, pr.bias, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)
     d = to_device(pr)
     ws = workspace(M, N, K)
     with linear.tune_override(flags=DENSE):
-        y, t = linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, want_t=lora, workspace=ws)
-        dx, u = linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, want_u=lora, workspace=ws)
+        (y, t), n = launches(lambda: linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, want_t=lora, workspace=ws))
+        assert n == (3 if lora else 2)           # (the rank-16 projection,) the dequantisation pass, the GEMM
+        (dx, u), n = launches(lambda: linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, want_u=lora, workspace=ws))
+        assert n == (4 if lora else 2)           # lora_B is transposed too
         linear.check_status()
         assert_close("y", y, ref["y"])
         assert_close("dx", dx, ref["dx"])
@@ -50,6 +66,63 @@ def test_tile_edges(N, K, M, lora, dropout, bias):
     if lora:
         assert_close("t", t, ref["t"])
         assert_close("u", u, ref["u"])
+
+
+@pytest.mark.parametrize("N,K,M,fwd,bwd", [(2048, 2048, 5000, BOTH + 4, BOTH + 4), (4096, 2112, 2560, BOTH + 3, WHOLE), (2112, 4096, 2560, WHOLE, BOTH + 3)])
+@pytest.mark.parametrize("dropout", [0.05, 0.0])
+def test_more_tiles_than_pairs(N, K, M, fwd, bwd, dropout):
+    """Pairs that take several tiles, whole waves and then a short one cut in two launches, with everything fused. The oracle
+    computes the rows around the tiles' edges; the kernels that decode give all of them."""
+    assert (_lib.lib().nf4ll_test_dense_plan(M, N, K), _lib.lib().nf4ll_test_dense_plan(M, K, N)) == (fwd, bwd)
+    pr = make_problem(N, K, M, seed=7, lora=True, dropout=dropout, bias=True)
+    rows = torch.tensor(sorted({r for e in range(0, M + 1, 512) for r in (e - 1, e, e + 127, e + 128, e + 300) if 0 <= r < M} | {M - 1}))
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x[rows], pr.dy[rows], pr.bias, pr.A16, pr.B16, pr.scale,
+                                    None if pr.mask is None else pr.mask[rows], pr.keep_scale)
+    d = to_device(pr)
+    ws = workspace(M, N, K)
+
+    def forward():
+        return linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, workspace=ws)[0]
+
+    def backward(out=None):
+        return linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, out=out, accumulate=out is not None, workspace=ws)[0]
+
+    with linear.tune_override(flags=DENSE):
+        y, n = launches(forward)
+        assert n == (4 if fwd > BOTH else 3)
+        dx, n = launches(backward)
+        assert n == (5 if bwd > BOTH else 4)
+        twice = backward(dx.clone())
+    with linear.tune_override(flags=8):
+        ws = None
+        y_decoded, dx_decoded = forward(), backward()
+    linear.check_status()
+    for name, got, want, full in (("y", y, ref["y"], y_decoded), ("dx", dx, ref["dx"], dx_decoded), ("dx + dx", twice, 2 * ref["dx"], 2 * dx_decoded.float())):
+        assert_close(name, got[rows.cuda()], want)
+        assert_close(name, got, full.double().cpu())
+
+
+def test_stacked_projections_cut_into_parts():
+    """Q|K|V with LoRA on q and v whose boundary lies inside a tile, in tiles cut into parts of the contraction."""
+    M, rows, K = 700, (1408, 384, 256), 1536
+    N = sum(rows)
+    assert _lib.lib().nf4ll_test_dense_plan(M, N, K) == 3
+    pr = make_problem(N, K, M, seed=12, lora=True, dropout=0.05, bias=True)
+    d = to_device(pr)
+    w16, at, segments, branches = oracle_weight(pr), 0, [], []
+    for i, r in enumerate(rows):
+        l = None if i == 1 else (pr.A16 * (i + 1), pr.B16[at:at + r].contiguous(), 2.0)
+        branches.append((at, r, l))
+        segments.append((r, None if l is None else (l[0].cuda(), l[1].cuda(), l[2]), None if l is None else d.mask, pr.keep_scale))
+        at += r
+    with linear.tune_override(flags=DENSE):
+        (y, _), n = launches(lambda: linear.forward_multi(d.w, d.x, segments, bias=d.bias, workspace=workspace(M, N, K)))
+    linear.check_status()
+    assert n == 4                                  # two projections, the dequantisation pass, the GEMM
+    for at, r, l in branches:
+        A, B, s = (None, None, 1.0) if l is None else l
+        ref = nf4_oracle.lora_linear_o1(w16[at:at + r], pr.x, None, pr.bias[at:at + r], A, B, s, None if l is None else pr.mask, pr.keep_scale if l else 1.0)
+        assert_close(f"rows {at}", y[:, at:at + r], ref["y"])
 
 
 @pytest.mark.parametrize("M,H,KV,I", [(300, 512, 128, 1024), (1100, 384, 128, 896)])
