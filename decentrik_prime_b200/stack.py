@@ -266,6 +266,7 @@ def _rows_aligned(t):
 _ATTN_OWN_US = {128: (23, 3.75e-6, 1.25e-3, 0.070), 64: (18, 1.69e-6, 0.57e-3, 0.060)}
 _ATTN_TORCH_US = {128: (48, 0.60e-6, 42.8e-6, 65), 64: (66, 0.73e-6, 24.6e-6, 60)}
 _ATTN_TORCH_HOST_US = (630, 210)        # issuing PyTorch's launches, some 70 a sequence: start, per sequence
+_ATTN_SURELY_OWN_ROWS = 1024            # up to here the library's are ahead by those figures for any heads and lengths
 
 
 class PackedAttention:
@@ -346,7 +347,7 @@ class PackedAttention:
         if sum(seq_lens) != qkv.shape[0]:
             raise ValueError(f"sequence lengths {seq_lens} do not add up to {qkv.shape[0]} rows")
         if (self.hd in _ATTN_OWN_US and qkv.is_cuda and qkv.dtype == torch.float16
-                and self._own_kernels(seq_lens, torch.cuda.is_current_stream_capturing())):
+                and (qkv.shape[0] <= _ATTN_SURELY_OWN_ROWS or self._own_kernels(seq_lens, torch.cuda.is_current_stream_capturing()))):
             qkv = _rows_aligned(qkv.detach())
             trig = self._trig_table(max(seq_lens), qkv.device)
             a, roped, lse = _lib.host().attention_forward(qkv, seq_lens, self.nh, self.nkv, self.hd, trig)

@@ -20,3 +20,10 @@ def test_the_faster_kernels(nh, nkv, hd, lens, own, graph, issued):
     att = stack.PackedAttention(nh, nkv, hd)
     assert att._own_kernels(lens, True) == (own <= graph)
     assert att._own_kernels(lens, False) == (own <= issued)
+
+
+def test_short_batches_need_no_model():
+    for nh, nkv, hd in ((1, 1, 64), (1, 1, 128), (8, 1, 64), (28, 4, 128), (64, 8, 128), (64, 64, 64), (128, 1, 128), (128, 1, 64)):
+        att = stack.PackedAttention(nh, nkv, hd)
+        for n in (1, 100, 500, 1000, stack._ATTN_SURELY_OWN_ROWS):
+            assert att._own_kernels([n], True) and att._own_kernels([n // 2, n - n // 2], True)
