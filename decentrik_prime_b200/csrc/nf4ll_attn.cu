@@ -7,6 +7,9 @@
 // per sequence is the whole gain (through PyTorch: 280 launches per layer and step). The contractions use mma.sync:
 // tiles of 64 rows are too small to feed tcgen05, and at a few microseconds per launch there is nothing to win.
 // Sequence boundaries travel in the kernel parameters, so no copy to the device is needed per batch.
+// That holds for short sequences. One of 2048 rows, 28 heads, takes 655 us forward and backward (161 TFLOP/s, chained by the
+// latencies of mma.sync and ldmatrix at one CTA of four warps per SM and tile), one of 4096 rows 2257 (187); the caller
+// (stack.py) takes other kernels for such batches.
 //
 //   rope     q, k rotated once into a buffer (a key row is read by every query tile after it)
 //   forward  one CTA per 64 query rows and head, 4 warps of 16 rows, keys and values in 64-row blocks by cp.async
