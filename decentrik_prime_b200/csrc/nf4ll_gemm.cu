@@ -1196,6 +1196,13 @@ static int check_lora(const nf4ll_lora* l, const char* who, int64_t K) {
   return NF4LL_OK;
 }
 
+// the kernels read a branch's rank-16 product four floats at a time
+static int check_product(const void* t, const char* who) {
+  if (!(reinterpret_cast<uintptr_t>(t) & 15)) return NF4LL_OK;
+  set_detail("%s: t_out / u_out must be 16-byte aligned", who);
+  return NF4LL_ERR_ALIGN;
+}
+
 int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_t ld_mask, float keep_scale,
                      const void* R, float scale, int64_t M, int64_t C, void* t32, int* zero_ptr, int zero_words,
                      cudaStream_t stream);
@@ -1408,6 +1415,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   if (int rc = check_act(act, ldact, KC, who, mode == kFwd ? "x" : "dy")) return rc;
   if (int rc = check_act(out, ldo, NO, who, mode == kFwd ? "y" : "dx")) return rc;
   if (int rc = check_lora(lora, who, W->K)) return rc;
+  if (int rc = check_product(lora ? side_out : nullptr, who)) return rc;
   if (bias && (reinterpret_cast<uintptr_t>(bias) & 15)) { set_detail("%s: bias must be 16-byte aligned", who); return NF4LL_ERR_ALIGN; }
   if (M > (int64_t(1) << 30)) { set_detail("%s: M too large", who); return NF4LL_ERR_SHAPE; }
   if (int rc = require_sm100()) return rc;
@@ -1426,6 +1434,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
       at += segments[i].rows;
       if (int rc = check_lora(segments[i].lora, who, W->K)) return rc;
       if (segments[i].lora && !segments[i].t_out) { set_detail("%s: segment %d has LoRA but no t_out", who, i); return NF4LL_ERR_NULL; }
+      if (int rc = check_product(segments[i].lora ? segments[i].t_out : nullptr, who)) return rc;
     }
     if (at != W->N) { set_detail("%s: segments cover %lld of %lld rows", who, static_cast<long long>(at), static_cast<long long>(W->N)); return NF4LL_ERR_SHAPE; }
   }
@@ -1618,6 +1627,8 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
   if (int rc = check_lora(lora_gate, who, W->K)) return rc;
   if (int rc = check_lora(lora_up, who, W->K)) return rc;
   if ((lora_gate && !t_gate) || (lora_up && !t_up)) { set_detail("%s: a LoRA branch needs its t_out", who); return NF4LL_ERR_NULL; }
+  if (int rc = check_product(lora_gate ? t_gate : nullptr, who)) return rc;
+  if (int rc = check_product(lora_up ? t_up : nullptr, who)) return rc;
   if (int rc = require_sm100()) return rc;
   if (M <= 128 || I % 128 || g_tune.any()) {
     // short batches and odd widths: the two projections on their own, then the stand-alone gated product

@@ -561,8 +561,9 @@ extern "C" int nf4ll_lora_grads(const void* dy, int64_t lddy, const void* x, int
   if (dA && (!x || !u32)) { set_detail("nf4ll_lora_grads: dA needs x and u"); return NF4LL_ERR_NULL; }
   if (dB && (!dy || !t32)) { set_detail("nf4ll_lora_grads: dB needs dy and t"); return NF4LL_ERR_NULL; }
   if ((dA && ((reinterpret_cast<uintptr_t>(x) & 15) || (ldx % 8))) || (dB && ((reinterpret_cast<uintptr_t>(dy) & 15) || (lddy % 8))) ||
-      (dA && mask && ((reinterpret_cast<uintptr_t>(mask) & 15) || ld_mask % 16))) {
-    set_detail("nf4ll_lora_grads: activations 16-byte aligned with leading dimensions multiples of 8; mask 16-byte aligned, ld_mask multiple of 16");
+      (dA && mask && ((reinterpret_cast<uintptr_t>(mask) & 15) || ld_mask % 16)) || (dA && (reinterpret_cast<uintptr_t>(u32) & 15)) ||
+      (dB && (reinterpret_cast<uintptr_t>(t32) & 15))) {
+    set_detail("nf4ll_lora_grads: activations, t and u 16-byte aligned, leading dimensions multiples of 8; mask 16-byte aligned, ld_mask multiple of 16");
     return NF4LL_ERR_ALIGN;
   }
   if (int rc = require_sm100()) return rc;

@@ -113,7 +113,7 @@ int64_t nf4ll_workspace_bytes_tuned(int64_t M, int64_t N, int64_t K, int32_t r, 
  * 1112 and solution/k_rope.py:39-45, 56-58.
  * x [M,ldx] fp16, y [M,ldy] fp16, bias fp16 [N] or NULL, lora NULL = no LoRA branch.
  * t_out: optional fp32 [M,16] = drop(x) . A^T (unscaled), kept for nf4ll_lora_grads.
- * ldx, ldy multiples of 8; x, y 16-byte aligned. status: optional device int32, set non-zero if a
+ * ldx, ldy multiples of 8; x, y, t_out 16-byte aligned. status: optional device int32, set non-zero if a
  * bounded wait in the kernel expires (never reset by the library). */
 int nf4ll_forward(const nf4ll_mat* W, const void* x, int64_t ldx, const void* bias,
                   const nf4ll_lora* lora, void* t_out, int64_t M, void* y, int64_t ldy,

@@ -109,3 +109,16 @@ def test_longer_tensors_are_taken(d):
     one, _ = linear.forward(d.w, d.x[:1], lora=d.lora, mask=d.mask[0], keep_scale=d.keep_scale)
     two, _ = linear.forward(d.w, d.x[:1], lora=d.lora, mask=d.mask[:1], keep_scale=d.keep_scale)
     assert torch.equal(one, two)
+
+
+def test_rank_16_products_off_a_16_byte_boundary_are_refused(d):
+    """They are read four floats at a time. Gradients may lie anywhere in a flat bucket."""
+    t, odd = f32(M, 16), f32(M * 16 + 1)[1:].view(M, 16)
+    for call in (lambda: linear.forward_multi(d.w, d.x, [(N, d.lora, None, 1.0, odd)]),
+                 lambda: linear.lora_grads(d.dy, d.x, odd, t, 1.0), lambda: linear.lora_grads(d.dy, d.x, t, odd, 1.0)):
+        with pytest.raises(ValueError):
+            call()
+    flat = f32(16 * K + 16 * N + 1)
+    linear.lora_grads(d.dy, d.x, t + 1, t + 1, 1.0, dA=flat[1:1 + 16 * K].view(16, K), dB=flat[1 + 16 * K:].view(N, 16))
+    dA, dB = linear.lora_grads(d.dy, d.x, t + 1, t + 1, 1.0)
+    assert torch.allclose(flat[1:1 + 16 * K].view(16, K), dA, rtol=1e-4, atol=1e-3) and torch.allclose(flat[1 + 16 * K:].view(N, 16), dB, rtol=1e-4, atol=1e-3)
