@@ -1255,9 +1255,10 @@ constexpr int64_t kDenseHostRows = 3072;       // below, a caller may be bound b
 // to 16384 rows. The kernels that decode take about 1.0 per 64-wide step of a tile (their pace is the decode; 0.6 in 128-wide
 // tiles), 4 per round of tiles (7 with the gated product) and 10 for the exchange of a split contraction (8 in 128-wide
 // tiles, which stacked projections with odd boundaries take: `narrow`); the dense GEMM 0.7 per step of its 512-row tiles
-// and 4 per round, after a pass of 2.5 bytes a weight. The second launch costs a caller that is bound by the host, hence a
+// and 4 per round (5 with the gated product), after a pass of 2.5 bytes a weight. The second launch costs a caller that is bound by the host, hence a
 // margin of 3 at middling batches (2048 rows of 1536 x 1536: 29 / 26 on the GPU, but 91 / 97 for an eager forward and
-// backward). Of 960 calls 4 are more than 4 % slower than decoding; where large batches were dense without looking, 24 were.
+// backward). Of 960 calls 4 are put on the dense path where it is more than 4 % slower; with large batches dense without
+// looking, 24 were.
 // Measured, decoding / dense: 37888 x 3584 forward at 512 rows 140 / 160, 1500 rows 424 / 360, 3071 rows 939 / 693;
 // 5120 x 5120 at 951 rows 83 / 80, 2048 rows 144 / 110; 1536 x 8960 at 951 rows 42 / 46; 768 x 26496 at 5884 rows 205 / 282 (36
 // tiles of 414 steps: half the GPU idles); backward of 25984 x 896 at 4306 rows 271 / 333, of 18944 x 3584 at 512 rows
@@ -1275,7 +1276,7 @@ static bool dense_pays(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_i
   const double decoding = rounds * (nkb / t.splits * (t.bn == 128 ? 0.6 : 1.0) + (gu_inter ? 7 : 4)) + (t.splits > 1 ? (narrow ? 8 : 10) : 0);
   const DensePlan d = dense_plan(M, NO, KC, gu_inter, sms);
   double dense = 3 + 0.53e-6 * static_cast<double>(NO) * static_cast<double>(KC);
-  dense += static_cast<double>((d.whole + sms / 2 - 1) / (sms / 2)) * (nkb * 0.7 + 4);
+  dense += static_cast<double>((d.whole + sms / 2 - 1) / (sms / 2)) * (nkb * 0.7 + (gu_inter ? 5 : 4));
   if (d.whole < d.tiles) dense += (nkb / d.parts + kDnExchange(d.parts) + (d.whole ? kDnSecondLaunch : 0)) * 0.7 + 4;
   return dense + (M < kDenseHostRows ? 3 : 0) < decoding;
 }
