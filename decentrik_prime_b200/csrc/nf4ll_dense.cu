@@ -82,7 +82,8 @@ __device__ __forceinline__ void dense_tile_pos(const DenseParams& p, int tile, i
 
 // The rank-16 steps of a tile: one over all 256 columns when both 128-column halves belong to the same branch, else one
 // per half, of 128 columns: a branch whose product is infinite or NaN must not reach the other half's columns (times
-// zeros it would). A half without a branch gets zeros on both sides, which TMA supplies by reading outside the factors.
+// zeros it would). A half without a branch multiplies one block of zeros, which TMA supplies by reading outside a factor, by
+// itself.
 struct DenseLora {
   int n;              // steps: 0, 1 (whole tile) or 2 (halves)
   int seg[2];         // -1: no branch
@@ -182,17 +183,18 @@ dense_gemm_kernel(const __grid_constant__ DenseMaps maps, const __grid_constant_
         const int64_t o0 = static_cast<int64_t>(to) * (p.gu_inter ? 128 : 256);
         const DenseLora l = dense_lora<MODE>(p, o0);
         if (l.n == 0) return;
-        const uint32_t bar = acquire(l.n * 3 * kDnLoraStep);
+        const bool none0 = MODE == kFwd && l.n == 2 && l.seg[0] < 0, none1 = MODE == kFwd && l.n == 2 && l.seg[1] < 0;
+        const uint32_t bar = acquire((l.n * 3 - (none0 || none1 ? 2 : 0)) * kDnLoraStep);
         if (!ok) return;
         const uint32_t base = smem_u32(smem) + (n % S) * kDnStageBytes;
         const int m0 = tm * 512 + static_cast<int>(rank) * 128;
         for (int k = 0; k < l.n; ++k) {
-          const bool none = l.seg[k] < 0;
+          const bool none = k ? none1 : none0;
           const int sg = none ? l.seg[1 - k] : l.seg[k];
           const uint32_t kb = base + k * 3 * kDnLoraStep;
 #pragma unroll 1
-          for (int h = 0; h < 4; ++h) {
-            const int row = static_cast<int>((none ? p.n_lora : p.lora_index[sg]) * p.M) + m0 + (h >> 1) * 256;      // past all branches: zeros
+          for (int h = 0; h < 4 && !none; ++h) {
+            const int row = static_cast<int>(p.lora_index[sg] * p.M) + m0 + (h >> 1) * 256;
             tma_load_2d_pair(kb + h * 2048, &maps.left, (h & 1) * 8, row, bar);
           }
           const uint32_t rb = kb + 2 * kDnLoraStep;
@@ -292,11 +294,11 @@ dense_gemm_kernel(const __grid_constant__ DenseMaps maps, const __grid_constant_
       };
       // the rank-16 steps as the first products of accumulator mt
       auto mma_lora = [&](int mt) {
-        const bool halves = lora.n == 2;
+        const bool halves = MODE == kFwd && lora.n == 2;
 #pragma unroll 1
         for (int k = 0; k < lora.n; ++k) {
           const uint32_t kb = stage_base(lora_at) + k * 3 * kDnLoraStep, rb = kb + 2 * kDnLoraStep;
-          const uint64_t ad = make_smem_desc(kb + mt * kDnLoraStep, 2048, 128, kSwizzleNone);
+          const uint64_t ad = make_smem_desc(halves && lora.seg[k] < 0 ? rb : kb + mt * kDnLoraStep, 2048, 128, kSwizzleNone);
           const uint64_t bd = (MODE == kFwd) ? make_smem_desc(rb, 2048, 128, kSwizzleNone) : make_smem_desc(rb, 2048, 1024, kSwizzle128B);
           tc_mma2_f16(tmem_base + mt * 256 + (halves ? k * 128 : 0), ad, bd, halves ? idesc_half : idesc, 0u);
         }
