@@ -184,7 +184,7 @@ struct Workspace {
       v.push_back({c.device, c.stream, at::Tensor()});
       s = &v.back();
     }
-    const int64_t have = s->ws.defined() ? s->ws.numel() : 0;
+    const int64_t have = s->ws.defined() ? s->ws.numel() : -1;      // a call that needs none gets one too
     if (have < fast) {
       const bool ask = s->refused == 0 || fast < s->refused || --s->again < 0;
       const int64_t want = ask ? fast : least();

@@ -1,4 +1,4 @@
-"""Calls whose fast route wants an fp16 copy of the weight, on a GPU without that much memory left for this process: they take
+"""Scratch memory. Calls whose fast route wants an fp16 copy of the weight, on a GPU without that much memory left for this process: they take
 the route that decodes inside the GEMM, as they do with a workspace of nf4ll_workspace_bytes."""
 
 import pytest
@@ -45,3 +45,25 @@ def test_the_smaller_route_when_memory_is_short():
     for name, got in (("y", y), ("dx", dx)):
         err, rel = nf4_oracle.errors(got, ref[name])
         assert err <= 2e-2 and rel <= 1e-3, (name, err, rel)
+
+
+def test_a_first_call_that_needs_no_scratch():
+    """A contraction too short to be split, without LoRA: the first call on a stream, issued and captured."""
+    pr = make_problem(256, 64, 130, seed=4, lora=False)
+    d = to_device(pr)
+    assert _lib.lib().nf4ll_workspace_bytes_fast(130, 256, 64, 0) == 0
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x)
+    torch.cuda.synchronize()
+    for capture in (False, True):
+        side = torch.cuda.Stream()
+        with torch.cuda.stream(side):
+            if capture:
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=side):
+                    y, _ = linear.forward(d.w, d.x)
+                graph.replay()
+            else:
+                y, _ = linear.forward(d.w, d.x)
+        side.synchronize()
+        err, rel = nf4_oracle.errors(y, ref["y"])
+        assert err <= 2e-2 and rel <= 1e-3, (capture, err, rel)
