@@ -266,7 +266,7 @@ struct Lora {
     fit_mask(mask, M, K);
   }
   static void fit_mask(const at::Tensor* mask, int64_t M, int64_t K) {
-    if (!mask) return;
+    if (!mask || M == 0) return;
     if (!mask->is_cuda() || mask->size(-1) < K || (mask->dim() == 1 ? 1 : mask->size(0)) < M)
       value_error("mask must be a CUDA tensor of at least %lld rows of %lld", static_cast<long long>(M), static_cast<long long>(K));
   }

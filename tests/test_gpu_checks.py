@@ -106,6 +106,7 @@ def test_longer_tensors_are_taken(d):
     tall = torch.cat([d.mask, mask(5, K)])
     got, _ = linear.forward(d.w, d.x, bias=torch.cat([d.bias, zeros(8)]), lora=d.lora, mask=tall, keep_scale=d.keep_scale, out=out)
     assert got is out and torch.equal(out[:M], y) and not out[M:].any()
+    assert linear.forward(d.w, d.x[:0], lora=d.lora, mask=mask(0))[0].shape == (0, N)      # nothing is read
     one, _ = linear.forward(d.w, d.x[:1], lora=d.lora, mask=d.mask[0], keep_scale=d.keep_scale)
     two, _ = linear.forward(d.w, d.x[:1], lora=d.lora, mask=d.mask[:1], keep_scale=d.keep_scale)
     assert torch.equal(one, two)
