@@ -1251,20 +1251,23 @@ static int forward_kind(int mode, int64_t M, int64_t N, int64_t K, bool stacked,
 constexpr int64_t kDenseNeverRows = 128;       // up to one 128-row tile the weight is decoded once anyway
 constexpr int64_t kDenseHostRows = 3072;       // below, a caller may be bound by its host
 
-// Whether the dense path is the faster one: times in us of both ways, fitted to 40 weights of 512 x 512 to 27648 x 5120 at 130
-// to 16384 rows. The kernels that decode take about 1.0 per 64-wide step of a tile (their pace is the decode; 0.6 in 128-wide
-// tiles), 4 per round of tiles (7 with the gated product) and 10 for the exchange of a split contraction (8 in 128-wide
-// tiles, which stacked projections with odd boundaries take: `narrow`); the dense GEMM 0.7 per step of its 512-row tiles
-// and 4 per round (5 with the gated product), after a pass of 2.5 bytes a weight. The second launch costs a caller that is bound by the host, hence a
-// margin of 3 at middling batches (2048 rows of 1536 x 1536: 29 / 26 on the GPU, but 91 / 97 for an eager forward and
-// backward). Of 960 calls 4 are put on the dense path where it is more than 4 % slower; with large batches dense without
-// looking, 24 were.
+// Whether the dense path is the faster one: times in us of both ways in a row of calls, fitted to 70 weights of 512 x 512 to
+// 27648 x 5120 at 130 to 16384 rows. The kernels that decode take about 1.0 per 64-wide step of a tile (their pace is the
+// decode; 0.6 in 128-wide tiles), 4 per round of tiles (7 with the gated product) and 12 for the exchange of a split
+// contraction (8 in 128-wide tiles, which stacked projections with odd boundaries take: `narrow`); the dense GEMM 0.7 per
+// step of its 512-row tiles and 4 per round (6 with the gated product), after a pass of 2.5 bytes a weight. Each launch that
+// it takes more costs a caller that is bound by the host, hence a margin of 3 for it at middling batches (2048 rows of
+// 1536 x 1536 with LoRA: 29 / 26 on the GPU, but 91 / 97 for an eager forward and backward); a split contraction without
+// LoRA has its counters cleared by a launch of its own, so there is none more. Over 1680 calls the choice takes 0.8 % longer than
+// the faster way would, and 18 of them more than 4 % longer than decoding; with large batches dense without looking 3.3 %
+// and 64.
 // Measured, decoding / dense: 37888 x 3584 forward at 512 rows 140 / 160, 1500 rows 424 / 360, 3071 rows 939 / 693;
-// 5120 x 5120 at 951 rows 83 / 80, 2048 rows 144 / 110; 1536 x 8960 at 951 rows 42 / 46; 768 x 26496 at 5884 rows 205 / 282 (36
-// tiles of 414 steps: half the GPU idles); backward of 25984 x 896 at 4306 rows 271 / 333, of 18944 x 3584 at 512 rows
-// 86 / 101, 1500 rows 295 / 240, of 17920 x 1536 at 951 rows 67 / 70; gate|up of 17920 x 1536 at 951 rows 62 / 62, 2048 rows
-// 120 / 108; Q|K|V of 1280 x 1024 (narrow) at 2604 rows 22 / 26, of 2176 x 1664 (narrow) at 2943 rows 50 / 36.
-static bool dense_pays(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, int sms) {
+// 5120 x 5120 at 951 rows 83 / 80, 2048 rows 144 / 110; 1536 x 8960 at 951 rows 42 / 46; 1024 x 1024 at 596 rows 22.7 / 19.8;
+// 768 x 26496 at 5884 rows 205 / 282 (36 tiles of 414 steps: half the GPU idles); backward of 25984 x 896 at 4306 rows
+// 271 / 333, of 18944 x 3584 at 512 rows 86 / 101, 1500 rows 295 / 240, of 17920 x 1536 at 951 rows 67 / 70; gate|up of
+// 17920 x 1536 at 951 rows 62 / 62, 2048 rows 120 / 108; Q|K|V of 1280 x 1024 (narrow) at 2604 rows 22 / 26, of 2176 x 1664
+// (narrow) at 2943 rows 50 / 36.
+static bool dense_pays(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, bool lora, int sms) {
   if (M <= kDenseNeverRows) return false;
   const double nkb = static_cast<double>(KC / 64);
   Tune width;
@@ -1273,12 +1276,14 @@ static bool dense_pays(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_i
   if (gu_inter) { t.pair = 0; t.bn = 256; t.splits = 1; t.tiles_m = (M + 255) / 256; t.tiles_o = (gu_inter + 127) / 128; }
   const int64_t at_once = t.pair ? sms / 2 : sms;
   const double rounds = static_cast<double>((t.tiles_m * t.tiles_o * t.splits + at_once - 1) / at_once);
-  const double decoding = rounds * (nkb / t.splits * (t.bn == 128 ? 0.6 : 1.0) + (gu_inter ? 7 : 4)) + (t.splits > 1 ? (narrow ? 8 : 10) : 0);
+  const double decoding = rounds * (nkb / t.splits * (t.bn == 128 ? 0.6 : 1.0) + (gu_inter ? 7 : 4)) + (t.splits > 1 ? (narrow ? 8 : 12) : 0);
   const DensePlan d = dense_plan(M, NO, KC, gu_inter, sms);
+  const bool cut = d.whole < d.tiles;
   double dense = 3 + 0.53e-6 * static_cast<double>(NO) * static_cast<double>(KC);
-  dense += static_cast<double>((d.whole + sms / 2 - 1) / (sms / 2)) * (nkb * 0.7 + (gu_inter ? 5 : 4));
-  if (d.whole < d.tiles) dense += (nkb / d.parts + kDnExchange(d.parts) + (d.whole ? kDnSecondLaunch : 0)) * 0.7 + 4;
-  return dense + (M < kDenseHostRows ? 3 : 0) < decoding;
+  dense += static_cast<double>((d.whole + sms / 2 - 1) / (sms / 2)) * (nkb * 0.7 + (gu_inter ? 6 : 4));
+  if (cut) dense += (nkb / d.parts + kDnExchange(d.parts) - 2 + (d.whole ? kDnSecondLaunch : 0)) * 0.7 + 4;
+  const int more = (cut && d.whole ? 3 : 2) - (t.splits > 1 && !lora ? 2 : 1);      // launches
+  return dense + (M < kDenseHostRows ? 3 * more : 0) < decoding;
 }
 
 // Scratch of a dense call: the rank-16 products the caller does not keep, lora_B transposed (backward), the fp16
@@ -1299,9 +1304,9 @@ static DenseScratch dense_scratch(int64_t M, int64_t N, int64_t K, bool keep_lef
 }
 
 // Whether a call runs on the dense path, given a workspace that holds the fp16 weight.
-static bool dense_wanted(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, int sms, const Tune& tune) {
+static bool dense_wanted(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, bool lora, int sms, const Tune& tune) {
   if (tune.any() || (tune.flags & 8) || g_expire_polls != 0) return false;
-  return (tune.flags & 16) || ((!tune.flags || M >= kDenseHostRows) && dense_pays(mode, M, NO, KC, gu_inter, narrow, sms));
+  return (tune.flags & 16) || ((!tune.flags || M >= kDenseHostRows) && dense_pays(mode, M, NO, KC, gu_inter, narrow, lora, sms));
 }
 
 struct DenseCall {
@@ -1422,6 +1427,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   if (int rc = require_sm100()) return rc;
   int sms = 148;
   if (int rc = device_sms(&sms)) return rc;
+  bool any_lora = lora != nullptr;
   bool narrow_tiles = false;       // a segment boundary that is not a multiple of 256 columns needs 128-column tiles
   if (segments) {
     if (n_segments < 1 || n_segments > kMaxSegments) { set_detail("%s: %d segments (1..%d)", who, n_segments, kMaxSegments); return NF4LL_ERR_SHAPE; }
@@ -1434,13 +1440,14 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
       if (at % 256) narrow_tiles = true;
       at += segments[i].rows;
       if (int rc = check_lora(segments[i].lora, who, W->K)) return rc;
+      if (segments[i].lora) any_lora = true;
       if (segments[i].lora && !segments[i].t_out) { set_detail("%s: segment %d has LoRA but no t_out", who, i); return NF4LL_ERR_NULL; }
       if (int rc = check_product(segments[i].lora ? segments[i].t_out : nullptr, who)) return rc;
     }
     if (at != W->N) { set_detail("%s: segments cover %lld of %lld rows", who, static_cast<long long>(at), static_cast<long long>(W->N)); return NF4LL_ERR_SHAPE; }
   }
   Tune tune = g_tune;
-  if (dense_wanted(mode, M, NO, KC, 0, narrow_tiles, sms, tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
+  if (dense_wanted(mode, M, NO, KC, 0, narrow_tiles, any_lora, sms, tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
     DenseCall c{};
     c.mode = mode; c.W = W; c.act = act; c.ldact = ldact; c.bias = bias; c.M = M; c.out = out; c.ldo = ldo; c.accumulate = accumulate;
     c.stacked = segments != nullptr;
@@ -1678,7 +1685,7 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
   }
   int sms = 148;
   if (int rc = device_sms(&sms)) return rc;
-  if (dense_wanted(kFwd, M, W->N, W->K, I, false, sms, g_tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
+  if (dense_wanted(kFwd, M, W->N, W->K, I, false, lora_gate || lora_up, sms, g_tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
     DenseCall c{};
     c.mode = kFwd; c.W = W; c.act = x; c.ldact = ldx; c.M = M; c.out = g; c.ldo = ldg;
     c.out_u = u; c.ldu = ldu; c.out_h = h; c.ldh = ldh; c.gu_inter = I; c.n_branch = 2;
@@ -1787,9 +1794,10 @@ extern "C" int64_t nf4ll_workspace_bytes_fast(int64_t M, int64_t N, int64_t K, i
   int64_t need = nf4ll_workspace_bytes(M, N, K, r);
   if (M <= kDenseNeverRows || N <= 0 || K <= 0) return need;
   const int sms = sms_or_default();
-  // any of the calls that the matrix may serve: forward, backward, stacked with odd boundaries, gate|up
-  if (!dense_pays(kFwd, M, N, K, 0, false, sms) && !dense_pays(kBwd, M, K, N, 0, false, sms) && (N % 128 || !dense_pays(kFwd, M, N, K, 0, true, sms)) &&
-      (N % 256 || !dense_pays(kFwd, M, N, K, N / 2, false, sms))) return need;
+  // any of the calls that the matrix may serve: forward, backward, stacked with odd boundaries, gate|up; without LoRA, which
+  // pays at more sizes than with
+  if (!dense_pays(kFwd, M, N, K, 0, false, false, sms) && !dense_pays(kBwd, M, K, N, 0, false, false, sms) &&
+      (N % 128 || !dense_pays(kFwd, M, N, K, 0, true, false, sms)) && (N % 256 || !dense_pays(kFwd, M, N, K, N / 2, false, false, sms))) return need;
   const int64_t n = dense_scratch(M, N, K, r > 0, r > 0, r > 0 ? kMaxSegments : 0).total;
   if (n > need) need = n;
   return need;
