@@ -20,7 +20,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libnf4ll.so")
 HOST_PATH = os.path.join(HERE, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "torch_host.cpp")
-SOURCES = ("nf4ll_api.cu", "nf4ll_dequant.cu", "nf4ll_dense.cu", "nf4ll_gemm.cu", "nf4ll_gemm2.cu", "nf4ll_lora.cu", "nf4ll_swiglu.cu", "nf4ll_stream.cu", "nf4ll_swap.cu", "nf4ll_norm.cu", "nf4ll_attn.cu")
+SOURCES = ("nf4ll_api.cu", "nf4ll_dequant.cu", "nf4ll_dense.cu", "nf4ll_gemm.cu", "nf4ll_gemm2.cu", "nf4ll_lora.cu", "nf4ll_mid.cu", "nf4ll_swiglu.cu", "nf4ll_stream.cu", "nf4ll_swap.cu", "nf4ll_norm.cu", "nf4ll_attn.cu")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "--fmad=true", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall", "-shared"]
@@ -165,6 +165,7 @@ SIGNATURES = {
     "nf4ll_tune_override": (None, [_i32, _i32, _i32, _i32]),
     "nf4ll_test_expire_wait": (None, [ctypes.c_uint32]),
     "nf4ll_test_dense_plan": (_i32, [_i64, _i64, _i64]),
+    "nf4ll_test_mid": (None, [_i32, _i32, _i32, _i32]),
     "nf4ll_launch_count": (_i64, []),
     "nf4ll_kernel_events": (None, [_vp, _vp]),
     "nf4ll_rms_forward": (_i32, [_vp, _vp, _vp, _vp, _f32, _i64, _i64, _vp, _i64, _vp, _LORA, _vp, _LORA, _vp, _vp]),

@@ -29,6 +29,7 @@
 #include "nf4ll_dense.cuh"
 #include "nf4ll_dequant.cuh"
 #include "nf4ll_gemm_shared.cuh"
+#include "nf4ll_mid.cuh"
 #include "nf4ll_stream.cuh"
 
 namespace nf4ll {
@@ -1041,6 +1042,10 @@ struct Tune {
   bool any() const { return bm || bn || splits; }
 };
 static thread_local Tune g_tune;
+struct MidTune {                      // nf4ll_test_mid
+  int on = 0, rb = 0, nt = 0, cl = 0;
+};
+static thread_local MidTune g_mid;
 static thread_local uint32_t g_expire_polls = 0;      // nf4ll_test_expire_wait: one-shot
 static thread_local cudaEvent_t g_ev_start = nullptr, g_ev_stop = nullptr;
 
@@ -1267,8 +1272,10 @@ constexpr int64_t kDenseHostRows = 3072;       // below, a caller may be bound b
 // 271 / 333, of 18944 x 3584 at 512 rows 86 / 101, 1500 rows 295 / 240, of 17920 x 1536 at 951 rows 67 / 70; gate|up of
 // 17920 x 1536 at 951 rows 62 / 62, 2048 rows 120 / 108; Q|K|V of 1280 x 1024 (narrow) at 2604 rows 22 / 26, of 2176 x 1664
 // (narrow) at 2943 rows 50 / 36.
-static bool dense_pays(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, bool lora, int sms) {
-  if (M <= kDenseNeverRows) return false;
+struct RowTimes {
+  double decoding, dense;          // dense: with the margin for its launches
+};
+static RowTimes row_times(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, bool lora, int sms) {
   const double nkb = static_cast<double>(KC / 64);
   Tune width;
   if (narrow) width.bn = 128;
@@ -1283,7 +1290,12 @@ static bool dense_pays(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_i
   dense += static_cast<double>((d.whole + sms / 2 - 1) / (sms / 2)) * (nkb * 0.7 + (gu_inter ? 6 : 4));
   if (cut) dense += (nkb / d.parts + kDnExchange(d.parts) - 2 + (d.whole ? kDnSecondLaunch : 0)) * 0.7 + 4;
   const int more = (cut && d.whole ? 3 : 2) - (t.splits > 1 && !lora ? 2 : 1);      // launches
-  return dense + (M < kDenseHostRows ? 3 * more : 0) < decoding;
+  return {decoding, dense + (M < kDenseHostRows ? 3 * more : 0)};
+}
+static bool dense_pays(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, bool lora, int sms) {
+  if (M <= kDenseNeverRows) return false;
+  const RowTimes t = row_times(mode, M, NO, KC, gu_inter, narrow, lora, sms);
+  return t.dense < t.decoding;
 }
 
 // Scratch of a dense call: the rank-16 products the caller does not keep, lora_B transposed (backward), the fp16
@@ -1406,6 +1418,68 @@ static int run_dense(const DenseCall& c, const DensePlan& d, int sms, const Dens
   return rc;
 }
 
+// Whether a call runs on the kernel for middling batches (nf4ll_mid.cu)
+constexpr int64_t kMidMostRows = 1024;
+static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int sms, const Tune& tune, MidPlan* mp) {
+  if (tune.any() || tune.flags || g_expire_polls != 0 || g_mid.on < 0) return false;
+  const int64_t NO = c.mode == kFwd ? c.W->N : c.W->K, KC = c.mode == kFwd ? c.W->K : c.W->N;
+  if (c.W->N * (c.W->K / 64) >= (int64_t(1) << 31) || c.M >= (1 << 24)) return false;      // the kernel's indices have 32 bits
+  if (g_mid.on > 0) return mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, g_mid.rb, g_mid.nt, g_mid.cl, mp);
+  if (c.M > kMidMostRows || (c.mode == kFwd && c.M <= kStreamMaxRows)) return false;
+  if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
+  if (c.M <= kDenseNeverRows) return true;
+  const RowTimes t = row_times(c.mode, c.M, NO, KC, c.gu_inter, narrow, lora, sms);
+  const double us = mp->us * (c.M <= 512 ? 1.08 : 1.2);      // the model's error: it knows nothing of clocks that fall under load
+  return us < t.decoding && us < t.dense;
+}
+
+// Scratch: the rank-16 product where the caller keeps none, lora_B transposed (backward).
+static int run_mid(MidCall& c, const MidPlan& mp, const nf4ll_lora* const* br, void* const* side, const bool* ready, void* workspace,
+                   int64_t workspace_bytes, int32_t* status, cudaStream_t stream, const char* who) {
+  const nf4ll_mat* W = c.W;
+  const bool fwd = c.mode == kFwd;
+  const int64_t left_bytes = br[0] && !side[0] ? align256(c.M * 16 * 4) : 0;
+  const int64_t need = left_bytes + (!fwd && br[0] && !br[0]->Bt ? align256(W->N * 16 * 2) : 0);
+  if (need > 0 && (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < need)) {
+    set_detail("%s: needs a 256-byte aligned workspace of %lld bytes (got %lld)", who, static_cast<long long>(need), static_cast<long long>(workspace_bytes));
+    return NF4LL_ERR_WORKSPACE;
+  }
+  uint8_t* ws = static_cast<uint8_t*>(workspace);
+  bool projected = false;
+  for (int i = 0; i < c.n_seg; ++i) {
+    const nf4ll_lora* l = br[i];
+    if (!l) continue;
+    float* left = side[i] ? static_cast<float*>(side[i]) : reinterpret_cast<float*>(ws);
+    if (fwd) {
+      if (!ready[i]) {
+        if (int rc = lora_down_launch(c.act, c.ldact, l->mask, l->ld_mask, l->keep_scale, l->A, 1.0f, c.M, W->K, left, nullptr, 0, stream)) return rc;
+        projected = true;
+      }
+      c.seg_right[i] = static_cast<const __half*>(l->B) - (i ? c.seg_end[i - 1] * 16 : 0);      // indexed by the row of W
+      c.seg_scale[i] = l->scale;
+    } else {
+      const void* bt = l->Bt;
+      if (!bt) {
+        if (int rc = transpose_n16_launch(l->B, ws + left_bytes, W->N, stream)) return rc;
+        bt = ws + left_bytes;
+      }
+      if (int rc = lora_down_launch(c.act, c.ldact, nullptr, 0, 1.0f, bt, l->scale, c.M, W->N, left, nullptr, 0, stream)) return rc;
+      projected = true;
+      c.seg_right[i] = static_cast<const __half*>(l->A);
+      c.seg_scale[i] = 1.0f;
+      c.mask = l->mask; c.ld_mask = l->ld_mask; c.keep_scale = l->keep_scale;
+    }
+    c.seg_left[i] = left;
+  }
+  // the measurement hook is one-shot: whichever kernel computes this call's product consumes it
+  cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
+  g_ev_start = g_ev_stop = nullptr;
+  if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
+  const int rc = mid_launch(c, mp, projected && !ev0, status, stream);
+  if (rc == NF4LL_OK && ev1) { if (int rce = record_event(ev1, stream)) return rce; }
+  return rc;
+}
+
 // `segments` (forward only): the weight is several projections stacked along N, each with its own
 // optional LoRA branch; `lora` / `side_out` are then unused.
 static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact, const void* bias,
@@ -1447,6 +1521,22 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     if (at != W->N) { set_detail("%s: segments cover %lld of %lld rows", who, static_cast<long long>(at), static_cast<long long>(W->N)); return NF4LL_ERR_SHAPE; }
   }
   Tune tune = g_tune;
+  {
+    MidCall c{};
+    c.mode = mode; c.W = W; c.act = act; c.ldact = ldact; c.M = M; c.bias = bias; c.out = out; c.ldo = ldo; c.accumulate = accumulate;
+    c.n_seg = segments ? n_segments : 1;
+    const nf4ll_lora* br[kMaxSegments] = {lora};
+    void* side[kMaxSegments] = {side_out};
+    bool ready[kMaxSegments] = {};
+    int64_t at = 0;
+    for (int i = 0; i < c.n_seg; ++i) {
+      if (segments) { br[i] = segments[i].lora; side[i] = segments[i].t_out; ready[i] = segments[i].t_ready != 0; }
+      at += segments ? segments[i].rows : W->N;
+      c.seg_end[i] = at;
+    }
+    MidPlan mp;
+    if (mid_wanted(c, narrow_tiles, any_lora, lora && lora->mask, sms, tune, &mp)) return run_mid(c, mp, br, side, ready, workspace, workspace_bytes, status, stream, who);
+  }
   if (dense_wanted(mode, M, NO, KC, 0, narrow_tiles, any_lora, sms, tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
     DenseCall c{};
     c.mode = mode; c.W = W; c.act = act; c.ldact = ldact; c.bias = bias; c.M = M; c.out = out; c.ldo = ldo; c.accumulate = accumulate;
@@ -1638,6 +1728,20 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
   if (int rc = check_product(lora_gate ? t_gate : nullptr, who)) return rc;
   if (int rc = check_product(lora_up ? t_up : nullptr, who)) return rc;
   if (int rc = require_sm100()) return rc;
+  {
+    int sms = 148;
+    if (int rc = device_sms(&sms)) return rc;
+    MidCall c{};
+    c.mode = kFwd; c.W = W; c.act = x; c.ldact = ldx; c.M = M; c.out = g; c.ldo = ldg;
+    c.out_u = u; c.ldu = ldu; c.out_h = h; c.ldh = ldh; c.gu_inter = I;
+    c.n_seg = 2;
+    c.seg_end[0] = I; c.seg_end[1] = W->N;
+    const nf4ll_lora* br[kMaxSegments] = {lora_gate, lora_up};
+    void* tout[kMaxSegments] = {t_gate, t_up};
+    const bool ready[kMaxSegments] = {};
+    MidPlan mp;
+    if (mid_wanted(c, false, lora_gate || lora_up, false, sms, g_tune, &mp)) return run_mid(c, mp, br, tout, ready, workspace, workspace_bytes, status, stream, who);
+  }
   if (M <= 128 || I % 128 || g_tune.any()) {
     // short batches and odd widths: the two projections on their own, then the stand-alone gated product
     int sms = 148;
@@ -1839,6 +1943,11 @@ extern "C" void nf4ll_tune_override(int32_t bm_tiles, int32_t bn, int32_t splits
 extern "C" void nf4ll_kernel_events(void* start, void* stop) {
   nf4ll::g_ev_start = static_cast<cudaEvent_t>(start);
   nf4ll::g_ev_stop = static_cast<cudaEvent_t>(stop);
+}
+
+// Testing hook (no counterpart in the reference)
+extern "C" void nf4ll_test_mid(int32_t on, int32_t rb, int32_t nt, int32_t cl) {
+  nf4ll::g_mid.on = on; nf4ll::g_mid.rb = rb; nf4ll::g_mid.nt = nt; nf4ll::g_mid.cl = cl;
 }
 
 // Failure-detection test hook (no counterpart in the reference). One-shot.

@@ -316,6 +316,11 @@ void nf4ll_test_expire_wait(uint32_t polls);
  * before them. */
 int32_t nf4ll_test_dense_plan(int64_t M, int64_t NO, int64_t KC);
 
+/* Testing hook; no counterpart in the reference. For the calling thread's next calls: on > 0 makes the kernel for middling
+ * batches take every call that it can, cut into units of 128 * rb weight rows x nt tokens over clusters of cl CTAs (0: its own
+ * choice); on < 0 keeps it out; zeros restore the built-in choice. */
+void nf4ll_test_mid(int32_t on, int32_t rb, int32_t nt, int32_t cl);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,142 @@
+"""The kernel for middling batches (csrc/nf4ll_mid.cu) against the CPU oracle O1 (fp64), at the sizes where its cutting can go
+wrong: row tiles, contractions and token tiles with remainders, blocks that do not come in aligned pairs (K a multiple of 64
+only), every cluster size, several units in a row per cluster, and both directions with LoRA, mask, bias and accumulation.
+Its weights are the bit-exact fp16 ones and every output is one fp32 sum rounded once, so the path's tolerance applies:
+max-abs-err <= 2e-2 and rel-L2 <= 1e-3."""
+
+import contextlib
+
+import pytest
+import torch
+
+from decentrik_prime_b200 import _lib, linear
+from oracle import nf4_oracle
+from tests.problem import make_problem, oracle_weight, to_device
+
+pytestmark = pytest.mark.gpu
+MAX_ABS, REL_L2 = 2e-2, 1e-3
+
+
+@contextlib.contextmanager
+def mid(rb=0, nt=0, cl=0, on=1):
+    _lib.lib().nf4ll_test_mid(on, rb, nt, cl)
+    try:
+        yield
+    finally:
+        _lib.lib().nf4ll_test_mid(0, 0, 0, 0)
+
+
+def assert_close(name, got, ref):
+    err, rel = nf4_oracle.errors(got, ref)
+    assert err <= MAX_ABS and rel <= REL_L2, f"{name}: max-abs {err:.3e} rel-L2 {rel:.3e}"
+
+
+def launches(f):
+    n0 = _lib.lib().nf4ll_launch_count()
+    out = f()
+    return out, _lib.lib().nf4ll_launch_count() - n0
+
+
+# (N, K): whole tiles; half a row tile and K of 6 steps; K of 21 steps (blocks in no pairs); K of 10 steps (pairs, no quads)
+@pytest.mark.parametrize("N,K", [(256, 512), (320, 384), (1280, 1344), (1024, 640)])
+@pytest.mark.parametrize("M,rb,nt,cl", [(1, 1, 16, 1), (17, 1, 32, 2), (33, 2, 48, 1), (100, 1, 64, 3), (129, 2, 80, 2), (187, 1, 192, 2),
+                                        (256, 1, 208, 1), (300, 2, 112, 1)])
+def test_forward_and_backward(N, K, M, rb, nt, cl):
+    if (N * K) % 16384:
+        N *= 2
+    pr = make_problem(N, K, M, seed=N + M, lora=True, dropout=0.05, bias=True)
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, pr.dy, pr.bias, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)
+    d = to_device(pr)
+    with mid(rb, nt, cl):
+        (y, _), n = launches(lambda: linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale))
+        dx, _ = linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)
+        old = torch.randn(M, K).half()
+        acc, _ = linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, out=old.cuda(), accumulate=True)
+        plain = linear.forward(d.w, d.x)[0]
+    linear.check_status()
+    assert n == 2                                 # rank-16 projection and the product
+    assert_close("y", y, ref["y"])
+    assert_close("dx", dx, ref["dx"])
+    assert_close("dx accumulated", acc, ref["dx"] + old.double())
+    assert_close("y without LoRA", plain, pr.x.double() @ oracle_weight(pr).double().t())
+
+
+@pytest.mark.parametrize("cl", range(1, 9))
+def test_cluster_sizes_give_the_same_bits_every_time(cl):
+    """Many units per cluster (3000 tokens in tiles of 32), the sums of the slices exchanged between the CTAs: compared with the
+    oracle on some rows, and bit for bit between repeated calls that race with one another."""
+    pr = make_problem(1024, 2048, 3000, seed=cl, lora=True, dropout=0.05)
+    d = to_device(pr)
+    rows = [0, 31, 32, 1501, 2999]
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x[rows], pr.dy[rows], None, pr.A16, pr.B16, pr.scale, pr.mask[rows], pr.keep_scale)
+
+    def both():
+        return (linear.forward(d.w, d.x, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0],
+                linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0])
+    with mid(1, 32, cl):
+        first = both()
+        again = [both() for _ in range(10)]
+    linear.check_status()
+    assert_close("y", first[0][rows], ref["y"])
+    assert_close("dx", first[1][rows], ref["dx"])
+    for other in again:
+        assert torch.equal(other[0], first[0]) and torch.equal(other[1], first[1])
+
+
+@pytest.mark.parametrize("I,K,M,nt,cl", [(256, 512, 20, 32, 1), (320, 1024, 130, 80, 2), (1088, 1024, 300, 112, 3), (256, 512, 187, 192, 1)])
+def test_gate_up(I, K, M, nt, cl):
+    """A branch whose rank-16 product is not finite does not reach the other one's columns."""
+    pr = make_problem(2 * I, K, M, seed=I, lora=False)
+    w = oracle_weight(pr).double()
+    g = torch.Generator().manual_seed(M)
+    lora = [((torch.randn(16, K, generator=g) / K ** 0.5).half(), (torch.randn(I, 16, generator=g) * 0.02).half(), 2.0) for _ in range(2)]
+    d = to_device(pr)
+    dev = [(a.cuda(), b.cuda(), s) for a, b, s in lora]
+    with mid(2, nt, cl):
+        gate, up, h, _, _ = linear.forward_gate_up(d.w, d.x, lora_gate=dev[0], lora_up=dev[1])
+        bad = (torch.full_like(dev[0][0], float("inf")), dev[0][1], 2.0)
+        _, up_beside, _, _, _ = linear.forward_gate_up(d.w, d.x, lora_gate=bad, lora_up=dev[1])
+    linear.check_status()
+    for i, got in enumerate((gate, up)):
+        t = pr.x.double() @ lora[i][0].double().t()
+        assert_close(f"half {i}", got, pr.x.double() @ w[i * I:(i + 1) * I].t() + 2.0 * t @ lora[i][1].double().t())
+    hg, hu = gate.cpu().double(), up.cpu().double()
+    assert_close("h", h, hg * torch.sigmoid(hg) * hu)
+    assert torch.equal(up_beside, up)
+
+
+def test_stacked_projections():
+    """Row tiles of 128 or 256 over segments of 128-row multiples, a branch on the first and on the last."""
+    K, M, parts = 512, 70, (384, 128, 256)
+    pr = make_problem(sum(parts), K, M, seed=5, lora=False, bias=True)
+    w = oracle_weight(pr).double()
+    g = torch.Generator().manual_seed(3)
+    lora = [((torch.randn(16, K, generator=g) / K ** 0.5).half(), (torch.randn(n, 16, generator=g) * 0.02).half(), 2.0) for n in parts]
+    d = to_device(pr)
+    segs = [(n, None if i == 1 else (lora[i][0].cuda(), lora[i][1].cuda(), 2.0), None, 1.0) for i, n in enumerate(parts)]
+    ref = pr.x.double() @ w.t() + pr.bias.double()
+    at = 0
+    for i, n in enumerate(parts):
+        if i != 1:
+            ref[:, at:at + n] += 2.0 * (pr.x.double() @ lora[i][0].double().t()) @ lora[i][1].double().t()
+        at += n
+    for rb in (1, 2):
+        with mid(rb, 0, 2):
+            y, _ = linear.forward_multi(d.w, d.x, segs, bias=d.bias)
+        assert_close(f"y, {rb} row blocks", y, ref)
+    linear.check_status()
+
+
+def test_values_that_are_not_finite_stay_in_their_rows():
+    """Padding tokens, rows past the weight and steps past the contraction contribute nothing, whatever the neighbours hold."""
+    pr = make_problem(320, 384 * 2, 50, seed=9, lora=False)
+    d = to_device(pr)
+    x = d.x.clone()
+    x[7] = float("inf")
+    x[9, 3] = float("nan")
+    with mid(1, 64, 2):
+        clean, y = linear.forward(d.w, d.x)[0], linear.forward(d.w, x)[0]
+    keep = [i for i in range(50) if i not in (7, 9)]
+    assert torch.equal(y[keep], clean[keep])
+    assert not torch.isfinite(y[[7, 9]]).any()
+    linear.check_status()
