@@ -20,7 +20,7 @@ INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 LIB_PATH = os.path.join(HERE, "libnf4ll.so")
 HOST_PATH = os.path.join(HERE, "_host.so")
 HOST_SOURCE = os.path.join(CSRC, "torch_host.cpp")
-SOURCES = ("nf4ll_api.cu", "nf4ll_dequant.cu", "nf4ll_dense.cu", "nf4ll_gemm.cu", "nf4ll_gemm2.cu", "nf4ll_lora.cu", "nf4ll_mid.cu", "nf4ll_swiglu.cu", "nf4ll_stream.cu", "nf4ll_swap.cu", "nf4ll_norm.cu", "nf4ll_attn.cu")
+SOURCES = ("nf4ll_api.cu", "nf4ll_dequant.cu", "nf4ll_dense.cu", "nf4ll_gemm.cu", "nf4ll_gemm2.cu", "nf4ll_lora.cu", "nf4ll_mid.cu", "nf4ll_swiglu.cu", "nf4ll_stream.cu", "nf4ll_norm.cu", "nf4ll_attn.cu")
 
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-lineinfo",
               "--fmad=true", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall", "-shared"]

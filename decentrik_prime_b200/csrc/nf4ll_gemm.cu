@@ -1216,38 +1216,24 @@ int launch_pair(int mode, int bm_tiles, const CUtensorMap& map, const CUtensorMa
                 const GemmParams& p, int64_t tiles_o, int64_t tiles_mp, int splits, int launch_splits, cudaStream_t stream);
 constexpr int64_t kStreamMaxRows = 16;     // most token rows of the weight-streaming kernel's own choice
 constexpr int64_t kStreamCapRows = 64;     // its limit (reachable through the tuning hook)
-constexpr int64_t kSwapMaxRows = 64;       // limit of the swapped-operand kernel (weights as the MMA's M operand)
-// From 9 to 16 rows the faster of the two by fits of their times: the streaming kernel's depends on how evenly its units go
-// round the SMs (and on the tokens), the swapped-operand kernel cuts the contraction too and pays for that. Measured:
-// 27648 x 5120 at 9 / 16 rows 38 / 40 us against 52 / 54, 5120 x 27648 55 / 62 against 45, 5120 x 5120 14 / 15 against 19,
-// 3584 x 18944 27 / 29 against 26 / 27. From 17 rows on the swapped-operand kernel wins over the 128-row tiles on weights of at
-// least 2^24 elements, and up to 64 rows on weights of at least 2^26. The streaming kernel is behind it there (27648 x 5120 at
-// 17 / 32 / 64 rows 70 / 74 / 133 us against 56; 5120 x 27648 108 / 117 / 160 against 54 / 56 / 60); on smaller weights, which
-// take the tiles, it would be ahead of them (3584 x 3584 at 17 / 32 / 48 rows 18 / 21 / 25 against 26, 8960 x 1536
-// 16 / 18 / 23 against 26), but is not asked.
-constexpr int64_t kSwapMinRows = 9;        // below, the streaming kernel keeps its exact fp32 scales
-constexpr int64_t kSwapMidRows = 32;
-constexpr int64_t kSwapMinWeights = int64_t(1) << 24;
-constexpr int64_t kSwapBigWeights = int64_t(1) << 26;
-static double swap_time_us(int64_t N, int64_t K) { return 11.0 + 0.245e-6 * static_cast<double>(N) * static_cast<double>(K); }
+// From 9 to 16 rows of one projection against at least 2^24 weights, the kernel for middling batches where a fit of its time lies
+// below one of the streaming kernel's, which depends on how evenly its units go round the SMs (and on the tokens). Measured,
+// streaming / middling: 5120 x 27648 at 9 / 16 rows 55 / 62 against 42, 3584 x 18944 27 / 29 against 25, 27648 x 5120 38 / 40
+// against 39. From 17 rows on the latter is ahead everywhere (1536 x 1536 at 17 rows 7.5; the streaming kernel 4.7 at 16).
+constexpr int64_t kMidLeastRows = 9;       // below, the streaming kernel keeps its exact fp32 scales
+constexpr int64_t kMidSmallWeights = int64_t(1) << 24;
+static double mid_small_us(int64_t N, int64_t K) { return 11.0 + 0.245e-6 * static_cast<double>(N) * static_cast<double>(K); }
 
-// Which kernel computes a forward of M rows: the 256 x 256 / 128-row tile kernels (kTiles), the register-level
-// weight-streaming kernel for decode-sized batches (kStream), or the swapped-operand tensor-core kernel for
-// short batches of 9 to 64 rows against a large weight (kSwap). Bits 1 and 2 of the tuning flags force kStream /
-// kSwap up to that kernel's limit.
-enum : int { kTiles = 0, kStream = 1, kSwap = 2 };
-static int forward_kind(int mode, int64_t M, int64_t N, int64_t K, bool stacked, int sms, const Tune& tune) {
+// Which kernel computes a forward of M rows that neither the kernel for middling batches nor the dense GEMM takes: the tile
+// kernels (kTiles) or the register-level weight-streaming kernel for decode-sized batches (kStream). Bit 1 of the tuning flags
+// forces kStream up to that kernel's limit.
+enum : int { kTiles = 0, kStream = 1 };
+static int forward_kind(int mode, int64_t M, bool stacked, const Tune& tune) {
   if (mode != kFwd) return kTiles;
-  // stacked projections never took the swapped-operand kernel, whose scales are rounded to fp16: they keep their precision
   if (stacked) return M <= kStreamMaxRows && !tune.any() && !tune.flags ? kStream : kTiles;
   if (tune.flags & 2) return M <= kStreamCapRows ? kStream : kTiles;
-  const bool swap_ok = M <= kSwapMaxRows && N * (K / 64) < (int64_t(1) << 31);      // the kernel indexes quantisation blocks with 32 bits
-  if (tune.flags & 4) return swap_ok ? kSwap : kTiles;
-  if (tune.any()) return kTiles;
-  const bool large = N * K >= (M <= kSwapMidRows ? kSwapMinWeights : kSwapBigWeights);
-  if (M < kSwapMinRows) return kStream;
-  if (M <= kStreamMaxRows) return swap_ok && large && swap_time_us(N, K) < stream_time_us(N, K, M, sms) ? kSwap : kStream;
-  return swap_ok && large ? kSwap : kTiles;
+  if (tune.any() || (tune.flags & 4)) return kTiles;
+  return M <= kStreamMaxRows ? kStream : kTiles;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1421,15 +1407,30 @@ static int run_dense(const DenseCall& c, const DensePlan& d, int sms, const Dens
 // Whether a call runs on the kernel for middling batches (nf4ll_mid.cu)
 constexpr int64_t kMidMostRows = 1024;
 static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int sms, const Tune& tune, MidPlan* mp) {
-  if (tune.any() || tune.flags || g_expire_polls != 0 || g_mid.on < 0) return false;
-  const int64_t NO = c.mode == kFwd ? c.W->N : c.W->K, KC = c.mode == kFwd ? c.W->K : c.W->N;
-  if (c.W->N * (c.W->K / 64) >= (int64_t(1) << 31) || c.M >= (1 << 24)) return false;      // the kernel's indices have 32 bits
+  if (g_expire_polls != 0 || g_mid.on < 0) return false;
+  const int64_t N = c.W->N, K = c.W->K, NO = c.mode == kFwd ? N : K, KC = c.mode == kFwd ? K : N;
+  if (N * (K / 64) >= (int64_t(1) << 31) || c.M >= (1 << 24)) return false;      // the kernel's indices have 32 bits
+  if ((tune.flags & 4) && c.mode == kFwd && c.n_seg == 1 && c.M <= kStreamCapRows) {
+    int64_t cl = tune.splits < 8 ? tune.splits : 8;
+    if (cl > (K + 255) / 256) cl = (K + 255) / 256;
+    return mid_plan(kFwd, c.M, NO, KC, false, 0, lora, 0, 0, static_cast<int>(cl), mp);
+  }
+  if (tune.any() || tune.flags) return false;
   if (g_mid.on > 0) return mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, g_mid.rb, g_mid.nt, g_mid.cl, mp);
-  if (c.M > kMidMostRows || (c.mode == kFwd && c.M <= kStreamMaxRows)) return false;
+  if (c.M > kMidMostRows) return false;
+  if (c.mode == kFwd && c.M <= kStreamMaxRows) {
+    // gate|up: the streaming kernel, whose scales stay fp32, unless this one's single launch is far ahead
+    if (c.M < kMidLeastRows || (c.n_seg > 1 && !c.gu_inter) || (c.gu_inter ? N / 2 : N) * K < kMidSmallWeights) return false;
+    const double own = mid_small_us(N, K) + (c.gu_inter ? 11 : 0);
+    if (!(own < stream_time_us(N, K, c.M, sms))) return false;
+  }
   if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
   if (c.M <= kDenseNeverRows) return true;
   const RowTimes t = row_times(c.mode, c.M, NO, KC, c.gu_inter, narrow, lora, sms);
-  const double us = mp->us * (c.M <= 512 ? 1.08 : 1.2);      // the model's error: it knows nothing of clocks that fall under load
+  // the model's margin: it knows nothing of clocks that fall under load. At the same work per launch it is 3 % low for 25 GFLOP
+  // and 20 % for 250 (backward of 27648 x 5120 at 951 rows: 288 us, where the tiles take 250).
+  const double work = 2e-9 * static_cast<double>(c.M) * static_cast<double>(N) * static_cast<double>(K);
+  const double us = mp->us * (1.05 + 0.15 * (work < 250 ? work / 250 : 1.0));
   return us < t.decoding && us < t.dense;
 }
 
@@ -1558,11 +1559,10 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   }
   if (segments && (narrow_tiles || tune.bn == 512)) tune.bn = narrow_tiles ? 128 : 256;
   Plan pl = make_plan(mode, M, NO, KC, lora ? lora->r : 0, sms, tune);
-  int kind = forward_kind(mode, M, W->N, W->K, segments != nullptr, sms, g_tune);
+  int kind = forward_kind(mode, M, segments != nullptr, g_tune);
   if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;      // it copies the absmax codes word by word
-  const int force_slices = (tune.flags & 6) ? tune.splits : 0;
-  const int64_t need = kind == kTiles ? pl.total()
-                                      : pl.left_bytes + pl.bt_bytes + (kind == kSwap ? swap_workspace_bytes(W->N, W->K, M, sms, force_slices) : 0);
+  const int force_slices = (tune.flags & 2) ? tune.splits : 0;
+  const int64_t need = kind == kTiles ? pl.total() : pl.left_bytes + pl.bt_bytes;
   if (need > 0) {
     if (!workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) || workspace_bytes < need) {
       set_detail("%s: needs a 256-byte aligned workspace of %lld bytes (got %lld)", who,
@@ -1595,10 +1595,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   }
   int* counters = nullptr;
   int counter_words = 0;
-  if (kind == kSwap) {
-    counters = reinterpret_cast<int*>(ws + pl.left_bytes + pl.bt_bytes);      // one per tile of 128 weight rows
-    counter_words = static_cast<int>((W->N + 127) / 128);
-  } else if (kind == kTiles && pl.splits > 1) {
+  if (kind == kTiles && pl.splits > 1) {
     counters = reinterpret_cast<int*>(ws + pl.left_bytes + pl.bt_bytes);
     counter_words = static_cast<int>(pl.counter_bytes / sizeof(int));
   }
@@ -1665,8 +1662,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
       c.seg_b[i] = segments ? p.seg_right[i] : (lora ? p.lora_right : nullptr);
       c.seg_scale[i] = segments ? p.seg_scale[i] : (lora ? lora->scale : 0.f);
     }
-    const int rc = kind == kStream ? stream_forward_launch(c, projected && !ev0, force_slices, stream)
-                                   : swap_forward_launch(c, counters, projected, force_slices, status, stream);
+    const int rc = stream_forward_launch(c, projected && !ev0, force_slices, stream);
     if (rc == NF4LL_OK && ev1) { if (int rce = record_event(ev1, stream)) return rce; }
     return rc;
   }
@@ -1746,14 +1742,8 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     // short batches and odd widths: the two projections on their own, then the stand-alone gated product
     int sms = 148;
     if (int rc = device_sms(&sms)) return rc;
-    int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, I, W->K, false, sms, g_tune);
-    // up to 16 rows the streaming kernel, whose scales stay fp32, unless the other one's single launch is far ahead: streaming /
-    // swapped in us, 2 x 18944 x 3584 at 9 / 16 rows 52 / 54 against 50, 2 x 27648 x 5120 85 / 91 against 81 / 83,
-    // 2 x 11008 x 2048 30 / 32 against 36
-    if (kind != kTiles && M <= kStreamMaxRows && stream_time_us(W->N, W->K, M, sms) < swap_time_us(W->N, W->K) + 11) kind = kStream;
+    int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, false, g_tune);
     if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;
-    if (kind == kSwap && (I % 128 || W->N * (W->K / 64) >= (int64_t(1) << 31) || !workspace || (reinterpret_cast<uintptr_t>(workspace) & 255) ||
-                          workspace_bytes < swap_workspace_bytes(W->N, W->K, M, sms, 0))) kind = kTiles;
     if (kind != kTiles) {
       // both halves in one pass over the weights
       StreamCall c{};
@@ -1766,9 +1756,8 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
       for (int i = 0; i < 2; ++i) {
         c.seg_end[i] = (i + 1) * I;
         if (!br[i]) continue;
-        const bool zero = kind == kSwap && !projected;
         if (int rc = lora_down_launch(x, ldx, br[i]->mask, br[i]->ld_mask, br[i]->keep_scale, br[i]->A, 1.0f, M, W->K, tout[i],
-                                      zero ? static_cast<int*>(workspace) : nullptr, zero ? static_cast<int>(W->N / 128) : 0, stream)) return rc;
+                                      nullptr, 0, stream)) return rc;
         projected = true;
         c.seg_t[i] = static_cast<const float*>(tout[i]);
         c.seg_b[i] = static_cast<const __half*>(br[i]->B) - i * I * 16;
@@ -1777,8 +1766,7 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
       cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
       g_ev_start = g_ev_stop = nullptr;
       if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
-      if (int rc = kind == kStream ? stream_forward_launch(c, projected && !ev0, 0, stream)
-                                   : swap_forward_launch(c, workspace, projected, 0, status, stream)) return rc;
+      if (int rc = stream_forward_launch(c, projected && !ev0, 0, stream)) return rc;
       if (ev1) { if (int rce = record_event(ev1, stream)) return rce; }
       return nf4ll_swiglu_forward(g, ldg, u, ldu, h, ldh, M, I, stream_v);
     }
@@ -1859,13 +1847,6 @@ static int sms_or_default() {
 static int64_t forward_need(int64_t M, int64_t N, int64_t K, int r, int sms, const Tune& tune) {
   const Plan base = make_plan(kFwd, M, N, K, r, sms, tune);
   int64_t need = base.total();
-  // the swapped-operand kernel keeps counters and partial sums in the workspace too; with it forced by the tuning flags a
-  // split count may be forced as well
-  const int fs = tune.splits;
-  if (M <= kSwapMaxRows) {
-    const int64_t st = base.left_bytes + base.bt_bytes + swap_workspace_bytes(N, K, M, sms, fs);
-    if (st > need) need = st;
-  }
   if (!tune.bn) {
     Tune narrow = tune;
     narrow.bn = 128;

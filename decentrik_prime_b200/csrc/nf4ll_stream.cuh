@@ -1,4 +1,4 @@
-// One call of the short-batch forwards: weight-streaming (nf4ll_stream.cu) or with swapped operands (nf4ll_swap.cu).
+// One call of the weight-streaming forward (nf4ll_stream.cu).
 #pragma once
 
 #include "nf4ll_gemm_shared.cuh"
@@ -28,8 +28,5 @@ double stream_time_us(int64_t N, int64_t K, int64_t M, int sms);
 int stream_forward_launch(const StreamCall& c, bool early, int force_team, cudaStream_t stream);
 
 int zero_words_launch(int* words, int n, cudaStream_t stream);      // nf4ll_lora.cu
-
-int64_t swap_workspace_bytes(int64_t N, int64_t K, int64_t M, int sms, int force_slices);
-int swap_forward_launch(const StreamCall& c, void* scratch, bool counters_zeroed, int force_slices, int32_t* status, cudaStream_t stream);
 
 }  // namespace nf4ll
