@@ -29,6 +29,7 @@
 #include "nf4ll_dense.cuh"
 #include "nf4ll_dequant.cuh"
 #include "nf4ll_gemm_shared.cuh"
+#include "nf4ll_lora.cuh"
 #include "nf4ll_mid.cuh"
 #include "nf4ll_stream.cuh"
 
@@ -1201,6 +1202,27 @@ static int check_lora(const nf4ll_lora* l, const char* who, int64_t K) {
   return NF4LL_OK;
 }
 
+// Rank-16 products of forward branches over the same activation, gathered so that they go out two to a launch.
+struct Projections {
+  const void* act;
+  int64_t ldact, M, K;
+  cudaStream_t stream;
+  DownBranch br[2];
+  int n = 0;
+  bool any = false;
+  int add(const nf4ll_lora* l, void* t) {
+    br[n++] = {l->mask, l->ld_mask, l->keep_scale, static_cast<const __half*>(l->A), static_cast<float*>(t)};
+    return n == 2 ? flush() : NF4LL_OK;
+  }
+  int flush() {
+    if (!n) return NF4LL_OK;
+    const int rc = lora_down_launch(act, ldact, br, n, 1.0f, M, K, nullptr, 0, stream);
+    n = 0;
+    any = true;
+    return rc;
+  }
+};
+
 // the kernels read a branch's rank-16 product four floats at a time
 static int check_product(const void* t, const char* who) {
   if (!(reinterpret_cast<uintptr_t>(t) & 15)) return NF4LL_OK;
@@ -1208,9 +1230,6 @@ static int check_product(const void* t, const char* who) {
   return NF4LL_ERR_ALIGN;
 }
 
-int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_t ld_mask, float keep_scale,
-                     const void* R, float scale, int64_t M, int64_t C, void* t32, int* zero_ptr, int zero_words,
-                     cudaStream_t stream);
 int transpose_n16_launch(const void* B, void* Bt, int64_t N, cudaStream_t stream);
 int launch_pair(int mode, int bm_tiles, const CUtensorMap& map, const CUtensorMap& nib_map, const CUtensorMap& out_map,
                 const GemmParams& p, int64_t tiles_o, int64_t tiles_mp, int splits, int launch_splits, cudaStream_t stream);
@@ -1447,15 +1466,14 @@ static int run_mid(MidCall& c, const MidPlan& mp, const nf4ll_lora* const* br, v
   }
   uint8_t* ws = static_cast<uint8_t*>(workspace);
   bool projected = false;
+  Projections t{c.act, c.ldact, c.M, W->K, stream};
   for (int i = 0; i < c.n_seg; ++i) {
     const nf4ll_lora* l = br[i];
     if (!l) continue;
     float* left = side[i] ? static_cast<float*>(side[i]) : reinterpret_cast<float*>(ws);
     if (fwd) {
-      if (!ready[i]) {
-        if (int rc = lora_down_launch(c.act, c.ldact, l->mask, l->ld_mask, l->keep_scale, l->A, 1.0f, c.M, W->K, left, nullptr, 0, stream)) return rc;
-        projected = true;
-      }
+      if (!ready[i])
+        if (int rc = t.add(l, left)) return rc;
       c.seg_right[i] = static_cast<const __half*>(l->B) - (i ? c.seg_end[i - 1] * 16 : 0);      // indexed by the row of W
       c.seg_scale[i] = l->scale;
     } else {
@@ -1472,6 +1490,8 @@ static int run_mid(MidCall& c, const MidPlan& mp, const nf4ll_lora* const* br, v
     }
     c.seg_left[i] = left;
   }
+  if (int rc = t.flush()) return rc;
+  projected |= t.any;
   // the measurement hook is one-shot: whichever kernel computes this call's product consumes it
   cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
   g_ev_start = g_ev_stop = nullptr;
@@ -1601,6 +1621,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   }
   bool projected = false;          // a rank-16 projection is what this call has launched last
   if (segments) {
+    Projections t{act, ldact, M, W->K, stream};
     int64_t at = 0;
     p.n_seg = n_segments;
     for (int i = 0; i < n_segments; ++i) {
@@ -1608,17 +1629,16 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
       p.seg_begin[i] = at;
       if (l) {
         // the rank-16 projection of this segment: computed here unless the producer of x already wrote it
-        if (!segments[i].t_ready) {
-          if (int rc = lora_down_launch(act, ldact, l->mask, l->ld_mask, l->keep_scale, l->A, 1.0f, M, W->K, segments[i].t_out,
-                                        nullptr, 0, stream)) return rc;
-          projected = true;
-        }
+        if (!segments[i].t_ready)
+          if (int rc = t.add(l, segments[i].t_out)) return rc;
         p.seg_left[i] = static_cast<const float*>(segments[i].t_out);
         p.seg_right[i] = static_cast<const __half*>(l->B) - at * 16;      // indexed by the fused output column
         p.seg_scale[i] = l->scale;
       }
       at += segments[i].rows;
     }
+    if (int rc = t.flush()) return rc;
+    projected = t.any;
   }
   if (lora) {
     // rank-16 projection of the activation, fp32: T = drop(x).A^T (forward) or U = s.dy.B (backward);
@@ -1752,21 +1772,20 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
       c.n_seg = 2;
       const nf4ll_lora* br[2] = {lora_gate, lora_up};
       void* tout[2] = {t_gate, t_up};
-      bool projected = false;
+      Projections t{x, ldx, M, W->K, stream};
       for (int i = 0; i < 2; ++i) {
         c.seg_end[i] = (i + 1) * I;
         if (!br[i]) continue;
-        if (int rc = lora_down_launch(x, ldx, br[i]->mask, br[i]->ld_mask, br[i]->keep_scale, br[i]->A, 1.0f, M, W->K, tout[i],
-                                      nullptr, 0, stream)) return rc;
-        projected = true;
+        if (int rc = t.add(br[i], tout[i])) return rc;
         c.seg_t[i] = static_cast<const float*>(tout[i]);
         c.seg_b[i] = static_cast<const __half*>(br[i]->B) - i * I * 16;
         c.seg_scale[i] = br[i]->scale;
       }
+      if (int rc = t.flush()) return rc;
       cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
       g_ev_start = g_ev_stop = nullptr;
       if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
-      if (int rc = stream_forward_launch(c, projected && !ev0, 0, stream)) return rc;
+      if (int rc = stream_forward_launch(c, t.any && !ev0, 0, stream)) return rc;
       if (ev1) { if (int rce = record_event(ev1, stream)) return rce; }
       return nf4ll_swiglu_forward(g, ldg, u, ldu, h, ldh, M, I, stream_v);
     }
@@ -1795,14 +1814,15 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
   p.gu_inter = I;
   const nf4ll_lora* br[2] = {lora_gate, lora_up};
   void* tout[2] = {t_gate, t_up};
+  Projections t{x, ldx, M, W->K, stream};
   for (int i = 0; i < 2; ++i) {
     if (!br[i]) continue;
-    if (int rc = lora_down_launch(x, ldx, br[i]->mask, br[i]->ld_mask, br[i]->keep_scale, br[i]->A, 1.0f, M, W->K, tout[i],
-                                  nullptr, 0, stream)) return rc;
+    if (int rc = t.add(br[i], tout[i])) return rc;
     p.seg_left[i] = static_cast<const float*>(tout[i]);
     p.seg_right[i] = static_cast<const __half*>(br[i]->B);
     p.seg_scale[i] = br[i]->scale;
   }
+  if (int rc = t.flush()) return rc;
   p.has_lora = (lora_gate || lora_up) ? 1 : 0;
   Plan pl{};
   pl.bm_tiles = 2; pl.bn = 256; pl.splits = 1; pl.launch_splits = 1; pl.pair = 0;

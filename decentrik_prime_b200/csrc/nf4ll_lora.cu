@@ -10,7 +10,7 @@
 // Both kernels are bandwidth-bound passes over x / dy (32 multiply-adds per fp16 element read), so
 // they use warp-level mma.sync.m16n8k16 with operands loaded straight from global memory with
 // 128-bit loads; there is nothing for TMA staging or tensor memory to win here.
-#include "nf4ll_common.cuh"
+#include "nf4ll_lora.cuh"
 
 namespace nf4ll {
 
@@ -53,16 +53,21 @@ __device__ __forceinline__ float down_peer_load(const float* local, uint32_t ran
 
 template <int RG, int COMBINE, int NW>
 __global__ void __launch_bounds__(NW * 32)
-lora_down_kernel(const __half* __restrict__ act, int64_t ldact, const uint8_t* __restrict__ mask, int64_t ld_mask,
-                 float keep_scale, const __half* __restrict__ R, float scale, int64_t M, int64_t C, int64_t c_per_cta,
-                 float* __restrict__ t32, int* __restrict__ zero_ptr, int zero_words) {
+lora_down_kernel(const __half* __restrict__ act, int64_t ldact, const DownBranch first, const DownBranch second, float scale, int64_t M, int64_t C,
+                 int64_t c_per_cta, int* __restrict__ zero_ptr, int zero_words) {
   pdl_wait();
   pdl_launch_dependents();
+  const DownBranch& br = blockIdx.z ? second : first;
+  const uint8_t* __restrict__ mask = br.mask;
+  const __half* __restrict__ R = br.R;
+  float* __restrict__ t32 = br.t32;
+  const int64_t ld_mask = br.ld_mask;
+  const float keep_scale = br.keep_scale;
   constexpr int ROWS = 8 * RG;
   __shared__ float part[NW][ROWS][17];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  if (blockIdx.x == 0 && blockIdx.y == 0) {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) {
     for (int i = threadIdx.x; i < zero_words; i += NW * 32) zero_ptr[i] = 0;
   }
   const int64_t m0 = static_cast<int64_t>(blockIdx.x) * ROWS;
@@ -88,7 +93,7 @@ lora_down_kernel(const __half* __restrict__ act, int64_t ldact, const uint8_t* _
   const uint4 zero = make_uint4(0, 0, 0, 0);
   // U chunks per trip, every load of the trip issued before the first use: the loop is bound by the
   // number of bytes a warp keeps in flight, not by arithmetic
-  constexpr int U = (RG == 2) ? 4 : 2;
+  constexpr int U = RG <= 2 ? 4 : 2;
   for (int64_t k0 = c_begin + static_cast<int64_t>(warp) * 32 + t * 8; k0 < c_end; k0 += U * NW * 32) {
     uint4 x[U][RG], ra[U], rb[U];
     uint2 mk[U][RG];
@@ -225,10 +230,19 @@ int zero_words_launch(int* words, int n, cudaStream_t stream) {
   return NF4LL_OK;
 }
 
-// R is [16,C] row-major. t32 (fp32 [M,16], required) = scale * (drop(act) . R^T). `zero_ptr` / `zero_words`:
-// optional 32-bit words the kernel clears on the way (see the kernel).
-int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_t ld_mask, float keep_scale,
-                     const void* R, float scale, int64_t M, int64_t C, void* t32, int* zero_ptr, int zero_words,
+template <int RG, int COMBINE, int NW>
+static int down_run(dim3 grid, unsigned cluster_y, const __half* a, int64_t ldact, const DownBranch* br, int n, float scale, int64_t M, int64_t C,
+                    int64_t c_per_cta, int* zero_ptr, int zero_words, cudaStream_t stream) {
+  grid.z = static_cast<unsigned>(n);
+  PdlLaunch lc(grid, dim3(NW * 32), 0, stream, cluster_y ? 1 : 0, cluster_y);
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<RG, COMBINE, NW>, a, ldact, br[0], br[n - 1], scale, M, C, c_per_cta, zero_ptr, zero_words));
+  return NF4LL_OK;
+}
+
+// t32 (fp32 [M,16]) = scale * (drop(act) . R^T), R [16,C] row-major, for one branch or for two over the same rows in one launch
+// (q and v of a layer, gate and up: a second launch cost a decoded layer 4 us). `zero_ptr` / `zero_words`: optional 32-bit words
+// the kernel clears on the way (see the kernel).
+int lora_down_launch(const void* act, int64_t ldact, const DownBranch* br, int n, float scale, int64_t M, int64_t C, int* zero_ptr, int zero_words,
                      cudaStream_t stream) {
   if (M == 0) {
     if (zero_words > 0) NF4LL_CUDA(cudaMemsetAsync(zero_ptr, 0, sizeof(int) * zero_words, stream));
@@ -238,43 +252,49 @@ int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_
   NF4LL_CUDA(cudaGetDevice(&dev));
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const __half* a = static_cast<const __half*>(act);
-  const __half* r = static_cast<const __half*>(R);
-  float* t = static_cast<float*>(t32);
   const int64_t groups16 = (M + 15) / 16;
   if (groups16 * 4 >= 3 * static_cast<int64_t>(sms)) {
     // enough rows for (nearly) one CTA per SM at 16 rows each: a CTA takes the whole contraction,
     // sixteen warps deep, and stores its rows directly
-    PdlLaunch lc(dim3(static_cast<unsigned>(groups16), 1), dim3(16 * 32), 0, stream);
-    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<2, kDownDirect, 16>, a, ldact, mask, ld_mask, keep_scale, r, scale, M, C,
-                                  C, t, zero_ptr, zero_words));
-    return NF4LL_OK;
+    return down_run<2, kDownDirect, 16>(dim3(static_cast<unsigned>(groups16), 1), 0, a, ldact, br, n, scale, M, C, C, zero_ptr, zero_words, stream);
   }
   const int64_t row_groups = (M + 31) / 32;
   const int64_t units = (C + kDownWarps * 32 - 1) / (kDownWarps * 32);     // 256-column units
-  int64_t ks = (2 * static_cast<int64_t>(sms)) / row_groups;     // at most two CTAs per SM: one wave, no tail
+  int64_t ks = (2 * static_cast<int64_t>(sms)) / (row_groups * n);     // at most two CTAs per SM: one wave, no tail
   if (ks > units) ks = units;
   if (ks < 1) ks = 1;
   // decode-sized batches are all latency: eight CTAs in one cluster (no zero-fill, no atomics) beat more CTAs + a memset
   if (ks > 8 && M * C <= (int64_t(1) << 21)) ks = 8;
   const int64_t c_per_cta = (units + ks - 1) / ks * (kDownWarps * 32);
   ks = (C + c_per_cta - 1) / c_per_cta;
-  dim3 grid(static_cast<unsigned>(row_groups), static_cast<unsigned>(ks));
-  if (ks == 1) {
-    PdlLaunch lc(grid, dim3(kDownWarps * 32), 0, stream);
-    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<4, kDownDirect, kDownWarps>, a, ldact, mask, ld_mask, keep_scale, r, scale, M, C,
-                                  c_per_cta, t, zero_ptr, zero_words));
-  } else if (ks <= 8) {
-    PdlLaunch lc(grid, dim3(kDownWarps * 32), 0, stream, 1, static_cast<unsigned>(ks));
-    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<4, kDownCluster, kDownWarps>, a, ldact, mask, ld_mask, keep_scale, r, scale, M, C,
-                                  c_per_cta, t, zero_ptr, zero_words));
-  } else {
-    NF4LL_CUDA(cudaMemsetAsync(t32, 0, sizeof(float) * 16 * M, stream));
-    count_launch();
-    lora_down_kernel<4, kDownAtomic, kDownWarps><<<grid, kDownWarps * 32, 0, stream>>>(
-        a, ldact, mask, ld_mask, keep_scale, r, scale, M, C, c_per_cta, t, zero_ptr, zero_words);
+  const dim3 grid(static_cast<unsigned>(row_groups), static_cast<unsigned>(ks));
+  if (ks == 1) return down_run<4, kDownDirect, kDownWarps>(grid, 0, a, ldact, br, n, scale, M, C, c_per_cta, zero_ptr, zero_words, stream);
+  if (ks <= 8) {
+    // fewer rows per CTA while the grid stays within two CTAs per SM: more CTAs, each with more of its loads in flight. But not
+    // where the kernel for middling batches streams a long contraction's weights meanwhile: it needs whole SMs, and the fewer
+    // this one holds the better (5120 x 27648 at 64 rows, both kernels: 46 us beside 16 CTAs of 32 rows, 53 behind 64 of 8)
+    const int64_t groups8 = (M + 7) / 8;
+    const unsigned k = static_cast<unsigned>(ks);
+    const bool aside = M > 16 && C > 16384;
+    if (!aside && groups8 * ks * n <= 2 * static_cast<int64_t>(sms))
+      return down_run<1, kDownCluster, kDownWarps>(dim3(static_cast<unsigned>(groups8), k), k, a, ldact, br, n, scale, M, C, c_per_cta, zero_ptr, zero_words, stream);
+    if (!aside && groups16 * ks * n <= 2 * static_cast<int64_t>(sms))
+      return down_run<2, kDownCluster, kDownWarps>(dim3(static_cast<unsigned>(groups16), k), k, a, ldact, br, n, scale, M, C, c_per_cta, zero_ptr, zero_words, stream);
+    return down_run<4, kDownCluster, kDownWarps>(grid, k, a, ldact, br, n, scale, M, C, c_per_cta, zero_ptr, zero_words, stream);
   }
+  for (int i = 0; i < n; ++i) NF4LL_CUDA(cudaMemsetAsync(br[i].t32, 0, sizeof(float) * 16 * M, stream));
+  count_launch();
+  lora_down_kernel<4, kDownAtomic, kDownWarps><<<dim3(grid.x, grid.y, n), kDownWarps * 32, 0, stream>>>(a, ldact, br[0], br[n - 1], scale, M, C,
+                                                                                                    c_per_cta, zero_ptr, zero_words);
   NF4LL_CUDA(cudaGetLastError());
   return NF4LL_OK;
+}
+
+int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_t ld_mask, float keep_scale,
+                     const void* R, float scale, int64_t M, int64_t C, void* t32, int* zero_ptr, int zero_words,
+                     cudaStream_t stream) {
+  const DownBranch one{mask, ld_mask, keep_scale, static_cast<const __half*>(R), static_cast<float*>(t32)};
+  return lora_down_launch(act, ldact, &one, 1, scale, M, C, zero_ptr, zero_words, stream);
 }
 
 // ---------------------------------------------------------------------------------------------
