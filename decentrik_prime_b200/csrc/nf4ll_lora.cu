@@ -301,11 +301,12 @@ int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_
 // Column reduction: out[c][j] (+)= scale * sum_m drop(act)[m][c] * side[m][j]   (j < 16)
 // as out^T[16, C] = side^T[16, M] . drop(act)[M, C]. One CTA = 64 columns x a range of rows, 4
 // warps. The rows arrive in 64-row stages through a ring of shared-memory buffers filled by
-// cp.async (act, mask and side as they lie in memory, two stages always in flight per CTA and
-// several CTAs per SM: the kernel is a pass over act at memory speed). A stage is then prepared in
-// place - dropout applied to the act tile, side transposed and split into fp16 hi + lo parts (two
-// MMAs recover ~22 mantissa bits) - and warp w contracts rows 16w..16w+15 of it against all 64
-// columns (ldmatrix.trans delivers the row-major act tile as the MMA's k-by-n operand). Row ranges
+// cp.async (act, mask and side as they lie in memory, two stages always in flight per CTA and four CTAs per SM: the kernel is
+// a pass over act at memory speed). A warp fetches its own sixteen rows of every stage, applies the dropout to them in place,
+// splits their side values into fp16 hi + lo fragments in registers (two MMAs recover ~22 mantissa bits) and contracts them
+// against all 64 columns (ldmatrix.trans delivers the row-major act tile as the MMA's k-by-n operand), so that the warps of a CTA
+// meet once, at the end: with three block barriers per stage and the side transposed through shared memory 2048 rows of
+// 8960 + 1536 columns took 25 us, LORAGRADNOW now. Row ranges
 // of different CTAs are combined with fp32 atomics, so the summation order across ranges is not fixed.
 // out index = j * ld_j + c * ld_c: dA[16,K] uses (K, 1), dB[N,16] uses (1, 16).
 // ---------------------------------------------------------------------------------------------
@@ -316,10 +317,10 @@ constexpr int kGradRing = 3;
 constexpr int kActStride = 72;     // halves per shared row: 144 B keeps ldmatrix rows on distinct banks
 constexpr int kGradActBytes = kGradStage * kActStride * 2;
 constexpr int kGradMaskBytes = kGradStage * kGradCols;
-constexpr int kGradSideBytes = kGradStage * 16 * 4;
+constexpr int kSideStride = 20;    // floats per shared row of side: a fragment's reads fall on distinct banks
+constexpr int kGradSideBytes = kGradStage * kSideStride * 4;
 constexpr int kGradStageBytes = kGradActBytes + kGradMaskBytes + kGradSideBytes;
-constexpr int kGradHiLoBytes = 2 * 16 * kActStride * 2;
-constexpr int kGradSmemBytes = kGradRing * kGradStageBytes + kGradHiLoBytes;
+constexpr int kGradSmemBytes = kGradRing * kGradStageBytes;
 static_assert(4 * 16 * (kGradCols + 1) * 4 <= kGradRing * kGradStageBytes, "the final reduction reuses the ring");
 
 __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
@@ -371,8 +372,6 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
   if (static_cast<int64_t>(blockIdx.y) * rows_per_cta >= M) return;      // this reduction has fewer row ranges than the other
   extern __shared__ __align__(16) uint8_t g_smem[];
   const uint32_t ring = smem_u32(g_smem);
-  __half (*s_hi)[kActStride] = reinterpret_cast<__half (*)[kActStride]>(g_smem + kGradRing * kGradStageBytes);
-  __half (*s_lo)[kActStride] = s_hi + 16;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int64_t c0 = static_cast<int64_t>(is_first ? blockIdx.x : blockIdx.x - tiles_first) * kGradCols;
@@ -384,13 +383,14 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[n][i] = 0.f;
 
-  // one stage of loads: 64 rows x (128 B of act, 64 B of mask, 64 B of side), one commit group
+  const int kb = warp * 16;        // this warp's sixteen rows of a stage
+  // its part of a stage of loads: 16 rows x (128 B of act, 64 B of mask, 64 B of side), one commit group
   auto issue = [&](int64_t r0, int slot) {
     const uint32_t base = ring + slot * kGradStageBytes;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int idx = threadIdx.x + i * kGradThreads;
-      const int r = idx >> 3, ch = idx & 7;
+      const int idx = lane + i * 32;
+      const int r = kb + (idx >> 3), ch = idx & 7;
       const int64_t row = r0 + r, col = c0 + ch * 8;
       const bool v = row < r_end && col < C;
       cp_async16(base + r * (kActStride * 2) + ch * 16, v ? act + row * ldact + col : act, v);
@@ -398,8 +398,8 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
     if (mask) {
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        const int idx = threadIdx.x + i * kGradThreads;
-        const int r = idx >> 2, ch = idx & 3;
+        const int idx = lane + i * 32;
+        const int r = kb + (idx >> 2), ch = idx & 3;
         const int64_t row = r0 + r, col = c0 + ch * 16;
         const bool v = row < r_end && col < C;
         cp_async16(base + kGradActBytes + r * kGradCols + ch * 16, v ? mask + row * ld_mask + col : mask, v);
@@ -407,12 +407,18 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
     }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
-      const int idx = threadIdx.x + i * kGradThreads;
-      const int r = idx >> 2, ch = idx & 3;
+      const int idx = lane + i * 32;
+      const int r = kb + (idx >> 2), ch = idx & 3;
       const bool v = r0 + r < r_end;
-      cp_async16(base + kGradActBytes + kGradMaskBytes + r * 64 + ch * 16, v ? side + (r0 + r) * 16 + ch * 4 : side, v);
+      cp_async16(base + kGradActBytes + kGradMaskBytes + r * (kSideStride * 4) + ch * 16, v ? side + (r0 + r) * 16 + ch * 4 : side, v);
     }
     cp_async_commit();
+  };
+  // two values of side as fp16 pairs hi + lo
+  auto split = [](float a, float b, uint32_t& hi, uint32_t& lo) {
+    hi = pack_half2_rn(a, b);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+    lo = pack_half2_rn(a - f.x, b - f.y);
   };
 #pragma unroll
   for (int s0 = 0; s0 < kGradRing - 1; ++s0) issue(r_begin + s0 * kGradStage, s0);
@@ -420,40 +426,26 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
   for (int64_t r0 = r_begin; r0 < r_end; r0 += kGradStage, ++it) {
     issue(r0 + (kGradRing - 1) * kGradStage, (it + kGradRing - 1) % kGradRing);   // past the range: empty, zero-filled
     cp_async_wait<kGradRing - 1>();
-    __syncthreads();
+    __syncwarp();
     uint8_t* st = g_smem + (it % kGradRing) * kGradStageBytes;
     if (mask) {
-      // dropout in place: 64 rows x 8 chunks of 8 columns over 128 threads
+      // dropout in place: 16 rows x 8 chunks of 8 columns over the warp
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int idx = threadIdx.x + i * kGradThreads;
-        const int r = idx >> 3, ch = idx & 7;
+        const int idx = lane + i * 32;
+        const int r = kb + (idx >> 3), ch = idx & 7;
         uint4* ap = reinterpret_cast<uint4*>(st + r * (kActStride * 2) + ch * 16);
         const uint2 m = *reinterpret_cast<const uint2*>(st + kGradActBytes + r * kGradCols + ch * 8);
         *ap = drop8(*ap, m, keep_scale);
       }
+      __syncwarp();
     }
-    // side transposed, split into hi + lo: 64 rows x 16 = 1024 values over 128 threads
-    const float* sd = reinterpret_cast<const float*>(st + kGradActBytes + kGradMaskBytes);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int idx = threadIdx.x + i * kGradThreads;
-      const int r = idx >> 4, j = idx & 15;
-      const float v = sd[idx];
-      const __half hi = __float2half_rn(v);
-      s_hi[j][r] = hi;
-      s_lo[j][r] = __float2half_rn(v - __half2float(hi));
-    }
-    __syncthreads();
-    const int kb = warp * 16;      // this warp's 16 rows of the stage
-    const uint32_t ah0 = *reinterpret_cast<const uint32_t*>(&s_hi[g][kb + 2 * t]);
-    const uint32_t ah1 = *reinterpret_cast<const uint32_t*>(&s_hi[g + 8][kb + 2 * t]);
-    const uint32_t ah2 = *reinterpret_cast<const uint32_t*>(&s_hi[g][kb + 2 * t + 8]);
-    const uint32_t ah3 = *reinterpret_cast<const uint32_t*>(&s_hi[g + 8][kb + 2 * t + 8]);
-    const uint32_t al0 = *reinterpret_cast<const uint32_t*>(&s_lo[g][kb + 2 * t]);
-    const uint32_t al1 = *reinterpret_cast<const uint32_t*>(&s_lo[g + 8][kb + 2 * t]);
-    const uint32_t al2 = *reinterpret_cast<const uint32_t*>(&s_lo[g][kb + 2 * t + 8]);
-    const uint32_t al3 = *reinterpret_cast<const uint32_t*>(&s_lo[g + 8][kb + 2 * t + 8]);
+    const float* sd = reinterpret_cast<const float*>(st + kGradActBytes + kGradMaskBytes) + (kb + 2 * t) * kSideStride + g;
+    uint32_t ah0, ah1, ah2, ah3, al0, al1, al2, al3;
+    split(sd[0], sd[kSideStride], ah0, al0);
+    split(sd[8], sd[kSideStride + 8], ah1, al1);
+    split(sd[8 * kSideStride], sd[9 * kSideStride], ah2, al2);
+    split(sd[8 * kSideStride + 8], sd[9 * kSideStride + 8], ah3, al3);
     const uint32_t act_base = ring + (it % kGradRing) * kGradStageBytes;
 #pragma unroll
     for (int np = 0; np < 4; ++np) {     // pairs of 8-column tiles
@@ -467,7 +459,7 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
       mma16816(acc[2 * np + 1], ah0, ah1, ah2, ah3, b2, b3);
       mma16816(acc[2 * np + 1], al0, al1, al2, al3, b2, b3);
     }
-    __syncthreads();
+    __syncwarp();                  // the slot is filled anew by the next trip
   }
   cp_async_wait<0>();
   __syncthreads();
@@ -499,8 +491,8 @@ static GradPlan grad_plan(int64_t M, int64_t C, int64_t sms, int64_t other_tiles
   GradPlan g;
   g.col_tiles = (C + kGradCols - 1) / kGradCols;
   const int64_t stages = (M + kGradStage - 1) / kGradStage;
-  // three CTAs per SM (shared memory): one wave over both reductions of the launch, no tail
-  int64_t msplit = (3 * sms + (g.col_tiles + other_tiles) - 1) / (g.col_tiles + other_tiles);
+  // four CTAs per SM (shared memory): one wave over both reductions of the launch, no tail
+  int64_t msplit = 4 * sms / (g.col_tiles + other_tiles);
   if (msplit > stages) msplit = stages;
   if (msplit < 1) msplit = 1;
   g.rows_per = (stages + msplit - 1) / msplit * kGradStage;
