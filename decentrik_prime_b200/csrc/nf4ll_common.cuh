@@ -145,7 +145,7 @@ __device__ __forceinline__ uint4 decode_word(const BlockTable& t, uint32_t w) {
 // has completed and its writes are visible, and must come before the first access to global
 // memory. Three kernels read earlier, all of them behind a kernel of the same call that has itself waited before it let
 // them start, so that only what that kernel writes is not there yet: the streaming kernel behind a rank-16 projection and
-// the swapped-operand kernel (x, weights, tables), the dense GEMM behind the dequantisation pass (activations, mask).
+// the kernel for middling batches (activations, weights, mask, tables), the dense GEMM behind the dequantisation pass (activations, mask).
 // pdl_launch_dependents() lets the NEXT kernel's blocks start as soon as every block of this
 // one has called it (or exited). Both are no-ops for an ordinary launch.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -306,7 +306,7 @@ int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_
 // splits their side values into fp16 hi + lo fragments in registers (two MMAs recover ~22 mantissa bits) and contracts them
 // against all 64 columns (ldmatrix.trans delivers the row-major act tile as the MMA's k-by-n operand), so that the warps of a CTA
 // meet once, at the end: with three block barriers per stage and the side transposed through shared memory 2048 rows of
-// 8960 + 1536 columns took 25 us, LORAGRADNOW now. Row ranges
+// 8960 + 1536 columns took 25 us, 20.5 now. Row ranges
 // of different CTAs are combined with fp32 atomics, so the summation order across ranges is not fixed.
 // out index = j * ld_j + c * ld_c: dA[16,K] uses (K, 1), dB[N,16] uses (1, 16).
 // ---------------------------------------------------------------------------------------------
