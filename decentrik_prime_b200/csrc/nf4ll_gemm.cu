@@ -1424,7 +1424,7 @@ static int run_dense(const DenseCall& c, const DensePlan& d, int sms, const Dens
 }
 
 // Whether a call runs on the kernel for middling batches (nf4ll_mid.cu)
-constexpr int64_t kMidMostRows = 1024;
+constexpr int64_t kMidMostRows = 2560;      // beyond, the dense GEMM or the tiles without asking
 static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int sms, const Tune& tune, MidPlan* mp) {
   if (g_expire_polls != 0 || g_mid.on < 0) return false;
   const int64_t N = c.W->N, K = c.W->K, NO = c.mode == kFwd ? N : K, KC = c.mode == kFwd ? K : N;
@@ -1449,7 +1449,10 @@ static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int 
   // the model's margin: it knows nothing of clocks that fall under load. At the same work per launch it is 3 % low for 25 GFLOP
   // and 20 % for 250 (backward of 27648 x 5120 at 951 rows: 288 us, where the tiles take 250).
   const double work = 2e-9 * static_cast<double>(c.M) * static_cast<double>(N) * static_cast<double>(K);
-  const double us = mp->us * (1.05 + 0.15 * (work < 250 ? work / 250 : 1.0));
+  // Beyond the rows that it was fitted to, a wider one still: without, 1536 x 8960 backward at 2048 rows took 63 us for 50,
+  // 5120 x 5120 backward 109 for 103; with it 1536 x 1536 at 2048 rows still goes from 24.5 to 14.3 us, 3584 x 3584 at 1100 from 41 to 29.
+  const double beyond = c.M <= 1024 ? 1.0 : c.mode == kFwd ? 1.15 : 1.29;
+  const double us = mp->us * (1.05 + 0.15 * (work < 250 ? work / 250 : 1.0)) * beyond;
   return us < t.decoding && us < t.dense;
 }
 
