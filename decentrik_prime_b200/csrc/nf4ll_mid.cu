@@ -1,4 +1,4 @@
-// Middling batches (17 to some hundreds of token rows), forward and backward-dX: the WEIGHTS are the 128-row operand of
+// Middling batches (17 to some hundreds of token rows, 2560 against small weights), forward and backward-dX: the WEIGHTS are the 128-row operand of
 // tcgen05.mma, the tokens its N operand (any multiple of 16 up to 256 columns), the contraction is cut over the CTAs of a
 // thread-block cluster. Serves the reference call sites solution/fast_qwen.py:947, 1037, 1080-1112 and, backward, 1310-1364.
 //
