@@ -52,6 +52,12 @@ constexpr int kMidMaxCodes = 8;
 constexpr int kMidLutBytes = 256 * 128;
 constexpr int kMidTurnRow = 32 * 4 + 16, kMidTurnBytes = 8 * kMidTurnRow;      // eight tokens of a warp's 32 columns, fp32, padded
 constexpr int kMidSmem = 227 * 1024;
+// Forward, up to so many rows: the rank-16 product keeps its 32 bits, as in the streaming kernel: two fp16 parts of it are
+// multiplied (22 bits), and values that fp16 cannot hold are added in fp32. Longer batches round it to fp16 like the tile kernels and the dense GEMM.
+// Where the branch is most of the output, rel-L2 against fp64 of 5120 x 27648 / 27648 x 5120 at 64 rows 2.6e-4 / 2.9e-4
+// rounded, 2.07e-4 / 2.08e-4 in two parts, which is the output's own rounding. Time with LoRA, rounded / in two parts: 5120 x 27648 at 64 rows
+// 47.0 / 47.2 us, 27648 x 5120 at 64 rows 43.0 / 43.7, gate|up of it at 24 rows 44.4 / 44.6, 1536 x 1536 at 24 rows 9.3 / 9.5.
+constexpr int64_t kMidSplitRows = 64;
 
 struct MidParams {
   const uint8_t* qabs;
@@ -63,6 +69,7 @@ struct MidParams {
   int ts;                          // token columns that a CTA of the cluster finishes
   int off_a, off_x, off_lora, off_xch, off_lut, off_turn, off_misc;      // shared memory
   int early, qabs_mode, x_alias, any_lora;
+  int split;                       // forward: the tokens' side of the rank-16 operands in two fp16 parts
   __half* out;
   int64_t ldo;
   const __half* bias;
@@ -116,6 +123,13 @@ __device__ __forceinline__ void mid_tmem_ld8(uint32_t taddr, float (&f)[8]) {
   tmem_ld_wait();
 #pragma unroll
   for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(v[j]);
+}
+__device__ __forceinline__ void mid_tmem_add(uint32_t taddr, float d) {      // one column
+  uint32_t v;
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x1.b32 {%0}, [%1];" : "=r"(v) : "r"(taddr) : "memory");
+  tmem_ld_wait();
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x1.b32 [%0], {%1};" ::"r"(taddr), "r"(__float_as_uint(__uint_as_float(v) + d)) : "memory");
+  tmem_st_wait();
 }
 __device__ __forceinline__ void mid_st_cluster(uint32_t addr, float a, float b, float c, float d) {
   asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
@@ -179,7 +193,9 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   uint64_t* xch_free = xch_full + 1;             // the other CTAs are ready for this CTA's partial sums
   uint64_t* drain = xch_free + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  static_assert((1024 + 64 + 8 * (2 * kMidBars + 2 * kMidMaxCodes + 9) + 8) % 16 == 0, "the words of `wide` are read sixteen bytes at a time");
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  uint32_t* wide = tmem_slot + 2;                // [2 units in turn][RB][4]: tokens beyond fp16's range, sixteen to a word, bits 0, 2, 4, ... (16-byte aligned)
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const Abort ab{abort_flag, p.status};
@@ -348,6 +364,8 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             const uint64_t tdesc = make_smem_desc(sL + RB * 4096 + rb * p.nt * 32, 128, 256, kSwizzleNone);
             if (MODE == kBwd && p.mask) tc_mma_f16(tmem_base + l_col + rb * p.nt, wdesc, tdesc, idesc, 0u);
             else tc_mma_f16(d0 + rb * p.nt, wdesc, tdesc, idesc, 1u);
+            if (MODE == kFwd && p.split)
+              tc_mma_f16(d0 + rb * p.nt, wdesc, make_smem_desc(sCode + p.off_turn + rb * 256, 128, kMidTurnBytes / 2, kSwizzleNone), idesc, 1u);
           }
           tc_commit(smem_u32(l_empty));
         }
@@ -526,17 +544,40 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
               }
               sts128(sL + rb * 4096 + at, v);
             }
-            // tokens' side, scaled and rounded to fp16
-            for (int c = tid; c < 2 * p.nt; c += 128) {
-              const int row = c >> 1, h = c & 1;
-              uint4 v = make_uint4(0, 0, 0, 0);
-              if (left && row < vt) {
-                const float4* src = reinterpret_cast<const float4*>(left + static_cast<int64_t>(t0 + row) * 16 + h * 8);
-                const float4 a = __ldcg(src), b = __ldcg(src + 1);       // the kernel before this one wrote them
-                v = make_uint4(pack_half2_rn(a.x * sc, a.y * sc), pack_half2_rn(a.z * sc, a.w * sc), pack_half2_rn(b.x * sc, b.y * sc),
-                               pack_half2_rn(b.z * sc, b.w * sc));
+            // tokens' side, scaled and rounded to fp16; or in two parts, fp16 each, a token with values beyond fp16's range
+            // left out here, its bit set, and added in fp32 by the epilogue
+            auto side = [&](int row, int h, float (&v)[8]) {
+              const float4* src = reinterpret_cast<const float4*>(left + static_cast<int64_t>(t0 + row) * 16 + h * 8);
+              const bool there = left && row < vt;
+              const float4 a = there ? __ldcg(src) : make_float4(0.f, 0.f, 0.f, 0.f), b = there ? __ldcg(src + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+              v[0] = a.x * sc; v[1] = a.y * sc; v[2] = a.z * sc; v[3] = a.w * sc;      // the kernel before this one wrote them
+              v[4] = b.x * sc; v[5] = b.y * sc; v[6] = b.z * sc; v[7] = b.w * sc;
+            };
+            const uint32_t sT = sL + RB * 4096 + rb * p.nt * 32;
+            if (MODE == kFwd && p.split) {
+              const int row = tid >> 1, h = tid & 1;               // 64 tokens at most; two lanes hold the halves of a token's rank
+              float v[8], r[8];
+              side(row, h, v);
+              uint4 hi = pack8(v);
+              auto off = [](uint32_t w) { return ((w & 0x7c007c00u) + 0x04000400u) & 0x80008000u; };      // an infinity or NaN of the two
+              const uint32_t out = __ballot_sync(0xffffffffu, (off(hi.x) | off(hi.y) | off(hi.z) | off(hi.w)) != 0);
+              const uint32_t pair = (out | (out >> 1)) & 0x55555555u;
+              if (lane == 0) wide[((ul & 1) * RB + rb) * 4 + q] = pair;
+              unpack8(hi, r);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) r[j] = v[j] - r[j];
+              uint4 lo = pack8(r);
+              if ((pair >> (lane & 30)) & 1) hi = lo = make_uint4(0, 0, 0, 0);
+              // the low parts lie in the warps' scratch (this warp's sixteen tokens in its own), idle until the unit's epilogue
+              sts128(sCode + p.off_turn + (row >> 3) * (kMidTurnBytes / 2) + rb * 256 + h * 128 + (row & 7) * 16, lo);
+              if (row < p.nt) sts128(sT + (row >> 3) * 256 + h * 128 + (row & 7) * 16, hi);
+            } else {
+              for (int c = tid; c < 2 * p.nt; c += 128) {
+                const int row = c >> 1, h = c & 1;
+                float v[8];
+                side(row, h, v);
+                sts128(sT + (row >> 3) * 256 + h * 128 + (row & 7) * 16, pack8(v));
               }
-              sts128(sL + RB * 4096 + rb * p.nt * 32 + (row >> 3) * 256 + h * 128 + (row & 7) * 16, v);
             }
           }
           fence_proxy_async_smem();
@@ -545,7 +586,38 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         }
       }
       const int buf = p.nbuf == 2 ? ul & 1 : 0;
+      const bool split = MODE == kFwd && p.split && p.any_lora && crank == 0 && crew == 0;
+      if (split && ok) ok = wait_or_abort(smem_u32(l_full), ul & 1, ab, 0x070d);      // the other warps' bits are there
       if (crew == 0 && ok) ok = wait_or_abort(smem_u32(acc_full + buf), (p.nbuf == 2 ? ul >> 1 : ul) & 1, ab, 0x070a);
+      if (split && ok) {
+        // rank-16 terms of tokens beyond fp16's range: added to their columns of the accumulator in fp32
+        uint32_t any = 0;
+#pragma unroll
+        for (int rb = 0; rb < RB; ++rb) {
+          const uint4 w = lds128(smem_u32(wide + ((ul & 1) * RB + rb) * 4));
+          any |= w.x | w.y | w.z | w.w;
+        }
+        tc_fence_after();
+#pragma unroll 1
+        for (int i = 0; any && i < RB * 4; ++i) {
+          const int rb = i >> 2, tg = (i & 3) * 16;
+          uint32_t bits = wide[(ul & 1) * RB * 4 + i];
+          const int n = row0_of(u, rb) + r;
+          int sg = 0;
+          while (sg + 1 < p.n_seg && n - r >= p.seg_end[sg]) ++sg;
+          for (; bits; bits &= bits - 1) {
+            const int t = tg + ((__ffs(bits) - 1) >> 1);
+            const uint32_t at = tmem_base + (static_cast<uint32_t>(q * 32) << 16) + buf * d_cols + rb * p.nt + t;
+            const float* left = p.seg_left[sg] + static_cast<int64_t>(t0 + t) * 16;
+            float l = 0.f;
+            if (n < p.seg_end[sg])
+              for (int k = 0; k < 16; ++k) l = fmaf(__ldcg(left + k), __half2float(p.seg_right[sg][static_cast<int64_t>(n) * 16 + k]) * p.seg_scale[sg], l);
+            __syncwarp();
+            mid_tmem_add(at, l);
+          }
+        }
+        tc_fence_before();
+      }
       if (crews > 1) {
         // the decoding warps have met none of the earlier phases of the barriers below: they go on behind the first crew
         named_barrier(2, 128 * (1 + kMidTeams));
@@ -791,7 +863,7 @@ static MidLayout mid_layout(int mode, const MidPlan& p, bool lora) {
   l.off_turn = at;
   at += 4 * kMidTurnBytes;
   l.off_misc = at;
-  at += 1024 + 64 + 8 * (2 * kMidBars + 2 * kMidMaxCodes + 16) + 16;
+  at += 1024 + 64 + 8 * (2 * kMidBars + 2 * kMidMaxCodes + 16) + 16 + 2 * 2 * 4 * 4;
   l.total = at + 1024;                          // the base is rounded up to 1024
   if (p.x_alias && xch + 4 * kMidTeams * kMidTurnBytes > ring) l.total = kMidSmem + 1;
   return l;
@@ -853,6 +925,7 @@ static bool mid_search(int mode, int64_t M, int64_t NO, int64_t KC, bool mask, i
         if (most <= 0) continue;
         MidPlan p{};
         p.rb = rb; p.nt = nt; p.cl = cl;
+        p.split = mode == kFwd && M <= kMidSplitRows && nt <= kMidSplitRows;
         p.tiles_o = static_cast<int>(tiles_o); p.tiles_t = static_cast<int>(tt); p.units = static_cast<int>(units);
         const int64_t rounds = (units + most - 1) / most;
         p.clusters = static_cast<int>((units + rounds - 1) / rounds);
@@ -914,6 +987,7 @@ int mid_launch(const MidCall& c, const MidPlan& pl, bool early, int32_t* status,
   p.nt = pl.nt; p.cl = pl.cl; p.tiles_t = pl.tiles_t; p.units = pl.units; p.nbuf = pl.nbuf; p.na = pl.na; p.nx = pl.nx; p.nc = pl.nc;
   p.nc_log = pl.nc == 8 ? 3 : pl.nc == 4 ? 2 : 1;
   p.ts = (pl.nt / 8 + pl.cl - 1) / pl.cl * 8;
+  p.split = pl.split ? 1 : 0;
   p.n_seg = c.n_seg;
   for (int i = 0; i < c.n_seg; ++i) {
     p.seg_end[i] = static_cast<int>(c.seg_end[i]);

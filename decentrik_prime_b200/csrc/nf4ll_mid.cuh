@@ -36,6 +36,7 @@ struct MidPlan {
   int clusters;                // launched; units / clusters rounded up = units one after another in a cluster
   int nbuf, na, nx, nc;        // accumulators, slots of decoded weights, slots of token tiles, slots of codes
   bool x_alias;                // the exchange of partial sums reuses the operand rings
+  bool split;                  // forward: the rank-16 product as two fp16 parts
   double us;                   // expected time
 };
 

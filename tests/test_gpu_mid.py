@@ -140,3 +140,36 @@ def test_values_that_are_not_finite_stay_in_their_rows():
     assert torch.equal(y[keep], clean[keep])
     assert not torch.isfinite(y[[7, 9]]).any()
     linear.check_status()
+
+
+@pytest.mark.parametrize("M,rb,nt,cl", [(1, 1, 16, 1), (9, 2, 16, 2), (17, 1, 32, 3), (33, 2, 48, 1), (40, 1, 16, 1), (64, 1, 64, 4), (64, 2, 64, 2)])
+def test_short_batches_keep_the_rank16_product_in_32_bits(M, rb, nt, cl):
+    """Up to 64 rows, with a branch that is nearly all of the output. In two fp16 parts the product is off by 2^-22, and so little
+    moves a result to its other neighbour in fp16 (steps of 2^-11 to 2^-10) with a probability of some 2^-11 per term; the fp32
+    sums' own error (about 2^-22 of a result) as much: 1 % allowed. A product rounded to fp16 (2^-12) moves two fifths of them.
+    A token whose scaled product fp16 cannot hold is finite and as close to fp64 as any; one that is not finite stays alone."""
+    N, K = 640, 1024                              # four groups of 256: as many CTAs in a cluster at most
+    pr = make_problem(N, K, M, seed=M + nt, lora=False, w_std=1e-3)
+    w = oracle_weight(pr).double()
+    g = torch.Generator().manual_seed(nt)
+    A, B = (torch.randn(16, K, generator=g) / K ** 0.5).half(), torch.randn(N, 16, generator=g).half()
+    d = to_device(pr)
+
+    def check(x, B, scale, rows):
+        with mid(rb, nt, cl):
+            y, _ = linear.forward(d.w, x.cuda(), lora=(A.cuda(), B.cuda(), scale))
+            multi, _ = linear.forward_multi(d.w, x.cuda(), [(256, None, None, 1.0), (384, (A.cuda(), B[:384].contiguous().cuda(), scale), None, 1.0)])
+        linear.check_status()
+        ref = x.double() @ w.t() + scale * (x.double() @ A.double().t()) @ B.double().t()
+        assert (y.cpu()[rows] != ref.half()[rows]).sum() <= 0.01 * N * len(rows)
+        ref2 = x.double() @ w[256:].t() + scale * (x.double() @ A.double().t()) @ B[:384].double().t()
+        assert (multi.cpu()[rows, 256:] != ref2.half()[rows]).sum() <= 0.01 * 384 * len(rows)
+        return y.cpu()
+    every = list(range(M))
+    check(pr.x, B, 2.0, every)
+    x = pr.x.clone()
+    x[M // 2] = (x[M // 2].float() * 2.0 ** 12).half()                # its product, times the scale: 2^17 and more
+    check(x, (B.float() * 2.0 ** -12).half(), 48.0, every)
+    x[M - 1, 5] = float("inf")
+    y = check(x, (B.float() * 2.0 ** -12).half(), 48.0, every[:-1])
+    assert not torch.isfinite(y[-1]).all()
