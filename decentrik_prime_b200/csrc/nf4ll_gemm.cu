@@ -1038,6 +1038,7 @@ struct Plan {
 
 // Tile shape / split count forced by a test (zeros: the built-in heuristic). flags bit 0: never use the
 // cooperative (shared) split reduction.
+constexpr int kFlagNoCoop = 1, kFlagNoDense = 8;
 struct Tune {
   int bm = 0, bn = 0, splits = 0, flags = 0;
   bool any() const { return bm || bn || splits; }
@@ -1434,7 +1435,7 @@ static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int 
     if (cl > (K + 255) / 256) cl = (K + 255) / 256;
     return mid_plan(kFwd, c.M, NO, KC, false, 0, lora, 0, 0, static_cast<int>(cl), mp);
   }
-  if (tune.any() || tune.flags) return false;
+  if (tune.any() || (tune.flags & ~(kFlagNoCoop | kFlagNoDense))) return false;      // those two say nothing about this kernel
   if (g_mid.on > 0) return mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, g_mid.rb, g_mid.nt, g_mid.cl, mp);
   if (c.M > kMidMostRows) return false;
   if (c.mode == kFwd && c.M <= kStreamMaxRows) {
@@ -1453,7 +1454,7 @@ static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int 
   // 5120 x 5120 backward 109 for 103; with it 1536 x 1536 at 2048 rows still goes from 24.5 to 14.3 us, 3584 x 3584 at 1100 from 41 to 29.
   const double beyond = c.M <= 1024 ? 1.0 : c.mode == kFwd ? 1.15 : 1.29;
   const double us = mp->us * (1.05 + 0.15 * (work < 250 ? work / 250 : 1.0)) * beyond;
-  return us < t.decoding && us < t.dense;
+  return us < t.decoding && (tune.flags || us < t.dense);      // under a flag the dense GEMM is not open to these batches
 }
 
 // Scratch: the rank-16 product where the caller keeps none, lora_B transposed (backward).

@@ -173,3 +173,20 @@ def test_short_batches_keep_the_rank16_product_in_32_bits(M, rb, nt, cl):
     x[M - 1, 5] = float("inf")
     y = check(x, (B.float() * 2.0 ** -12).half(), 48.0, every[:-1])
     assert not torch.isfinite(y[-1]).all()
+
+
+@pytest.mark.parametrize("N,K,M", [(1536, 1536, 24), (4096, 4096, 64), (8960, 1536, 187)])
+@pytest.mark.parametrize("flags", [1, 8, 9])
+def test_flags_about_other_kernels_do_not_keep_it_out(N, K, M, flags):
+    """Bit 0 (no cooperative reduction) and bit 3 (no dequantisation): the same kernel as without them, bit for bit."""
+    d = to_device(make_problem(N, K, M, seed=M, lora=True, dropout=0.05, bias=True))
+
+    def both():
+        return (linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0],
+                linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0])
+    default = both()
+    with mid():
+        assert all(torch.equal(a, b) for a, b in zip(default, both()))
+    with linear.tune_override(flags=flags):
+        assert all(torch.equal(a, b) for a, b in zip(default, both()))
+    linear.check_status()
