@@ -1038,7 +1038,7 @@ struct Plan {
 
 // Tile shape / split count forced by a test (zeros: the built-in heuristic). flags bit 0: never use the
 // cooperative (shared) split reduction.
-constexpr int kFlagNoCoop = 1, kFlagNoDense = 8;
+constexpr int kFlagNoCoop = 1, kFlagNoDense = 8, kFlagDense = 16;
 struct Tune {
   int bm = 0, bn = 0, splits = 0, flags = 0;
   bool any() const { return bm || bn || splits; }
@@ -1321,12 +1321,6 @@ static DenseScratch dense_scratch(int64_t M, int64_t N, int64_t K, bool keep_lef
   return s;
 }
 
-// Whether a call runs on the dense path, given a workspace that holds the fp16 weight.
-static bool dense_wanted(int mode, int64_t M, int64_t NO, int64_t KC, int64_t gu_inter, bool narrow, bool lora, int sms, const Tune& tune) {
-  if (tune.any() || (tune.flags & 8) || g_expire_polls != 0) return false;
-  return (tune.flags & 16) || ((!tune.flags || M >= kDenseHostRows) && dense_pays(mode, M, NO, KC, gu_inter, narrow, lora, sms));
-}
-
 struct DenseCall {
   int mode;
   const nf4ll_mat* W;
@@ -1361,7 +1355,16 @@ static DenseScratch dense_call_scratch(const DenseCall& c) {
   return dense_scratch(c.M, c.W->N, c.W->K, one && !c.side[0], c.mode == kBwd && one && !c.lora[0]->Bt, dense_branches(c));
 }
 
-static int run_dense(const DenseCall& c, const DensePlan& d, int sms, const DenseScratch& sc, uint8_t* ws, int32_t* status, cudaStream_t stream) {
+// Whether the dense path is open to a call: the hooks allow it and the workspace holds the fp16 weight.
+static bool dense_open(const DenseCall& c, const Tune& tune, const void* workspace, int64_t workspace_bytes) {
+  if (tune.any() || (tune.flags & kFlagNoDense) || g_expire_polls != 0) return false;
+  if (!(tune.flags & kFlagDense) && (c.M <= kDenseNeverRows || (tune.flags && c.M < kDenseHostRows))) return false;
+  return workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255) && workspace_bytes >= dense_call_scratch(c).total;
+}
+
+static int run_dense(const DenseCall& c, int sms, uint8_t* ws, int32_t* status, cudaStream_t stream) {
+  const DensePlan d = dense_call_plan(c, sms);
+  const DenseScratch sc = dense_call_scratch(c);
   const nf4ll_mat* W = c.W;
   const bool fwd = c.mode == kFwd;
   const int64_t NO = fwd ? W->N : W->K, KC = fwd ? W->K : W->N;
@@ -1426,7 +1429,8 @@ static int run_dense(const DenseCall& c, const DensePlan& d, int sms, const Dens
 
 // Whether a call runs on the kernel for middling batches (nf4ll_mid.cu)
 constexpr int64_t kMidMostRows = 2560;      // beyond, the dense GEMM or the tiles without asking
-static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int sms, const Tune& tune, MidPlan* mp) {
+// `t`: the times of the other ways beyond kDenseNeverRows rows; `dense`: the dense GEMM is one of them
+static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lora, bool mask, int sms, const Tune& tune, MidPlan* mp) {
   if (g_expire_polls != 0 || g_mid.on < 0) return false;
   const int64_t N = c.W->N, K = c.W->K, NO = c.mode == kFwd ? N : K, KC = c.mode == kFwd ? K : N;
   if (N * (K / 64) >= (int64_t(1) << 31) || c.M >= (1 << 24)) return false;      // the kernel's indices have 32 bits
@@ -1446,7 +1450,6 @@ static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int 
   }
   if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
   if (c.M <= kDenseNeverRows) return true;
-  const RowTimes t = row_times(c.mode, c.M, NO, KC, c.gu_inter, narrow, lora, sms);
   // the model's margin: it knows nothing of clocks that fall under load. At the same work per launch it is 3 % low for 25 GFLOP
   // and 20 % for 250 (backward of 27648 x 5120 at 951 rows: 288 us, where the tiles take 250).
   const double work = 2e-9 * static_cast<double>(c.M) * static_cast<double>(N) * static_cast<double>(K);
@@ -1454,7 +1457,7 @@ static bool mid_wanted(const MidCall& c, bool narrow, bool lora, bool mask, int 
   // 5120 x 5120 backward 109 for 103; with it 1536 x 1536 at 2048 rows still goes from 24.5 to 14.3 us, 3584 x 3584 at 1100 from 41 to 29.
   const double beyond = c.M <= 1024 ? 1.0 : c.mode == kFwd ? 1.15 : 1.29;
   const double us = mp->us * (1.05 + 0.15 * (work < 250 ? work / 250 : 1.0)) * beyond;
-  return us < t.decoding && (tune.flags || us < t.dense);      // under a flag the dense GEMM is not open to these batches
+  return us < t.decoding && !(dense && us >= t.dense);
 }
 
 // Scratch: the rank-16 product where the caller keeps none, lora_B transposed (backward).
@@ -1550,36 +1553,27 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     MidCall c{};
     c.mode = mode; c.W = W; c.act = act; c.ldact = ldact; c.M = M; c.bias = bias; c.out = out; c.ldo = ldo; c.accumulate = accumulate;
     c.n_seg = segments ? n_segments : 1;
-    const nf4ll_lora* br[kMaxSegments] = {lora};
-    void* side[kMaxSegments] = {side_out};
-    bool ready[kMaxSegments] = {};
+    DenseCall dc{};
+    dc.mode = mode; dc.W = W; dc.act = act; dc.ldact = ldact; dc.bias = bias; dc.M = M; dc.out = out; dc.ldo = ldo; dc.accumulate = accumulate;
+    dc.stacked = segments != nullptr;
+    dc.n_branch = c.n_seg;
     int64_t at = 0;
     for (int i = 0; i < c.n_seg; ++i) {
-      if (segments) { br[i] = segments[i].lora; side[i] = segments[i].t_out; ready[i] = segments[i].t_ready != 0; }
+      dc.lora[i] = segments ? segments[i].lora : lora;
+      dc.side[i] = segments ? segments[i].t_out : side_out;
+      dc.side_ready[i] = segments && segments[i].t_ready != 0;
+      dc.begin[i] = at;
+      dc.rows[i] = segments ? segments[i].rows : NO;
       at += segments ? segments[i].rows : W->N;
       c.seg_end[i] = at;
     }
+    const bool dense = dense_open(dc, tune, workspace, workspace_bytes);
+    RowTimes t{};
+    if (M > kDenseNeverRows && (dense || M <= kMidMostRows)) t = row_times(mode, M, NO, KC, 0, narrow_tiles, any_lora, sms);
     MidPlan mp;
-    if (mid_wanted(c, narrow_tiles, any_lora, lora && lora->mask, sms, tune, &mp)) return run_mid(c, mp, br, side, ready, workspace, workspace_bytes, status, stream, who);
-  }
-  if (dense_wanted(mode, M, NO, KC, 0, narrow_tiles, any_lora, sms, tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
-    DenseCall c{};
-    c.mode = mode; c.W = W; c.act = act; c.ldact = ldact; c.bias = bias; c.M = M; c.out = out; c.ldo = ldo; c.accumulate = accumulate;
-    c.stacked = segments != nullptr;
-    c.n_branch = segments ? n_segments : 1;
-    if (segments) {
-      int64_t at = 0;
-      for (int i = 0; i < n_segments; ++i) {
-        c.begin[i] = at; c.rows[i] = segments[i].rows; c.lora[i] = segments[i].lora;
-        c.side[i] = segments[i].t_out; c.side_ready[i] = segments[i].t_ready != 0;
-        at += segments[i].rows;
-      }
-    } else {
-      c.rows[0] = NO; c.lora[0] = lora; c.side[0] = side_out;
-    }
-    const DensePlan d = dense_call_plan(c, sms);
-    const DenseScratch sc = dense_call_scratch(c);
-    if (workspace_bytes >= sc.total) return run_dense(c, d, sms, sc, static_cast<uint8_t*>(workspace), status, stream);
+    if (mid_wanted(c, t, dense, any_lora, lora && lora->mask, sms, tune, &mp))
+      return run_mid(c, mp, dc.lora, dc.side, dc.side_ready, workspace, workspace_bytes, status, stream, who);
+    if (dense && ((tune.flags & kFlagDense) || t.dense < t.decoding)) return run_dense(dc, sms, static_cast<uint8_t*>(workspace), status, stream);
   }
   if (segments && (narrow_tiles || tune.bn == 512)) tune.bn = narrow_tiles ? 128 : 256;
   Plan pl = make_plan(mode, M, NO, KC, lora ? lora->r : 0, sms, tune);
@@ -1748,24 +1742,30 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
   if (int rc = check_product(lora_gate ? t_gate : nullptr, who)) return rc;
   if (int rc = check_product(lora_up ? t_up : nullptr, who)) return rc;
   if (int rc = require_sm100()) return rc;
+  int sms = 148;
+  if (int rc = device_sms(&sms)) return rc;
+  const bool odd = M <= 128 || I % 128 || g_tune.any();      // left to the two projections on their own by the kernels of large batches
   {
-    int sms = 148;
-    if (int rc = device_sms(&sms)) return rc;
     MidCall c{};
     c.mode = kFwd; c.W = W; c.act = x; c.ldact = ldx; c.M = M; c.out = g; c.ldo = ldg;
     c.out_u = u; c.ldu = ldu; c.out_h = h; c.ldh = ldh; c.gu_inter = I;
     c.n_seg = 2;
     c.seg_end[0] = I; c.seg_end[1] = W->N;
-    const nf4ll_lora* br[kMaxSegments] = {lora_gate, lora_up};
-    void* tout[kMaxSegments] = {t_gate, t_up};
-    const bool ready[kMaxSegments] = {};
+    DenseCall dc{};
+    dc.mode = kFwd; dc.W = W; dc.act = x; dc.ldact = ldx; dc.M = M; dc.out = g; dc.ldo = ldg;
+    dc.out_u = u; dc.ldu = ldu; dc.out_h = h; dc.ldh = ldh; dc.gu_inter = I; dc.n_branch = 2;
+    dc.rows[0] = dc.rows[1] = I; dc.begin[1] = I;
+    dc.lora[0] = lora_gate; dc.lora[1] = lora_up; dc.side[0] = t_gate; dc.side[1] = t_up;
+    const bool dense = dense_open(dc, g_tune, workspace, workspace_bytes);
+    RowTimes t{};
+    if (M > kDenseNeverRows && (dense || M <= kMidMostRows)) t = row_times(kFwd, M, W->N, W->K, I, false, lora_gate || lora_up, sms);
     MidPlan mp;
-    if (mid_wanted(c, false, lora_gate || lora_up, false, sms, g_tune, &mp)) return run_mid(c, mp, br, tout, ready, workspace, workspace_bytes, status, stream, who);
+    if (mid_wanted(c, t, dense, lora_gate || lora_up, false, sms, g_tune, &mp))
+      return run_mid(c, mp, dc.lora, dc.side, dc.side_ready, workspace, workspace_bytes, status, stream, who);
+    if (!odd && dense && ((g_tune.flags & kFlagDense) || t.dense < t.decoding)) return run_dense(dc, sms, static_cast<uint8_t*>(workspace), status, stream);
   }
-  if (M <= 128 || I % 128 || g_tune.any()) {
+  if (odd) {
     // short batches and odd widths: the two projections on their own, then the stand-alone gated product
-    int sms = 148;
-    if (int rc = device_sms(&sms)) return rc;
     int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, false, g_tune);
     if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;
     if (kind != kTiles) {
@@ -1797,18 +1797,6 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     if (int rc = run_gemm(kFwd, &wg, x, ldx, nullptr, lora_gate, t_gate, M, g, ldg, 0, workspace, workspace_bytes, status, stream_v)) return rc;
     if (int rc = run_gemm(kFwd, &wu, x, ldx, nullptr, lora_up, t_up, M, u, ldu, 0, workspace, workspace_bytes, status, stream_v)) return rc;
     return nf4ll_swiglu_forward(g, ldg, u, ldu, h, ldh, M, I, stream_v);
-  }
-  int sms = 148;
-  if (int rc = device_sms(&sms)) return rc;
-  if (dense_wanted(kFwd, M, W->N, W->K, I, false, lora_gate || lora_up, sms, g_tune) && workspace && !(reinterpret_cast<uintptr_t>(workspace) & 255)) {
-    DenseCall c{};
-    c.mode = kFwd; c.W = W; c.act = x; c.ldact = ldx; c.M = M; c.out = g; c.ldo = ldg;
-    c.out_u = u; c.ldu = ldu; c.out_h = h; c.ldh = ldh; c.gu_inter = I; c.n_branch = 2;
-    c.rows[0] = c.rows[1] = I; c.begin[1] = I;
-    c.lora[0] = lora_gate; c.lora[1] = lora_up; c.side[0] = t_gate; c.side[1] = t_up;
-    const DensePlan d = dense_call_plan(c, sms);
-    const DenseScratch sc = dense_call_scratch(c);
-    if (workspace_bytes >= sc.total) return run_dense(c, d, sms, sc, static_cast<uint8_t*>(workspace), status, stream);
   }
   GemmParams p{};
   p.nib = W->nib; p.qabs = W->qabs; p.scale2 = W->scale2; p.offset2 = W->offset2; p.code2 = W->code2;

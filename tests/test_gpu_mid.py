@@ -190,3 +190,26 @@ def test_flags_about_other_kernels_do_not_keep_it_out(N, K, M, flags):
     with linear.tune_override(flags=flags):
         assert all(torch.equal(a, b) for a, b in zip(default, both()))
     linear.check_status()
+
+
+@pytest.mark.parametrize("N,K,M,backward", [(5120, 5120, 2300, False), (5120, 5120, 1800, True)])
+def test_it_takes_what_the_dense_gemm_would_where_the_workspace_is_too_small(N, K, M, backward):
+    """Calls for which the models put the dense GEMM first and this kernel second: with the least workspace, this one. The order
+    of the sums, the rank-16 branch's place in it included, tells the three ways apart."""
+    h = _lib.lib()
+    d = to_device(make_problem(N, K, M, seed=1, lora=True, dropout=0.0, device="cuda"))
+    sizes = [h.nf4ll_workspace_bytes(M, N, K, 16), h.nf4ll_workspace_bytes_fast(M, N, K, 16)]
+    assert sizes[0] < 2 * N * K <= sizes[1]
+    least, fast = (torch.empty(n, dtype=torch.uint8, device="cuda") for n in sizes)
+
+    def run(ws):
+        return (linear.backward_dx(d.w, d.dy, lora=d.lora, workspace=ws) if backward else linear.forward(d.w, d.x, lora=d.lora, workspace=ws))[0]
+    with mid():
+        own = run(least)
+    with mid(on=-1):
+        tiles = run(least)
+    with linear.tune_override(flags=16):
+        dense = run(fast)
+    assert not torch.equal(own, dense) and not torch.equal(own, tiles)
+    assert torch.equal(run(fast), dense) and torch.equal(run(least), own)
+    linear.check_status()
