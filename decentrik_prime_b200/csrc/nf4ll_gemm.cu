@@ -1943,6 +1943,8 @@ extern "C" void nf4ll_test_mid(int32_t on, int32_t rb, int32_t nt, int32_t cl) {
   nf4ll::g_mid.on = on; nf4ll::g_mid.rb = rb; nf4ll::g_mid.nt = nt; nf4ll::g_mid.cl = cl;
 }
 
+extern "C" int64_t nf4ll_test_mid_searches(void) { return nf4ll::mid_searches(); }
+
 // Failure-detection test hook (no counterpart in the reference). One-shot.
 extern "C" void nf4ll_test_expire_wait(uint32_t polls) { nf4ll::g_expire_polls = polls; }
 

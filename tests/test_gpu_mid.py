@@ -213,3 +213,24 @@ def test_it_takes_what_the_dense_gemm_would_where_the_workspace_is_too_small(N, 
     assert not torch.equal(own, dense) and not torch.equal(own, tiles)
     assert torch.equal(run(fast), dense) and torch.equal(run(least), own)
     linear.check_status()
+
+
+def test_plans_of_a_layer_are_searched_for_once():
+    """The products of a small layer, forward and backward with and without a mask, at a hundred batch sizes: a second pass over
+    the same sizes finds every plan of a batch size it has just made."""
+    h = _lib.lib()
+    ds = [to_device(make_problem(N, K, 600, seed=N + K, lora=True, dropout=0.05, device="cuda")) for N, K in ((512, 512), (1024, 512), (512, 1024), (768, 512))]
+
+    def layer(M):
+        for d in ds:
+            x, dy, mask = d.x[:M], d.dy[:M], d.mask[:M]
+            linear.forward(d.w, x, lora=d.lora, mask=mask, keep_scale=d.keep_scale)
+            linear.forward(d.w, x)
+            linear.backward_dx(d.w, dy, lora=d.lora, mask=mask, keep_scale=d.keep_scale)
+            linear.backward_dx(d.w, dy)
+    for M in range(17, 600, 6):
+        layer(M)
+        before = h.nf4ll_test_mid_searches()
+        layer(M)
+        assert h.nf4ll_test_mid_searches() == before, M
+    linear.check_status()
