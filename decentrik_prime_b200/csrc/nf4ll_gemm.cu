@@ -1236,13 +1236,18 @@ int launch_pair(int mode, int bm_tiles, const CUtensorMap& map, const CUtensorMa
                 const GemmParams& p, int64_t tiles_o, int64_t tiles_mp, int splits, int launch_splits, cudaStream_t stream);
 constexpr int64_t kStreamMaxRows = 16;     // most token rows of the weight-streaming kernel's own choice
 constexpr int64_t kStreamCapRows = 64;     // its limit (reachable through the tuning hook)
-// From 9 to 16 rows of one projection against at least 2^24 weights, the kernel for middling batches where a fit of its time lies
-// below one of the streaming kernel's, which depends on how evenly its units go round the SMs (and on the tokens). Measured,
-// streaming / middling: 5120 x 27648 at 9 / 16 rows 55 / 62 against 42, 3584 x 18944 27 / 29 against 25, 27648 x 5120 38 / 40
-// against 39. From 17 rows on the latter is ahead everywhere (1536 x 1536 at 17 rows 7.5; the streaming kernel 4.7 at 16).
-constexpr int64_t kMidLeastRows = 9;       // below, the streaming kernel keeps its exact fp32 scales
+// From 9 to 16 rows of one projection (or of each half of gate|up) against at least 2^24 weights, the kernel for middling batches
+// where its model (mid_plan; 5 % low there) lies below the streaming kernel's, which depends on how evenly its units go round the
+// SMs and on the tokens, and to which gate|up adds a launch. Measured, streaming / middling, us at 9 and 16 rows: 5120 x 27648
+// 55 / 41 and 63 / 41, 27648 x 5120 38 / 36 and 41 / 36, 18944 x 3584 22 / 19 and 23 / 19, 5120 x 5120 14.0 / 13.6 and 15.6 / 13.6,
+// 10240 x 2560 13.2 / 15.0 and 14.3 / 15.0, gate|up of 2 x 9472 x 3584 26 / 21 and 27 / 21; below 2^24 the streaming kernel is
+// ahead (3584 x 3584 9.2 / 10.8, 1536 x 8960 10.6 / 12.0 at 16 rows),
+// but not for gate|up of such halves, which is not asked (2 x 5504 x 2048 15.8 / 13.6). Over 51 such calls the choice takes 0.3 % longer than the
+// faster kernel, 9 % at worst (27648 x 1024). Against fp64 sums over the fp16 weights, which are the result that this path is
+// held to, the rel-L2 is 3.4e-4 in the streaming kernel and 2.1e-4 in this one; over the unrounded weights 2.8e-4 and 2.9e-4.
+// From 17 rows on the latter is ahead everywhere (1536 x 1536 at 17 rows 7.5; the streaming kernel 4.8 at 16).
+constexpr int64_t kMidLeastRows = 9;       // below, the streaming kernel keeps its exact fp32 scales, and is the faster one nearly everywhere
 constexpr int64_t kMidSmallWeights = int64_t(1) << 24;
-static double mid_small_us(int64_t N, int64_t K) { return 11.0 + 0.245e-6 * static_cast<double>(N) * static_cast<double>(K); }
 
 // Which kernel computes a forward of M rows that neither the kernel for middling batches nor the dense GEMM takes: the tile
 // kernels (kTiles) or the register-level weight-streaming kernel for decode-sized batches (kStream). Bit 1 of the tuning flags
@@ -1443,10 +1448,8 @@ static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lor
   if (g_mid.on > 0) return mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, g_mid.rb, g_mid.nt, g_mid.cl, mp);
   if (c.M > kMidMostRows) return false;
   if (c.mode == kFwd && c.M <= kStreamMaxRows) {
-    // gate|up: the streaming kernel, whose scales stay fp32, unless this one's single launch is far ahead
     if (c.M < kMidLeastRows || (c.n_seg > 1 && !c.gu_inter) || (c.gu_inter ? N / 2 : N) * K < kMidSmallWeights) return false;
-    const double own = mid_small_us(N, K) + (c.gu_inter ? 11 : 0);
-    if (!(own < stream_time_us(N, K, c.M, sms))) return false;
+    return mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp) && 1.05 * mp->us < stream_time_us(N, K, c.M, sms) + (c.gu_inter ? 4 : 0);
   }
   if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
   if (c.M <= kDenseNeverRows) return true;

@@ -285,7 +285,7 @@ int nf4ll_read_status(const int32_t* status, void* stream);
  * flags bit 1: run a forward of at most 64 rows on the register-level weight-streaming kernel (default: up to
  * 16 rows); flags bit 2: run a forward of one projection and at most 64 rows on the kernel for middling batches (weights
  * as the MMA's row operand; default: from 17 rows on while a model of its time is ahead, and 9 to 16 rows against weights of
- * at least 2^24 elements where a fit of both kernels' times says so); flags bit 3: never
+ * at least 2^24 elements where models of both kernels' times say so); flags bit 3: never
  * dequantise into the workspace, whatever its size (the kernel for middling batches stays open); flags bit 4: do so for any number of rows if the workspace holds
  * 2 N K + 192 M + 32 N + 2048 bytes. With bit 1 `splits` forces the number of warps
  * that share a unit of rows (even: units of 16 rows, odd: of 32), with bit 2 the number of slices of the contraction (8 at most). Size the workspace of such calls with nf4ll_workspace_bytes_tuned. */

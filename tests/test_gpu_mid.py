@@ -234,3 +234,21 @@ def test_plans_of_a_layer_are_searched_for_once():
         layer(M)
         assert h.nf4ll_test_mid_searches() == before, M
     linear.check_status()
+
+
+@pytest.mark.parametrize("N,K,M,gate_up,taken", [(5120, 27648, 9, False, True), (27648, 5120, 16, False, True), (18944, 3584, 16, False, True),
+                                                 (18944, 3584, 9, True, True), (27648, 5120, 16, True, True), (27648, 5120, 8, False, False),
+                                                 (3584, 3584, 16, False, False), (10240, 2560, 9, False, False), (27648, 5120, 9, True, False)])
+def test_nine_to_sixteen_rows_take_the_faster_kernel(N, K, M, gate_up, taken):
+    """Calls on which the two kernels differ by 5 % or more (but the last, 2 %): the default gives one's bits or the other's."""
+    d = to_device(make_problem(N, K, M, seed=N + M, lora=False, device="cuda"))
+
+    def run():
+        return linear.forward_gate_up(d.w, d.x)[0] if gate_up else linear.forward(d.w, d.x)[0]
+    with mid():
+        own = run()
+    with mid(on=-1):
+        streamed = run()
+    assert not torch.equal(own, streamed)
+    assert torch.equal(run(), own if taken else streamed)
+    linear.check_status()
