@@ -167,6 +167,7 @@ SIGNATURES = {
     "nf4ll_test_dense_plan": (_i32, [_i64, _i64, _i64]),
     "nf4ll_test_mid": (None, [_i32, _i32, _i32, _i32]),
     "nf4ll_test_mid_searches": (_i64, []),
+    "nf4ll_test_mid_withhold": (None, [_i32, ctypes.c_uint32]),
     "nf4ll_launch_count": (_i64, []),
     "nf4ll_kernel_events": (None, [_vp, _vp]),
     "nf4ll_rms_forward": (_i32, [_vp, _vp, _vp, _vp, _f32, _i64, _i64, _vp, _i64, _vp, _LORA, _vp, _LORA, _vp, _vp]),

@@ -1048,8 +1048,19 @@ struct MidTune {                      // nf4ll_test_mid
   int on = 0, rb = 0, nt = 0, cl = 0;
 };
 static thread_local MidTune g_mid;
+struct Withhold {                     // nf4ll_test_mid_withhold
+  int what = 0;
+  uint32_t wait_us = 0;
+};
+static thread_local Withhold g_withhold;
 static thread_local uint32_t g_expire_polls = 0;      // nf4ll_test_expire_wait: one-shot
 static thread_local cudaEvent_t g_ev_start = nullptr, g_ev_stop = nullptr;
+// The failure-detection hooks hold for one call, whichever kernel it takes
+struct OneShot {
+  const Withhold withhold = g_withhold;
+  OneShot() { g_withhold = Withhold{}; }
+  ~OneShot() { g_expire_polls = 0; }
+};
 
 // Record a measurement event on `stream`; inside a stream capture the record becomes a node of the graph that is
 // executed (and timed) at every replay
@@ -1519,6 +1530,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
                     const nf4ll_segment* segments = nullptr, int n_segments = 0) {
   const char* who = segments ? "nf4ll_forward_multi" : (mode == kFwd ? "nf4ll_forward" : "nf4ll_backward_dx");
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  const OneShot hooks;
   if (int rc = check_mat(W, who)) return rc;
   if (M < 0) { set_detail("%s: M=%lld", who, static_cast<long long>(M)); return NF4LL_ERR_SHAPE; }
   if (M == 0) return NF4LL_OK;
@@ -1556,6 +1568,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     MidCall c{};
     c.mode = mode; c.W = W; c.act = act; c.ldact = ldact; c.M = M; c.bias = bias; c.out = out; c.ldo = ldo; c.accumulate = accumulate;
     c.n_seg = segments ? n_segments : 1;
+    c.withhold = hooks.withhold.what; c.wait_us = hooks.withhold.wait_us;
     DenseCall dc{};
     dc.mode = mode; dc.W = W; dc.act = act; dc.ldact = ldact; dc.bias = bias; dc.M = M; dc.out = out; dc.ldo = ldo; dc.accumulate = accumulate;
     dc.stacked = segments != nullptr;
@@ -1610,7 +1623,6 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   if (expire && p.coop && pl.splits > 1) {
     // test hook: launch one split short, so that every tile's counter stays below `splits` and each CTA's
     // bounded wait on it runs out after `expire` polls
-    g_expire_polls = 0;
     pl.launch_splits = pl.splits - 1;
     p.spin_limit = expire;
   }
@@ -1730,6 +1742,7 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
                        void* workspace, int64_t workspace_bytes, int32_t* status, void* stream_v) {
   const char* who = "nf4ll_forward_gate_up";
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  const OneShot hooks;
   if (int rc = check_mat(W, who)) return rc;
   if (M < 0 || W->N % 2) { set_detail("%s: M=%lld, %lld stacked rows", who, (long long)M, (long long)W->N); return NF4LL_ERR_SHAPE; }
   if (M == 0) return NF4LL_OK;
@@ -1754,6 +1767,7 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     c.out_u = u; c.ldu = ldu; c.out_h = h; c.ldh = ldh; c.gu_inter = I;
     c.n_seg = 2;
     c.seg_end[0] = I; c.seg_end[1] = W->N;
+    c.withhold = hooks.withhold.what; c.wait_us = hooks.withhold.wait_us;
     DenseCall dc{};
     dc.mode = kFwd; dc.W = W; dc.act = x; dc.ldact = ldx; dc.M = M; dc.out = g; dc.ldo = ldg;
     dc.out_u = u; dc.ldu = ldu; dc.out_h = h; dc.ldh = ldh; dc.gu_inter = I; dc.n_branch = 2;
@@ -1944,6 +1958,11 @@ extern "C" void nf4ll_kernel_events(void* start, void* stop) {
 // Testing hook (no counterpart in the reference)
 extern "C" void nf4ll_test_mid(int32_t on, int32_t rb, int32_t nt, int32_t cl) {
   nf4ll::g_mid.on = on; nf4ll::g_mid.rb = rb; nf4ll::g_mid.nt = nt; nf4ll::g_mid.cl = cl;
+}
+
+// Failure-detection test hook (no counterpart in the reference). One-shot.
+extern "C" void nf4ll_test_mid_withhold(int32_t what, uint32_t wait_us) {
+  nf4ll::g_withhold.what = what; nf4ll::g_withhold.wait_us = wait_us;
 }
 
 extern "C" int64_t nf4ll_test_mid_searches(void) { return nf4ll::mid_searches(); }

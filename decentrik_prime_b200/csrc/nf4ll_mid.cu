@@ -34,8 +34,8 @@
 // 18944 x 3584 at 333 rows 57, now 46; 27648 x 5120 at 333 rows 148, now 96. Backward 1536 x 8960 at 187 rows 24.4, now 14.7;
 // 18944 x 3584 at 187 rows 69, now 40; 5120 x 27648 at 333 rows 164, now 99.
 //
-// Every wait is bounded and reports through the status word. Warp roles: 0 codes, 1 MMA issue, 2 token tiles, 3 idle, 4-7 rank-16
-// operands and epilogue, 8-23 decode.
+// Every wait is bounded and reports through the status word (tested by withholding codes, rank-16 operands and partial sums).
+// Warp roles: 0 codes, 1 MMA issue, 2 token tiles, 3 idle, 4-7 rank-16 operands and epilogue, 8-23 decode.
 #include <cuda.h>
 
 #include "nf4ll_mid.cuh"
@@ -59,6 +59,8 @@ constexpr int kMidSmem = 227 * 1024;
 // 47.0 / 47.2 us, 27648 x 5120 at 64 rows 43.0 / 43.7, gate|up of it at 24 rows 44.4 / 44.6, 1536 x 1536 at 24 rows 9.3 / 9.5.
 constexpr int64_t kMidSplitRows = 64;
 
+enum : int { kHoldCodes = 1, kHoldRank16 = 2, kHoldSums = 3 };      // nf4ll_test_mid_withhold
+
 struct MidParams {
   const uint8_t* qabs;
   const float* scale2;
@@ -69,6 +71,8 @@ struct MidParams {
   int ts;                          // token columns that a CTA of the cluster finishes
   int off_a, off_x, off_lora, off_xch, off_lut, off_turn, off_misc;      // shared memory
   int early, qabs_mode, x_alias, any_lora;
+  int withhold;                    // failure-detection hook: what is never signalled
+  uint64_t wait_ns;                // limit of the waits
   int split;                       // forward: the tokens' side of the rank-16 operands in two fp16 parts
   __half* out;
   int64_t ldo;
@@ -157,12 +161,32 @@ __device__ __forceinline__ uint64_t mid_twice(float v) {
   return d;
 }
 
-// Barrier waits of whole warps on the kernel's critical path
-__device__ __forceinline__ bool mid_wait(uint32_t bar, uint32_t parity, const Abort& ab, int code) {
+// A wait of a whole warp. Its lanes vote, so that they agree on the outcome: the tensor-memory instructions, elect.sync and the
+// barriers behind it want all of them, and a lane that saw the phase complete while another saw the abort flag would go on alone.
+// (Time without / with the vote, us: 18944 x 3584 at 333 rows forward 45.4 / 45.8, backward 72.0 / 73.0, 8960 x 1536 at 187 rows 12.2 / 11.7.)
+// Bounded by polls and by time; CLUSTER: for barriers on which other CTAs arrive (polled, their arrivals wake a parked thread slowly).
+struct MidAbort : Abort {
+  uint64_t limit_ns;
+};
+template <bool CLUSTER = false>
+__device__ __forceinline__ bool mid_wait(uint32_t bar, uint32_t parity, const MidAbort& ab, int code) {
 #pragma unroll 1
   for (int i = 0; i < 64; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return wait_or_abort(bar, parity, ab, code);
+    if (__all_sync(0xffffffffu, CLUSTER ? mbar_test_wait_cluster(bar, parity) : mbar_try_wait(bar, parity))) return true;
+  const uint64_t t0 = global_timer_ns();
+#pragma unroll 1
+  for (uint32_t i = 0; i < (CLUSTER ? kSpinLimit << 4 : kSpinLimit); ++i) {
+    if (__all_sync(0xffffffffu, CLUSTER ? mbar_test_wait_cluster(bar, parity) : mbar_try_wait_hint(bar, parity, kParkNs))) return true;
+    if (__any_sync(0xffffffffu, *ab.flag != 0)) return false;
+    if (__any_sync(0xffffffffu, global_timer_ns() - t0 > ab.limit_ns)) break;
+  }
+  ab.raise(code);
+  return false;
+}
+// Copies or MMAs that may be under way when the kernel gives up get a millisecond to finish
+__device__ __forceinline__ void mid_drain(uint32_t bar, uint32_t parity) {
+  const uint64_t t0 = global_timer_ns();
+  for (int i = 0; i < (1 << 16) && !mbar_test_wait(bar, parity) && global_timer_ns() - t0 < 1000000; ++i) {}
 }
 
 template <int MODE, int RB>
@@ -198,7 +222,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   uint32_t* wide = tmem_slot + 2;                // [2 units in turn][RB][4]: tokens beyond fp16's range, sixteen to a word, bits 0, 2, 4, ... (16-byte aligned)
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const Abort ab{abort_flag, p.status};
+  const MidAbort ab{{abort_flag, p.status}, p.wait_ns};
   const int cl = p.cl;
   const int crank = cl > 1 ? static_cast<int>(cluster_ctarank()) : 0;
   const int cluster = blockIdx.x / cl, n_clusters = gridDim.x / cl;
@@ -273,6 +297,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         for (int g = grp0; ok && g < grp1; ++g)
 #pragma unroll
           for (int rb = 0; rb < (MODE == kFwd ? RB : 1); ++rb, ++i) {
+            if (p.withhold == kHoldCodes && i == 1) { ok = false; break; }
             const int c = i & (p.nc - 1);
             if (!wait_or_abort(smem_u32(c_empty + c), ((i >> p.nc_log) & 1) ^ 1, ab, 0x0701)) { ok = false; break; }
             mbar_arrive_expect_tx(smem_u32(c_full + c), kStage);
@@ -281,8 +306,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             else tma_load_2d(sCode + c * kStage, &tmap_nib, r0 / 2, g * 128, smem_u32(c_full + c));
           }
       if (*abort_flag)        // copies still in flight get a bounded chance to land before the CTA goes away
-        for (int k = (i > p.nc ? i - p.nc : 0); k < i; ++k)
-          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(smem_u32(c_full + (k & (p.nc - 1))), (k >> p.nc_log) & 1); ++spin) {}
+        for (int k = (i > p.nc ? i - p.nc : 0); k < i; ++k) mid_drain(smem_u32(c_full + (k & (p.nc - 1))), (k >> p.nc_log) & 1);
     }
   } else if (warp == 2) {
     // ----------------------------------------------------------------------------- token tiles
@@ -307,8 +331,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         }
       }
       if (*abort_flag)        // copies still in flight get a bounded chance to land
-        for (int k = (hi > p.nx ? hi - p.nx : 0); k < hi; ++k)
-          for (int spin = 0; spin < (1 << 16) && !mbar_try_wait(smem_u32(a_full + k * RB % kMidBars), (k * RB / kMidBars) & 1); ++spin) {}
+        for (int k = (hi > p.nx ? hi - p.nx : 0); k < hi; ++k) mid_drain(smem_u32(a_full + k * RB % kMidBars), (k * RB / kMidBars) & 1);
     }
   } else if (warp == 1) {
     // ----------------------------------------------------------------------------- MMA issue: the whole warp walks the loop, one elected
@@ -373,12 +396,6 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       }
       if (mid_elect()) tc_commit(smem_u32(acc_full + buf));
       __syncwarp();
-    }
-    if (!ok) {
-      // none of this warp's MMAs may still be running when tensor memory is freed
-      if (mid_elect()) tc_commit(smem_u32(drain));
-      __syncwarp();
-      for (int spin = 0; spin < (1 << 18) && !mbar_try_wait(smem_u32(drain), 0); ++spin) {}
     }
   }
   bool ok = true;
@@ -519,7 +536,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
       const int u = cluster + ul * n_clusters, crews = ul == last ? 1 + kMidTeams : 1;
       const int t0 = (u % p.tiles_t) * p.nt, vt = min(p.nt, p.M - t0);
       if (p.any_lora && crank == 0 && crew == 0 && ok) {
-        ok = wait_or_abort(smem_u32(l_empty), (ul & 1) ^ 1, ab, 0x0709);
+        ok = mid_wait(smem_u32(l_empty), (ul & 1) ^ 1, ab, 0x0709);
         if (ok) {
 #pragma unroll
           for (int rb = 0; rb < RB; ++rb) {
@@ -582,13 +599,13 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
           }
           fence_proxy_async_smem();
           __syncwarp();
-          if (lane == 0) mbar_arrive(smem_u32(l_full));
+          if (lane == 0 && p.withhold != kHoldRank16) mbar_arrive(smem_u32(l_full));
         }
       }
       const int buf = p.nbuf == 2 ? ul & 1 : 0;
       const bool split = MODE == kFwd && p.split && p.any_lora && crank == 0 && crew == 0;
-      if (split && ok) ok = wait_or_abort(smem_u32(l_full), ul & 1, ab, 0x070d);      // the other warps' bits are there
-      if (crew == 0 && ok) ok = wait_or_abort(smem_u32(acc_full + buf), (p.nbuf == 2 ? ul >> 1 : ul) & 1, ab, 0x070a);
+      if (split && ok) ok = mid_wait(smem_u32(l_full), ul & 1, ab, 0x070d);      // the other warps' bits are there
+      if (crew == 0 && ok) ok = mid_wait(smem_u32(acc_full + buf), (p.nbuf == 2 ? ul >> 1 : ul) & 1, ab, 0x070a);
       if (split && ok) {
         // rank-16 terms of tokens beyond fp16's range: added to their columns of the accumulator in fp32
         uint32_t any = 0;
@@ -675,7 +692,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         tb = min(crank * p.ts, vt); te = min(tb + p.ts, vt);
         int turn = 0;                            // chunks of eight columns go round the crews
         if (p.x_alias && warp == kMidEpiWarp && ok) peers(xch_free);       // this CTA's operand rings are idle
-        if (ok) ok = wait_cluster_or_abort(smem_u32(xch_free), ul & 1, ab, 0x070b);
+        if (ok) ok = mid_wait<true>(smem_u32(xch_free), ul & 1, ab, 0x070b);
         if (ok) {
           for (int k = 1; k < cl; ++k) {
             int dst = crank + k;                 // peers in turn, so that not all write to the same one
@@ -703,8 +720,8 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         if (crews > 1) named_barrier(2, 128 * (1 + kMidTeams));
         if (ok) {
           __syncwarp();
-          if (crew == 0) peers(xch_full);
-          ok = wait_cluster_or_abort(smem_u32(xch_full), ul & 1, ab, 0x070c);
+          if (crew == 0 && !(p.withhold == kHoldSums && crank == cl - 1)) peers(xch_full);
+          ok = mid_wait<true>(smem_u32(xch_full), ul & 1, ab, 0x070c);
         }
       }
       if (ok) {
@@ -781,6 +798,12 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
+    if (*abort_flag) {                         // none of this warp's MMAs may still be running when tensor memory is freed
+      if (mid_elect()) tc_commit(smem_u32(drain));
+      __syncwarp();
+      mid_drain(smem_u32(drain), 0);
+      __syncwarp();
+    }
     tmem_dealloc(tmem_base, 512);
   }
   if (cl > 1) cluster_sync_all();                // nobody leaves while a peer may still write to its shared memory
@@ -1023,6 +1046,8 @@ int mid_launch(const MidCall& c, const MidPlan& pl, bool early, int32_t* status,
   p.out_u = static_cast<__half*>(c.out_u); p.ldu = c.ldu;
   p.out_h = static_cast<__half*>(c.out_h); p.ldh = c.ldh;
   p.status = status;
+  p.withhold = c.withhold;
+  p.wait_ns = c.withhold ? static_cast<uint64_t>(c.wait_us) * 1000 : kWaitLimitNs;
   const bool wide = fwd || pl.rb == 2;           // backward with one row block: its 128 columns are 64 bytes of codes
   CUtensorMap mx, mn;
   if (int rc = mid_encode(&mx, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, c.act, static_cast<uint64_t>(p.steps) * 64, static_cast<uint64_t>(c.M),

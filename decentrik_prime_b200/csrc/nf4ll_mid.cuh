@@ -27,6 +27,8 @@ struct MidCall {
   int64_t ldu;
   void* out_h;
   int64_t ldh;
+  int withhold;                          // failure-detection hook (nf4ll_test_mid_withhold), 0: off
+  uint32_t wait_us;
 };
 
 // How a call is cut up. A unit is (128 * rb weight rows / output columns) x (nt tokens), worked on by one cluster.

@@ -303,13 +303,14 @@ void nf4ll_kernel_events(void* start, void* stop);
  * across one step to report how many of the library's kernels a step consists of. */
 int64_t nf4ll_launch_count(void);
 
-/* Failure-detection test hook; no counterpart in the reference. The calling thread's NEXT call whose
- * contraction is split with the cooperative reduction is launched one split short and with a limit of
+/* Failure-detection test hook; no counterpart in the reference. The calling thread's NEXT call, if its
+ * contraction is split with the cooperative reduction, is launched one split short and with a limit of
  * `polls` polls (instead of 2^22) on the wait for a tile's other splits. Nothing ever completes those
  * tiles' counters, so every CTA's wait runs out: each one records NF4LL_ERR_DEVICE_WAIT's cause in the
  * status word, releases its tensor memory and returns; the call's output is undefined, the context stays
- * usable and later calls are unaffected (the tile counters are cleared before every use). One-shot;
- * ignored by calls that do not split cooperatively. */
+ * usable and later calls are unaffected (the tile counters are cleared before every use). One-shot: forgotten after the
+ * next forward or backward-dX call, which leaves the kernel for middling batches and the dense GEMM out, and ignored by
+ * one that does not split cooperatively. */
 void nf4ll_test_expire_wait(uint32_t polls);
 
 /* Testing hook; no counterpart in the reference. How the large-batch GEMM over a dequantised weight distributes [M, NO] with a
@@ -325,6 +326,13 @@ void nf4ll_test_mid(int32_t on, int32_t rb, int32_t nt, int32_t cl);
 /* Testing hook; no counterpart in the reference. How often the calling thread has searched for the cutting of a call to that
  * kernel; a call whose cutting it still holds does not search. */
 int64_t nf4ll_test_mid_searches(void);
+
+/* Failure-detection test hook; no counterpart in the reference. In the calling thread's NEXT forward or backward-dX call, if the
+ * kernel for middling batches takes it, no CTA loads codes after its first stage (what = 1), the rank-16 operands are never
+ * announced (2), or the last CTA of every cluster never announces its partial sums (3), and the waits of whole warps end after
+ * wait_us microseconds (instead of a second). The waits for what is missing run out: the cause is recorded in the status word, the
+ * kernel ends, the call's output is undefined, the context stays usable and later calls are unaffected. One-shot. */
+void nf4ll_test_mid_withhold(int32_t what, uint32_t wait_us);
 
 #ifdef __cplusplus
 }
