@@ -1464,13 +1464,23 @@ static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lor
   }
   if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
   if (c.M <= kDenseNeverRows) return true;
-  // the model's margin: it knows nothing of clocks that fall under load. At the same work per launch it is 3 % low for 25 GFLOP
+  // The model's margin: it knows nothing of clocks that fall under load. At the same work per launch it is 3 % low for 25 GFLOP
   // and 20 % for 250 (backward of 27648 x 5120 at 951 rows: 288 us, where the tiles take 250).
   const double work = 2e-9 * static_cast<double>(c.M) * static_cast<double>(N) * static_cast<double>(K);
-  // Beyond the rows that it was fitted to, a wider one still: without, 1536 x 8960 backward at 2048 rows took 63 us for 50,
-  // 5120 x 5120 backward 109 for 103; with it 1536 x 1536 at 2048 rows still goes from 24.5 to 14.3 us, 3584 x 3584 at 1100 from 41 to 29.
+  double margin = 1.05 + 0.15 * (work < 250 ? work / 250 : 1.0);
+  // Forward with one row block and only two slots of token tiles (from 128 tokens a tile on), an item takes a quarter longer than the
+  // model has it, which tells in a long chain of them: 2048 x 11008 at 1024 rows (86 items) 62.8 us, the tiles 54.7.
+  if (c.mode == kFwd && mp->rb == 1 && mp->nx == 2 && mp->items > 40) {
+    const double chain = 1.05 + 0.1 * (mp->items < 64 ? static_cast<double>(mp->items - 40) / 24 : 1.0);
+    if (chain > margin) margin = chain;
+  }
+  // Beyond the rows that it was fitted to, wider still. Measured without this kernel, with it and as chosen, 1840 calls (30 weights from
+  // 256 x 1536 to 27648 x 5120, forward, backward and gate|up, 23 batch sizes of 129 to 2560 rows): the choice takes 1.4 % longer than
+  // the best would, 6 calls 3 to 5 % longer than without this kernel, 96 more than 5 % longer than with it, most of them
+  // backward beyond 1024 rows (1024 x 4096 at 1400 rows 22.0 us, 19.9 with it). With 1.15 there too, 14 calls would be slower than without,
+  // 1536 x 8960 backward at 2560 rows by 17 %.
   const double beyond = c.M <= 1024 ? 1.0 : c.mode == kFwd ? 1.15 : 1.29;
-  const double us = mp->us * (1.05 + 0.15 * (work < 250 ? work / 250 : 1.0)) * beyond;
+  const double us = mp->us * margin * beyond;
   return us < t.decoding && !(dense && us >= t.dense);
 }
 

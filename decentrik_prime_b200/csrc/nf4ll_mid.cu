@@ -953,6 +953,7 @@ static bool mid_search(int mode, int64_t M, int64_t NO, int64_t KC, bool mask, i
         const int64_t rounds = (units + most - 1) / most;
         p.clusters = static_cast<int>((units + rounds - 1) / rounds);
         const int64_t items = (groups + cl - 1) / cl * halves * rb;
+        p.items = rounds * items;
         p.us = mid_us(mode, rb, nt, cl, rounds, items, 2);
         if (found && p.us >= plan->us) continue;
         if (!mid_buffers(mode, mask, lora, &p)) continue;

@@ -39,6 +39,7 @@ struct MidPlan {
   int nbuf, na, nx, nc;        // accumulators, slots of decoded weights, slots of token tiles, slots of codes
   bool x_alias;                // the exchange of partial sums reuses the operand rings
   bool split;                  // forward: the rank-16 product as two fp16 parts
+  int64_t items;               // items of 128 x 128 weights that a CTA takes one after another
   double us;                   // expected time
 };
 

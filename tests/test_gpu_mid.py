@@ -252,3 +252,22 @@ def test_nine_to_sixteen_rows_take_the_faster_kernel(N, K, M, gate_up, taken):
     assert not torch.equal(own, streamed)
     assert torch.equal(run(), own if taken else streamed)
     linear.check_status()
+
+
+@pytest.mark.parametrize("M,taken", [(951, True), (1024, False), (1025, True)])
+def test_long_chains_with_two_token_slots_are_left_to_the_tiles_where_those_are_ahead(M, taken):
+    """2048 x 11008 forward: 144 units of 112 tokens and four slots, 128 units of 128 tokens and two slots, and one row more, for
+    which the tiles take another round."""
+    d = to_device(make_problem(2048, 11008, M, seed=M, lora=True, dropout=0.0, device="cuda"))
+    ws = torch.empty(_lib.lib().nf4ll_workspace_bytes(M, 2048, 11008, 16), dtype=torch.uint8, device="cuda")      # no room for the dense GEMM
+    t = d.x.float() @ d.A16.float().t()
+
+    def run():                                        # the rank-16 product given: its sum over a row uses atomics here
+        return linear.forward_multi(d.w, d.x, [(2048, d.lora, None, 1.0, t)], workspace=ws)[0]
+    with mid():
+        own = run()
+    with mid(on=-1):
+        tiles = run()
+    assert not torch.equal(own, tiles)
+    assert torch.equal(run(), own if taken else tiles)
+    linear.check_status()
