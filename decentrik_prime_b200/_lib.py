@@ -166,6 +166,7 @@ SIGNATURES = {
     "nf4ll_test_expire_wait": (None, [ctypes.c_uint32]),
     "nf4ll_test_dense_plan": (_i32, [_i64, _i64, _i64]),
     "nf4ll_test_mid": (None, [_i32, _i32, _i32, _i32]),
+    "nf4ll_test_mid_calls": (_i64, []),
     "nf4ll_test_mid_searches": (_i64, []),
     "nf4ll_test_mid_withhold": (None, [_i32, ctypes.c_uint32]),
     "nf4ll_launch_count": (_i64, []),

@@ -1975,6 +1975,8 @@ extern "C" void nf4ll_test_mid_withhold(int32_t what, uint32_t wait_us) {
   nf4ll::g_withhold.what = what; nf4ll::g_withhold.wait_us = wait_us;
 }
 
+extern "C" int64_t nf4ll_test_mid_calls(void) { return nf4ll::mid_calls(); }
+
 extern "C" int64_t nf4ll_test_mid_searches(void) { return nf4ll::mid_searches(); }
 
 // Failure-detection test hook (no counterpart in the reference). One-shot.

@@ -1,5 +1,5 @@
 // Middling batches (17 to some hundreds of token rows, 2560 against small weights), forward and backward-dX: the WEIGHTS are the 128-row operand of
-// tcgen05.mma, the tokens its N operand (any multiple of 16 up to 256 columns), the contraction is cut over the CTAs of a
+// tcgen05.mma, the tokens its N operand (any multiple of 16 up to 240 columns, 224 with LoRA: what shared memory holds two tiles of), the contraction is cut over the CTAs of a
 // thread-block cluster. Serves the reference call sites solution/fast_qwen.py:947, 1037, 1080-1112 and, backward, 1310-1364.
 //
 //   forward    y^T[128 weight rows, tokens] = W[rows, K] . x^T
@@ -1005,6 +1005,8 @@ bool mid_plan(int mode, int64_t M, int64_t NO, int64_t KC, bool mask, int64_t gu
   return e->found;
 }
 int64_t mid_searches() { return g_mid_searches; }
+static thread_local int64_t g_mid_calls = 0;
+int64_t mid_calls() { return g_mid_calls; }
 
 template <int MODE, int RB>
 static int mid_launch_cfg(const CUtensorMap& mx, const CUtensorMap& mn, const MidParams& p, const MidPlan& pl, int smem, cudaStream_t stream) {
@@ -1016,6 +1018,7 @@ static int mid_launch_cfg(const CUtensorMap& mx, const CUtensorMap& mn, const Mi
 }
 
 int mid_launch(const MidCall& c, const MidPlan& pl, bool early, int32_t* status, cudaStream_t stream) {
+  ++g_mid_calls;
   const nf4ll_mat* W = c.W;
   const bool fwd = c.mode == kFwd;
   MidParams p{};

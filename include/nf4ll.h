@@ -323,6 +323,9 @@ int32_t nf4ll_test_dense_plan(int64_t M, int64_t NO, int64_t KC);
  * choice); on < 0 keeps it out; zeros restore the built-in choice. */
 void nf4ll_test_mid(int32_t on, int32_t rb, int32_t nt, int32_t cl);
 
+/* Testing hook; no counterpart in the reference. How many calls of the calling thread that kernel has taken. */
+int64_t nf4ll_test_mid_calls(void);
+
 /* Testing hook; no counterpart in the reference. How often the calling thread has searched for the cutting of a call to that
  * kernel; a call whose cutting it still holds does not search. */
 int64_t nf4ll_test_mid_searches(void);

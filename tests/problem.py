@@ -3,12 +3,34 @@ fp16 weight ~ N(0, 0.02) quantised to NF4 (block 64, double-quantised absmax), f
 ~ N(0, 1), LoRA r=16 / alpha=32 with kaiming-uniform A and B ~ N(0, 0.01), dropout p=0.05 with the
 keep-mask drawn from the seed, keep_scale = 1 / float32(1 - p)."""
 
+import contextlib
 import math
 
 import numpy as np
 import torch
 
 from decentrik_prime_b200 import k_nf4, quantize
+
+
+@contextlib.contextmanager
+def mid(rb=0, nt=0, cl=0, on=1):
+    """Calls of this thread inside the block run on the kernel for middling batches, cut as given (0: its own choice), or with
+    on = -1 never do: tests of the kernels that otherwise get only what that one leaves."""
+    from decentrik_prime_b200 import _lib
+    _lib.lib().nf4ll_test_mid(on, rb, nt, cl)
+    try:
+        yield
+    finally:
+        _lib.lib().nf4ll_test_mid(0, 0, 0, 0)
+
+
+@contextlib.contextmanager
+def tiles_only():
+    """Neither the kernel for middling batches nor the dense GEMM: the kernels that decode inside the GEMM (up to 16 rows forward, the
+    streaming kernel), whatever the models of times say."""
+    from decentrik_prime_b200 import linear
+    with mid(on=-1), linear.tune_override(flags=8):
+        yield
 
 
 class Problem:

@@ -1,30 +1,32 @@
 """Failure detection on the device: a bounded wait that runs out must end the kernel with an error status
-the host can read, leave the CUDA context usable and not disturb later calls. The failure is staged
-without faulting anything: the library's test hook launches a split contraction one split short (with a
-short poll limit), so the wait of every CTA on its tile's other splits can never be satisfied."""
+the host can read, leave the CUDA context usable and not disturb later calls. The failures are staged
+without faulting anything, by hooks of the library: a split contraction launched one split short (with a short poll
+limit), so that the wait of every CTA on its tile's other splits can never be satisfied, and something in the kernel for middling
+batches that is never signalled."""
 
 import pytest
 import torch
 
 from decentrik_prime_b200 import _lib, linear
-from tests.problem import make_problem, to_device
+from tests.problem import make_problem, tiles_only, to_device
 
 pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("direction", ["forward", "backward"])
 def test_expired_wait_is_reported_and_the_next_call_is_correct(direction):
-    # 1536 x 1536 at M = 2048: 48 output tiles, so the plan splits the contraction three ways and the 144
-    # CTAs share the reduction (single-CTA kernel forward, CTA-pair kernel backward)
+    # 1536 x 1536 at M = 2048 on the tile kernels: 48 output tiles, so the plan splits the contraction three
+    # ways and the 144 CTAs share the reduction (single-CTA kernel forward, CTA-pair kernel backward)
     pr = make_problem(1536, 1536, 2048, seed=71, lora=True, dropout=0.05, bias=True)
     d = to_device(pr)
     dev = d.x.device
     h = _lib.lib()
 
     def run():
-        if direction == "forward":
-            return linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0]
-        return linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0]
+        with tiles_only():
+            if direction == "forward":
+                return linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0]
+            return linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0]
 
     good = run().clone()
     linear.check_status()

@@ -1,12 +1,14 @@
 """A captured call's scratch belongs to its graph: a replay neither writes to memory that has gone to somebody else since, nor
 meets the scratch of eager calls on the same stream."""
 
+import contextlib
+
 import pytest
 import torch
 
 from decentrik_prime_b200 import linear
 from oracle import nf4_oracle
-from tests.problem import make_problem, oracle_weight, to_device
+from tests.problem import make_problem, oracle_weight, tiles_only, to_device
 
 pytestmark = pytest.mark.gpu
 
@@ -18,8 +20,9 @@ def calls(pr, d):
 
 
 @pytest.mark.parametrize("warm", [True, False])
-@pytest.mark.parametrize("N,K,M", [(512, 2048, 70), (4096, 4096, 24), (1024, 2048, 3100)])      # split tiles, swapped operands, fp16 weight
-def test_replay_after_the_workspace_has_grown(N, K, M, warm):
+@pytest.mark.parametrize("N,K,M,way", [(512, 2048, 70, tiles_only), (4096, 4096, 24, contextlib.nullcontext),      # split tiles, middling batches,
+                                       (1024, 2048, 3100, contextlib.nullcontext)])                               # fp16 weight
+def test_replay_after_the_workspace_has_grown(N, K, M, way, warm):
     pr = make_problem(N, K, M, seed=N + M, lora=True, dropout=0.05, bias=True)
     d = to_device(pr)
     ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, pr.dy, pr.bias, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)
@@ -27,11 +30,12 @@ def test_replay_after_the_workspace_has_grown(N, K, M, warm):
     torch.cuda.synchronize()
     side = torch.cuda.Stream()
     with torch.cuda.stream(side):
-        if warm:
-            calls(pr, d)
-        graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, stream=side):
-            y, dx = calls(pr, d)
+        with way():
+            if warm:
+                calls(pr, d)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=side):
+                y, dx = calls(pr, d)
         big_y, _ = linear.forward(big.w, big.x, lora=big.lora)      # grows the stream's workspace
         expected = big_y.clone()
         # memory of every size class, so that whatever has been released is somebody's now

@@ -2,12 +2,14 @@
 on identical seeded inputs. Tolerance (the task statement): max-abs-err <= 2e-2 and rel-L2 <= 1e-3
 against the fp32/fp64-accumulated oracle O1; dequantised weights bit-exact."""
 
+import contextlib
+
 import pytest
 import torch
 
 from decentrik_prime_b200 import _lib, linear
 from oracle import nf4_oracle
-from tests.problem import make_problem, oracle_weight, to_device
+from tests.problem import make_problem, oracle_weight, tiles_only, to_device
 
 pytestmark = pytest.mark.gpu
 MAX_ABS, REL_L2 = 2e-2, 1e-3
@@ -42,27 +44,40 @@ def run_case(N, K, M, lora=True, dropout=0.05, bias=False, force=(0, 0, 0), seed
     return pr, d, ref
 
 
+BOTH = pytest.mark.parametrize("way", [contextlib.nullcontext, tiles_only], ids=["default", "tiles"])
+
+
+@BOTH
 @pytest.mark.parametrize("M", [1, 8, 63, 64, 65, 127, 128, 129, 300])
-def test_ragged_rows(M):
-    run_case(256, 256, M, seed=M)
+def test_ragged_rows(M, way):
+    with way():
+        run_case(256, 256, M, seed=M)
 
 
+@BOTH
 @pytest.mark.parametrize("N,K", [(256, 128), (128, 128), (384, 128), (128, 384)])
-def test_toy_layer_shapes(N, K):
+def test_toy_layer_shapes(N, K, way):
     """The shapes of the reference's GPU test layer (solution/test_kernels.py:48-49)."""
-    run_case(N, K, 200, bias=True, seed=N + K)
+    with way():
+        run_case(N, K, 200, bias=True, seed=N + K)
 
 
-def test_no_lora_no_bias():
-    run_case(256, 512, 150, lora=False)
+@BOTH
+def test_no_lora_no_bias(way):
+    with way():
+        run_case(256, 512, 150, lora=False)
 
 
-def test_lora_without_dropout():
-    run_case(256, 256, 256, dropout=0.0, bias=True)
+@BOTH
+def test_lora_without_dropout(way):
+    with way():
+        run_case(256, 256, 256, dropout=0.0, bias=True)
 
 
-def test_leading_dimensions():
-    run_case(256, 256, 130, padded=True, bias=True)
+@BOTH
+def test_leading_dimensions(way):
+    with way():
+        run_case(256, 256, 130, padded=True, bias=True)
 
 
 @pytest.mark.parametrize("force", [(1, 128, 1), (2, 128, 1), (1, 256, 1), (2, 256, 1), (1, 128, 3), (2, 256, 2), (2, 256, 4),
@@ -80,8 +95,9 @@ def test_split_contraction_on_a_grid_larger_than_one_wave(force):
     run_case(1536, 1536, 2048, bias=True, force=force, seed=5 + force[1])
 
 
+@BOTH
 @pytest.mark.parametrize("M", [200, 1300])
-def test_stacked_projections_in_one_launch_match_separate_calls(M):
+def test_stacked_projections_in_one_launch_match_separate_calls(M, way):
     """nf4ll_forward_multi on Q|K|V of a packed layer (LoRA on q and v, bias on all, k narrower than a
     256-column tile) and on gate|up equals the three / two single-projection calls."""
     from decentrik_prime_b200 import k_nf4, quantize
@@ -109,7 +125,8 @@ def test_stacked_projections_in_one_launch_match_separate_calls(M):
             y, t = linear.forward(w, x, bias=b, lora=l, mask=m, keep_scale=ks, want_t=True)
             ref_y.append(y); ref_t.append(t)
         wg = linear.Nf4Weight.from_layer_group(layer, names, code2)
-        y, ts = linear.forward_multi(wg, x, [(w.N, l, m, ks) for w, l, m in zip(ws, loras, masks)], bias=torch.cat(bias))
+        with way():
+            y, ts = linear.forward_multi(wg, x, [(w.N, l, m, ks) for w, l, m in zip(ws, loras, masks)], bias=torch.cat(bias))
         linear.check_status()
         assert_close("stacked y", y, torch.cat(ref_y, 1).double())
         for t, rt in zip(ts, ref_t):
@@ -120,11 +137,13 @@ def test_stacked_projections_in_one_launch_match_separate_calls(M):
         linear.forward_multi(wg, x, [(wg.N - 64, None, None, 1.0), (64, None, None, 1.0)])
 
 
+@BOTH
 @pytest.mark.parametrize("M,lora_up,I", [(300, True, 896), (1100, False, 896), (100, True, 896), (300, True, 960)])
-def test_gate_up_forward_with_the_gated_product_in_its_epilogue(M, lora_up, I):
+def test_gate_up_forward_with_the_gated_product_in_its_epilogue(M, lora_up, I, way):
     """nf4ll_forward_gate_up against the two single-projection forwards and the stand-alone gated-SiLU
     kernel: g, u within the GEMM tolerance, h bit-identical to the stand-alone kernel applied to the
-    stored g, u; M = 100 (short batch) and I = 960 (not a multiple of 128) take the composite path."""
+    stored g, u. On the tile kernels M = 100 (short batch) and I = 960 (not a multiple of 128) take
+    the composite path."""
     from decentrik_prime_b200 import k_nf4, quantize
     H = 512
     names = ("gate_proj", "up_proj")
@@ -143,7 +162,8 @@ def test_gate_up_forward_with_the_gated_product_in_its_epilogue(M, lora_up, I):
     g0, tg0 = linear.forward(wg, x, lora=lg, mask=mg, keep_scale=ks, want_t=True)
     u0, tu0 = linear.forward(wu, x, lora=lu, mask=mu, keep_scale=ks, want_t=True)
     w = linear.Nf4Weight.from_layer_group(layer, names, code2)
-    g, u, h, tg, tu = linear.forward_gate_up(w, x, lg, mg, lu, mu, ks)
+    with way():
+        g, u, h, tg, tu = linear.forward_gate_up(w, x, lg, mg, lu, mu, ks)
     linear.check_status()
     assert_close("g", g, g0.double())
     assert_close("u", u, u0.double())
@@ -269,14 +289,21 @@ def test_mlp_block_fused_glue_matches_pytorch_glue():
         assert rel <= 2e-3, (err, rel)
 
 
-def test_block_step_replays_from_a_cuda_graph():
+@BOTH
+def test_block_step_replays_from_a_cuda_graph(way):
     """Every launch of a block step (cluster, cooperative and programmatic-dependent launches included)
     can be captured into a CUDA graph; the replay gives the eager results bit for bit (the gradient
-    reductions use atomics, so gradients are compared with a tolerance)."""
+    reductions use atomics, so gradients are compared with a tolerance). On the tile kernels down_proj's
+    contraction is split and its reduction cooperative."""
+    with way():
+        replay_block_step()
+
+
+def replay_block_step():
     from decentrik_prime_b200 import blocks
     dev = torch.device("cuda")
     bucket = blocks.GradBucket(blocks.MlpBlock.grad_numel(1536, 1024), dev)
-    blk = blocks.MlpBlock(1536, 1024, seed=21, device=dev, bucket=bucket)     # down_proj: 1536-wide output, split contraction
+    blk = blocks.MlpBlock(1536, 1024, seed=21, device=dev, bucket=bucket)
     gen = torch.Generator().manual_seed(2)
     M = 2048
     x = torch.randn(M, 1536, generator=gen).half().cuda()
@@ -352,16 +379,21 @@ def test_split_contraction_is_stable_under_back_to_back_launches():
     d = to_device(pr)
     with linear.tune_override(splits=1):
         y0, _ = linear.forward(d.w, d.x, bias=d.bias)
-    outs = [linear.forward(d.w, d.x, bias=d.bias)[0] for _ in range(100)]
+    with linear.tune_override(bm_tiles=2, bn=256, splits=3):
+        split, _ = linear.forward(d.w, d.x, bias=d.bias)
+    with tiles_only():
+        outs = [linear.forward(d.w, d.x, bias=d.bias)[0] for _ in range(100)]
     linear.check_status()
+    assert torch.equal(outs[0], split) and not torch.equal(split, y0)      # the default plan: three parts, added up in order
     assert all(torch.equal(o, outs[0]) for o in outs), "split-K results differ between launches"
     err, rel = nf4_oracle.errors(outs[0], y0.float())
     assert err <= 2e-3 and rel <= 1e-4, (err, rel)      # same sums, only the fp32 addition order differs
     # with LoRA too: at this batch size the rank-16 projection is computed without atomics
     pl = make_problem(1536, 1536, 2048, seed=62, lora=True, dropout=0.05)
     dl = to_device(pl)
-    outs = [linear.forward(dl.w, dl.x, lora=dl.lora, mask=dl.mask, keep_scale=dl.keep_scale)[0] for _ in range(50)]
-    dxs = [linear.backward_dx(dl.w, dl.dy, lora=dl.lora, mask=dl.mask, keep_scale=dl.keep_scale)[0] for _ in range(50)]
+    with tiles_only():
+        outs = [linear.forward(dl.w, dl.x, lora=dl.lora, mask=dl.mask, keep_scale=dl.keep_scale)[0] for _ in range(50)]
+        dxs = [linear.backward_dx(dl.w, dl.dy, lora=dl.lora, mask=dl.mask, keep_scale=dl.keep_scale)[0] for _ in range(50)]
     linear.check_status()
     assert all(torch.equal(o, outs[0]) for o in outs), "forward with LoRA differs between launches"
     assert all(torch.equal(o, dxs[0]) for o in dxs), "backward-dX with LoRA differs between launches"

@@ -1,29 +1,18 @@
 """The kernel for middling batches (csrc/nf4ll_mid.cu) against the CPU oracle O1 (fp64), at the sizes where its cutting can go
 wrong: row tiles, contractions and token tiles with remainders, blocks that do not come in aligned pairs (K a multiple of 64
-only), every cluster size, several units in a row per cluster, and both directions with LoRA, mask, bias and accumulation.
+only), every cluster size, several units in a row per cluster with one accumulator and with two, and both directions with LoRA, mask, bias and accumulation.
 Its weights are the bit-exact fp16 ones and every output is one fp32 sum rounded once, so the path's tolerance applies:
 max-abs-err <= 2e-2 and rel-L2 <= 1e-3."""
-
-import contextlib
 
 import pytest
 import torch
 
 from decentrik_prime_b200 import _lib, linear
 from oracle import nf4_oracle
-from tests.problem import make_problem, oracle_weight, to_device
+from tests.problem import make_problem, mid, oracle_weight, to_device
 
 pytestmark = pytest.mark.gpu
 MAX_ABS, REL_L2 = 2e-2, 1e-3
-
-
-@contextlib.contextmanager
-def mid(rb=0, nt=0, cl=0, on=1):
-    _lib.lib().nf4ll_test_mid(on, rb, nt, cl)
-    try:
-        yield
-    finally:
-        _lib.lib().nf4ll_test_mid(0, 0, 0, 0)
 
 
 def assert_close(name, got, ref):
@@ -37,6 +26,10 @@ def launches(f):
     return out, _lib.lib().nf4ll_launch_count() - n0
 
 
+def taken():
+    return _lib.lib().nf4ll_test_mid_calls()
+
+
 # (N, K): whole tiles; half a row tile and K of 6 steps; K of 21 steps (blocks in no pairs); K of 10 steps (pairs, no quads)
 @pytest.mark.parametrize("N,K", [(256, 512), (320, 384), (1280, 1344), (1024, 640)])
 @pytest.mark.parametrize("M,rb,nt,cl", [(1, 1, 16, 1), (17, 1, 32, 2), (33, 2, 48, 1), (100, 1, 64, 3), (129, 2, 80, 2), (187, 1, 192, 2),
@@ -47,14 +40,15 @@ def test_forward_and_backward(N, K, M, rb, nt, cl):
     pr = make_problem(N, K, M, seed=N + M, lora=True, dropout=0.05, bias=True)
     ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, pr.dy, pr.bias, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)
     d = to_device(pr)
-    with mid(rb, nt, cl):
+    before = taken()
+    with mid(rb, nt, min(cl, -(-K // 256), N // 128)):                 # a cluster's CTAs take 256 steps forward, 128 backward at least
         (y, _), n = launches(lambda: linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale))
         dx, _ = linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)
         old = torch.randn(M, K).half()
         acc, _ = linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale, out=old.cuda(), accumulate=True)
         plain = linear.forward(d.w, d.x)[0]
     linear.check_status()
-    assert n == 2                                 # rank-16 projection and the product
+    assert n == 2 and taken() - before == 4       # rank-16 projection and the product
     assert_close("y", y, ref["y"])
     assert_close("dx", dx, ref["dx"])
     assert_close("dx accumulated", acc, ref["dx"] + old.double())
@@ -83,6 +77,60 @@ def test_cluster_sizes_give_the_same_bits_every_time(cl):
         assert torch.equal(other[0], first[0]) and torch.equal(other[1], first[1])
 
 
+# Units beyond the 148 CTAs or 74 pairs that a B200 holds at once. `accumulators`: how many of a unit's columns tensor memory has room for,
+# beside the slots of weights (forward) or the masked rank-16 product (backward).
+@pytest.mark.parametrize("backward,N,K,M,rb,nt,cl,mask,accumulators", [(False, 2304, 512, 3000, 2, 176, 1, False, 1), (False, 1024, 512, 3000, 2, 64, 1, False, 2),
+                                                                       (False, 1024, 512, 2600, 2, 64, 2, False, 2), (False, 1280, 768, 3100, 2, 96, 2, True, 1),
+                                                                       (True, 512, 1536, 3000, 2, 112, 1, True, 1), (True, 512, 1536, 3000, 2, 112, 1, False, 2),
+                                                                       (True, 512, 1536, 1650, 2, 64, 2, True, 2), (True, 256, 1408, 3000, 1, 224, 1, True, 1),
+                                                                       (True, 512, 1280, 3500, 1, 128, 2, True, 2)])
+def test_several_units_in_a_row(backward, N, K, M, rb, nt, cl, mask, accumulators):
+    beside = rb * nt if backward and mask else 0 if backward else 256
+    assert accumulators == (2 if 2 * rb * nt + beside <= 512 else 1)
+    pr = make_problem(N, K, M, seed=N + nt, lora=True, dropout=0.05 if mask else 0.0, bias=not backward)
+    d = to_device(pr)
+    rows = sorted({0, nt - 1, nt, M // 2, M - nt, M - 1})
+    ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x[rows], pr.dy[rows], pr.bias, pr.A16, pr.B16, pr.scale,
+                                    pr.mask[rows] if mask else None, pr.keep_scale)
+    blocks = -(-(K if backward else N) // (128 * rb))
+    assert blocks * -(-M // nt) > {1: 148, 2: 74}[cl]
+
+    def run():
+        if backward:
+            return linear.backward_dx(d.w, d.dy, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0]
+        return linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0]
+    before = taken()
+    with mid(rb, nt, cl):
+        first = run()
+        again = [run() for _ in range(5)]
+    linear.check_status()
+    assert taken() - before == 6
+    assert_close("dx" if backward else "y", first[rows], ref["dx" if backward else "y"])
+    assert all(torch.equal(a, first) for a in again)
+
+
+def test_gate_up_with_several_units_in_a_row():
+    """2 x 1152 rows, 3000 tokens in tiles of 176: 162 units on 148 CTAs, one accumulator, two slots of weights, LoRA on both halves."""
+    I, K, M = 1152, 512, 3000
+    pr = make_problem(2 * I, K, M, seed=I, lora=False)
+    g = torch.Generator().manual_seed(M)
+    lora = [((torch.randn(16, K, generator=g) / K ** 0.5).half(), (torch.randn(I, 16, generator=g) * 0.02).half(), 2.0) for _ in range(2)]
+    d = to_device(pr)
+    dev = [(a.cuda(), b.cuda(), s) for a, b, s in lora]
+    before = taken()
+    with mid(2, 176, 1):
+        first = linear.forward_gate_up(d.w, d.x, lora_gate=dev[0], lora_up=dev[1])[:3]
+        again = [linear.forward_gate_up(d.w, d.x, lora_gate=dev[0], lora_up=dev[1])[:3] for _ in range(5)]
+    linear.check_status()
+    assert taken() - before == 6
+    rows = [0, 175, 176, 1500, 2999]
+    x, w = pr.x[rows].double(), oracle_weight(pr).double()
+    for i in range(2):
+        assert_close(f"half {i}", first[i][rows], x @ w[i * I:(i + 1) * I].t() + 2.0 * (x @ lora[i][0].double().t()) @ lora[i][1].double().t())
+    assert torch.equal(first[2], linear.swiglu_forward(first[0].contiguous(), first[1].contiguous()))
+    assert all(torch.equal(a, b) for other in again for a, b in zip(other, first))
+
+
 @pytest.mark.parametrize("I,K,M,nt,cl", [(256, 512, 20, 32, 1), (320, 1024, 130, 80, 2), (1088, 1024, 300, 112, 3), (256, 512, 187, 192, 1)])
 def test_gate_up(I, K, M, nt, cl):
     """A branch whose rank-16 product is not finite does not reach the other one's columns."""
@@ -92,11 +140,13 @@ def test_gate_up(I, K, M, nt, cl):
     lora = [((torch.randn(16, K, generator=g) / K ** 0.5).half(), (torch.randn(I, 16, generator=g) * 0.02).half(), 2.0) for _ in range(2)]
     d = to_device(pr)
     dev = [(a.cuda(), b.cuda(), s) for a, b, s in lora]
+    before = taken()
     with mid(2, nt, cl):
         gate, up, h, _, _ = linear.forward_gate_up(d.w, d.x, lora_gate=dev[0], lora_up=dev[1])
         bad = (torch.full_like(dev[0][0], float("inf")), dev[0][1], 2.0)
         _, up_beside, _, _, _ = linear.forward_gate_up(d.w, d.x, lora_gate=bad, lora_up=dev[1])
     linear.check_status()
+    assert taken() - before == 2
     for i, got in enumerate((gate, up)):
         t = pr.x.double() @ lora[i][0].double().t()
         assert_close(f"half {i}", got, pr.x.double() @ w[i * I:(i + 1) * I].t() + 2.0 * t @ lora[i][1].double().t())
@@ -121,8 +171,10 @@ def test_stacked_projections():
             ref[:, at:at + n] += 2.0 * (pr.x.double() @ lora[i][0].double().t()) @ lora[i][1].double().t()
         at += n
     for rb in (1, 2):
+        before = taken()
         with mid(rb, 0, 2):
             y, _ = linear.forward_multi(d.w, d.x, segs, bias=d.bias)
+        assert taken() - before == 1
         assert_close(f"y, {rb} row blocks", y, ref)
     linear.check_status()
 
@@ -134,8 +186,10 @@ def test_values_that_are_not_finite_stay_in_their_rows():
     x = d.x.clone()
     x[7] = float("inf")
     x[9, 3] = float("nan")
+    before = taken()
     with mid(1, 64, 2):
         clean, y = linear.forward(d.w, d.x)[0], linear.forward(d.w, x)[0]
+    assert taken() - before == 2
     keep = [i for i in range(50) if i not in (7, 9)]
     assert torch.equal(y[keep], clean[keep])
     assert not torch.isfinite(y[[7, 9]]).any()
@@ -156,10 +210,12 @@ def test_short_batches_keep_the_rank16_product_in_32_bits(M, rb, nt, cl):
     d = to_device(pr)
 
     def check(x, B, scale, rows):
+        before = taken()
         with mid(rb, nt, cl):
             y, _ = linear.forward(d.w, x.cuda(), lora=(A.cuda(), B.cuda(), scale))
             multi, _ = linear.forward_multi(d.w, x.cuda(), [(256, None, None, 1.0), (384, (A.cuda(), B[:384].contiguous().cuda(), scale), None, 1.0)])
         linear.check_status()
+        assert taken() - before == 2
         ref = x.double() @ w.t() + scale * (x.double() @ A.double().t()) @ B.double().t()
         assert (y.cpu()[rows] != ref.half()[rows]).sum() <= 0.01 * N * len(rows)
         ref2 = x.double() @ w[256:].t() + scale * (x.double() @ A.double().t()) @ B[:384].double().t()

@@ -1,5 +1,5 @@
 """The rank-16 passes at the edges of their row and column tiles, against fp64: projections T of one and of two branches over the
-same rows, one launch (cluster and direct combination, 8 / 16 / 32 rows per CTA), and the gradients dA, dB whose warps each
+same rows, one launch (direct with 16 and 32 rows per CTA, through a cluster with 8, 16 and 32, by atomics), and the gradients dA, dB whose warps each
 take sixteen rows of a 64-row stage. fp32 sums of n fp16 products: relative error in the 2-norm below n 2^-24 / sqrt(n), here
 1e-5 with the hi + lo split of the fp32 operand (2^-22) included."""
 
@@ -20,8 +20,35 @@ def dropped(x, mask, ks):
     return (x.float() * ks).half().double() * mask if mask is not None else x.double()
 
 
-@pytest.mark.parametrize("M,K", [(1, 512), (7, 5120), (8, 1536), (9, 512), (17, 2048), (31, 320), (64, 4096), (65, 1536), (187, 1536), (300, 512), (2300, 512)])
-def test_projections_of_two_branches(M, K):
+def variant(M, C, n):
+    """How lora_down_launch (csrc/nf4ll_lora.cu) combines the parts of a row's sum, and the rows of a CTA, on a B200's 148 SMs."""
+    sms = 148
+    groups = {r: -(-M // r) for r in (8, 16, 32)}
+    if groups[16] * 4 >= 3 * sms:
+        return "direct", 16
+    units = -(-C // 256)
+    ks = max(1, min(2 * sms // (groups[32] * n), units))
+    if ks > 8 and M * C <= 1 << 21:
+        ks = 8
+    per = -(-units // ks)
+    ks = -(-C // (per * 256))
+    if ks == 1:
+        return "direct", 32
+    if ks > 8:
+        return "atomic", 32
+    aside = M > 16 and C > 16384
+    return "cluster", next((r for r in (8, 16) if not aside and groups[r] * ks * n <= 2 * sms), 32)
+
+
+CASES = [(1, 512, "cluster", 8), (7, 5120, "cluster", 8), (8, 1536, "cluster", 8), (9, 512, "cluster", 8), (17, 2048, "cluster", 8),
+         (31, 320, "cluster", 8), (64, 4096, "cluster", 8), (65, 1536, "cluster", 8), (187, 1536, "cluster", 8), (300, 512, "cluster", 8),
+         (2300, 512, "direct", 16), (333, 3584, "cluster", 16), (511, 3584, "cluster", 32), (63, 27648, "cluster", 32),
+         (701, 256, "direct", 32), (187, 18944, "atomic", 32)]
+
+
+@pytest.mark.parametrize("M,K,combined,rows", CASES)
+def test_projections_of_two_branches(M, K, combined, rows):
+    assert torch.cuda.get_device_properties(0).multi_processor_count != 148 or variant(M, K, 2) == (combined, rows)
     parts = (128, 128, 256)
     pr = make_problem(sum(parts), K, M, seed=M + K, lora=False)
     d = to_device(pr)

@@ -72,8 +72,8 @@ def test_small_batch_forward_variants(N, K, M):
 
 @pytest.mark.parametrize("N,K", [(256, 256), (192, 256), (256, 384), (640, 1024), (4096, 512), (256, 320), (512, 2112)])
 @pytest.mark.parametrize("M", [1, 16, 17, 33, 64])
-def test_swapped_operand_kernel_variants(N, K, M):
-    """The swapped-operand tensor-core kernel (weights as the MMA's 128-row operand, 16 / 32 / 64 token columns),
+def test_kernel_for_middling_batches_under_the_tuning_flag(N, K, M):
+    """The kernel for middling batches (weights as the MMA's 128-row operand, 16 to 64 token columns),
     forced through the tuning hook: one and several slices of the contraction, tiles with fewer than 128 weight
     rows (N = 192), last groups of one and two quantisation blocks (K = 320, 2112, 384),
     row lengths that are not a multiple of four blocks (K = 384, 320: absmax codes fetched byte by byte)."""
@@ -141,8 +141,8 @@ def test_config4_weight_stream_shapes(which):
 
 @pytest.mark.parametrize("N,K", [(18944, 3584), (3584, 18944), (3584, 3584)])
 def test_short_batches_on_7b_shapes(N, K):
-    """Every batch size class of the default dispatch (streaming kernel, swapped-operand kernel with 16 / 32 / 64
-    token columns, 128-row tiles) at the Qwen2.5-7B shapes, whose rows are 56 and 296 quantisation blocks long
+    """Every class of short batches of the default dispatch (streaming kernel, kernel for middling batches with 16 to 80
+    token columns) at the Qwen2.5-7B shapes, whose rows are 56 and 296 quantisation blocks long
     (14 and 74 groups of four): M in {1, 8, 9, 16, 24, 33, 64, 65} with LoRA, dropout and bias; y on sampled output
     columns for every token, t in full."""
     pr = make_problem(N, K, 65, seed=4500 + N % 89, lora=True, dropout=0.05, bias=True, device="cuda")

@@ -1,4 +1,4 @@
-"""The weight-streaming forward of decode-sized batches, and the swapped-operand one for gate|up: single, stacked (Q|K|V) and
+"""The weight-streaming forward of decode-sized batches, and the kernel for middling batches for gate|up: single, stacked (Q|K|V) and
 gate|up calls against the fp64 oracle of each projection, at rows of a whole and of an odd number of four quantisation
 blocks, at the edges of the token tiles, with and without the rank-16 branch (behind whose kernel the weight stream starts
 early). Tolerance as for every forward: fp16 outputs of fp32 sums."""
@@ -70,7 +70,7 @@ def test_stacked(K, M, with_lora):
         at += r
 
 
-# M = 20 on two weights of 2^24 elements: one launch of the swapped-operand kernel
+# M = 20 and 33 on two weights of 2^24 elements: one launch of the kernel for middling batches
 @pytest.mark.parametrize("I,K,M", [(256, K, M) for K in (512, 576) for M in (1, 8, 9, 16)] + [(8192, 2048, 20), (4096, 4096, 33)])
 def test_gate_up(I, K, M):
     gen = torch.Generator().manual_seed(K + M)

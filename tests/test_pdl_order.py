@@ -20,6 +20,10 @@ def kernels():
             yield os.path.basename(path), m.group(1), m.group(2), text[m.end():end]
 
 
+def body_of(name):
+    return next(k[3] for k in kernels() if k[1] == name)
+
+
 def waiting():
     return [k for k in kernels() if re.search(r"^  pdl_wait\(\);", k[3], re.M)]
 
@@ -38,3 +42,21 @@ def test_wait_comes_before_global_memory(file, name, params, body):
         assert not re.search(rf"\b{p}\s*(\[|\+)|\*\s*{p}\b|__ldg\(\s*{p}\b", before), f"{file}: {name} reads {p} before pdl_wait()"
     for s in structs:
         assert not re.search(rf"\b{s}\.\w+\s*\[", before), f"{file}: {name} reads through {s} before pdl_wait()"
+
+
+def test_the_kernel_for_middling_batches_reads_early_only_what_its_projection_does_not_write():
+    """Behind a projection of the same call (p.early) its producers, tables and decoding warps go on at once and the epilogue warps
+    wait before they touch the rank-16 product or an output; otherwise every warp waits before anything is read."""
+    body = body_of("nf4_mid_kernel")
+    roles = body.index("if (warp == 0) {")
+    prologue, rest = body[:roles], body[roles:]
+    waits = [m.start() for m in re.finditer(r"if \(!p\.early\)( \{\n)?\s+pdl_wait\(\);", prologue)]
+    assert len(waits) == 2                                      # the table warps' and the two producers'
+    assert not re.search(r"p\.(qabs|scale2|offset2|code2|mask|seg_left|seg_right|bias|out)\w*\s*(\[|\+)|tma_load", prologue[:waits[0]])
+    assert prologue.index("p.code2[") > waits[0]
+    late = rest.index("if (p.early) pdl_wait();")
+    assert rest[:late].rstrip().endswith("if (warp >= kMidEpiWarp) {")
+    assert not re.search(r"p\.(seg_left|seg_right|bias|out|out_u|out_h)\b|p\.mask\s*[+\[]", rest[:late])      # the epilogue's, all behind its wait
+    # and the host says "early" only behind a projection of the same call that it has just launched
+    host = open(os.path.join(CSRC, "nf4ll_gemm.cu")).read()
+    assert "mid_launch(c, mp, projected && !ev0, status, stream)" in host

@@ -6,6 +6,7 @@ reuse that buffer with different problems, and it must refuse problems that do n
 Collected last on purpose: a run that stops at the first failure has then already run every other test.
 """
 
+import contextlib
 import ctypes
 
 import pytest
@@ -13,7 +14,7 @@ import torch
 
 from decentrik_prime_b200 import _lib, linear
 from oracle import nf4_oracle
-from tests.problem import make_problem, oracle_weight, to_device
+from tests.problem import make_problem, oracle_weight, tiles_only, to_device
 
 pytestmark = pytest.mark.gpu
 MAX_ABS, REL_L2 = 2e-2, 1e-3
@@ -32,10 +33,11 @@ def _call(h, static, d, y, t, ws=None):
                            t.data_ptr(), M, y.data_ptr(), y.stride(0), ws.data_ptr(), ws.numel(), st.data_ptr(), stream)
 
 
-def test_static_scratch_forward_matches_workspace_forward_twice():
+@pytest.mark.parametrize("way", [contextlib.nullcontext, tiles_only], ids=["default", "tiles"])
+def test_static_scratch_forward_matches_workspace_forward_twice(way):
     h = _lib.lib()
     # two different problems in a row through the same built-in buffer: the first splits its contraction
-    # (partial sums and tile counters live in the scratch), the second does not
+    # (partial sums and tile counters live in the scratch) on the tile kernels, the second does not
     for N, K, M, seed in ((1536, 1536, 2048, 51), (512, 256, 300, 52)):
         pr = make_problem(N, K, M, seed=seed, lora=True, dropout=0.05, bias=True)
         d = to_device(pr)
@@ -46,10 +48,12 @@ def test_static_scratch_forward_matches_workspace_forward_twice():
         y_new = torch.full((M, N), float("nan"), dtype=torch.float16, device="cuda")
         t_ref = torch.empty(M, 16, dtype=torch.float32, device="cuda")
         t_new = torch.full((M, 16), float("nan"), dtype=torch.float32, device="cuda")
-        _lib.check(_call(h, False, d, y_ref, t_ref, ws))
-        torch.cuda.synchronize()
-        free_before = torch.cuda.mem_get_info()[0]
-        _lib.check(_call(h, True, d, y_new, t_new))
+        assert (need >= 3 * M * N * 4) == (N == 1536)      # three fp32 slabs of partial sums
+        with way():
+            _lib.check(_call(h, False, d, y_ref, t_ref, ws))
+            torch.cuda.synchronize()
+            free_before = torch.cuda.mem_get_info()[0]
+            _lib.check(_call(h, True, d, y_new, t_new))
         linear.check_status()
         # the call took nothing from the device: not through the runtime, not through torch's allocator
         assert torch.cuda.mem_get_info()[0] == free_before
