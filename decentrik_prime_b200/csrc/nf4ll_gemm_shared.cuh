@@ -55,6 +55,12 @@ struct GemmParams {
 constexpr uint32_t kCoopSpinLimit = 1u << 22;   // default for GemmParams::spin_limit
 constexpr int kFixSlots = 8;     // 16 KB slots of the split-K fix-up ring (fits every tile shape's operand rings)
 
+// cuTensorMapEncodeTiled, asked from the driver once (nf4ll_gemm.cu)
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                  CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+int get_encode_fn(EncodeTiledFn* out);
+
 struct Abort {
   volatile int* flag;
   int32_t* status;

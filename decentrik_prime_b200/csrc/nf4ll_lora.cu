@@ -270,9 +270,13 @@ int lora_down_launch(const void* act, int64_t ldact, const DownBranch* br, int n
   const dim3 grid(static_cast<unsigned>(row_groups), static_cast<unsigned>(ks));
   if (ks == 1) return down_run<4, kDownDirect, kDownWarps>(grid, 0, a, ldact, br, n, scale, M, C, c_per_cta, zero_ptr, zero_words, stream);
   if (ks <= 8) {
-    // fewer rows per CTA while the grid stays within two CTAs per SM: more CTAs, each with more of its loads in flight. But not
+    // Fewer rows per CTA while the grid stays within two CTAs per SM: more CTAs, each with more of its loads in flight. But not
     // where the kernel for middling batches streams a long contraction's weights meanwhile: it needs whole SMs, and the fewer
-    // this one holds the better (5120 x 27648 at 64 rows, both kernels: 46 us beside 16 CTAs of 32 rows, 53 behind 64 of 8)
+    // this one holds the better. Both kernels, 32 rows per CTA / fewer, us: 5120 x 27648 at 32, 64, 128 rows 43.8 / 47.2, 47.3 / 52.8,
+    // 56.9 / 57.0, 3584 x 18944 at 64 and 96 rows 28.8 / 31.1 and 30.2 / 35.4, 8192 x 28672 at 64 rows 66.0 / 69.4, 1536 x 17920 at 96 rows
+    // 20.6 / 24.5 (but at 187 and 333 rows 33.5 / 31.3 and 38.7 / 36.4, the worst of 33 calls beyond 128 rows), backward over the same
+    // contractions alike. With shorter ones this kernel's own time tells: 4096 x 14336 at 64 and 128 rows 35.4 / 29.9 and 38.5 / 33.2,
+    // 2048 x 11008 at 128 rows 29.8 / 25.9 (5120 x 5120 at 128 rows 19.6 / 21.6).
     const int64_t groups8 = (M + 7) / 8;
     const unsigned k = static_cast<unsigned>(ks);
     const bool aside = M > 16 && C > 16384;

@@ -812,28 +812,15 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 // ---------------------------------------------------------------------------------------------
 // Host side
 // ---------------------------------------------------------------------------------------------
-typedef CUresult (*MidEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
-                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
 static int mid_encode(CUtensorMap* map, CUtensorMapDataType type, const void* base, uint64_t inner, uint64_t outer, uint64_t stride_bytes,
                       uint32_t box_inner, uint32_t box_outer, CUtensorMapSwizzle swizzle, const char* what) {
-  static MidEncodeFn cached = nullptr;       // written once with the same value by any thread
-  if (!cached) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    NF4LL_CUDA(cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres));
-    if (qres != cudaDriverEntryPointSuccess || !fn) {
-      set_detail("cuTensorMapEncodeTiled not available from the driver");
-      return NF4LL_ERR_CUDA;
-    }
-    cached = reinterpret_cast<MidEncodeFn>(fn);
-  }
+  EncodeTiledFn encode = nullptr;
+  if (int rc = get_encode_fn(&encode)) return rc;
   const cuuint64_t dims[2] = {inner, outer};
   const cuuint64_t strides[1] = {stride_bytes};
   const cuuint32_t box[2] = {box_inner, box_outer};
   const cuuint32_t estr[2] = {1, 1};
-  const CUresult r = cached(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
+  const CUresult r = encode(map, type, 2, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_detail("cuTensorMapEncodeTiled (%s) failed with CUresult %d", what, static_cast<int>(r));
