@@ -57,7 +57,9 @@ lora_down_kernel(const __half* __restrict__ act, int64_t ldact, const DownBranch
                  int64_t c_per_cta, int* __restrict__ zero_ptr, int zero_words) {
   pdl_wait();
   pdl_launch_dependents();
-  const DownBranch& br = blockIdx.z ? second : first;
+  // Two branches in one launch only where a row's sum is cut up (short batches). The choice costs registers that the direct variant's
+  // loads need: with it 2048 x 8960 / 16384 x 18944 under a mask take 21.0 / 230 us, without 16.0 / 178.
+  const DownBranch& br = COMBINE != kDownDirect && blockIdx.z ? second : first;
   const uint8_t* __restrict__ mask = br.mask;
   const __half* __restrict__ R = br.R;
   float* __restrict__ t32 = br.t32;
@@ -233,14 +235,18 @@ int zero_words_launch(int* words, int n, cudaStream_t stream) {
 template <int RG, int COMBINE, int NW>
 static int down_run(dim3 grid, unsigned cluster_y, const __half* a, int64_t ldact, const DownBranch* br, int n, float scale, int64_t M, int64_t C,
                     int64_t c_per_cta, int* zero_ptr, int zero_words, cudaStream_t stream) {
-  grid.z = static_cast<unsigned>(n);
-  PdlLaunch lc(grid, dim3(NW * 32), 0, stream, cluster_y ? 1 : 0, cluster_y);
-  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<RG, COMBINE, NW>, a, ldact, br[0], br[n - 1], scale, M, C, c_per_cta, zero_ptr, zero_words));
+  const int launches = COMBINE == kDownDirect ? n : 1;
+  grid.z = static_cast<unsigned>(n / launches);
+  for (int i = 0; i < launches; ++i) {
+    PdlLaunch lc(grid, dim3(NW * 32), 0, stream, cluster_y ? 1 : 0, cluster_y);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_down_kernel<RG, COMBINE, NW>, a, ldact, br[i], br[n - 1], scale, M, C, c_per_cta, zero_ptr,
+                                  i == 0 ? zero_words : 0));
+  }
   return NF4LL_OK;
 }
 
-// t32 (fp32 [M,16]) = scale * (drop(act) . R^T), R [16,C] row-major, for one branch or for two over the same rows in one launch
-// (q and v of a layer, gate and up: a second launch cost a decoded layer 4 us). `zero_ptr` / `zero_words`: optional 32-bit words
+// t32 (fp32 [M,16]) = scale * (drop(act) . R^T), R [16,C] row-major, for one branch or for two over the same rows, in one launch
+// where the rows are few (q and v of a layer, gate and up: a second launch cost a decoded layer 4 us). `zero_ptr` / `zero_words`: optional 32-bit words
 // the kernel clears on the way (see the kernel).
 int lora_down_launch(const void* act, int64_t ldact, const DownBranch* br, int n, float scale, int64_t M, int64_t C, int* zero_ptr, int zero_words,
                      cudaStream_t stream) {
@@ -310,7 +316,8 @@ int lora_down_launch(const void* act, int64_t ldact, const uint8_t* mask, int64_
 // splits their side values into fp16 hi + lo fragments in registers (two MMAs recover ~22 mantissa bits) and contracts them
 // against all 64 columns (ldmatrix.trans delivers the row-major act tile as the MMA's k-by-n operand), so that the warps of a CTA
 // meet once, at the end: with three block barriers per stage and the side transposed through shared memory 2048 rows of
-// 8960 + 1536 columns took 25 us, 20.5 now. Row ranges
+// 8960 + 1536 columns took 21.3 us (dropout on the 1536) and 24.0 (on the 8960) with operands out of HBM, 18.2 and 21.6 now; 21.0 and 23.5
+// with operands in L2, 17.1 and 20.0 now. The three of them in an MLP block's step at 2048 rows: 578 us with the former kernel, 568 with this. Row ranges
 // of different CTAs are combined with fp32 atomics, so the summation order across ranges is not fixed.
 // out index = j * ld_j + c * ld_c: dA[16,K] uses (K, 1), dB[N,16] uses (1, 16).
 // ---------------------------------------------------------------------------------------------

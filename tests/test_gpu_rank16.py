@@ -6,7 +6,7 @@ take sixteen rows of a 64-row stage. fp32 sums of n fp16 products: relative erro
 import pytest
 import torch
 
-from decentrik_prime_b200 import linear
+from decentrik_prime_b200 import _lib, linear
 from tests.problem import make_problem, to_device
 
 pytestmark = pytest.mark.gpu
@@ -59,8 +59,16 @@ def test_projections_of_two_branches(M, K, combined, rows):
     for on in ((0, 2), (0, 1, 2), (1,)):
         segs = [(n, (lora[i][0].cuda(), lora[i][1].cuda(), 2.0) if i in on else None, masks[i].cuda() if i in on and masks[i] is not None else None, ks[i])
                 for i, n in enumerate(parts)]
+        before = _lib.lib().nf4ll_launch_count()
         _, t = linear.forward_multi(d.w, d.x, segs)
+        launches = _lib.lib().nf4ll_launch_count() - before
         linear.check_status()
+        with_t = [(*s, ti) if ti is not None else s for s, ti in zip(segs, t)]
+        before = _lib.lib().nf4ll_launch_count()
+        linear.forward_multi(d.w, d.x, with_t)
+        launches -= _lib.lib().nf4ll_launch_count() - before
+        # two branches in a launch but where a CTA has whole rows: the choice between them costs those kernels a fifth of their speed
+        assert launches == (len(on) if combined == "direct" else (len(on) + 1) // 2)
         for i in on:
             assert rel(t[i], dropped(pr.x, masks[i], ks[i]) @ lora[i][0].double().t()) < 1e-5, (on, i)
 
