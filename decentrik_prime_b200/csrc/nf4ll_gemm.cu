@@ -1256,7 +1256,8 @@ constexpr int64_t kStreamCapRows = 64;     // its limit (reachable through the t
 constexpr int64_t kMidLeastRows = 9;       // below, the streaming kernel keeps its exact fp32 scales, and is the faster one nearly everywhere
 constexpr int64_t kMidSmallWeights = int64_t(1) << 24;
 
-// Which kernel computes a forward of M rows that neither the kernel for middling batches nor the dense GEMM takes: the tile
+// Which kernel computes a forward of M rows that neither the kernel for middling batches nor the dense GEMM takes (from 17 to 128
+// rows: only weights of 2^31 quantisation blocks and more, forced tiles, the hooks that keep the former out): the tile
 // kernels (kTiles) or the register-level weight-streaming kernel for decode-sized batches (kStream). Bit 1 of the tuning flags
 // forces kStream up to that kernel's limit.
 enum : int { kTiles = 0, kStream = 1 };
@@ -1788,7 +1789,8 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     if (!odd && dense && ((g_tune.flags & kFlagDense) || t.dense < t.decoding)) return run_dense(dc, sms, static_cast<uint8_t*>(workspace), status, stream);
   }
   if (odd) {
-    // short batches and odd widths: the two projections on their own, then the stand-alone gated product
+    // What the kernel for middling batches leaves of short batches and odd widths: up to 16 rows, both halves in one pass; otherwise
+    // the two projections on their own, then the stand-alone gated product.
     int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, false, g_tune);
     if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;
     if (kind != kTiles) {
