@@ -1457,7 +1457,10 @@ static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lor
   if (c.M > kMidMostRows) return false;
   if (c.mode == kFwd && c.M <= kStreamMaxRows) {
     if (c.M < kMidLeastRows || (c.n_seg > 1 && !c.gu_inter) || (c.gu_inter ? N / 2 : N) * K < kMidSmallWeights) return false;
-    return mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp) && 1.05 * mp->us < stream_time_us(N, K, c.M, sms) + (c.gu_inter ? 4 : 0);
+    if (!mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
+    // The streaming kernel where both models put it 5 % ahead. At 16 rows, that one / this one, us: 27648 x 5120 33.9 / 35.4, 18944 x 3584
+    // 17.5 / 18.7, 5120 x 27648 39.9 / 40.3; 3584 x 18944 21.2 / 24.6, 9728 x 2560 9.5 / 17.4, 4096 x 4096 9.3 / 11.3.
+    return c.gu_inter ? 1.05 * mp->us < stream_gate_up_line_us(N, K, c.M, sms) : mp->us < 1.05 * stream_time_us(N, K);
   }
   if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
   if (c.M <= kDenseNeverRows) return true;
@@ -1601,7 +1604,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   if (segments && (narrow_tiles || tune.bn == 512)) tune.bn = narrow_tiles ? 128 : 256;
   Plan pl = make_plan(mode, M, NO, KC, lora ? lora->r : 0, sms, tune);
   int kind = forward_kind(mode, M, segments != nullptr, g_tune);
-  if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;      // it copies the absmax codes word by word
+  if (kind == kStream && ((reinterpret_cast<uintptr_t>(W->qabs) & 3) || !stream_takes(W->N, W->K, false))) kind = kTiles;
   const int force_slices = (tune.flags & 2) ? tune.splits : 0;
   const int64_t need = kind == kTiles ? pl.total() : pl.left_bytes + pl.bt_bytes;
   if (need > 0) {
@@ -1702,7 +1705,8 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
       c.seg_b[i] = segments ? p.seg_right[i] : (lora ? p.lora_right : nullptr);
       c.seg_scale[i] = segments ? p.seg_scale[i] : (lora ? lora->scale : 0.f);
     }
-    const int rc = stream_forward_launch(c, projected && !ev0, force_slices, stream);
+    c.withhold = hooks.withhold.what; c.wait_us = hooks.withhold.wait_us;
+    const int rc = stream_forward_launch(c, projected && !ev0, force_slices, status, stream);
     if (rc == NF4LL_OK && ev1) { if (int rce = record_event(ev1, stream)) return rce; }
     return rc;
   }
@@ -1792,12 +1796,13 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     // What the kernel for middling batches leaves of short batches and odd widths: up to 16 rows, both halves in one pass; otherwise
     // the two projections on their own, then the stand-alone gated product.
     int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, false, g_tune);
-    if (kind == kStream && (reinterpret_cast<uintptr_t>(W->qabs) & 3)) kind = kTiles;
+    if (kind == kStream && ((reinterpret_cast<uintptr_t>(W->qabs) & 3) || !stream_takes(W->N, W->K, true))) kind = kTiles;
     if (kind != kTiles) {
       // both halves in one pass over the weights
       StreamCall c{};
       c.W = W; c.x = x; c.ldx = ldx; c.M = M;
-      c.y = g; c.ldy = ldg; c.y2 = u; c.ldy2 = ldu; c.split = I;
+      c.withhold = hooks.withhold.what; c.wait_us = hooks.withhold.wait_us;
+      c.y = g; c.ldy = ldg; c.split = I; c.y2 = u; c.ldy2 = ldu; c.h = h; c.ldh = ldh;
       c.n_seg = 2;
       const nf4ll_lora* br[2] = {lora_gate, lora_up};
       void* tout[2] = {t_gate, t_up};
@@ -1814,9 +1819,9 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
       cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
       g_ev_start = g_ev_stop = nullptr;
       if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
-      if (int rc = stream_forward_launch(c, t.any && !ev0, 0, stream)) return rc;
+      if (int rc = stream_forward_launch(c, t.any && !ev0, 0, status, stream)) return rc;
       if (ev1) { if (int rce = record_event(ev1, stream)) return rce; }
-      return nf4ll_swiglu_forward(g, ldg, u, ldu, h, ldh, M, I, stream_v);
+      return NF4LL_OK;
     }
     const nf4ll_mat wg = sub_rows(W, 0, I), wu = sub_rows(W, I, I);
     if (int rc = run_gemm(kFwd, &wg, x, ldx, nullptr, lora_gate, t_gate, M, g, ldg, 0, workspace, workspace_bytes, status, stream_v)) return rc;

@@ -12,20 +12,28 @@ struct StreamCall {
   const void* bias;
   void* y;
   int64_t ldy;
-  void* y2;                              // rows from `split` on go here, null: one output
-  int64_t ldy2, split;
+  int64_t split;                         // gate|up: rows of a half
+  void* y2;                              // its second half's output
+  int64_t ldy2;
+  void* h;                               // silu(first half) * second half; null: not gate|up
+  int64_t ldh;
   int n_seg;                             // projections stacked along N
   int64_t seg_end[kMaxSegments];         // first row after the segment
   const float* seg_t[kMaxSegments];      // [M, 16] fp32 rank-16 product of the segment, null: no LoRA
   const __half* seg_b[kMaxSegments];     // its lora_B, indexed by the row of W
   float seg_scale[kMaxSegments];
+  int withhold;                          // failure-detection hook
+  uint32_t wait_us;
 };
 
-// What the streaming kernel takes for M <= 16 tokens, up to the fixed cost of a launch: a fit through the times of five
-// shapes from 3584 x 3584 to 27648 x 5120 at 1 to 16 tokens (0.6 us per block of the busiest warp, and the token rows).
-double stream_time_us(int64_t N, int64_t K, int64_t M, int sms);
+// What the kernel takes for 9 to 16 tokens, behind other calls and without a rank-16 branch: a fit (nf4ll_stream.cu, stream_us)
+double stream_time_us(int64_t N, int64_t K);
+// Gate|up of 9 to 16 rows goes to the kernel for middling batches where its model is below this
+double stream_gate_up_line_us(int64_t N, int64_t K, int64_t M, int sms);
+// Whether the kernel takes weights of this size (rows as long as eight CTAs hold the tokens of them in registers: 43008 weights)
+bool stream_takes(int64_t N, int64_t K, bool gate_up);
 // `early`: the kernel launched right before on the stream is a rank-16 projection of the same call
-int stream_forward_launch(const StreamCall& c, bool early, int force_team, cudaStream_t stream);
+int stream_forward_launch(const StreamCall& c, bool early, int force, int32_t* status, cudaStream_t stream);
 
 int zero_words_launch(int* words, int n, cudaStream_t stream);      // nf4ll_lora.cu
 

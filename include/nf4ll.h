@@ -285,10 +285,11 @@ int nf4ll_read_status(const int32_t* status, void* stream);
  * flags bit 1: run a forward of at most 64 rows on the register-level weight-streaming kernel (default: up to
  * 16 rows); flags bit 2: run a forward of one projection and at most 64 rows on the kernel for middling batches (weights
  * as the MMA's row operand; default: from 17 rows on while a model of its time is ahead, and 9 to 16 rows against weights of
- * at least 2^24 elements where models of both kernels' times say so); flags bit 3: never
+ * at least 2^24 elements unless models of both kernels' times put the streaming kernel 5 % ahead); flags bit 3: never
  * dequantise into the workspace, whatever its size (the kernel for middling batches stays open); flags bit 4: do so for any number of rows if the workspace holds
  * 2 N K + 192 M + 32 N + 2048 bytes. With bit 1 `splits` forces the number of warps
- * that share a unit of rows (even: units of 16 rows, odd: of 32), with bit 2 the number of slices of the contraction (8 at most). Size the workspace of such calls with nf4ll_workspace_bytes_tuned. */
+ * that share a tile of rows (low byte; as many as its rows are blocks long, and as hold the tokens), CTAs of a cluster (next byte)
+ * and teams of warps (next byte), zeros leave the choice to the kernel; with bit 2 the number of slices of the contraction (8 at most). Size the workspace of such calls with nf4ll_workspace_bytes_tuned. */
 void nf4ll_tune_override(int32_t bm_tiles, int32_t bn, int32_t splits, int32_t flags);
 
 /* Measurement hook; no counterpart in the reference. The calling thread's NEXT nf4ll_forward /
@@ -333,7 +334,8 @@ int64_t nf4ll_test_mid_searches(void);
 /* Failure-detection test hook; no counterpart in the reference. In the calling thread's NEXT forward or backward-dX call, if the
  * kernel for middling batches takes it, no CTA loads codes after its first stage (what = 1), the rank-16 operands are never
  * announced (2), or the last CTA of every cluster never announces its partial sums (3), and the waits of whole warps end after
- * wait_us microseconds (instead of a second). The waits for what is missing run out: the cause is recorded in the status word, the
+ * wait_us microseconds (instead of a second); if the weight-streaming kernel takes it, no codes are copied (1), or the last CTA of
+ * every cluster never announces its sums (3). The waits for what is missing run out: the cause is recorded in the status word, the
  * kernel ends, the call's output is undefined, the context stays usable and later calls are unaffected. One-shot. */
 void nf4ll_test_mid_withhold(int32_t what, uint32_t wait_us);
 

@@ -1,0 +1,100 @@
+"""How the streaming kernel cuts a call up, at its edges: rows of one quantisation block and of as many as one CTA holds and one more
+(a cluster), tiles that go round teams, stages and buffers several times, clusters whose last CTA has fewer blocks, absmax codes off a
+16-byte boundary, gate|up with its product in the launch and behind it. Against the fp64 oracle, with the tolerance of every forward."""
+
+import pytest
+import torch
+
+from decentrik_prime_b200 import _lib, linear
+from oracle import nf4_oracle
+from tests.problem import make_problem, oracle_weight, tiles_only, to_device
+from tests.test_gpu_linear import assert_close
+
+pytestmark = pytest.mark.gpu
+COPIES, CLUSTER_SUMS = 1, 3
+
+
+def reference(pr):
+    return nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, None, pr.bias, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)["y"]
+
+
+def forward(d, w=None):
+    y = linear.forward(w or d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)[0]
+    linear.check_status()
+    return y
+
+
+# 84 blocks to a CTA up to 8 tokens (5376 weights), 60 beyond (3840); 9728 rows: five tiles for some CTAs, four for others
+@pytest.mark.parametrize("N,K", [(256, 64), (256, 448), (192, 5376), (256, 5440), (256, 8128), (192, 3840), (256, 3904), (9728, 512), (19456, 64)])
+@pytest.mark.parametrize("M", [1, 5, 8, 9, 16])
+def test_edges(N, K, M):
+    pr = make_problem(N, K, M, seed=N + K + M, lora=True, dropout=0.05, bias=True, device="cuda" if N * K > 1 << 22 else "cpu")
+    with tiles_only():
+        assert_close("y", forward(to_device(pr)), reference(pr))
+
+
+# warps of a team | CTAs of a cluster | teams (beyond 8 tokens two at most): every size of a cluster, parts of one to seven blocks
+@pytest.mark.parametrize("np,cl,teams", [(12, 1, 1), (2, 1, 4), (3, 1, 2), (6, 1, 2), (1, 2, 1), (5, 3, 2), (2, 4, 2), (4, 5, 1), (1, 6, 4), (7, 7, 1), (2, 8, 1), (3, 2, 4)])
+@pytest.mark.parametrize("M", [3, 13])
+def test_forced_cuts(np, cl, teams, M):
+    pr = make_problem(9728, 832, M, seed=np + cl + teams, lora=True, dropout=0.05, bias=True, device="cuda")      # 13 blocks a row, 608 tiles
+    d = to_device(pr)
+    with linear.tune_override(splits=np | cl << 8 | teams << 16, flags=2):
+        y = forward(d)
+    assert_close("y", y, reference(pr))
+
+
+@pytest.mark.parametrize("K", [512, 5440])
+def test_absmax_codes_off_a_boundary(K):
+    d = to_device(make_problem(256, K, 6, seed=K, lora=True, dropout=0.05, bias=True))
+    room = torch.empty(d.w.qabs.numel() + 16, dtype=torch.uint8, device="cuda")
+    room[4:4 + d.w.qabs.numel()] = d.w.qabs
+    shifted = linear.Nf4Weight(d.w.packed, room[4:4 + d.w.qabs.numel()], d.w.scale2, d.w.offset2, d.w.code2, d.w.N, d.w.K)
+    assert shifted.qabs.data_ptr() % 16 == 4
+    assert torch.equal(forward(d, shifted), forward(d))
+
+
+# halves of 640 and 9472 rows; in one launch up to 8 tokens, beyond only where a CTA holds a row
+@pytest.mark.parametrize("inter,K,launches", [(640, 512, (1, 1)), (9472, 256, (1, 1)), (640, 5632, (1, 2))])
+@pytest.mark.parametrize("M", [1, 8, 11])
+def test_gate_up(inter, K, launches, M):
+    gate, up = (make_problem(inter, K, M, seed=inter + K + i, lora=True, dropout=0.05, device="cuda") for i in (0, 1))
+    d = [to_device(p) for p in (gate, up)]
+    stacked = [torch.cat([getattr(e.w, n) for e in d]) for n in ("packed", "qabs", "scale2", "offset2")]
+    w = linear.Nf4Weight(*stacked, d[0].w.code2, 2 * inter, K)
+    h = _lib.lib()
+    with tiles_only():
+        linear.forward_gate_up(w, d[0].x)      # (its scratch)
+    _lib.lib().nf4ll_test_mid(-1, 0, 0, 0)
+    try:
+        before = h.nf4ll_launch_count()
+        linear.forward_gate_up(w, d[0].x)
+        assert h.nf4ll_launch_count() - before == launches[M > 8]
+        g, u, product, _, _ = linear.forward_gate_up(w, d[0].x, d[0].lora, d[0].mask, d[1].lora, d[1].mask, gate.keep_scale)
+    finally:
+        _lib.lib().nf4ll_test_mid(0, 0, 0, 0)
+    linear.check_status()
+    up.x = gate.x
+    assert_close("g", g, reference(gate))
+    assert_close("u", u, reference(up))
+    assert torch.equal(product, linear.swiglu_forward(g.contiguous(), u.contiguous()))
+
+
+@pytest.mark.parametrize("what,K,M,words", [(COPIES, 512, 1, {0x0801, 0x0802, 0x0806}), (COPIES, 512, 16, {0x0801, 0x0802, 0x0806}),
+                                            (COPIES, 6144, 8, {0x0801, 0x0802, 0x0806, 0x0807}), (CLUSTER_SUMS, 6144, 8, {0x0807, 0x0804, 0x0806})])
+def test_expired_waits(what, K, M, words):
+    """Copies that are never asked for, sums of a cluster that are never announced (nf4ll_test_mid_withhold; limit 20 ms): the kernel
+    ends, the status word holds a wait that depends on them, and the same call gives the same bits again."""
+    d = to_device(make_problem(4096, K, M, seed=K + M, lora=True, dropout=0.05, bias=True, device="cuda"))
+    with tiles_only():
+        good = forward(d).clone()
+        _lib.lib().nf4ll_test_mid_withhold(what, 20000)
+        linear.forward(d.w, d.x, bias=d.bias, lora=d.lora, mask=d.mask, keep_scale=d.keep_scale)
+        with pytest.raises(_lib.Nf4llError) as info:
+            linear.check_status()
+        assert "wait" in str(info.value)
+        word = int(linear.status_word(d.x.device).item())
+        linear.status_word(d.x.device).zero_()
+        assert word in words, hex(word)
+        for _ in range(3):
+            assert torch.equal(forward(d), good)
