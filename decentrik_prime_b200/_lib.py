@@ -141,6 +141,29 @@ class Segment(ctypes.Structure):
                 ("t_ready", ctypes.c_int32)]
 
 
+class Grad(ctypes.Structure):
+    """struct nf4ll_grad (include/nf4ll.h)."""
+    _fields_ = [("dy", ctypes.c_void_p), ("lddy", ctypes.c_int64), ("x", ctypes.c_void_p), ("ldx", ctypes.c_int64),
+                ("mask", ctypes.c_void_p), ("ld_mask", ctypes.c_int64), ("keep_scale", ctypes.c_float), ("t", ctypes.c_void_p),
+                ("u", ctypes.c_void_p), ("scale", ctypes.c_float), ("N", ctypes.c_int64), ("K", ctypes.c_int64),
+                ("dA", ctypes.c_void_p), ("dB", ctypes.c_void_p)]
+
+
+class Gated(ctypes.Structure):
+    """struct nf4ll_gated (include/nf4ll.h)."""
+    _fields_ = ([f for n in ("g", "u", "dh", "dg", "du") for f in ((n, ctypes.c_void_p), ("ld" + n, ctypes.c_int64))]
+                + [("mask", ctypes.c_void_p), ("ld_mask", ctypes.c_int64), ("keep_scale", ctypes.c_float)]
+                + [(n, ctypes.c_void_p) for n in ("t_gate", "t_up", "u_down", "Bt_gate", "Bt_up")]
+                + [("scale_gate", ctypes.c_float), ("scale_up", ctypes.c_float)]
+                + [(n, ctypes.c_void_p) for n in ("u_gate", "u_up", "dB_gate", "dB_up", "dA_down")])
+
+
+class Expand(ctypes.Structure):
+    """struct nf4ll_expand (include/nf4ll.h)."""
+    _fields_ = [("u", ctypes.c_void_p), ("A", ctypes.c_void_p), ("mask", ctypes.c_void_p), ("ld_mask", ctypes.c_int64),
+                ("keep_scale", ctypes.c_float)]
+
+
 _vp, _i64, _i32, _f32 = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int32, ctypes.c_float
 _MAT, _LORA, _SEG = ctypes.POINTER(Nf4Mat), ctypes.POINTER(LoraArgs), ctypes.POINTER(Segment)
 
@@ -160,6 +183,8 @@ SIGNATURES = {
     "nf4ll_lora_down": (_i32, [_vp, _i64, _vp, _i64, _f32, _vp, _f32, _i32, _i64, _i64, _vp, _vp, _vp]),
     "nf4ll_lora_grads": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _f32, _vp, _vp, _f32, _i32, _i64, _i64, _i64,
                                 _vp, _vp, _i32, _vp]),
+    "nf4ll_lora_grads_batch": (_i32, [ctypes.POINTER(Grad), _i32, _i64, _i32, _vp]),
+    "nf4ll_lora_expand": (_i32, [ctypes.POINTER(Expand), _i32, _i64, _i64, _vp, _i64, _vp]),
     "nf4ll_workspace_bytes_fast": (_i64, [_i64, _i64, _i64, _i32]),
     "nf4ll_workspace_bytes_tuned": (_i64, [_i64, _i64, _i64, _i32, _i32, _i32, _i32]),
     "nf4ll_tune_override": (None, [_i32, _i32, _i32, _i32]),
@@ -175,6 +200,8 @@ SIGNATURES = {
     "nf4ll_rms_backward": (_i32, [_vp, _i64, _f32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _LORA, _vp, _LORA, _vp, _vp]),
     "nf4ll_swiglu_forward": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _vp]),
     "nf4ll_swiglu_backward": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _vp]),
+    "nf4ll_gated_backward_bytes": (_i64, [_i64, _i64]),
+    "nf4ll_gated_backward": (_i32, [ctypes.POINTER(Gated), _i64, _i64, _i32, _vp, _i64, _vp]),
     "nf4ll_lora_project": (_i32, [_vp, _i64, _vp, _i64, _f32, _vp, _f32, _i64, _i64, _vp, _vp]),
     "nf4ll_lora_shadow": (_i32, [_vp, _vp, _i64, _i64, _vp, _vp, _vp, _vp]),
     "nf4ll_attention_forward": (_i32, [_vp, _i64, _vp, _i32, _i64, _i32, _i32, _i32, _vp, _vp, _i64, _vp, _i64, _vp, _vp]),

@@ -212,6 +212,45 @@ class MlpBlock:
         if self._grad_slice is not None and not accumulate_grads:
             self._grad_slice.zero_()
             accumulate_grads = True
+        if self.fused_glue and self.gate.has_lora and self.up.has_lora and self.down.has_lora:
+            dx = self._backward_joined(g, u, dy, need_dx, accumulate_grads, out)
+        else:
+            dx = self._backward_each(g, u, dy, need_dx, accumulate_grads, out)
+        self._saved = None
+        return dx
+
+    def _backward_joined(self, g, u, dy, need_dx, accumulate_grads, out):
+        """With LoRA on every projection. One pass over g, u and dh forms dg and du and takes from them, and from h, all that the
+        branches need of [M, inter] matrices; the LoRA terms of dx are expanded first (two dropout masks) and one product over
+        the stacked weight adds [dg | du] . W to them; what is left of the factors' gradients is one more launch. Two roundings
+        of dx, like the reference's fp16 add (solution/fast_qwen.py:1320-1323), the first of them of the small LoRA terms."""
+        gate, up, down = self.projections
+        (x, mg, kg, tg), (_, mu, ku, tu), (h, md, kd, td) = (p._saved for p in self.projections)
+        gs = self.grad_stream
+        gu = g._base
+        dh, ud = linear.backward_dx(down.w, dy, lora=down.lora, mask=md, keep_scale=kd, want_u=True)
+        ug, uu = linear.gated_backward(g, u, dh, md, kd, tg, tu, ud, (gate.B16t, gate.scale), (up.B16t, up.scale), gate.dB, up.dB,
+                                       down.dA, accumulate_grads)
+        grads = [(dy, h, td, ud, down.scale, None, 1.0, None, down.dB), (g, x, tg, ug, gate.scale, mg, kg, gate.dA, None),
+                 (u, x, tu, uu, up.scale, mu, ku, up.dA, None)]
+        if gs is not None:
+            gs.wait_stream(torch.cuda.current_stream(dy.device))
+            with torch.cuda.stream(gs):
+                linear.lora_grads_batch(grads, accumulate_grads)
+        dx = None
+        if need_dx:
+            dx = out if out is not None else torch.empty(dy.shape[0], self.hidden, dtype=torch.float16, device=dy.device)
+            linear.lora_expand([(ug, gate.A16, mg, kg), (uu, up.A16, mu, ku)], dx)
+            linear.backward_dx(self.w_gu, gu, out=dx, accumulate=True)
+        if gs is not None:
+            torch.cuda.current_stream(dy.device).wait_stream(gs)
+        else:
+            linear.lora_grads_batch(grads, accumulate_grads)
+        for p in self.projections:
+            p._saved = None
+        return dx
+
+    def _backward_each(self, g, u, dy, need_dx, accumulate_grads, out):
         gs, pend = self.grad_stream, self._pending
         dh = self.down.backward(dy, accumulate_grads=accumulate_grads, grad_stream=gs, pending=pend)
         if self.fused_glue:
@@ -223,13 +262,10 @@ class MlpBlock:
             du = (dhf * gf * sig).half()
             dg = (dhf * u.float() * sig * (1.0 + gf * (1.0 - sig))).half()
         dx = self.gate.backward(dg, out=out, need_dx=need_dx, accumulate_grads=accumulate_grads, grad_stream=gs, pending=pend)
-        # d(input) of gate and up are summed into one buffer: the second launch adds its fp32 result to the
-        # fp16 values the first one stored and rounds again (two roundings, like the reference's fp16 add,
-        # solution/fast_qwen.py:1320-1323)
+        # the second launch adds its fp32 result to the fp16 values the first one stored and rounds again
         dx = self.up.backward(du, out=dx, accumulate=need_dx, need_dx=need_dx, accumulate_grads=accumulate_grads,
                               grad_stream=gs, pending=pend)
         if gs is not None:
             torch.cuda.current_stream(dy.device).wait_stream(gs)
             pend.clear()
-        self._saved = None
         return dx

@@ -367,19 +367,59 @@ __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
+// Two fp32 values side by side in a register pair: one instruction for both, each rounded as the scalar one.
+__device__ __forceinline__ uint64_t f32x2(float lo, float hi) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ float2 f32x2_split(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ uint64_t half2_to_f32x2(uint32_t w) {
+  const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w));
+  return f32x2(v.x, v.y);
+}
+__device__ __forceinline__ uint32_t f32x2_to_half2(uint64_t v) {
+  const float2 f = f32x2_split(v);
+  return pack_half2_rn(f.x, f.y);
+}
+
 // drop(x) on 8 packed fp16 values: fp16(x * keep_scale) where the mask byte is non-zero, else 0
-// (reference solution/k_norm.py:49-53: scale in fp32, then one rounding to fp16).
+// (reference solution/k_norm.py:49-53: scale in fp32, then one rounding to fp16). Four bytes of the mask at a time: the top bit of each
+// is set where it is not zero, and prmt spreads that bit over the value's sixteen.
 __device__ __forceinline__ uint4 drop8(uint4 raw, uint2 m, float keep_scale) {
-  uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
+  const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};
   const uint32_t mw[2] = {m.x, m.y};
+  const uint64_t ks = f32x2(keep_scale, keep_scale);
+  uint32_t o[4];
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float2 v = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-    const bool k0 = ((mw[j >> 1] >> ((2 * j & 3) * 8)) & 0xffu) != 0;
-    const bool k1 = ((mw[j >> 1] >> (((2 * j + 1) & 3) * 8)) & 0xffu) != 0;
-    w[j] = pack_half2_rn(k0 ? v.x * keep_scale : 0.f, k1 ? v.y * keep_scale : 0.f);
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t on = ((mw[j] & 0x7f7f7f7fu) + 0x7f7f7f7fu) | mw[j];
+    uint32_t lo, hi;
+    asm("prmt.b32 %0, %1, 0, 0x9988;" : "=r"(lo) : "r"(on));
+    asm("prmt.b32 %0, %1, 0, 0xbbaa;" : "=r"(hi) : "r"(on));
+    o[2 * j] = f32x2_to_half2(mul2(half2_to_f32x2(w[2 * j]), ks)) & lo;
+    o[2 * j + 1] = f32x2_to_half2(mul2(half2_to_f32x2(w[2 * j + 1]), ks)) & hi;
   }
-  return make_uint4(w[0], w[1], w[2], w[3]);
+  return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
 // one whole 32-byte sector (dst 32-byte aligned)
@@ -407,28 +447,54 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
                     pack_half2_rn(f[6], f[7]));
 }
 
-// sigmoid through the special-function unit: ex2.approx and rcp.approx, a few ulp of fp32 - far inside
-// the fp16 rounding of the results
-__device__ __forceinline__ float fast_sigmoid(float a) { return __fdividef(1.0f, 1.0f + __expf(-a)); }
-
-__device__ __forceinline__ uint4 swiglu_fwd8(const uint4& gv, const uint4& uv) {
-  float a[8], b[8], o[8];
-  unpack8(gv, a); unpack8(uv, b);
-#pragma unroll
-  for (int j = 0; j < 8; ++j) o[j] = a[j] * fast_sigmoid(a[j]) * b[j];
-  return pack8(o);
+// sigmoid = 1 / (1 + 2^(-a log2 e)) through the special-function unit: ex2.approx and rcp.approx, a few ulp of fp32 - far inside
+// the fp16 rounding of the results. Their flushing forms: a power that underflows adds nothing to the 1, and a sigmoid that does comes
+// with a result that is zero in fp16.
+constexpr float kMinusLog2e = -1.4426950408889634f;
+__device__ __forceinline__ float ex2_ftz(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float fast_sigmoid(float a) { return rcp_ftz(1.0f + ex2_ftz(a * kMinusLog2e)); }
+__device__ __forceinline__ uint64_t fast_sigmoid2(uint64_t a) {
+  const float2 e = f32x2_split(mul2(a, f32x2(kMinusLog2e, kMinusLog2e)));
+  const float2 d = f32x2_split(add2(f32x2(ex2_ftz(e.x), ex2_ftz(e.y)), f32x2(1.0f, 1.0f)));
+  return f32x2(rcp_ftz(d.x), rcp_ftz(d.y));
 }
 
-__device__ __forceinline__ void swiglu_bwd8(const uint4& gv, const uint4& uv, const uint4& dv, uint4& og4, uint4& ou4) {
-  float a[8], b[8], d[8], og[8], ou[8];
-  unpack8(gv, a); unpack8(uv, b); unpack8(dv, d);
+__device__ __forceinline__ uint4 swiglu_fwd8(const uint4& gv, const uint4& uv) {
+  const uint32_t g[4] = {gv.x, gv.y, gv.z, gv.w}, u[4] = {uv.x, uv.y, uv.z, uv.w};
+  uint32_t o[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) {
-    const float sig = fast_sigmoid(a[j]);
-    ou[j] = d[j] * (a[j] * sig);
-    og[j] = (d[j] * b[j]) * sig * (1.0f + a[j] * (1.0f - sig));
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t a = half2_to_f32x2(g[j]);
+    o[j] = f32x2_to_half2(mul2(mul2(a, fast_sigmoid2(a)), half2_to_f32x2(u[j])));
   }
-  og4 = pack8(og); ou4 = pack8(ou);
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// dg, du; and h once more, as swiglu_fwd8 gives it (unused, it costs nothing)
+__device__ __forceinline__ void swiglu_bwd8(const uint4& gv, const uint4& uv, const uint4& dv, uint4& og4, uint4& ou4, uint4& oh4) {
+  const uint32_t g[4] = {gv.x, gv.y, gv.z, gv.w}, u[4] = {uv.x, uv.y, uv.z, uv.w}, dh[4] = {dv.x, dv.y, dv.z, dv.w};
+  uint32_t og[4], ou[4], oh[4];
+  const uint64_t one = f32x2(1.0f, 1.0f), minus = f32x2(-1.0f, -1.0f);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const uint64_t a = half2_to_f32x2(g[j]), b = half2_to_f32x2(u[j]), d = half2_to_f32x2(dh[j]);
+    const uint64_t sig = fast_sigmoid2(a), silu = mul2(a, sig);
+    ou[j] = f32x2_to_half2(mul2(d, silu));
+    oh[j] = f32x2_to_half2(mul2(silu, b));
+    og[j] = f32x2_to_half2(mul2(mul2(mul2(d, b), sig), fma2(a, fma2(sig, minus, one), one)));
+  }
+  og4 = make_uint4(og[0], og[1], og[2], og[3]);
+  ou4 = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+  oh4 = make_uint4(oh[0], oh[1], oh[2], oh[3]);
 }
 
 }  // namespace nf4ll

@@ -334,22 +334,8 @@ constexpr int kGradStageBytes = kGradActBytes + kGradMaskBytes + kGradSideBytes;
 constexpr int kGradSmemBytes = kGradRing * kGradStageBytes;
 static_assert(4 * 16 * (kGradCols + 1) * 4 <= kGradRing * kGradStageBytes, "the final reduction reuses the ring");
 
-__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
-  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
-               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
-               : "r"(addr));
-}
-// 16 bytes global -> shared, or 16 zero bytes when `valid` is false (src must still be an address)
-__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
-  const int n = valid ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// One column reduction. A launch carries up to two of them (dA and dB of one projection): column
-// tiles [0, tiles_first) of the grid belong to the first, the rest to the second.
+// One column reduction. A launch carries several of them (dA and dB of one projection or of three): column
+// tiles [end[i-1], end[i]) of the grid belong to problem i.
 struct GradProblem {
   const __half* act;
   int64_t ldact;
@@ -364,12 +350,20 @@ struct GradProblem {
   int64_t ld_j, ld_c;
 };
 
+constexpr int kGradProblems = 6;
+struct GradBatch {
+  GradProblem problem[kGradProblems];
+  int end[kGradProblems];
+  int n;
+};
+
 __global__ void __launch_bounds__(kGradThreads, 4)
-lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_first, int64_t M) {
+lora_grad_kernel(const __grid_constant__ GradBatch batch, int64_t M) {
   pdl_wait();
   pdl_launch_dependents();
-  const bool is_first = static_cast<int>(blockIdx.x) < tiles_first;
-  const GradProblem& pb = is_first ? first : second;
+  int which = 0;
+  while (static_cast<int>(blockIdx.x) >= batch.end[which]) ++which;
+  const GradProblem& pb = batch.problem[which];
   const __half* __restrict__ act = pb.act;
   const int64_t ldact = pb.ldact;
   const uint8_t* __restrict__ mask = pb.mask;
@@ -385,7 +379,7 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
   const uint32_t ring = smem_u32(g_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int64_t c0 = static_cast<int64_t>(is_first ? blockIdx.x : blockIdx.x - tiles_first) * kGradCols;
+  const int64_t c0 = static_cast<int64_t>(static_cast<int>(blockIdx.x) - (which ? batch.end[which - 1] : 0)) * kGradCols;
   const int64_t r_begin = static_cast<int64_t>(blockIdx.y) * rows_per_cta;
   const int64_t r_end = (r_begin + rows_per_cta < M) ? r_begin + rows_per_cta : M;
   float acc[8][4];
@@ -425,12 +419,6 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
     }
     cp_async_commit();
   };
-  // two values of side as fp16 pairs hi + lo
-  auto split = [](float a, float b, uint32_t& hi, uint32_t& lo) {
-    hi = pack_half2_rn(a, b);
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
-    lo = pack_half2_rn(a - f.x, b - f.y);
-  };
 #pragma unroll
   for (int s0 = 0; s0 < kGradRing - 1; ++s0) issue(r_begin + s0 * kGradStage, s0);
   int it = 0;
@@ -453,10 +441,10 @@ lora_grad_kernel(const GradProblem first, const GradProblem second, int tiles_fi
     }
     const float* sd = reinterpret_cast<const float*>(st + kGradActBytes + kGradMaskBytes) + (kb + 2 * t) * kSideStride + g;
     uint32_t ah0, ah1, ah2, ah3, al0, al1, al2, al3;
-    split(sd[0], sd[kSideStride], ah0, al0);
-    split(sd[8], sd[kSideStride + 8], ah1, al1);
-    split(sd[8 * kSideStride], sd[9 * kSideStride], ah2, al2);
-    split(sd[8 * kSideStride + 8], sd[9 * kSideStride + 8], ah3, al3);
+    split_half2(sd[0], sd[kSideStride], ah0, al0);
+    split_half2(sd[8], sd[kSideStride + 8], ah1, al1);
+    split_half2(sd[8 * kSideStride], sd[9 * kSideStride], ah2, al2);
+    split_half2(sd[8 * kSideStride + 8], sd[9 * kSideStride + 8], ah3, al3);
     const uint32_t act_base = ring + (it % kGradRing) * kGradStageBytes;
 #pragma unroll
     for (int np = 0; np < 4; ++np) {     // pairs of 8-column tiles
@@ -511,35 +499,144 @@ static GradPlan grad_plan(int64_t M, int64_t C, int64_t sms, int64_t other_tiles
   return g;
 }
 
-// dA = u^T . drop(x) (u carries the LoRA scale, reference solution/fast_qwen.py:1370-1371) and / or
-// dB = scale * dy^T . t (fast_qwen.py:1369), in one launch.
-static int lora_grads_launch(const void* dy, int64_t lddy, const void* x, int64_t ldx, const uint8_t* mask, int64_t ld_mask,
-                             float keep_scale, const void* t32, const void* u32, float scale, int64_t M, int64_t N, int64_t K,
-                             void* dA, void* dB, cudaStream_t stream) {
+// For each of n projections dA = u^T . drop(x) (u carries the LoRA scale, reference solution/fast_qwen.py:1370-1371) and / or
+// dB = scale * dy^T . t (fast_qwen.py:1369), all in one launch: row ranges are as long as one wave of CTAs over all of them allows.
+static int lora_grads_launch(const nf4ll_grad* grads, int n, int64_t M, cudaStream_t stream) {
   int dev = 0, sms = 148;
   NF4LL_CUDA(cudaGetDevice(&dev));
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   NF4LL_CUDA(cudaFuncSetAttribute(lora_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmemBytes));
-  const int64_t tiles_a = dA ? (K + kGradCols - 1) / kGradCols : 0;
-  const int64_t tiles_b = dB ? (N + kGradCols - 1) / kGradCols : 0;
-  GradProblem pa{}, pbb{};
-  int64_t ms = 1;
-  if (dA) {
-    const GradPlan g = grad_plan(M, K, sms, tiles_b);
-    pa = GradProblem{static_cast<const __half*>(x), ldx, mask, ld_mask, keep_scale, static_cast<const float*>(u32), 1.0f, K,
-                     g.rows_per, static_cast<float*>(dA), K, 1};
-    ms = g.msplit;
+  int64_t tiles = 0;
+  for (int i = 0; i < n; ++i) tiles += (grads[i].dA ? (grads[i].K + kGradCols - 1) / kGradCols : 0) + (grads[i].dB ? (grads[i].N + kGradCols - 1) / kGradCols : 0);
+  GradBatch b{};
+  int64_t ranges = 1, at = 0;
+  auto add = [&](GradProblem pr) {
+    const GradPlan g = grad_plan(M, pr.C, sms, tiles - (pr.C + kGradCols - 1) / kGradCols);
+    pr.rows_per_cta = g.rows_per;
+    at += g.col_tiles;
+    b.problem[b.n] = pr;
+    b.end[b.n++] = static_cast<int>(at);
+    if (g.msplit > ranges) ranges = g.msplit;
+  };
+  for (int i = 0; i < n; ++i) {
+    const nf4ll_grad& g = grads[i];
+    if (g.dA) add(GradProblem{static_cast<const __half*>(g.x), g.ldx, g.mask, g.ld_mask, g.keep_scale, static_cast<const float*>(g.u), 1.0f, g.K, 0, static_cast<float*>(g.dA), g.K, 1});
+    if (g.dB) add(GradProblem{static_cast<const __half*>(g.dy), g.lddy, nullptr, 0, 1.0f, static_cast<const float*>(g.t), g.scale, g.N, 0, static_cast<float*>(g.dB), 1, 16});
   }
-  if (dB) {
-    const GradPlan g = grad_plan(M, N, sms, tiles_a);
-    pbb = GradProblem{static_cast<const __half*>(dy), lddy, nullptr, 0, 1.0f, static_cast<const float*>(t32), scale, N,
-                      g.rows_per, static_cast<float*>(dB), 1, 16};
-    if (g.msplit > ms) ms = g.msplit;
-  }
-  dim3 grid(static_cast<unsigned>(tiles_a + tiles_b), static_cast<unsigned>(ms));
-  PdlLaunch lc(grid, dim3(kGradThreads), kGradSmemBytes, stream);
-  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_grad_kernel, pa, pbb, static_cast<int>(tiles_a), M));
+  PdlLaunch lc(dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(ranges)), dim3(kGradThreads), kGradSmemBytes, stream);
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_grad_kernel, b, M));
   return NF4LL_OK;
+}
+
+static int clear_grad(const nf4ll_grad& g, cudaStream_t stream) {
+  // gradients that lie back to back are cleared by one fill
+  const bool joined = g.dA && g.dB && static_cast<float*>(g.dB) == static_cast<float*>(g.dA) + 16 * g.K;
+  if (g.dA) NF4LL_CUDA(cudaMemsetAsync(g.dA, 0, sizeof(float) * 16 * (joined ? g.K + g.N : g.K), stream));
+  if (g.dB && !joined) NF4LL_CUDA(cudaMemsetAsync(g.dB, 0, sizeof(float) * 16 * g.N, stream));
+  return NF4LL_OK;
+}
+
+static int check_grad(const nf4ll_grad& g, const char* who) {
+  if (g.N <= 0 || g.K <= 0 || g.N % 8 || g.K % 8) {
+    set_detail("%s: N=%lld K=%lld (multiples of 8)", who, static_cast<long long>(g.N), static_cast<long long>(g.K));
+    return NF4LL_ERR_SHAPE;
+  }
+  if (g.dA && (!g.x || !g.u)) { set_detail("%s: dA needs x and u", who); return NF4LL_ERR_NULL; }
+  if (g.dB && (!g.dy || !g.t)) { set_detail("%s: dB needs dy and t", who); return NF4LL_ERR_NULL; }
+  auto off = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
+  if ((g.dA && (off(g.x) || g.ldx % 8 || off(g.u) || (g.mask && (off(g.mask) || g.ld_mask % 16)))) || (g.dB && (off(g.dy) || g.lddy % 8 || off(g.t)))) {
+    set_detail("%s: activations, t and u 16-byte aligned, leading dimensions multiples of 8; mask 16-byte aligned, ld_mask multiple of 16", who);
+    return NF4LL_ERR_ALIGN;
+  }
+  return NF4LL_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// out[M,K] = fp16(sum over branches of drop(u . A)), A [16,K] fp16, u [M,16] fp32 (two fp16 parts of it: 22 bits), under the keep-mask of
+// the branch's input: the LoRA terms of d(input) of projections that share an input, whose base terms one product adds to it. Two of
+// them could not share a GEMM's epilogue otherwise (two masks on one tile). A CTA takes 64 columns, whose factors its warps
+// keep in registers, and goes through blocks of sixteen rows. 2 B written and 1 B of mask read per branch and element.
+// ---------------------------------------------------------------------------------------------
+constexpr int kExpandWarps = 4, kExpandCols = 64;
+struct ExpandBranch {
+  const float* u;
+  const __half* A;
+  const uint8_t* mask;
+  int64_t ld_mask;
+  float keep_scale;
+};
+
+template <int N>
+__global__ void __launch_bounds__(kExpandWarps * 32)
+lora_expand_kernel(const ExpandBranch first, const ExpandBranch second, __half* __restrict__ out, int64_t ldo, int64_t M, int64_t K) {
+  pdl_wait();
+  pdl_launch_dependents();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int64_t c0 = static_cast<int64_t>(blockIdx.x) * kExpandCols;
+  // Tile j of a group of 32 columns holds columns 8 i + 2 j, + 1 for i = 0..3, so that lane (g, t) ends with columns 8 t .. 8 t + 7 of
+  // its rows in registers: 16-byte stores, 8-byte reads of the mask
+  constexpr int kGroups = kExpandCols / 32;
+  uint32_t b0[N][kGroups][4], b1[N][kGroups][4];   // ranks 2 t, 2 t + 1 and + 8 of the tile's column g
+#pragma unroll
+  for (int n = 0; n < N; ++n) {
+    const __half* A = n ? second.A : first.A;
+#pragma unroll
+    for (int q = 0; q < kGroups; ++q)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t c = c0 + 32 * q + 8 * (g >> 1) + 2 * j + (g & 1);
+        auto at = [&](int rank) { return c < K ? static_cast<uint32_t>(__half_as_ushort(__ldg(A + rank * K + c))) : 0u; };
+        b0[n][q][j] = at(2 * t) | at(2 * t + 1) << 16;
+        b1[n][q][j] = at(2 * t + 8) | at(2 * t + 9) << 16;
+      }
+  }
+  const int64_t step = static_cast<int64_t>(gridDim.y) * kExpandWarps * 16;
+  for (int64_t m0 = (static_cast<int64_t>(blockIdx.y) * kExpandWarps + warp) * 16; m0 < M; m0 += step) {
+    const int64_t row[2] = {m0 + g, m0 + g + 8};
+    float v[kGroups][2][8];                        // columns 8 t .. 8 t + 7 of each row
+#pragma unroll
+    for (int n = 0; n < N; ++n) {
+      const ExpandBranch& br = n ? second : first;
+      uint32_t hi[4], lo[4];                       // (row g, ranks 2t..), (row g + 8, same), (row g, ranks 2t + 8..), (row g + 8, same)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int64_t r = row[i & 1];
+        const float2 f = r < M ? __ldcg(reinterpret_cast<const float2*>(br.u + r * 16 + 2 * t + 8 * (i >> 1))) : make_float2(0.f, 0.f);
+        split_half2(f.x, f.y, hi[i], lo[i]);
+      }
+      uint2 keep[kGroups][2];
+#pragma unroll
+      for (int q = 0; q < kGroups; ++q)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int64_t c = c0 + 32 * q + 8 * t;
+          keep[q][i] = br.mask && row[i] < M && c < K ? __ldg(reinterpret_cast<const uint2*>(br.mask + row[i] * br.ld_mask + c)) : make_uint2(0, 0);
+        }
+#pragma unroll
+      for (int q = 0; q < kGroups; ++q)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float c[4] = {0.f, 0.f, 0.f, 0.f};
+          mma16816(c, hi[0], hi[1], hi[2], hi[3], b0[n][q][j], b1[n][q][j]);
+          mma16816(c, lo[0], lo[1], lo[2], lo[3], b0[n][q][j], b1[n][q][j]);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int e = 2 * j + (i & 1);
+            const uint32_t k = (e < 4 ? keep[q][i >> 1].x : keep[q][i >> 1].y) & 0xffu << 8 * (e & 3);
+            const float d = !br.mask ? c[i] : k ? c[i] * br.keep_scale : 0.f;
+            v[q][i >> 1][e] = n ? v[q][i >> 1][e] + d : d;
+          }
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < kGroups; ++q)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int64_t c = c0 + 32 * q + 8 * t;
+        if (row[i] < M && c < K) *reinterpret_cast<uint4*>(out + row[i] * ldo + c) = pack8(v[q][i]);
+      }
+  }
 }
 
 }  // namespace nf4ll
@@ -577,27 +674,60 @@ extern "C" int nf4ll_lora_grads(const void* dy, int64_t lddy, const void* x, int
   using namespace nf4ll;
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   if (r != 16) { set_detail("nf4ll_lora_grads: rank %d", r); return NF4LL_ERR_RANK; }
-  if (M < 0 || N <= 0 || K <= 0 || (N % 8) || (K % 8)) {
-    set_detail("nf4ll_lora_grads: M=%lld N=%lld K=%lld (N, K multiples of 8)", (long long)M, (long long)N, (long long)K);
-    return NF4LL_ERR_SHAPE;
-  }
-  if (dA && (!x || !u32)) { set_detail("nf4ll_lora_grads: dA needs x and u"); return NF4LL_ERR_NULL; }
-  if (dB && (!dy || !t32)) { set_detail("nf4ll_lora_grads: dB needs dy and t"); return NF4LL_ERR_NULL; }
-  if ((dA && ((reinterpret_cast<uintptr_t>(x) & 15) || (ldx % 8))) || (dB && ((reinterpret_cast<uintptr_t>(dy) & 15) || (lddy % 8))) ||
-      (dA && mask && ((reinterpret_cast<uintptr_t>(mask) & 15) || ld_mask % 16)) || (dA && (reinterpret_cast<uintptr_t>(u32) & 15)) ||
-      (dB && (reinterpret_cast<uintptr_t>(t32) & 15))) {
-    set_detail("nf4ll_lora_grads: activations, t and u 16-byte aligned, leading dimensions multiples of 8; mask 16-byte aligned, ld_mask multiple of 16");
-    return NF4LL_ERR_ALIGN;
-  }
+  if (M < 0) { set_detail("nf4ll_lora_grads: M=%lld", static_cast<long long>(M)); return NF4LL_ERR_SHAPE; }
+  const nf4ll_grad one{dy, lddy, x, ldx, mask, ld_mask, keep_scale, t32, u32, scale, N, K, dA, dB};
+  if (int rc = check_grad(one, "nf4ll_lora_grads")) return rc;
   if (int rc = require_sm100()) return rc;
-  if (!accumulate) {
-    // gradients that lie back to back are cleared by one fill
-    const bool joined = dA && dB && static_cast<float*>(dB) == static_cast<float*>(dA) + 16 * K;
-    if (dA) NF4LL_CUDA(cudaMemsetAsync(dA, 0, sizeof(float) * 16 * (joined ? K + N : K), stream));
-    if (dB && !joined) NF4LL_CUDA(cudaMemsetAsync(dB, 0, sizeof(float) * 16 * N, stream));
-  }
+  if (!accumulate)
+    if (int rc = clear_grad(one, stream)) return rc;
   if (M > 0 && (dA || dB))
-    if (int rc = lora_grads_launch(dy, lddy, x, ldx, mask, ld_mask, keep_scale, t32, u32, scale, M, N, K, dA, dB, stream)) return rc;
+    if (int rc = lora_grads_launch(&one, 1, M, stream)) return rc;
+  return NF4LL_OK;
+}
+
+extern "C" int nf4ll_lora_grads_batch(const nf4ll_grad* grads, int32_t n, int64_t M, int32_t accumulate, void* stream_v) {
+  using namespace nf4ll;
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  const char* who = "nf4ll_lora_grads_batch";
+  if (!grads) { set_detail("%s: null pointer", who); return NF4LL_ERR_NULL; }
+  if (M < 0 || n < 1 || n > kGradProblems / 2) { set_detail("%s: M=%lld, %d projections (1..%d)", who, static_cast<long long>(M), n, kGradProblems / 2); return NF4LL_ERR_SHAPE; }
+  bool any = false;
+  for (int i = 0; i < n; ++i) {
+    if (int rc = check_grad(grads[i], who)) return rc;
+    any |= grads[i].dA || grads[i].dB;
+  }
+  if (!any) return NF4LL_OK;
+  if (int rc = require_sm100()) return rc;
+  for (int i = 0; i < n && !accumulate; ++i)
+    if (int rc = clear_grad(grads[i], stream)) return rc;
+  return M > 0 ? lora_grads_launch(grads, n, M, stream) : static_cast<int>(NF4LL_OK);
+}
+
+extern "C" int nf4ll_lora_expand(const nf4ll_expand* branches, int32_t n, int64_t M, int64_t K, void* out, int64_t ldo, void* stream) {
+  using namespace nf4ll;
+  const char* who = "nf4ll_lora_expand";
+  if (!branches || !out) { set_detail("%s: null pointer", who); return NF4LL_ERR_NULL; }
+  if (M < 0 || K <= 0 || K % 8 || n < 1 || n > 2) { set_detail("%s: M=%lld K=%lld, %d branches (1..2)", who, static_cast<long long>(M), static_cast<long long>(K), n); return NF4LL_ERR_SHAPE; }
+  auto off = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) & 15) != 0; };
+  ExpandBranch br[2]{};
+  for (int i = 0; i < n; ++i) {
+    const nf4ll_expand& b = branches[i];
+    if (!b.u || !b.A) { set_detail("%s: a branch needs u and A", who); return NF4LL_ERR_NULL; }
+    if (off(b.u) || off(b.A) || (b.mask && (off(b.mask) || b.ld_mask % 16))) { set_detail("%s: u, A and mask 16-byte aligned, ld_mask a multiple of 16", who); return NF4LL_ERR_ALIGN; }
+    br[i] = ExpandBranch{static_cast<const float*>(b.u), static_cast<const __half*>(b.A), b.mask, b.ld_mask, b.keep_scale};
+  }
+  if (off(out) || ldo % 8 || ldo < K) { set_detail("%s: out 16-byte aligned, its leading dimension a multiple of 8 and >= K", who); return NF4LL_ERR_ALIGN; }
+  if (M == 0) return NF4LL_OK;
+  if (int rc = require_sm100()) return rc;
+  int dev = 0, sms = 148;
+  NF4LL_CUDA(cudaGetDevice(&dev));
+  NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // four CTAs per SM at most, each with a block of rows per warp at least
+  const int64_t tiles = (K + kExpandCols - 1) / kExpandCols, blocks = (M + 16 * kExpandWarps - 1) / (16 * kExpandWarps);
+  int64_t y = (4 * static_cast<int64_t>(sms) + tiles - 1) / tiles;
+  y = y < blocks ? y : blocks;
+  PdlLaunch lc(dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(y)), dim3(kExpandWarps * 32), 0, static_cast<cudaStream_t>(stream));
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, n == 2 ? lora_expand_kernel<2> : lora_expand_kernel<1>, br[0], br[1], static_cast<__half*>(out), ldo, M, K));
   return NF4LL_OK;
 }
 

@@ -5,6 +5,27 @@
 
 namespace nf4ll {
 
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2, uint32_t& r3) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+               : "r"(addr));
+}
+// 16 bytes global -> shared, or 16 zero bytes when `valid` is false (src must still be an address)
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, bool valid) {
+  const int n = valid ? 16 : 0;
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// two values as fp16 pairs hi + lo: 22 bits of each
+__device__ __forceinline__ void split_half2(float a, float b, uint32_t& hi, uint32_t& lo) {
+  hi = pack_half2_rn(a, b);
+  const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
+  lo = pack_half2_rn(a - f.x, b - f.y);
+}
+
 struct DownBranch {
   const uint8_t* mask;      // keep-mask of the activation, may be null
   int64_t ld_mask;

@@ -490,6 +490,76 @@ PyObject* py_lora_grads(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   });
 }
 
+struct Items {                            // the elements of a tuple or list
+  PyObject* o;
+  explicit Items(PyObject* seq, const char* what) : o(PySequence_Fast(seq, what)) { if (!o) throw PyRaised(); }
+  ~Items() { Py_DECREF(o); }
+  Py_ssize_t size() const { return PySequence_Fast_GET_SIZE(o); }
+  PyObject* operator[](Py_ssize_t i) const { return PySequence_Fast_GET_ITEM(o, i); }
+};
+
+// lora_grads_batch(((dy, x, t, u, scale, mask, keep_scale, dA, dB), ...), accumulate)
+PyObject* py_lora_grads_batch(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  ARGS(2);
+  return guarded([&]() -> PyObject* {
+    const Items list(a[0], "projections must be a sequence");
+    if (list.size() < 1) value_error("one projection at least");
+    std::vector<nf4ll_grad> grads;
+    int64_t M = 0;
+    for (Py_ssize_t i = 0; i < list.size(); ++i) {
+      const Items it(list[i], "a projection is (dy, x, t, u, scale, mask, keep_scale, dA, dB)");
+      if (it.size() != 9) value_error("a projection is (dy, x, t, u, scale, mask, keep_scale, dA, dB)");
+      const at::Tensor &dy = tensor(it[0], "dy"), &x = tensor(it[1], "x"), &t = tensor(it[2], "t"), &u = tensor(it[3], "u");
+      if (x.dim() != 2 || dy.dim() != 2) value_error("x and dy must be matrices");
+      if (i == 0) M = x.size(0);
+      const int64_t K = x.size(1), N = dy.size(1);
+      if (x.size(0) != M) value_error("the projections of one call have as many rows each");
+      check_act(x, K, "x");
+      check_act(dy, N, "dy", M);
+      check_side(t, M * kRank, "t");
+      check_side(u, M * kRank, "u");
+      Lora m;
+      m.set_mask(optional(it[5], "mask"), true);
+      Lora::fit_mask(optional(it[5], "mask"), M, K);
+      const at::Tensor *dA = optional(it[7], "dA"), *dB = optional(it[8], "dB");
+      if (dA) check_side(*dA, kRank * K, "dA");
+      if (dB) check_side(*dB, kRank * N, "dB");
+      grads.push_back({dy.data_ptr(), ld(dy), x.data_ptr(), ld(x), m.c.mask, m.c.ld_mask, static_cast<float>(number(it[6])), t.data_ptr(), u.data_ptr(),
+                       static_cast<float>(number(it[4])), N, K, ptr(dA), ptr(dB)});
+    }
+    const Items first(list[0], "a projection");
+    check(nf4ll_lora_grads_batch(grads.data(), static_cast<int32_t>(grads.size()), M, PyObject_IsTrue(a[1]), Call(tensor(first[1], "x")).stream));
+    Py_RETURN_NONE;
+  });
+}
+
+// lora_expand(((u, A16, mask, keep_scale), ...), out)
+PyObject* py_lora_expand(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  ARGS(2);
+  return guarded([&]() -> PyObject* {
+    const at::Tensor& out = tensor(a[1], "out");
+    if (out.dim() != 2) value_error("out must be a matrix");
+    const int64_t M = out.size(0), K = out.size(1);
+    check_act(out, K, "out");
+    const Items list(a[0], "branches must be a sequence");
+    std::vector<nf4ll_expand> branches;
+    for (Py_ssize_t i = 0; i < list.size(); ++i) {
+      const Items it(list[i], "a branch is (u, A16, mask, keep_scale)");
+      if (it.size() != 4) value_error("a branch is (u, A16, mask, keep_scale)");
+      const at::Tensor &u = tensor(it[0], "u"), &A = tensor(it[1], "lora_A");
+      check_side(u, M * kRank, "u");
+      if (A.scalar_type() != at::kHalf || !A.is_contiguous() || !A.is_cuda() || A.dim() != 2 || A.size(0) != kRank || A.size(1) != K)
+        value_error("lora_A shadow must be contiguous CUDA fp16 [16, %lld]", static_cast<long long>(K));
+      Lora m;
+      m.set_mask(optional(it[2], "mask"));
+      Lora::fit_mask(optional(it[2], "mask"), M, K);
+      branches.push_back({u.data_ptr(), A.data_ptr(), m.c.mask, m.c.ld_mask, static_cast<float>(number(it[3]))});
+    }
+    check(nf4ll_lora_expand(branches.data(), static_cast<int32_t>(branches.size()), M, K, out.data_ptr(), ld(out), Call(out).stream));
+    Py_RETURN_NONE;
+  });
+}
+
 // lora_u(dy, B16t, scale) -> u fp32 [M, 16] = scale * dy . B
 PyObject* py_lora_u(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   ARGS(3);
@@ -553,6 +623,41 @@ PyObject* py_swiglu_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
     check(nf4ll_swiglu_backward(g.data_ptr(), ld(g), u.data_ptr(), ld(u), dh.data_ptr(), ld(dh), dg.data_ptr(), ld(dg), du.data_ptr(), ld(du), M, I,
                                 Call(g).stream));
     Py_RETURN_NONE;
+  });
+}
+
+// gated_backward(g, u, dh, dg, du, mask, keep_scale, t_gate, t_up, u_down, B16t_gate, B16t_up, scale_gate, scale_up, dB_gate, dB_up, dA_down,
+//                accumulate) -> (u_gate, u_up), fp32 [M, 16] each
+PyObject* py_gated_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  ARGS(18);
+  return guarded([&]() -> PyObject* {
+    const at::Tensor &g = tensor(a[0], "g"), &u = tensor(a[1], "u"), &dh = tensor(a[2], "dh"), &dg = tensor(a[3], "dg"), &du = tensor(a[4], "du");
+    if (g.dim() != 2) value_error("g must be a matrix");
+    const int64_t M = g.size(0), I = g.size(1);
+    check_act(g, I, "g");
+    check_act(u, I, "u", M);
+    check_act(dh, I, "dh", M);
+    check_act(dg, I, "dg", M);
+    check_act(du, I, "du", M);
+    Lora m;
+    m.set_mask(optional(a[5], "mask"), true);
+    Lora::fit_mask(optional(a[5], "mask"), M, I);
+    const at::Tensor &tg = tensor(a[7], "t_gate"), &tu = tensor(a[8], "t_up"), &ud = tensor(a[9], "u_down"), &bg = tensor(a[10], "B16t of gate"),
+                     &bu = tensor(a[11], "B16t of up"), &dbg = tensor(a[14], "dB of gate"), &dbu = tensor(a[15], "dB of up"), &dad = tensor(a[16], "dA of down");
+    for (const auto* t : {&tg, &tu, &ud}) check_side(*t, M * kRank, "t and u");
+    for (const auto* t : {&dbg, &dbu, &dad}) check_side(*t, I * kRank, "dA and dB");
+    for (const auto* b : {&bg, &bu})
+      if (b->scalar_type() != at::kHalf || b->dim() != 2 || b->size(0) != kRank || b->size(1) != I || !b->is_contiguous() || !b->is_cuda())
+        value_error("lora_B transposed shadow must be contiguous CUDA fp16 [16, %lld]", static_cast<long long>(I));
+    at::Tensor ug = empty({M, kRank}, at::kFloat, g), uu = empty({M, kRank}, at::kFloat, g);
+    const int64_t bytes = nf4ll_gated_backward_bytes(M, I);
+    at::Tensor scratch = empty({std::max<int64_t>(bytes, 1)}, at::kByte, g);
+    const nf4ll_gated p{g.data_ptr(), ld(g), u.data_ptr(), ld(u), dh.data_ptr(), ld(dh), dg.data_ptr(), ld(dg), du.data_ptr(), ld(du), m.c.mask, m.c.ld_mask,
+                        static_cast<float>(number(a[6])), tg.data_ptr(), tu.data_ptr(), ud.data_ptr(), bg.data_ptr(), bu.data_ptr(),
+                        static_cast<float>(number(a[12])), static_cast<float>(number(a[13])), ug.data_ptr(), uu.data_ptr(), dbg.data_ptr(), dbu.data_ptr(),
+                        dad.data_ptr()};
+    check(nf4ll_gated_backward(&p, M, I, PyObject_IsTrue(a[17]), scratch.data_ptr(), bytes, Call(g).stream));
+    return pair(wrap(&ug), wrap(&uu));
   });
 }
 
@@ -891,6 +996,7 @@ PyObject* py_setup(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
 
 #define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(py_##name)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {METHOD(forward), METHOD(forward_multi), METHOD(forward_gate_up), METHOD(backward_dx), METHOD(lora_grads), METHOD(lora_u), METHOD(lora_shadow),
+                         METHOD(lora_grads_batch), METHOD(lora_expand), METHOD(gated_backward),
                          METHOD(swiglu_forward), METHOD(swiglu_backward), METHOD(rms_forward), METHOD(rms_backward), METHOD(dequant),
                          METHOD(attention_forward), METHOD(attention_backward), METHOD(linear), METHOD(set_tune), METHOD(setup), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "host path between PyTorch tensors and libnf4ll.so", -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -149,6 +149,20 @@ def lora_u(dy, B16t, scale):
     return _lib.host().lora_u(dy, B16t, scale)
 
 
+def lora_grads_batch(projections, accumulate=False):
+    """lora_grads of up to three projections over as many rows each, in one launch: (dy, x, t, u, scale, mask, keep_scale,
+    dA, dB) of each, dA or dB None to leave it out."""
+    _lib.host().lora_grads_batch(projections, accumulate)
+
+
+def lora_expand(branches, out):
+    """out[M,K] = fp16(sum over one or two branches (u, A16, mask, keep_scale) of keep_scale * mask (.) (u . A)): the LoRA
+    terms of d(input) of projections that share an input (reference solution/fast_qwen.py:1376-1377), to which one
+    backward_dx(..., out=out, accumulate=True) over the stacked weight adds the rest."""
+    _lib.host().lora_expand(branches, out)
+    return out
+
+
 def nf4_lora_linear(x, w: Nf4Weight, bias=None, lora=None, mask=None, keep_scale=1.0):
     """Differentiable y = NF4Linear(x) + LoRA(x). `lora` = (A fp32 [16,K], B fp32 [N,16], scale) with
     A and B ordinary parameters: they receive fp32 gradients; W is frozen (no dW)."""
@@ -168,3 +182,11 @@ def swiglu_backward(g, u, dh, inplace=True):
     du = u if inplace else torch.empty_like(u)
     _lib.host().swiglu_backward(g, u, dh, dg, du)
     return dg, du
+
+
+def gated_backward(g, u, dh, mask, keep_scale, t_gate, t_up, u_down, gate, up, dB_gate, dB_up, dA_down, accumulate=False):
+    """swiglu_backward in place (g becomes dg, u becomes du), and in the same pass what LoRA branches on gate, up and down take
+    from the matrices it holds: returns (u_gate, u_up), fp32 [M,16] = scale * dg . B (lora_u would read dg again for it), and
+    writes dB_gate, dB_up (scale * dg^T . t) and dA_down (u_down^T . drop(silu(g) * u)). `gate`, `up`: (B16t, scale) of each."""
+    return _lib.host().gated_backward(g, u, dh, g, u, mask, keep_scale, t_gate, t_up, u_down, gate[0], up[0], gate[1], up[1],
+                                      dB_gate, dB_up, dA_down, accumulate)

@@ -473,8 +473,8 @@ class NormedDecoderLayer:
         pq, pv = P["q_proj"], P["v_proj"]
         uq = linear.lora_u(dqkv[:, :H], pq.B16t, pq.scale)
         uv = linear.lora_u(dqkv[:, H + KV:], pv.B16t, pv.scale)
-        linear.lora_grads(dqkv[:, :H], y1, tq, uq, pq.scale, mask=mq, keep_scale=ks, dA=pq.dA, dB=pq.dB, accumulate=True)
-        linear.lora_grads(dqkv[:, H + KV:], y1, tv, uv, pv.scale, mask=mv, keep_scale=ks, dA=pv.dA, dB=pv.dB, accumulate=True)
+        linear.lora_grads_batch([(dqkv[:, :H], y1, tq, uq, pq.scale, mq, ks, pq.dA, pq.dB),
+                                 (dqkv[:, H + KV:], y1, tv, uv, pv.scale, mv, ks, pv.dA, pv.dB)], accumulate=True)
         self._saved = None
         if not need_dx:
             return None, None

@@ -215,6 +215,38 @@ int nf4ll_lora_grads(const void* dy, int64_t lddy, const void* x, int64_t ldx, c
                      float scale, int32_t r, int64_t M, int64_t N, int64_t K,
                      void* dA, void* dB, int32_t accumulate, void* stream);
 
+/* The same for up to three projections over M rows each (gate, up and down of an MLP block) in one launch. */
+typedef struct nf4ll_grad {
+  const void* dy;           /* __half [M, lddy], N columns */
+  int64_t lddy;
+  const void* x;            /* __half [M, ldx], K columns */
+  int64_t ldx;
+  const uint8_t* mask;      /* [M, ld_mask] or NULL */
+  int64_t ld_mask;
+  float keep_scale;
+  const void* t;            /* fp32 [M,16] */
+  const void* u;            /* fp32 [M,16] */
+  float scale;
+  int64_t N, K;
+  void* dA;                 /* fp32 [16,K] or NULL */
+  void* dB;                 /* fp32 [N,16] or NULL */
+} nf4ll_grad;
+int nf4ll_lora_grads_batch(const nf4ll_grad* grads, int32_t n, int64_t M, int32_t accumulate, void* stream);
+
+/* LoRA terms of d(input) of one or two projections that share an input:
+ *   out[M,K] = fp16( sum_i keep_scale_i * mask_i (.) (u_i . A_i) ),   u_i fp32 [M,16] = scale_i * d(out_i) . B_i
+ * (`lqx`, `lvx` of solution/fast_qwen.py:1376-1377 and the masked add of solution/k_norm.py:64-71). One accumulating
+ * nf4ll_backward_dx over the stacked weight, without a LoRA branch, then completes dx: the two masks of gate and up (or q and v)
+ * would not fit one GEMM's epilogue. K a multiple of 8; pointers 16-byte aligned, ldo a multiple of 8, ld_mask of 16. */
+typedef struct nf4ll_expand {
+  const void* u;            /* fp32 [M,16] */
+  const void* A;            /* __half [16,K] */
+  const uint8_t* mask;      /* [M, ld_mask] or NULL */
+  int64_t ld_mask;
+  float keep_scale;
+} nf4ll_expand;
+int nf4ll_lora_expand(const nf4ll_expand* branches, int32_t n, int64_t M, int64_t K, void* out, int64_t ldo, void* stream);
+
 /* Fused residual add + RMSNorm that PRODUCES the inputs of the projections which follow it:
  *   xs = x (+ delta16);  rstd = rsqrt(mean(xs^2) + eps);  y = w * (xs * rstd);  y16 = fp16(y)
  *   t_i = fp16(keep_i ? y * keep_scale_i : 0) . A_i^T      for up to two LoRA branches (q and v), fp32 [M,16]
@@ -252,6 +284,44 @@ int nf4ll_swiglu_forward(const void* g, int64_t ldg, const void* u, int64_t ldu,
 int nf4ll_swiglu_backward(const void* g, int64_t ldg, const void* u, int64_t ldu, const void* dh,
                           int64_t lddh, void* dg, int64_t lddg, void* du, int64_t lddu, int64_t M,
                           int64_t I, void* stream);
+
+/* The backward of an MLP block's gated product with everything that LoRA branches on gate, up and down take from [M,I] matrices:
+ * dg and du as nf4ll_swiglu_backward forms them, and from the rounded results
+ *   u_gate[M,16] = scale_gate * dg . B_gate          u_up[M,16] = scale_up * du . B_up         (`daq`, `dav` of solution/fast_qwen.py:1370, 1373)
+ *   dB_gate[I,16] (+)= scale_gate * dg^T . t_gate    dB_up[I,16] (+)= scale_up * du^T . t_up
+ *   dA_down[16,I] (+)= u_down^T . drop(h),  h = fp16(silu(g) * u)                              (solution/fast_qwen.py:1369, 1371)
+ * all fp32. t_gate, t_up, u_down: fp32 [M,16] of nf4ll_forward_gate_up and nf4ll_backward_dx; Bt_*: lora_B transposed, __half [16,I];
+ * mask: of h. scratch: nf4ll_gated_backward_bytes(M, I) device bytes, 16-byte aligned (parts of u_gate and u_up, added up in a fixed order).
+ * dg / du may alias g / u. I a multiple of 8; matrices, t, u and Bt 16-byte aligned, their leading dimensions multiples of 8, ld_mask of 16. */
+typedef struct nf4ll_gated {
+  const void* g;
+  int64_t ldg;
+  const void* u;
+  int64_t ldu;
+  const void* dh;
+  int64_t lddh;
+  void* dg;
+  int64_t lddg;
+  void* du;
+  int64_t lddu;
+  const uint8_t* mask;      /* [M, ld_mask] or NULL */
+  int64_t ld_mask;
+  float keep_scale;
+  const void* t_gate;
+  const void* t_up;
+  const void* u_down;
+  const void* Bt_gate;
+  const void* Bt_up;
+  float scale_gate, scale_up;
+  void* u_gate;
+  void* u_up;
+  void* dB_gate;
+  void* dB_up;
+  void* dA_down;
+} nf4ll_gated;
+int64_t nf4ll_gated_backward_bytes(int64_t M, int64_t I);
+int nf4ll_gated_backward(const nf4ll_gated* p, int64_t M, int64_t I, int32_t accumulate, void* scratch, int64_t scratch_bytes,
+                         void* stream);
 
 /* Rotary embedding + causal grouped-query attention over packed varlen rows (the step between the Q|K|V and the O
  * projection; the reference's own kernels are solution/k_rope.py and solution/k_attn.py).

@@ -1,0 +1,104 @@
+"""The joined backward of an MLP block: gated-SiLU backward with what LoRA branches take from its matrices, the LoRA terms of dx
+expanded for two dropout masks, the factors' gradients of several projections in one launch, at the edges of their tiles."""
+
+import pytest
+import torch
+
+from decentrik_prime_b200 import linear
+from decentrik_prime_b200.blocks import MlpBlock
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def rand(*shape, scale=1.0, seed=0):
+    gen = torch.Generator().manual_seed(seed)
+    return (torch.randn(*shape, generator=gen) * scale).to(DEV)
+
+
+# stages of 16 rows, row ranges of several of them, warps of 64 and CTAs of 256 columns, 16-byte pieces of the mask
+@pytest.mark.parametrize("M,I", [(1, 8), (15, 40), (16, 256), (17, 264), (33, 2056), (187, 1000), (600, 8960), (4801, 520)])
+@pytest.mark.parametrize("masked,accumulate", [(True, True), (False, False)])
+def test_gated_backward_with_lora(M, I, masked, accumulate):
+    gu, dh = rand(M, 2 * I, seed=1).half(), rand(M, I + 8, seed=2).half()[:, :I]
+    Bg, Bu = (rand(16, I, scale=0.05, seed=3 + i).half() for i in range(2))
+    tg, tu, ud = (rand(M, 16, seed=5 + i) for i in range(3))
+    mask = (rand(M, (I + 15) // 16 * 16, seed=8) > -1.0).to(torch.uint8)[:, :I] if masked else None
+    grads = [rand(*s, seed=9) for s in ((I, 16), (I, 16), (16, I))]
+    before = [x.double() if accumulate else 0.0 for x in grads]
+    g, u = gu[:, :I], gu[:, I:]
+    dg, du = linear.swiglu_backward(g, u, dh, inplace=False)
+    h = linear.swiglu_forward(g, u)
+    h = h if mask is None else (h.float() * mask * 1.25).half()
+    ug, uu = linear.gated_backward(g, u, dh, mask, 1.25, tg, tu, ud, (Bg, 2.0), (Bu, 0.5), *grads, accumulate)
+    assert torch.equal(gu, torch.cat((dg, du), 1))
+    # exact products in fp32 sums: a unit in the last place of the absolute sum per addition
+    for d, b, s, got in ((dg, Bg, 2.0, ug), (du, Bu, 0.5, uu)):
+        bound = s * d.double().abs() @ b.double().abs().t()
+        assert ((got.double() - s * d.double() @ b.double().t()).abs() <= (I / 16 + 16) * 2.0 ** -23 * bound + 1e-12).all()
+    # and the sides in two fp16 parts (22 bits)
+    for d, side, s, got, old in ((dg, tg, 2.0, grads[0], before[0]), (du, tu, 0.5, grads[1], before[1]), (h, ud, 1.0, grads[2].t(), before[2])):
+        old = old.t() if got is not grads[0] and got is not grads[1] and accumulate else old
+        ref, bound = s * d.double().t() @ side.double() + old, s * d.double().abs().t() @ side.double().abs()
+        assert ((got.double() - ref).abs() <= (M / 16 + 16) * 2.0 ** -22 * (bound + abs(old))).all()
+
+
+@pytest.mark.parametrize("M,K", [(1, 8), (15, 56), (16, 64), (17, 72), (65, 136), (187, 1536), (3001, 200)])
+@pytest.mark.parametrize("masked", [(), (0,), (1,), (0, 1)])
+@pytest.mark.parametrize("n", [1, 2])
+def test_expanded_lora_terms(M, K, masked, n):
+    ldm = (K + 15) // 16 * 16
+    u = [rand(M, 16, scale=0.3, seed=i) for i in range(n)]
+    A = [rand(16, K, scale=0.2, seed=5 + i).half() for i in range(n)]
+    masks = [(rand(M, ldm, seed=9 + i) > -1.0).to(torch.uint8)[:, :K] if i in masked else None for i in range(n)]
+    out = torch.full((M, K + 8), 7.0, dtype=torch.float16, device=DEV)
+    linear.lora_expand([(u[i], A[i], masks[i], 1.25) for i in range(n)], out[:, :K])
+    ref, bound = 0.0, 0.0
+    for i in range(n):
+        keep = 1.0 if masks[i] is None else masks[i].double() * 1.25
+        ref = ref + keep * (u[i].double() @ A[i].double())
+        bound = bound + 1.25 * (u[i].double().abs() @ A[i].double().abs())
+    # u in two fp16 parts (22 bits) and fp32 sums, then one rounding to fp16
+    assert ((out[:, :K].double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -20 * bound + 2.0 ** -24).all()
+    assert (out[:, K:] == 7.0).all()
+
+
+@pytest.mark.parametrize("M", [1, 64, 187, 2048])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_gradients_of_three_projections(M, accumulate):
+    """Against one call each: the row ranges differ (fp32 sums of M terms in another order)."""
+    list_, want = [], []
+    for i, (N, K) in enumerate(((72, 200), (8, 1536), (1536, 64))):
+        dy, x, t, u = rand(M, N, seed=i).half(), rand(M, K, seed=10 + i).half(), rand(M, 16, seed=20 + i), rand(M, 16, seed=30 + i)
+        mask = (rand(M, (K + 15) // 16 * 16, seed=40 + i) > -1.0).to(torch.uint8)[:, :K] if i != 1 else None
+        dA, dB = rand(16, K, seed=50 + i), rand(N, 16, seed=60 + i)
+        want.append(linear.lora_grads(dy, x, t, u, 0.5, mask=mask, keep_scale=1.25, dA=dA.clone(), dB=dB.clone(), accumulate=accumulate))
+        list_.append((dy, x, t, u, 0.5, mask, 1.25, dA, dB))
+    linear.lora_grads_batch(list_, accumulate)
+    for (dy, x, t, u, s, _, ks, dA, dB), (wA, wB) in zip(list_, want):
+        tol = (M / 16 + 16) * 2.0 ** -22
+        assert ((dA - wA).abs() <= tol * (ks * (u.abs().t() @ x.float().abs()) + wA.abs() + 1)).all()
+        assert ((dB - wB).abs() <= tol * (s * (dy.float().abs().t() @ t.abs()) + wB.abs() + 1)).all()
+
+
+@pytest.mark.parametrize("M", [1, 24, 187])
+def test_joined_and_separate_backward(M):
+    """Both orders of the block's backward round dx twice to fp16: each within two half-ulps of the exact sum."""
+    H, I = 256, 512
+    x, dy = rand(M, H, seed=1).half(), rand(M, H, seed=2).half()
+    masks = [(rand(M, k, seed=3 + i) > -1.3).to(torch.uint8) for i, k in enumerate((H, H, I))]
+    block = MlpBlock(H, I, 0, DEV)
+    got = []
+    for joined in (True, False):
+        block.forward(x, masks, 1.1)
+        if not joined:
+            g, u = block._saved
+            dx = block._backward_each(g, u, dy, True, False, None)
+        else:
+            dx = block.backward(dy)
+        got.append((dx, [t.clone() for p in block.projections for t in (p.dA, p.dB)]))
+    (dx1, gr1), (dx2, gr2) = got
+    scale = dx2.float().abs().max()
+    assert ((dx1.float() - dx2.float()).abs() <= 2.0 ** -11 * 4 * scale).all()
+    for a, b in zip(gr1, gr2):
+        assert ((a - b).norm() / b.norm()) < 1e-3          # u of the joined order from fp32 sums in another order
