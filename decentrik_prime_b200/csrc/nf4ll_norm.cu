@@ -17,9 +17,9 @@
 //     out  = dres + dx  (fp32)  and its fp16 copy
 // The [M, D] LoRA input gradients of the reference never exist: the rank-16 factors are expanded per element.
 //
-// A CTA owns 16 (forward) or 8 (backward) token rows and the whole hidden dimension, sixteen warps deep; a
-// lane's values stay in registers between the row reduction and the second phase, so every input is read once.
-#include "nf4ll_common.cuh"
+// A group of 8 token rows (16 in the forward of a long batch) belongs to a CTA or, where the groups would leave SMs idle, to a cluster
+// whose CTAs share out the hidden dimension; a lane's values stay in registers between the row reduction and the second phase.
+#include "nf4ll_pair.cuh"
 
 namespace nf4ll {
 
@@ -36,6 +36,11 @@ struct NormBranch {
 
 __device__ __forceinline__ void load8_f32(const float* p, float (&v)[8]) {
   const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+  v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+// of memory that the kernel writes too
+__device__ __forceinline__ void load8_f32_rw(const float* p, float (&v)[8]) {
+  const float4 a = *reinterpret_cast<const float4*>(p), b = *(reinterpret_cast<const float4*>(p) + 1);
   v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
 }
 __device__ __forceinline__ void store8_f32(float* p, const float (&v)[8]) {
@@ -188,127 +193,328 @@ rms_fwd_kernel(const float* __restrict__ x, const __half* __restrict__ delta, fl
   }
 }
 
-// 8 rows per CTA
+// ---------------------------------------------------------------------------------------------
+// The forward for batches whose groups of rows do not fill the SMs: eight rows per cluster of up to eight CTAs (eight warps each),
+// which share out the columns. The row sums meet through distributed shared memory, every CTA adding them up in rank order, and the
+// rank-16 products in the first CTA likewise. Such a batch is bound by the chain load - sum - products - store of one CTA, so what
+// counts is how little of a row a CTA has, and that the loads of the second phase are on their way before the sum: one CTA of sixteen
+// warps per 16 (D > 2048: 8) rows against this, us, with two branches / without: 1536 columns, 8 rows 9.7 / 4.9 -> 4.6 / 2.9, 333 rows 13.2 / 7.4 ->
+// 6.2 / 3.9, 951 rows 20.2 / 9.4 -> 14.1 / 7.4; 3584 columns, 8 rows 15.2 / 9.0 -> 5.7 / 3.4, 333 rows 22.1 / 9.7 -> 11.8 / 6.2.
+// ---------------------------------------------------------------------------------------------
+constexpr int kSplitWarps = 8;
+
+__device__ __forceinline__ float peer_f32(const float* local, uint32_t rank) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(local), rank)) : "memory");
+  return v;
+}
+
+// total over the cluster of every row's sum, for row g: part[warp][row] of each CTA; s_sum is read by the others until the next cluster barrier
+template <int NW>
+__device__ __forceinline__ float split_row_total(const float (&part)[NW][8], float (&s_sum)[8], int g) {
+  __syncthreads();
+  if (threadIdx.x < 8) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) v += part[w][threadIdx.x];
+    s_sum[threadIdx.x] = v;
+  }
+  if (gridDim.y == 1) {
+    __syncthreads();
+    return s_sum[g];
+  }
+  cluster_sync_all();
+  float peer[8], v = 0.f;
+#pragma unroll
+  for (uint32_t r = 0; r < 8; ++r) peer[r] = r < gridDim.y ? peer_f32(&s_sum[g], r) : 0.f;      // all in flight at once
+#pragma unroll
+  for (uint32_t r = 0; r < 8; ++r) v += peer[r];
+  return v;
+}
+
+// CPW chunks of 32 columns per warp; `chunks` of them per CTA
 template <int CPW>
-__global__ void __launch_bounds__(kNormWarps * 32)
-rms_bwd_kernel(const __half* __restrict__ dy16, int64_t lddy, float gscale, const float* __restrict__ x,
-               const __half* __restrict__ delta, const float* __restrict__ w, const float* __restrict__ rstd,
-               const float* dres, float* out, __half* __restrict__ out16, int64_t M, int64_t D,
-               const NormBranch ba, const NormBranch bb) {
+__global__ void __launch_bounds__(kSplitWarps * 32, 2)
+rms_fwd_split_kernel(const float* __restrict__ x, const __half* __restrict__ delta, float* __restrict__ xout, const float* __restrict__ w, float eps,
+                     int64_t M, int64_t D, __half* __restrict__ y16, int64_t ldy, float* __restrict__ rstd_out, const NormBranch ba, const NormBranch bb,
+                     int chunks) {
   pdl_wait();
   pdl_launch_dependents();
-  __shared__ float s_part[kNormWarps][8];
-  __shared__ float s_c[8];
+  __shared__ float s_part[kSplitWarps][8];
+  __shared__ float s_sum[8];
+  __shared__ float s_t[2][kSplitWarps][8][17];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int64_t m0 = static_cast<int64_t>(blockIdx.x) * 8;
-  const bool ok = m0 + g < M;
-  const int64_t row = ok ? m0 + g : 0;
-  const float r = __ldg(rstd + row);
-  float ua[16], ub[16];
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + g;
+  const bool ok = row < M;
+  const int64_t col0 = static_cast<int64_t>(blockIdx.y) * chunks * 32;
+  const int64_t col1 = col0 + chunks * 32 < D ? col0 + chunks * 32 : D;
+  float xv[CPW][8], wv[CPW][8], ss = 0.f;
+  constexpr bool kEarly = CPW <= 2;                // lora_A of both branches, ranks g and g + 8, before the sums where registers allow
+  uint4 fr[kEarly ? CPW : 1][4];
+  auto load_fr = [&](int64_t k, uint4 (&f)[4]) {
 #pragma unroll
-  for (int j = 0; j < 16; ++j) { ua[j] = 0.f; ub[j] = 0.f; }
-  if (ba.A) {
-#pragma unroll
-    for (int j4 = 0; j4 < 4; ++j4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(ba.u + row * 16) + j4);
-      ua[4 * j4] = v.x * ba.keep_scale; ua[4 * j4 + 1] = v.y * ba.keep_scale; ua[4 * j4 + 2] = v.z * ba.keep_scale; ua[4 * j4 + 3] = v.w * ba.keep_scale;
+    for (int b = 0; b < 2; ++b) {
+      const __half* A = b ? bb.A : ba.A;
+      const uint4 zero = make_uint4(0, 0, 0, 0);
+      f[2 * b] = A && k < col1 ? __ldg(reinterpret_cast<const uint4*>(A + static_cast<int64_t>(g) * D + k)) : zero;
+      f[2 * b + 1] = A && k < col1 ? __ldg(reinterpret_cast<const uint4*>(A + static_cast<int64_t>(g + 8) * D + k)) : zero;
     }
-  }
-  if (bb.A) {
-#pragma unroll
-    for (int j4 = 0; j4 < 4; ++j4) {
-      const float4 v = __ldg(reinterpret_cast<const float4*>(bb.u + row * 16) + j4);
-      ub[4 * j4] = v.x * bb.keep_scale; ub[4 * j4 + 1] = v.y * bb.keep_scale; ub[4 * j4 + 2] = v.z * bb.keep_scale; ub[4 * j4 + 3] = v.w * bb.keep_scale;
-    }
-  }
-  float gv[CPW][8];
-  float cs = 0.f;
+  };
 #pragma unroll
   for (int c = 0; c < CPW; ++c) {
-    const int64_t k = (static_cast<int64_t>(c) * kNormWarps + warp) * 32 + t * 8;
+    const int64_t k = col0 + (c * kSplitWarps + warp) * 32 + t * 8;
+    const bool in = k < col1;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) gv[c][j] = 0.f;
-    if (k < D && ok) {
-      float dy[8], xr[8], wv[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(dy16 + row * lddy + k)), dy);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) dy[j] *= gscale;
-#pragma unroll
-      for (int br = 0; br < 2; ++br) {
-        const NormBranch& b = br ? bb : ba;
-        if (!b.A) continue;
-        const float* u = br ? ub : ua;
-        float l[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) l[j] = 0.f;
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-          float av[8];
-          unpack8(__ldg(reinterpret_cast<const uint4*>(b.A + static_cast<int64_t>(jj) * D + k)), av);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) l[j] = fmaf(u[jj], av[j], l[j]);
-        }
-        if (b.mask) {
-          const uint2 m = __ldg(reinterpret_cast<const uint2*>(b.mask + row * b.ld_mask + k));
-#pragma unroll
-          for (int j = 0; j < 8; ++j) dy[j] += keep_bit(m, j) ? l[j] : 0.f;
-        } else {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) dy[j] += l[j];
-        }
-      }
-      load8_f32(x + row * D + k, xr);
+    for (int j = 0; j < 8; ++j) xv[c][j] = wv[c][j] = 0.f;
+    if (in && ok) {
+      load8_f32(x + row * D + k, xv[c]);
       if (delta) {
         float dv[8];
         unpack8(__ldg(reinterpret_cast<const uint4*>(delta + row * D + k)), dv);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) xr[j] += dv[j];
+        for (int j = 0; j < 8; ++j) xv[c][j] += dv[j];
       }
-      load8_f32(w + k, wv);
+    }
+    if (in) load8_f32(w + k, wv[c]);
+    if (kEarly) load_fr(k, fr[c]);
+  }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        gv[c][j] = dy[j] * wv[j];
-        cs = fmaf(gv[c][j], xr[j] * r, cs);
+  for (int c = 0; c < CPW; ++c) {
+    const int64_t k = col0 + (c * kSplitWarps + warp) * 32 + t * 8;
+    if (xout && k < col1 && ok) store8_f32(xout + row * D + k, xv[c]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss = fmaf(xv[c][j], xv[c][j], ss);
+  }
+  ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+  ss += __shfl_xor_sync(0xffffffffu, ss, 2);
+  if (t == 0) s_part[warp][g] = ss;
+  const float r = rsqrtf(split_row_total(s_part, s_sum, g) * (1.0f / static_cast<float>(D)) + eps);
+  if (blockIdx.y == 0 && warp == 0 && t == 0 && ok) rstd_out[row] = r;
+  float acc[2][4];
+#pragma unroll
+  for (int b = 0; b < 2; ++b) acc[b][0] = acc[b][1] = acc[b][2] = acc[b][3] = 0.f;
+#pragma unroll
+  for (int c = 0; c < CPW; ++c) {
+    const int64_t k = col0 + (c * kSplitWarps + warp) * 32 + t * 8;
+    const bool live = k < col1 && ok;
+    uint4 (&f)[4] = fr[kEarly ? c : 0];
+    if (!kEarly) load_fr(k, f);
+    float y[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) y[j] = wv[c][j] * (xv[c][j] * r);
+    if (y16 && live) *reinterpret_cast<uint4*>(y16 + row * ldy + k) = pack8(y);
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const NormBranch& br = b ? bb : ba;
+      if (!br.A) continue;
+      float d[8];
+      const uint2 m = br.mask && live ? __ldg(reinterpret_cast<const uint2*>(br.mask + row * br.ld_mask + k)) : make_uint2(0, 0);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) d[j] = live ? (br.mask ? (keep_bit(m, j) ? y[j] * br.keep_scale : 0.f) : y[j]) : 0.f;
+      const uint4 q = pack8(d);
+      mma16816(acc[b], f[2 * b].x, f[2 * b + 1].x, f[2 * b].y, f[2 * b + 1].y, q.x, q.y);
+      mma16816(acc[b], f[2 * b].z, f[2 * b + 1].z, f[2 * b].w, f[2 * b + 1].w, q.z, q.w);
+    }
+  }
+  if (ba.A || bb.A) {
+    // acc[b][0], [1] = (rank g, rows 2t, 2t+1); [2], [3] = (rank g+8, same rows)
+#pragma unroll
+    for (int b = 0; b < 2; ++b)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s_t[b][warp][2 * t + (i & 1)][g + 8 * (i >> 1)] = acc[b][i];
+    __syncthreads();
+    const int b = threadIdx.x >> 7, rr = threadIdx.x >> 4 & 7, j = threadIdx.x & 15;
+    float v = 0.f;
+#pragma unroll
+    for (int wq = 0; wq < kSplitWarps; ++wq) v += s_t[b][wq][rr][j];
+    if (gridDim.y > 1) {
+      s_t[b][0][rr][j] = v;                        // read and written by this thread only
+      cluster_sync_all();
+      if (blockIdx.y == 0) {
+        float peer[8];
+#pragma unroll
+        for (uint32_t q = 1; q < 8; ++q) peer[q] = q < gridDim.y ? peer_f32(&s_t[b][0][rr][j], q) : 0.f;
+#pragma unroll
+        for (uint32_t q = 1; q < 8; ++q) v += peer[q];
       }
+    }
+    const NormBranch& br = b ? bb : ba;
+    const int64_t m = static_cast<int64_t>(blockIdx.x) * 8 + rr;
+    if (blockIdx.y == 0 && br.A && m < M) br.t[m * 16 + j] = v;
+  }
+  if (gridDim.y > 1) cluster_sync_all();           // shared memory stays until the others have read it
+}
+
+// An 8 x 8 block of 16-bit values, a row in four lanes: transposed
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+// a, b as fp16 pairs of descending weight: 33 bits, all of an fp32 value in fp16's range
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&p)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    p[i] = pack_half2_rn(a, b);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
+    a = fabsf(f.x) <= 65504.f ? a - f.x : 0.f;     // nothing is left of an infinity
+    b = fabsf(f.y) <= 65504.f ? b - f.y : 0.f;
+  }
+}
+
+// The expansion u . A on the tensor cores: a lane's sixteen bytes of a rank's row are four 2-column pieces, which movmatrix turns into the
+// right operand for columns 8 i + 2 w, + 1 (i = 0..3), so that over w = 0..3 lane (g, t) ends with its own columns 8 t .. + 7 of row g. u
+// goes in three fp16 parts under a power of two per row that brings its largest to [1, 2): no less than its 24 bits, whatever their size.
+// With fp32 FMAs it was 32 loads, 256 conversions and 256 FMAs per lane and chunk, and the larger error against fp64 (9.5e-8 of the
+// result's norm at u of 1 with 1536 columns, 7.2e-8 so). us with two branches / without, one CTA and FMAs before: 1536 columns, 8 rows 13.1 / 6.0 ->
+// 4.6 / 3.0, 951 rows 22.3 / 11.1 -> 15.6 / 10.6, 2048 rows (a CTA per group) 41.4 / 20.9 -> 31.5 / 20.4; 3584 columns, 333 rows 59.8 / 20.5 ->
+// 14.2 / 9.6, 2048 rows 120 / 45 -> 68 / 42.
+template <int CPW, int NW, bool KEEP>
+__global__ void __launch_bounds__(NW * 32, NW == kSplitWarps ? 2 : 1)
+rms_bwd_kernel(const __half* __restrict__ dy16, int64_t lddy, float gscale, const float* __restrict__ x, const __half* __restrict__ delta,
+                     const float* __restrict__ w, const float* __restrict__ rstd, const float* dres, float* out, __half* __restrict__ out16, int64_t M,
+                     int64_t D, const NormBranch ba, const NormBranch bb, int chunks) {
+  pdl_wait();
+  pdl_launch_dependents();
+  __shared__ float s_part[NW][8];
+  __shared__ float s_sum[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 8 + g;
+  const bool ok = row < M;
+  const int64_t col0 = static_cast<int64_t>(blockIdx.y) * chunks * 32;
+  const int64_t col1 = col0 + chunks * 32 < D ? col0 + chunks * 32 : D;
+  const float r = ok ? __ldg(rstd + row) : 0.f;
+  auto load_x = [&](int64_t k, float (&v)[8]) {
+    load8_f32(x + row * D + k, v);
+    if (delta) {
+      float dv[8];
+      unpack8(__ldg(reinterpret_cast<const uint4*>(delta + row * D + k)), dv);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] += dv[j];
+    }
+  };
+  // left operand: row g, ranks 2t, 2t+1 and + 8 (rows g + 8 are zeros)
+  uint32_t ul[2][3], uh[2][3];
+  float back[2] = {1.f, 1.f};
+#pragma unroll
+  for (int b = 0; b < 2; ++b) {
+    const NormBranch& br = b ? bb : ba;
+    if (!br.A) continue;
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 lo = ok ? __ldg(reinterpret_cast<const float2*>(br.u + row * 16 + 2 * t)) : zero;
+    float2 hi = ok ? __ldg(reinterpret_cast<const float2*>(br.u + row * 16 + 2 * t + 8)) : zero;
+    lo.x *= br.keep_scale; lo.y *= br.keep_scale; hi.x *= br.keep_scale; hi.y *= br.keep_scale;
+    float m = fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(hi.x), fabsf(hi.y)));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+    // the exponent of the row's largest, within what two normal powers of two can undo
+    int e = static_cast<int>(__float_as_uint(m) >> 23) - 127;
+    e = e < -126 ? -126 : e > 126 ? 126 : e;
+    const float f = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
+    back[b] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+    split3(lo.x * f, lo.y * f, ul[b]);
+    split3(hi.x * f, hi.y * f, uh[b]);
+  }
+  constexpr int KC = KEEP ? CPW : 1;               // chunks whose x and dres stay in registers
+  float gv[CPW][8], xh[KC][8], dr[KC][8], cs = 0.f;
+#pragma unroll
+  for (int c = 0; c < CPW; ++c) {
+    const int64_t k = col0 + (c * NW + warp) * 32 + t * 8;
+    const bool in = k < col1, live = in && ok;
+    const int kc = KEEP ? c : 0;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    float dy[8], wv[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) xh[kc][j] = dr[kc][j] = wv[j] = 0.f;
+    unpack8(live ? __ldg(reinterpret_cast<const uint4*>(dy16 + row * lddy + k)) : zero, dy);
+    if (live) {
+      load_x(k, xh[kc]);
+      if (KEEP && dres) load8_f32_rw(dres + row * D + k, dr[kc]);
+    }
+    if (in) load8_f32(w + k, wv);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dy[j] *= gscale;
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      const NormBranch& br = b ? bb : ba;
+      if (!br.A) continue;
+      const uint4 f0 = in ? __ldg(reinterpret_cast<const uint4*>(br.A + static_cast<int64_t>(g) * D + k)) : zero;
+      const uint4 f1 = in ? __ldg(reinterpret_cast<const uint4*>(br.A + static_cast<int64_t>(g + 8) * D + k)) : zero;
+      const uint2 m = br.mask && live ? __ldg(reinterpret_cast<const uint2*>(br.mask + row * br.ld_mask + k)) : make_uint2(0, 0);
+      const uint32_t p0[4] = {f0.x, f0.y, f0.z, f0.w}, p1[4] = {f1.x, f1.y, f1.z, f1.w};
+      uint32_t b0[4], b1[4];
+      float l[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        b0[q] = transpose8x8(p0[q]);
+        b1[q] = transpose8x8(p1[q]);
+        l[q][0] = l[q][1] = l[q][2] = l[q][3] = 0.f;
+      }
+#pragma unroll
+      for (int i = 2; i >= 0; --i)                 // the smallest part first
+#pragma unroll
+        for (int q = 0; q < 4; ++q) mma16816(l[q], ul[b][i], 0u, uh[b][i], 0u, b0[q], b1[q]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dy[j] += !br.mask || keep_bit(m, j) ? l[j >> 1][j & 1] * back[b] : 0.f;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      xh[kc][j] *= r;
+      gv[c][j] = dy[j] * wv[j];
+      cs = fmaf(gv[c][j], xh[kc][j], cs);
     }
   }
   cs += __shfl_xor_sync(0xffffffffu, cs, 1);
   cs += __shfl_xor_sync(0xffffffffu, cs, 2);
   if (t == 0) s_part[warp][g] = cs;
-  __syncthreads();
-  if (threadIdx.x < 8) {
-    float v = 0.f;
-#pragma unroll
-    for (int wq = 0; wq < kNormWarps; ++wq) v += s_part[wq][threadIdx.x];
-    s_c[threadIdx.x] = v * (1.0f / static_cast<float>(D));
-  }
-  __syncthreads();
-  const float cm = s_c[g];
+  const float cm = split_row_total(s_part, s_sum, g) * (1.0f / static_cast<float>(D));
 #pragma unroll
   for (int c = 0; c < CPW; ++c) {
-    const int64_t k = (static_cast<int64_t>(c) * kNormWarps + warp) * 32 + t * 8;
-    if (k < D && ok) {
-      float xr[8], o[8];
-      load8_f32(x + row * D + k, xr);          // second read of x: from L1 / L2
-      if (delta) {
-        float dv[8];
-        unpack8(__ldg(reinterpret_cast<const uint4*>(delta + row * D + k)), dv);
+    const int64_t k = col0 + (c * NW + warp) * 32 + t * 8;
+    if (k < col1 && ok) {
+      float o[8];
+      const int kc = KEEP ? c : 0;
+      if (!KEEP) {                                 // second read of x: from L1 / L2
+        load_x(k, xh[0]);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) xr[j] += dv[j];
+        for (int j = 0; j < 8; ++j) xh[0][j] *= r, dr[0][j] = 0.f;
+        if (dres) load8_f32_rw(dres + row * D + k, dr[0]);
       }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) o[j] = (gv[c][j] - (xr[j] * r) * cm) * r;
-      if (dres) {
-        float dv[8];
-        load8_f32(dres + row * D + k, dv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] += dv[j];
-      }
+      for (int j = 0; j < 8; ++j) o[j] = (gv[c][j] - xh[kc][j] * cm) * r + dr[kc][j];
       store8_f32(out + row * D + k, o);
       if (out16) *reinterpret_cast<uint4*>(out16 + row * D + k) = pack8(o);
     }
   }
+  if (gridDim.y > 1) cluster_sync_all();
+}
+
+// CTAs per group of eight rows and 32-column chunks per CTA: as many as find room at once, each warp with a chunk at least. Two per SM
+// in powers of two; clusters of other sizes leave SMs of a GPC idle, and at two per SM some of them wait for a second wave (42 groups in
+// sevens, 2048 columns: 8.5 us against 7.7 in fours; in sixes, 1536 columns, 6.3 against 7.3 in fours). parts = 0: a second wave would be
+// needed, or a row is too long for what is free; then a CTA of sixteen warps takes the whole row (951 rows of 1536 in two waves of clusters: 23.7 us
+// against 20.3). parts = 1 is worth it in the backward only (2048 rows of 1024: 12.6 us against 15.1; forward 9.1 against 8.4).
+struct NormSplit {
+  unsigned groups, parts;
+  int chunks, cpw;
+};
+static int norm_split(NormSplit* s, int64_t M, int64_t D) {
+  int dev = 0, sms = 148;
+  NF4LL_CUDA(cudaGetDevice(&dev));
+  NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t groups = (M + 7) / 8, all = (D + 31) / 32;
+  int64_t parts = 8;
+  auto fits = [&](int64_t n) { return groups * n <= (n & (n - 1) ? 7 : 8) * static_cast<int64_t>(sms) / 4; };
+  while (parts > 1 && (!fits(parts) || all < parts * kSplitWarps)) --parts;
+  *s = NormSplit{static_cast<unsigned>(groups), 0, 0, 0};
+  const int64_t chunks = (all + parts - 1) / parts;
+  if (!fits(parts) || chunks > 4 * kSplitWarps) return NF4LL_OK;
+  s->chunks = static_cast<int>(chunks);
+  s->parts = static_cast<unsigned>((all + chunks - 1) / chunks);
+  s->cpw = static_cast<int>((chunks + kSplitWarps - 1) / kSplitWarps);
+  return NF4LL_OK;
 }
 
 static int check_branch(const nf4ll_lora* l, const void* side, const char* who, int64_t D, NormBranch* out, bool forward) {
@@ -356,6 +562,14 @@ extern "C" int nf4ll_rms_forward(const float* x, const void* delta16, float* xou
   const int cpw = static_cast<int>((D + kNormWarps * 32 - 1) / (kNormWarps * 32));
   const __half* dl = static_cast<const __half*>(delta16);
   __half* y = static_cast<__half*>(y16);
+  NormSplit s;
+  if (int rc = norm_split(&s, M, D)) return rc;
+  if (s.parts > 1) {
+    PdlLaunch lc(dim3(s.groups, s.parts), dim3(kSplitWarps * 32), 0, st, 1, s.parts);
+    const auto kernel = s.cpw <= 1 ? rms_fwd_split_kernel<1> : s.cpw <= 2 ? rms_fwd_split_kernel<2> : s.cpw <= 3 ? rms_fwd_split_kernel<3> : rms_fwd_split_kernel<4>;
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, kernel, x, dl, xout, w, eps, M, D, y, ldy, rstd, ba, bb, s.chunks));
+    return NF4LL_OK;
+  }
   if (cpw <= 4) {
     PdlLaunch lc(dim3(static_cast<unsigned>((M + 15) / 16)), dim3(kNormWarps * 32), 0, st);
     NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, rms_fwd_kernel<2, 4>, x, dl, xout, w, eps, M, D, y, ldy, rstd, ba, bb));
@@ -384,15 +598,15 @@ extern "C" int nf4ll_rms_backward(const void* dy16, int64_t lddy, float gscale, 
   if (int rc = check_branch(lora_b, u_b, who, D, &bb, false)) return rc;
   if (int rc = require_sm100()) return rc;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int cpw = static_cast<int>((D + kNormWarps * 32 - 1) / (kNormWarps * 32));
-  PdlLaunch lc(dim3(static_cast<unsigned>((M + 7) / 8)), dim3(kNormWarps * 32), 0, st);
   const __half* dyp = static_cast<const __half*>(dy16);
   const __half* dl = static_cast<const __half*>(delta16);
   __half* o16 = static_cast<__half*>(out16);
-  if (cpw <= 4) {
-    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, rms_bwd_kernel<4>, dyp, lddy, gscale, x, dl, w, rstd, dres, out, o16, M, D, ba, bb));
-  } else {
-    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, rms_bwd_kernel<8>, dyp, lddy, gscale, x, dl, w, rstd, dres, out, o16, M, D, ba, bb));
-  }
+  NormSplit s;
+  if (int rc = norm_split(&s, M, D)) return rc;
+  const auto kernel = !s.parts ? (D <= kNormWarps * 32 * 4 ? rms_bwd_kernel<4, kNormWarps, false> : rms_bwd_kernel<8, kNormWarps, false>)
+                      : s.cpw <= 1 ? rms_bwd_kernel<1, kSplitWarps, true> : s.cpw <= 2 ? rms_bwd_kernel<2, kSplitWarps, true>
+                      : s.cpw <= 3 ? rms_bwd_kernel<3, kSplitWarps, true> : rms_bwd_kernel<4, kSplitWarps, true>;
+  PdlLaunch lc(dim3(s.groups, s.parts ? s.parts : 1), dim3((s.parts ? kSplitWarps : kNormWarps) * 32), 0, st, s.parts > 1 ? 1 : 0, s.parts > 1 ? s.parts : 0);
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, kernel, dyp, lddy, gscale, x, dl, w, rstd, dres, out, o16, M, D, ba, bb, s.parts ? s.chunks : static_cast<int>((D + 31) / 32)));
   return NF4LL_OK;
 }
