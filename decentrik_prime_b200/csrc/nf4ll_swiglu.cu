@@ -8,57 +8,64 @@
 
 namespace nf4ll {
 
-// Both kernels are one pass at memory speed: a thread takes two 16-byte chunks per trip, all loads
-// of the trip issued before the arithmetic, so that every SM keeps enough bytes in flight.
+// Both kernels are one pass at memory speed: a thread takes several 16-byte chunks per trip, all loads of the trip issued before the
+// arithmetic, so that every SM keeps enough bytes in flight. T: how wide a chunk's number is (its row comes out of a division, which
+// took a good part of a trip in 64 bits). us at 16384 x 18944 / 2048 x 8960 / 951 x 8960 / 187 x 8960, backward: 511 / 32.2 / 16.2 / 4.6 with two
+// chunks per trip and 64-bit divisions for all, 480 / 30.8 / 15.5 / 2.9 now; forward 343 / 22.2 / 11.7 / 3.2, now 304 / 19.6 / 10.6 / 2.9.
+template <typename T, int U>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __half* __restrict__ g, int64_t ldg, const __half* __restrict__ u, int64_t ldu,
-                  __half* __restrict__ h, int64_t ldh, int64_t M, int64_t chunks_per_row) {
+                  __half* __restrict__ h, int64_t ldh, T total, T chunks_per_row) {
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t total = M * chunks_per_row;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += 2 * stride) {
-    const int64_t i2 = i + stride;
-    const bool two = i2 < total;
-    const int64_t row = i / chunks_per_row, col = (i - row * chunks_per_row) * 8;
-    const int64_t row2 = two ? i2 / chunks_per_row : row, col2 = two ? (i2 - row2 * chunks_per_row) * 8 : col;
-    const uint4 ga = __ldcs(reinterpret_cast<const uint4*>(g + row * ldg + col));
-    const uint4 ua = __ldcs(reinterpret_cast<const uint4*>(u + row * ldu + col));
-    const uint4 gb = __ldcs(reinterpret_cast<const uint4*>(g + row2 * ldg + col2));
-    const uint4 ub = __ldcs(reinterpret_cast<const uint4*>(u + row2 * ldu + col2));
-    *reinterpret_cast<uint4*>(h + row * ldh + col) = swiglu_fwd8(ga, ua);
-    if (two) *reinterpret_cast<uint4*>(h + row2 * ldh + col2) = swiglu_fwd8(gb, ub);
+  const T stride = static_cast<T>(gridDim.x) * 256;
+  for (T i = static_cast<T>(blockIdx.x) * 256 + threadIdx.x; i < total; i += U * stride) {
+    uint4 gv[U], uv[U];
+    int64_t at[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const T j = i + k * stride < total ? i + k * stride : i;
+      const T row = j / chunks_per_row;
+      const int64_t col = static_cast<int64_t>(j - row * chunks_per_row) * 8;
+      gv[k] = __ldcs(reinterpret_cast<const uint4*>(g + row * ldg + col));
+      uv[k] = __ldcs(reinterpret_cast<const uint4*>(u + row * ldu + col));
+      at[k] = row * ldh + col;
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k)
+      if (k == 0 || i + k * stride < total) *reinterpret_cast<uint4*>(h + at[k]) = swiglu_fwd8(gv[k], uv[k]);
   }
 }
 
 // dg / du may alias g / u (in-place, as the reference overwrites [gate | up]): a chunk is read in
 // full before it is written, by the same thread.
+template <typename T, int U>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __half* g, int64_t ldg, const __half* u, int64_t ldu, const __half* __restrict__ dh, int64_t lddh,
-                  __half* dg, int64_t lddg, __half* du, int64_t lddu, int64_t M, int64_t chunks_per_row) {
+                  __half* dg, int64_t lddg, __half* du, int64_t lddu, T total, T chunks_per_row) {
   pdl_wait();
   pdl_launch_dependents();
-  const int64_t total = M * chunks_per_row;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += 2 * stride) {
-    const int64_t i2 = i + stride;
-    const bool two = i2 < total;
-    const int64_t row = i / chunks_per_row, col = (i - row * chunks_per_row) * 8;
-    const int64_t row2 = two ? i2 / chunks_per_row : row, col2 = two ? (i2 - row2 * chunks_per_row) * 8 : col;
-    const uint4 ga = *reinterpret_cast<const uint4*>(g + row * ldg + col);
-    const uint4 ua = *reinterpret_cast<const uint4*>(u + row * ldu + col);
-    const uint4 da = __ldcs(reinterpret_cast<const uint4*>(dh + row * lddh + col));
-    const uint4 gb = *reinterpret_cast<const uint4*>(g + row2 * ldg + col2);
-    const uint4 ub = *reinterpret_cast<const uint4*>(u + row2 * ldu + col2);
-    const uint4 db = __ldcs(reinterpret_cast<const uint4*>(dh + row2 * lddh + col2));
-    uint4 og, ou, oh;
-    swiglu_bwd8(ga, ua, da, og, ou, oh);
-    *reinterpret_cast<uint4*>(dg + row * lddg + col) = og;
-    *reinterpret_cast<uint4*>(du + row * lddu + col) = ou;
-    if (two) {
-      swiglu_bwd8(gb, ub, db, og, ou, oh);
-      *reinterpret_cast<uint4*>(dg + row2 * lddg + col2) = og;
-      *reinterpret_cast<uint4*>(du + row2 * lddu + col2) = ou;
+  const T stride = static_cast<T>(gridDim.x) * 256;
+  for (T i = static_cast<T>(blockIdx.x) * 256 + threadIdx.x; i < total; i += U * stride) {
+    uint4 gv[U], uv[U], dv[U];
+    int64_t row[U], col[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      const T j = i + k * stride < total ? i + k * stride : i;
+      const T r = j / chunks_per_row;
+      row[k] = r;
+      col[k] = static_cast<int64_t>(j - r * chunks_per_row) * 8;
+      gv[k] = *reinterpret_cast<const uint4*>(g + row[k] * ldg + col[k]);
+      uv[k] = *reinterpret_cast<const uint4*>(u + row[k] * ldu + col[k]);
+      dv[k] = __ldcs(reinterpret_cast<const uint4*>(dh + row[k] * lddh + col[k]));
+    }
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      if (k > 0 && i + k * stride >= total) break;
+      uint4 og, ou, oh;
+      swiglu_bwd8(gv[k], uv[k], dv[k], og, ou, oh);
+      *reinterpret_cast<uint4*>(dg + row[k] * lddg + col[k]) = og;
+      *reinterpret_cast<uint4*>(du + row[k] * lddu + col[k]) = ou;
     }
   }
 }
@@ -301,12 +308,15 @@ static int check_mat16(const void* p, int64_t ld, int64_t cols, const char* who,
   return NF4LL_OK;
 }
 
-static int grid_for(int64_t total, unsigned* blocks) {
+// `shortish`: so few chunks that one per thread and trip serves them best (with two or four some threads of a trip have none): up to four
+// trips of all resident threads; 951 x 8960 backward 15.5 us with one, 16.6 with two, 2048 x 8960 31.6 and 30.8
+static int grid_for(int64_t total, unsigned* blocks, bool* shortish) {
   int dev = 0, sms = 148;
   NF4LL_CUDA(cudaGetDevice(&dev));
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  int64_t b = (total + 511) / 512;              // two chunks per thread and trip
+  int64_t b = (total + 255) / 256;
   const int64_t cap = static_cast<int64_t>(sms) * 8;
+  *shortish = total <= 4 * cap * 256;
   *blocks = static_cast<unsigned>(b < cap ? b : cap);
   return NF4LL_OK;
 }
@@ -323,10 +333,18 @@ extern "C" int nf4ll_swiglu_forward(const void* g, int64_t ldg, const void* u, i
   if (int rc = check_mat16(h, ldh, I, "nf4ll_swiglu_forward", "h")) return rc;
   if (int rc = require_sm100()) return rc;
   unsigned blocks = 1;
-  if (int rc = grid_for(M * (I / 8), &blocks)) return rc;
+  const int64_t total = M * (I / 8);
+  bool shortish = false;
+  if (int rc = grid_for(total, &blocks, &shortish)) return rc;
   PdlLaunch lc(dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream));
-  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, swiglu_fwd_kernel, static_cast<const __half*>(g), ldg, static_cast<const __half*>(u), ldu,
-                                static_cast<__half*>(h), ldh, M, I / 8));
+  const __half *gp = static_cast<const __half*>(g), *up = static_cast<const __half*>(u);
+  __half* hp = static_cast<__half*>(h);
+  if (total < (int64_t(1) << 30)) {
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, shortish ? swiglu_fwd_kernel<uint32_t, 1> : swiglu_fwd_kernel<uint32_t, 4>, gp, ldg, up, ldu, hp, ldh,
+                                  static_cast<uint32_t>(total), static_cast<uint32_t>(I / 8)));
+  } else {
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, swiglu_fwd_kernel<int64_t, 4>, gp, ldg, up, ldu, hp, ldh, total, I / 8));
+  }
   return NF4LL_OK;
 }
 
@@ -342,11 +360,18 @@ extern "C" int nf4ll_swiglu_backward(const void* g, int64_t ldg, const void* u, 
   if (int rc = check_mat16(du, lddu, I, "nf4ll_swiglu_backward", "du")) return rc;
   if (int rc = require_sm100()) return rc;
   unsigned blocks = 1;
-  if (int rc = grid_for(M * (I / 8), &blocks)) return rc;
+  const int64_t total = M * (I / 8);
+  bool shortish = false;
+  if (int rc = grid_for(total, &blocks, &shortish)) return rc;
   PdlLaunch lc(dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream));
-  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, swiglu_bwd_kernel, static_cast<const __half*>(g), ldg, static_cast<const __half*>(u), ldu,
-                                static_cast<const __half*>(dh), lddh, static_cast<__half*>(dg), lddg, static_cast<__half*>(du), lddu,
-                                M, I / 8));
+  const __half *gp = static_cast<const __half*>(g), *up = static_cast<const __half*>(u), *dp = static_cast<const __half*>(dh);
+  __half *dgp = static_cast<__half*>(dg), *dup = static_cast<__half*>(du);
+  if (total < (int64_t(1) << 30)) {
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, shortish ? swiglu_bwd_kernel<uint32_t, 1> : swiglu_bwd_kernel<uint32_t, 2>, gp, ldg, up, ldu, dp, lddh, dgp, lddg,
+                                  dup, lddu, static_cast<uint32_t>(total), static_cast<uint32_t>(I / 8)));
+  } else {
+    NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, swiglu_bwd_kernel<int64_t, 2>, gp, ldg, up, ldu, dp, lddh, dgp, lddg, dup, lddu, total, I / 8));
+  }
   return NF4LL_OK;
 }
 
