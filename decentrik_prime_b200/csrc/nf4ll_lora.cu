@@ -260,9 +260,15 @@ int lora_down_launch(const void* act, int64_t ldact, const DownBranch* br, int n
   const __half* a = static_cast<const __half*>(act);
   const int64_t groups16 = (M + 15) / 16;
   if (groups16 * 4 >= 3 * static_cast<int64_t>(sms)) {
-    // enough rows for (nearly) one CTA per SM at 16 rows each: a CTA takes the whole contraction,
-    // sixteen warps deep, and stores its rows directly
-    return down_run<2, kDownDirect, 16>(dim3(static_cast<unsigned>(groups16), 1), 0, a, ldact, br, n, scale, M, C, C, zero_ptr, zero_words, stream);
+    // enough rows for (nearly) one CTA per SM at 16 rows each: a CTA takes the whole contraction and stores its rows directly. Sixteen warps
+    // deep where each SM has one CTA; of more rows an SM holds two CTAs of eight warps or four of four, one of which computes or ends
+    // while the others' loads are on their way. Under a mask / without, us, sixteen warps against this: 4096 x 8960 29.0 / 21.3 -> 23.7 / 17.0 (four
+    // warps 31.1 / 23.5), 8192 x 3584 28.2 / 20.4 -> 19.1 / 14.0 (eight 21.6 / 15.7), 16384 x 3584 48.4 / 34.6 -> 34.4 / 25.2, 16384 x 18944 178 / 126 ->
+    // 162 / 115; 2048 x 8960 16.0 / 11.8 with sixteen, 18.5 / 13.7 with eight.
+    const dim3 grid(static_cast<unsigned>(groups16), 1);
+    if (groups16 <= sms) return down_run<2, kDownDirect, 16>(grid, 0, a, ldact, br, n, scale, M, C, C, zero_ptr, zero_words, stream);
+    if (groups16 <= 2 * static_cast<int64_t>(sms)) return down_run<2, kDownDirect, 8>(grid, 0, a, ldact, br, n, scale, M, C, C, zero_ptr, zero_words, stream);
+    return down_run<2, kDownDirect, 4>(grid, 0, a, ldact, br, n, scale, M, C, C, zero_ptr, zero_words, stream);
   }
   const int64_t row_groups = (M + 31) / 32;
   const int64_t units = (C + kDownWarps * 32 - 1) / (kDownWarps * 32);     // 256-column units
