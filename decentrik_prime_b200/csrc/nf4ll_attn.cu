@@ -7,16 +7,17 @@
 // per sequence is the whole gain (through PyTorch: 280 launches per layer and step). The contractions use mma.sync:
 // tiles of 64 rows are too small to feed tcgen05, and at a few microseconds per launch there is nothing to win.
 // Sequence boundaries travel in the kernel parameters, so no copy to the device is needed per batch.
-// That holds for short sequences. One of 2048 rows, 28 heads, takes 655 us forward and backward (161 TFLOP/s, chained by the
-// latencies of mma.sync and ldmatrix at one CTA of four warps per SM and tile), one of 4096 rows 2257 (187); the caller
+// That holds for short sequences. One of 2048 rows, 28 heads, takes 618 us forward and backward (171 TFLOP/s, chained by the
+// latencies of mma.sync and ldmatrix at eight warps per SM), one of 4096 rows 2160 (196); the caller
 // (stack.py) takes other kernels for such batches.
 //
 //   rope     q, k rotated once into a buffer (a key row is read by every query tile after it)
-//   forward  one CTA per 64 query rows and head, 4 warps of 16 rows, keys and values in 64-row blocks by cp.async
+//   forward  one CTA per 64 query rows and head, 4 warps of 16 rows, keys and values in 64-row blocks by cp.async; of long sequences
+//            two times 4 warps, the blocks dealt out between them
 //   dK, dV   a cluster of up to 8 CTAs per 64 key rows and key-value head, the group's query heads dealt out among them,
 //            each looping over the later query rows; their sums meet through distributed shared memory in a fixed order. One
 //            CTA for the whole group left most SMs idle: 951 rows, 12 heads of 128 in groups of 6, 115 us, 28 now
-//   dQ       one CTA per 64 query rows and head, looping over the earlier key rows
+//   dQ       one CTA per 64 query rows and head, looping over the earlier key rows, shared out like the forward's
 // The backward kernels rotate dQ and dK back in their epilogue (both halves of a rotated pair sit in one thread).
 #include "nf4ll_pair.cuh"
 
@@ -78,12 +79,12 @@ template <int HD>
 __device__ __forceinline__ uint32_t tile_addr(uint32_t base, int row, int chunk) {
   return base + row * (HD * 2) + ((chunk ^ (row & 7)) << 4);
 }
-template <int HD, int ROWS>
+template <int HD, int ROWS, int THREADS = kAttnThreads>
 __device__ __forceinline__ void load_tile(uint32_t base, const __half* src, int64_t ld, int row0, int end) {
   constexpr int CH = HD / 8;
 #pragma unroll
-  for (int i = 0; i < ROWS * CH / kAttnThreads; ++i) {
-    const int idx = threadIdx.x + i * kAttnThreads, r = idx / CH, c = idx % CH;
+  for (int i = 0; i < ROWS * CH / THREADS; ++i) {
+    const int idx = threadIdx.x % THREADS + i * THREADS, r = idx / CH, c = idx % CH;
     const bool v = row0 + r < end;
     attn_cp16(tile_addr<HD>(base, r, c), v ? src + (row0 + r) * ld + c * 8 : src, v);
   }
@@ -103,6 +104,9 @@ template <int HD>
 __device__ __forceinline__ void frag_bt(uint32_t base, int k0, int n0, int lane, uint32_t (&b)[4]) {
   ldsm4t(tile_addr<HD>(base, k0 + (lane & 15), n0 / 8 + (lane >> 4)), b);
 }
+
+// the 128 threads of one half of a CTA
+__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, %1;" ::"r"(half + 1), "n"(kAttnThreads) : "memory"); }
 
 __device__ __forceinline__ void find_tile(const SeqTable& t, int tile, int& start, int& len, int& t0) {
   int lo = 0, hi = t.n - 1;
@@ -154,15 +158,15 @@ rope_kernel(const __half* __restrict__ src, int64_t lds, __half* __restrict__ ds
 }
 
 // ---------------------------------------------------------------------------------------------
-template <int HD>
-__global__ void __launch_bounds__(kAttnThreads)
+template <int HD, int HALVES>
+__global__ void __launch_bounds__(HALVES * kAttnThreads)
 attn_fwd_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ SeqTable seqs) {
   pdl_wait();
   pdl_launch_dependents();
   extern __shared__ __align__(128) uint8_t a_smem[];
   constexpr int TILE = kAttnRows * HD * 2, KS = HD / 16, NT = HD / 8;
-  const uint32_t sQ = smem_u32(a_smem), sK = sQ + TILE, sV = sK + 2 * TILE;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int half = HALVES == 1 ? 0 : threadIdx.x / kAttnThreads, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t sQ = smem_u32(a_smem), sK = sQ + TILE + half * 4 * TILE, sV = sK + 2 * TILE;
   int start, len, q0;
   find_tile(seqs, seqs.tile[seqs.n] - 1 - blockIdx.x, start, len, q0);      // later (longer) tiles first
   const int head = blockIdx.y, kvh = head / p.group;
@@ -170,25 +174,37 @@ attn_fwd_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Se
   const __half* kp = p.k + start * p.ldr + kvh * HD;
   const __half* vp = p.v + start * p.ldv + kvh * HD;
   const int n_blocks = q0 / kAttnRows + 1;
-  load_tile<HD, kAttnRows>(sQ, qp, p.ldr, q0, len);
-  load_tile<HD, kAttnRows>(sK, kp, p.ldr, 0, len);
-  load_tile<HD, kAttnRows>(sV, vp, p.ldv, 0, len);
-  attn_commit();
+  load_tile<HD, kAttnRows, HALVES * kAttnThreads>(sQ, qp, p.ldr, q0, len);
+  auto load = [&](int b, int slot) {
+    if (b < n_blocks) {
+      load_tile<HD, kAttnRows>(sK + slot * TILE, kp, p.ldr, b * kAttnRows, len);
+      load_tile<HD, kAttnRows>(sV + slot * TILE, vp, p.ldv, b * kAttnRows, len);
+    }
+    attn_commit();
+  };
+  auto sync = [&] {
+    if (HALVES == 1) __syncthreads();
+    else half_sync(half);
+  };
+  load(half, 0);
+  load(half + HALVES, 1);
   float o[NT][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
 #pragma unroll
   for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int i = 0; i < 4; ++i) o[n][i] = 0.f;
   const int row_a = q0 + warp * 16 + g;
-  for (int b = 0; b < n_blocks; ++b) {
-    const uint32_t kb = sK + (b & 1) * TILE, vb = sV + (b & 1) * TILE;
-    if (b + 1 < n_blocks) {
-      load_tile<HD, kAttnRows>(sK + ((b + 1) & 1) * TILE, kp, p.ldr, (b + 1) * kAttnRows, len);
-      load_tile<HD, kAttnRows>(sV + ((b + 1) & 1) * TILE, vp, p.ldv, (b + 1) * kAttnRows, len);
-    }
-    attn_commit();
-    attn_wait<1>();
-    __syncthreads();
+  attn_wait<1>();
+  __syncthreads();
+  // the queries stay in registers where four warps have an SM's share of them (40 sequences of 30 rows 17.8 -> 16.4 us; with eight 81 -> 85
+  // at 2048 rows, 12 heads)
+  uint32_t qf[HALVES == 2 ? 1 : KS][4];
+  if (HALVES == 1) {
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) frag_a<HD>(sQ, warp * 16, kk, lane, qf[kk]);
+  }
+  for (int b = half, slot = 0; b < n_blocks; b += HALVES, slot ^= 1) {
+    const uint32_t kb = sK + slot * TILE, vb = sV + slot * TILE;
     float s[8][4];
 #pragma unroll
     for (int n = 0; n < 8; ++n)
@@ -196,8 +212,8 @@ attn_fwd_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Se
       for (int i = 0; i < 4; ++i) s[n][i] = 0.f;
 #pragma unroll
     for (int kk = 0; kk < KS; ++kk) {
-      uint32_t a[4];
-      frag_a<HD>(sQ, warp * 16, kk, lane, a);
+      if (HALVES == 2) frag_a<HD>(sQ, warp * 16, kk, lane, qf[0]);
+      const uint32_t (&a)[4] = qf[HALVES == 2 ? 0 : kk];
 #pragma unroll
       for (int n2 = 0; n2 < 4; ++n2) {
         uint32_t bf[4];
@@ -246,7 +262,40 @@ attn_fwd_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Se
         mma16816(o[2 * n2 + 1], a0, a1, a2, a3, bf[2], bf[3]);
       }
     }
+    sync();
+    load(b + 2 * HALVES, slot);
+    attn_wait<1>();
+    sync();
+  }
+  if constexpr (HALVES == 2) {
+    // the second half's sums through shared memory (its own key and value blocks have been read)
+    attn_wait<0>();
+    float* const other = reinterpret_cast<float*>(a_smem + TILE + 4 * TILE);       // [4 + o][thread], two planes of m and l first
     __syncthreads();
+    const int tid = threadIdx.x % kAttnThreads;
+    if (half) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        other[h * kAttnThreads + tid] = m[h];
+        other[(2 + h) * kAttnThreads + tid] = l[h];
+      }
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) other[(4 + 4 * n + i) * kAttnThreads + tid] = o[n][i];
+    }
+    __syncthreads();
+    if (half) return;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const float m1 = other[h * kAttnThreads + tid], mn = fmaxf(m[h], m1), c0 = exp2_fast(m[h] - mn), c1 = exp2_fast(m1 - mn);
+      m[h] = mn;
+      l[h] = l[h] * c0 + other[(2 + h) * kAttnThreads + tid] * c1;
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 2 * h; i < 2 * h + 2; ++i) o[n][i] = o[n][i] * c0 + other[(4 + 4 * n + i) * kAttnThreads + tid] * c1;
+    }
   }
 #pragma unroll
   for (int h = 0; h < 2; ++h) {
@@ -317,26 +366,36 @@ __device__ __forceinline__ void attn_cp4(uint32_t dst, const void* src, bool val
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
 }
 
-template <int HD>
-__global__ void __launch_bounds__(kAttnThreads)
+template <int HD, int HALVES>
+__global__ void __launch_bounds__(HALVES * kAttnThreads)
 attn_dq_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ SeqTable seqs) {
   pdl_wait();
   pdl_launch_dependents();
   extern __shared__ __align__(128) uint8_t a_smem[];
   constexpr int TILE = kAttnRows * HD * 2, KS = HD / 16, NT = HD / 8;
-  const uint32_t sQ = smem_u32(a_smem), sO = sQ + TILE, sK = sO + TILE, sV = sK + 2 * TILE;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int half = HALVES == 1 ? 0 : threadIdx.x / kAttnThreads, warp = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const uint32_t sQ = smem_u32(a_smem), sO = sQ + TILE, sK = sO + TILE + half * 4 * TILE, sV = sK + 2 * TILE;
   int start, len, q0;
   find_tile(seqs, seqs.tile[seqs.n] - 1 - blockIdx.x, start, len, q0);
   const int head = blockIdx.y, kvh = head / p.group;
   const __half* kp = p.k + start * p.ldr + kvh * HD;
   const __half* vp = p.v + start * p.ldv + kvh * HD;
   const int n_blocks = q0 / kAttnRows + 1;
-  load_tile<HD, kAttnRows>(sQ, p.q + start * p.ldr + head * HD, p.ldr, q0, len);
-  load_tile<HD, kAttnRows>(sO, p.dout + start * p.lddo + head * HD, p.lddo, q0, len);
-  load_tile<HD, kAttnRows>(sK, kp, p.ldr, 0, len);
-  load_tile<HD, kAttnRows>(sV, vp, p.ldv, 0, len);
-  attn_commit();
+  load_tile<HD, kAttnRows, HALVES * kAttnThreads>(sQ, p.q + start * p.ldr + head * HD, p.ldr, q0, len);
+  load_tile<HD, kAttnRows, HALVES * kAttnThreads>(sO, p.dout + start * p.lddo + head * HD, p.lddo, q0, len);
+  auto load = [&](int b, int slot) {
+    if (b < n_blocks) {
+      load_tile<HD, kAttnRows>(sK + slot * TILE, kp, p.ldr, b * kAttnRows, len);
+      load_tile<HD, kAttnRows>(sV + slot * TILE, vp, p.ldv, b * kAttnRows, len);
+    }
+    attn_commit();
+  };
+  auto sync = [&] {
+    if (HALVES == 1) __syncthreads();
+    else half_sync(half);
+  };
+  load(half, 0);
+  load(half + HALVES, 1);
   const int row_a = q0 + warp * 16 + g;
   float lse[2], delta[2], dq[NT][4];
 #pragma unroll
@@ -349,15 +408,10 @@ attn_dq_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Seq
   for (int n = 0; n < NT; ++n)
 #pragma unroll
     for (int i = 0; i < 4; ++i) dq[n][i] = 0.f;
-  for (int b = 0; b < n_blocks; ++b) {
-    const uint32_t kb = sK + (b & 1) * TILE, vb = sV + (b & 1) * TILE;
-    if (b + 1 < n_blocks) {
-      load_tile<HD, kAttnRows>(sK + ((b + 1) & 1) * TILE, kp, p.ldr, (b + 1) * kAttnRows, len);
-      load_tile<HD, kAttnRows>(sV + ((b + 1) & 1) * TILE, vp, p.ldv, (b + 1) * kAttnRows, len);
-    }
-    attn_commit();
-    attn_wait<1>();
-    __syncthreads();
+  attn_wait<1>();
+  __syncthreads();
+  for (int b = half, slot = 0; b < n_blocks; b += HALVES, slot ^= 1) {
+    const uint32_t kb = sK + slot * TILE, vb = sV + slot * TILE;
 #pragma unroll
     for (int hb = 0; hb < 2; ++hb) {         // 32 keys at a time
       float s[4][4], dp[4][4];
@@ -402,7 +456,28 @@ attn_dq_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Seq
         }
       }
     }
+    sync();
+    load(b + 2 * HALVES, slot);
+    attn_wait<1>();
+    sync();
+  }
+  if constexpr (HALVES == 2) {
+    attn_wait<0>();
+    float* const other = reinterpret_cast<float*>(a_smem + 2 * TILE + 4 * TILE);   // the second half's sums, [value][thread]
     __syncthreads();
+    const int tid = threadIdx.x % kAttnThreads;
+    if (half) {
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int i = 0; i < 4; ++i) other[(4 * n + i) * kAttnThreads + tid] = dq[n][i];
+    }
+    __syncthreads();
+    if (half) return;
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) dq[n][i] += other[(4 * n + i) * kAttnThreads + tid];
   }
   store_unrotated<HD>(dq, p, p.dq + start * p.ldd + head * HD, row_a, len, t, p.scale);
 }
@@ -594,10 +669,22 @@ static int attn_table(SeqTable* t, const int32_t* lens, int n, int at, int64_t* 
   return at;
 }
 
+// Eight warps per CTA in two halves that take the key blocks in turn, each with a ring of its own, and add up at the end: half as long a
+// chain of blocks per tile. From four blocks in the longest sequence on; with fewer the second half idles and costs shared memory (sequences
+// of 130 and 129 rows, 28 heads of 128, forward 12.5 us with one half, 14.1 with two; of 190 and 150 rows 14.2 and 14.5). us, forward / backward, one half ->
+// two: 4 sequences of 951 rows, 12 heads of 128, 20.7 / 52.3 -> 18.4 / 49.0; 333 rows, 28 heads 19.6 / 53.1 -> 17.6 / 48.0; 1024 rows, 12 heads 44.0 /
+// 121 -> 32.0 / 104; 2048 rows, 28 heads 169 / 477 -> 158 / 460.
+static int attn_halves(const SeqTable& t) {
+  int longest = 0;
+  for (int i = 0; i < t.n; ++i) longest = t.tile[i + 1] - t.tile[i] > longest ? t.tile[i + 1] - t.tile[i] : longest;
+  return longest > 3 ? 2 : 1;
+}
+
 template <int HD>
 static int attn_forward_hd(AttnParams p, const __half* qkv, int64_t ldq, __half* roped, const int32_t* lens, int n, int kv_heads, cudaStream_t stream) {
-  constexpr int smem = 5 * kAttnRows * HD * 2;
-  NF4LL_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  constexpr int tile = kAttnRows * HD * 2;
+  NF4LL_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 5 * tile));
+  NF4LL_CUDA(cudaFuncSetAttribute(attn_fwd_kernel<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 9 * tile));
   int64_t row = 0;
   for (int at = 0; at < n;) {
     SeqTable t;
@@ -606,16 +693,18 @@ static int attn_forward_hd(AttnParams p, const __half* qkv, int64_t ldq, __half*
     const int64_t work = static_cast<int64_t>(t.start[t.n] - t.start[0]) * (p.heads + kv_heads) * (HD / 16);
     PdlLaunch lr(dim3(static_cast<unsigned>((work + 255) / 256 < 1184 ? (work + 255) / 256 : 1184)), dim3(256), 0, stream);
     NF4LL_CUDA(cudaLaunchKernelEx(&lr.cfg, rope_kernel, qkv, ldq, roped, p.ldr, p.trig, p.heads + kv_heads, HD, t));
-    PdlLaunch lf(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(kAttnThreads), smem, stream);
-    NF4LL_CUDA(cudaLaunchKernelEx(&lf.cfg, attn_fwd_kernel<HD>, p, t));
+    const int halves = attn_halves(t);
+    PdlLaunch lf(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(halves * kAttnThreads), (1 + 4 * halves) * tile, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lf.cfg, halves == 2 ? attn_fwd_kernel<HD, 2> : attn_fwd_kernel<HD, 1>, p, t));
   }
   return NF4LL_OK;
 }
 
 template <int HD>
 static int attn_backward_hd(AttnParams p, const int32_t* lens, int n, int kv_heads, cudaStream_t stream) {
-  constexpr int smem_q = 6 * kAttnRows * HD * 2, smem_kv = 4 * kAttnRows * HD * 2 + 4 * 32 * 4;
-  NF4LL_CUDA(cudaFuncSetAttribute(attn_dq_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_q));
+  constexpr int tile = kAttnRows * HD * 2, smem_kv = 4 * kAttnRows * HD * 2 + 4 * 32 * 4;
+  NF4LL_CUDA(cudaFuncSetAttribute(attn_dq_kernel<HD, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 6 * tile));
+  NF4LL_CUDA(cudaFuncSetAttribute(attn_dq_kernel<HD, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 10 * tile));
   NF4LL_CUDA(cudaFuncSetAttribute(attn_dkv_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_kv));
   int64_t row = 0;
   for (int at = 0; at < n;) {
@@ -628,8 +717,9 @@ static int attn_backward_hd(AttnParams p, const int32_t* lens, int n, int kv_hea
     const unsigned parts = static_cast<unsigned>(p.group < 8 ? p.group : 8);
     PdlLaunch lk(dim3(static_cast<unsigned>(t.tile[t.n]) * parts, static_cast<unsigned>(kv_heads)), dim3(kAttnThreads), smem_kv, stream, parts, 1);
     NF4LL_CUDA(cudaLaunchKernelEx(&lk.cfg, attn_dkv_kernel<HD>, p, t));
-    PdlLaunch lq(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(kAttnThreads), smem_q, stream);
-    NF4LL_CUDA(cudaLaunchKernelEx(&lq.cfg, attn_dq_kernel<HD>, p, t));
+    const int halves = attn_halves(t);
+    PdlLaunch lq(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(halves * kAttnThreads), (2 + 4 * halves) * tile, stream);
+    NF4LL_CUDA(cudaLaunchKernelEx(&lq.cfg, halves == 2 ? attn_dq_kernel<HD, 2> : attn_dq_kernel<HD, 1>, p, t));
   }
   return NF4LL_OK;
 }

@@ -274,8 +274,8 @@ class PackedAttention:
     over all sequences and heads (the library's nf4ll_attention_*; reference solution/k_rope.py, k_attn.py) for fp16 rows on
     the GPU in heads of 64 or 128, PyTorch's kernels per sequence (scaled_dot_product_attention, autograd for the backward)
     for others, and for long sequences: the library's use mma.sync on tiles of 64 rows, which is faster where launches and
-    short sequences count (4 sequences of 951 rows in all, 12 heads of 128: 77 us and 1507), and slower once the products do
-    (one of 2048 rows, 28 heads: 655 us, PyTorch's 557 replayed from a graph and 840 called one by one; of 4096 rows 2257 and
+    short sequences count (4 sequences of 951 rows in all, 12 heads of 128: 68 us and 1507), and slower once the products do
+    (one of 2048 rows, 28 heads: 618 us, PyTorch's 557 replayed from a graph and 840 called one by one; of 4096 rows 2160 and
     1342; 8 of 1024 rows 1317 and 2991). Rotary embedding as in Qwen2: the two halves of a head rotate against each other,
     positions restart at every sequence."""
 
