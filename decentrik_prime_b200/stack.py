@@ -83,6 +83,7 @@ class DecoderLayerProjections:
             self._Bv_pad = torch.zeros(2 * kv, linear.RANK, dtype=torch.float16, device=device)
             self._Bvt_pad = torch.zeros(linear.RANK, 2 * kv, dtype=torch.float16, device=device)
             self._pad_src = pv
+            pv.B16 = self._Bv_pad[kv:]                         # refreshed where the joint k | v backward reads it
             self.refresh16()
         # with a bucket the layer's gradients are one contiguous slice: cleared by one fill per backward
         self._grad_slice = bucket.flat[grad_lo:bucket._at] if bucket is not None and bucket._at > grad_lo else None
@@ -94,7 +95,6 @@ class DecoderLayerProjections:
             if p.has_lora:
                 p.refresh16()
         if self.kv_one_backward:
-            self._Bv_pad[self.kv:].copy_(self._pad_src.B16)
             self._Bvt_pad[:, self.kv:].copy_(self._pad_src.B16t)
 
     def grad_numel(self, lora_on):
@@ -510,7 +510,7 @@ class NormedStack:
         x, delta = x32, None
         for layer, masks in zip(self.layers, masks_per_layer):
             x, delta = layer.forward(x, delta, masks, keep_scale, seq_lens)
-        return x + delta.float()
+        return x + delta                                       # promoted to fp32 on the way in
 
     def backward(self, dres, need_input_grad=False):
         d, d16 = dres, dres.half()
