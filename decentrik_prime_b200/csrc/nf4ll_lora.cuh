@@ -19,6 +19,12 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
+// An 8 x 8 block of 16-bit values, a row in four lanes: transposed
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
 // two values as fp16 pairs hi + lo: 22 bits of each
 __device__ __forceinline__ void split_half2(float a, float b, uint32_t& hi, uint32_t& lo) {
   hi = pack_half2_rn(a, b);

@@ -19,6 +19,7 @@
 //
 // A group of 8 token rows (16 in the forward of a long batch) belongs to a CTA or, where the groups would leave SMs idle, to a cluster
 // whose CTAs share out the hidden dimension; a lane's values stay in registers between the row reduction and the second phase.
+#include "nf4ll_lora.cuh"
 #include "nf4ll_pair.cuh"
 
 namespace nf4ll {
@@ -346,12 +347,6 @@ rms_fwd_split_kernel(const float* __restrict__ x, const __half* __restrict__ del
   if (gridDim.y > 1) cluster_sync_all();           // shared memory stays until the others have read it
 }
 
-// An 8 x 8 block of 16-bit values, a row in four lanes: transposed
-__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
-  uint32_t r;
-  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
-  return r;
-}
 // a, b as fp16 pairs of descending weight: 33 bits, all of an fp32 value in fp16's range
 __device__ __forceinline__ void split3(float a, float b, uint32_t (&p)[3]) {
 #pragma unroll
