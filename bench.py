@@ -492,12 +492,12 @@ def run_ours(args):
                              "frac_of_burst": (achieved / pk["tflops_burst"]) if achieved else None,
                              "frac_of_sustained": (achieved / pk["tflops_sustained"]) if achieved else None,
                              "traffic": NCU_DRAM_BYTES_PER_LAUNCH,
-                             "traffic_source": "ncu capture of one step (mean DRAM bytes read + written per tensor-core launch), "
-                                               "not a measurement of this run",
+                             "traffic_source": "ncu capture of one step (mean DRAM bytes read + written per tensor-core launch, five of them: "
+                                               "gate and up apart in the backward), not a measurement of this run",
                              # NF4 bytes of the six weight passes of a step + every activation matrix a launch reads or
-                             # writes (x, g, u, h | h, y | dy, dh | dg, dx | du, dx read + written), over the five launches
+                             # writes (x, g, u, h | h, y | dy, dh | dg, du, dx read + written), over the four launches
                              "algorithmic_bytes_per_launch": (6 * INTER * HIDDEN * 0.516113
-                                                              + 2 * M * (6 * HIDDEN + 7 * INTER)) / 5,
+                                                              + 2 * M * (5 * HIDDEN + 7 * INTER)) / 4,
                              "kernel": "nf4_gemm_kernel / nf4_gemm_pair_kernel (forward and backward-dX launches)",
                              "events": events_where,
                              "launches_timed": n_kern, "avg_launch_us": kern_ms * 1e3 / max(n_kern, 1)},
@@ -837,9 +837,9 @@ def _fill_event_pool(n):
 
 
 def _hook_block(blk, ev_pairs, M):
-    """Arrange for the six tensor-core launches of this block step to be bracketed by CUDA events.
-    The library records a one-shot event pair around its next GEMM kernel, so each projection call
-    is wrapped to arm the hook right before it."""
+    """Arrange for the four tensor-core launches of this block step (gate|up and down, forward and backward-dX) to be
+    bracketed by CUDA events. The library records a one-shot event pair around its next GEMM kernel, so each call that
+    launches one is wrapped to arm the hook right before it."""
     import torch
     from decentrik_prime_b200 import _lib, linear
     h = _lib.lib()
@@ -848,38 +848,29 @@ def _hook_block(blk, ev_pairs, M):
         return
     blk._hooked, blk._ev_sink = True, ev_pairs
 
-    def arm(proj, n_out):
+    def arm(flops):
         if blk._ev_sink is None:
             return
         a, b = _event_pool.pop()
         h.nf4ll_kernel_events(a.cuda_event, b.cuda_event)
-        blk._ev_sink.append((a, b, 2 * M * proj.w.N * proj.w.K + 2 * M * 16 * n_out))
+        blk._ev_sink.append((a, b, flops))
 
-    if getattr(blk, "fused_glue", False):
-        # gate and up run as ONE tensor-core launch (gated product in its epilogue): arm the hook once for both
-        blk_fwd = blk.forward
+    def wrap(owner, name, flops):
+        call = getattr(owner, name)
 
-        def blk_fwd_hook(*a, _f=blk_fwd, **k):
-            if blk._ev_sink is not None:
-                ea, eb = _event_pool.pop()
-                h.nf4ll_kernel_events(ea.cuda_event, eb.cuda_event)
-                blk._ev_sink.append((ea, eb, sum(2 * M * pj.w.N * pj.w.K + 2 * M * 16 * pj.w.N for pj in (blk.gate, blk.up))))
-            return _f(*a, **k)
+        def hook(*a, **k):
+            arm(flops)
+            return call(*a, **k)
 
-        blk.forward = blk_fwd_hook
+        setattr(owner, name, hook)
 
-    for proj in blk.projections:
-        fwd, bwd = proj.forward, proj.backward
-
-        def fwd_hook(*a, _p=proj, _f=fwd, **k):
-            arm(_p, _p.w.N)
-            return _f(*a, **k)
-
-        def bwd_hook(*a, _p=proj, _f=bwd, **k):
-            arm(_p, _p.w.K)
-            return _f(*a, **k)
-
-        proj.forward, proj.backward = fwd_hook, bwd_hook
+    product = {p: 2 * M * p.w.N * p.w.K for p in blk.projections}
+    # gate and up run as ONE tensor-core launch each way: forward with both rank-16 terms (the gated product in its epilogue; the
+    # block's first launch of the kind), backward without (they are expanded before)
+    wrap(blk, "forward", sum(product[p] + 2 * M * 16 * p.w.N for p in (blk.gate, blk.up)))
+    wrap(blk.down, "forward", product[blk.down] + 2 * M * 16 * blk.down.w.N)
+    wrap(blk, "_down_dx", product[blk.down] + 2 * M * 16 * blk.down.w.K)
+    wrap(blk, "_gate_up_dx", product[blk.gate] + product[blk.up])
 
 
 def main():

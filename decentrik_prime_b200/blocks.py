@@ -227,8 +227,8 @@ class MlpBlock:
         gate, up, down = self.projections
         (x, mg, kg, tg), (_, mu, ku, tu), (h, md, kd, td) = (p._saved for p in self.projections)
         gs = self.grad_stream
-        gu = g._base
-        dh, ud = linear.backward_dx(down.w, dy, lora=down.lora, mask=md, keep_scale=kd, want_u=True)
+        gu = g.as_strided((g.shape[0], 2 * self.inter), g.stride())      # g and u lie side by side
+        dh, ud = self._down_dx(dy, md, kd)
         ug, uu = linear.gated_backward(g, u, dh, md, kd, tg, tu, ud, (gate.B16t, gate.scale), (up.B16t, up.scale), gate.dB, up.dB,
                                        down.dA, accumulate_grads)
         grads = [(dy, h, td, ud, down.scale, None, 1.0, None, down.dB), (g, x, tg, ug, gate.scale, mg, kg, gate.dA, None),
@@ -241,7 +241,7 @@ class MlpBlock:
         if need_dx:
             dx = out if out is not None else torch.empty(dy.shape[0], self.hidden, dtype=torch.float16, device=dy.device)
             linear.lora_expand([(ug, gate.A16, mg, kg), (uu, up.A16, mu, ku)], dx)
-            linear.backward_dx(self.w_gu, gu, out=dx, accumulate=True)
+            self._gate_up_dx(gu, dx)
         if gs is not None:
             torch.cuda.current_stream(dy.device).wait_stream(gs)
         else:
@@ -249,6 +249,12 @@ class MlpBlock:
         for p in self.projections:
             p._saved = None
         return dx
+
+    def _down_dx(self, dy, mask, keep_scale):
+        return linear.backward_dx(self.down.w, dy, lora=self.down.lora, mask=mask, keep_scale=keep_scale, want_u=True)
+
+    def _gate_up_dx(self, gu, dx):
+        linear.backward_dx(self.w_gu, gu, out=dx, accumulate=True)
 
     def _backward_each(self, g, u, dy, need_dx, accumulate_grads, out):
         gs, pend = self.grad_stream, self._pending

@@ -82,21 +82,23 @@ def test_gradients_of_three_projections(M, accumulate):
 
 
 @pytest.mark.parametrize("M", [1, 24, 187])
-def test_joined_and_separate_backward(M):
+@pytest.mark.parametrize("mode", [torch.no_grad, torch.inference_mode])
+def test_joined_and_separate_backward(M, mode):
     """Both orders of the block's backward round dx twice to fp16: each within two half-ulps of the exact sum."""
     H, I = 256, 512
     x, dy = rand(M, H, seed=1).half(), rand(M, H, seed=2).half()
     masks = [(rand(M, k, seed=3 + i) > -1.3).to(torch.uint8) for i, k in enumerate((H, H, I))]
     block = MlpBlock(H, I, 0, DEV)
     got = []
-    for joined in (True, False):
-        block.forward(x, masks, 1.1)
-        if not joined:
-            g, u = block._saved
-            dx = block._backward_each(g, u, dy, True, False, None)
-        else:
-            dx = block.backward(dy)
-        got.append((dx, [t.clone() for p in block.projections for t in (p.dA, p.dB)]))
+    with mode():
+        for joined in (True, False):
+            block.forward(x, masks, 1.1)
+            if not joined:
+                g, u = block._saved
+                dx = block._backward_each(g, u, dy, True, False, None)
+            else:
+                dx = block.backward(dy)
+            got.append((dx, [t.clone() for p in block.projections for t in (p.dA, p.dB)]))
     (dx1, gr1), (dx2, gr2) = got
     scale = dx2.float().abs().max()
     assert ((dx1.float() - dx2.float()).abs() <= 2.0 ** -11 * 4 * scale).all()
