@@ -176,9 +176,9 @@ class MlpBlock:
         self._pending = []
 
     def use_grad_stream(self, stream=None):
-        """Run the three dA/dB kernels of a backward on a side stream, beside the dX GEMMs (they are bound by
-        HBM latency, the GEMMs by the tensor and shared-memory pipes); `backward` joins the stream before it
-        returns. Works eagerly and under CUDA-graph capture (the fork and the join are captured as edges)."""
+        """Run the dA/dB kernel of a backward (the kernels, where only some projections carry LoRA) on a side stream, beside
+        the dX GEMMs (it is bound by HBM latency, the GEMMs by the tensor and shared-memory pipes); `backward` joins the stream
+        before it returns. Works eagerly and under CUDA-graph capture (the fork and the join are captured as edges)."""
         self.grad_stream = stream if stream is not None else torch.cuda.Stream(self.gate.w.device)
         return self
 
@@ -207,7 +207,7 @@ class MlpBlock:
         return y
 
     def backward(self, dy, need_dx=True, accumulate_grads=False, out=None):
-        """d(input) of the block (into `out` when given) and the LoRA gradients of its three projections."""
+        """d(input) of the block (into `out` when given, which may be `dy`) and the LoRA gradients of its three projections."""
         g, u = self._saved
         if self._grad_slice is not None and not accumulate_grads:
             self._grad_slice.zero_()
@@ -219,11 +219,17 @@ class MlpBlock:
         self._saved = None
         return dx
 
+    def _wait_before_writing(self, out, dy):
+        """What runs on the gradient stream reads dy: it ends before `out` is written where that shares its memory."""
+        if self.grad_stream is not None and out is not None and out.untyped_storage().data_ptr() == dy.untyped_storage().data_ptr():
+            torch.cuda.current_stream(dy.device).wait_stream(self.grad_stream)
+
     def _backward_joined(self, g, u, dy, need_dx, accumulate_grads, out):
         """With LoRA on every projection. One pass over g, u and dh forms dg and du and takes from them, and from h, all that the
-        branches need of [M, inter] matrices; the LoRA terms of dx are expanded first (two dropout masks) and one product over
-        the stacked weight adds [dg | du] . W to them; what is left of the factors' gradients is one more launch. Two roundings
-        of dx, like the reference's fp16 add (solution/fast_qwen.py:1320-1323), the first of them of the small LoRA terms."""
+        branches need of [M, inter] matrices; what is left of the factors' gradients is one more launch, before dx is written, which
+        may lie in dy's memory; the LoRA terms of dx are expanded first (two dropout masks) and one product over the
+        stacked weight adds [dg | du] . W to them. Two roundings of dx, like the reference's fp16 add
+        (solution/fast_qwen.py:1320-1323), the first of them of the small LoRA terms."""
         gate, up, down = self.projections
         (x, mg, kg, tg), (_, mu, ku, tu), (h, md, kd, td) = (p._saved for p in self.projections)
         gs = self.grad_stream
@@ -237,15 +243,16 @@ class MlpBlock:
             gs.wait_stream(torch.cuda.current_stream(dy.device))
             with torch.cuda.stream(gs):
                 linear.lora_grads_batch(grads, accumulate_grads)
+        else:
+            linear.lora_grads_batch(grads, accumulate_grads)
         dx = None
         if need_dx:
+            self._wait_before_writing(out, dy)
             dx = out if out is not None else torch.empty(dy.shape[0], self.hidden, dtype=torch.float16, device=dy.device)
             linear.lora_expand([(ug, gate.A16, mg, kg), (uu, up.A16, mu, ku)], dx)
             self._gate_up_dx(gu, dx)
         if gs is not None:
             torch.cuda.current_stream(dy.device).wait_stream(gs)
-        else:
-            linear.lora_grads_batch(grads, accumulate_grads)
         for p in self.projections:
             p._saved = None
         return dx
@@ -267,6 +274,7 @@ class MlpBlock:
             dhf = dh.float()
             du = (dhf * gf * sig).half()
             dg = (dhf * u.float() * sig * (1.0 + gf * (1.0 - sig))).half()
+        self._wait_before_writing(out, dy)
         dx = self.gate.backward(dg, out=out, need_dx=need_dx, accumulate_grads=accumulate_grads, grad_stream=gs, pending=pend)
         # the second launch adds its fp32 result to the fp16 values the first one stored and rounds again
         dx = self.up.backward(du, out=dx, accumulate=need_dx, need_dx=need_dx, accumulate_grads=accumulate_grads,

@@ -4,8 +4,8 @@ expanded for two dropout masks, the factors' gradients of several projections in
 import pytest
 import torch
 
-from decentrik_prime_b200 import linear
-from decentrik_prime_b200.blocks import MlpBlock
+from decentrik_prime_b200 import k_nf4, linear
+from decentrik_prime_b200.blocks import GradBucket, MlpBlock
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -104,3 +104,56 @@ def test_joined_and_separate_backward(M, mode):
     assert ((dx1.float() - dx2.float()).abs() <= 2.0 ** -11 * 4 * scale).all()
     for a, b in zip(gr1, gr2):
         assert ((a - b).norm() / b.norm()) < 1e-3          # u of the joined order from fp32 sums in another order
+
+
+def block_reference(block, x, masks, ks, dy):
+    """fp64 over the fp16 weights and factors: dx and dA, dB of gate, up, down. The forward's g, u and h are the block's own."""
+    flat = torch.empty(block.layer.numel, dtype=torch.float16, device=DEV)
+    k_nf4.dequant_layer(block.layer, block.code2, None, flat)
+    at, W = 0, []
+    for p in block.projections:
+        W.append(flat[at:at + p.w.N * p.w.K].view(p.w.N, p.w.K).double())
+        at += p.w.N * p.w.K
+    (Ag, Bg), (Au, Bu), (Ad, Bd) = ((p.A16.double(), p.B16.double()) for p in block.projections)
+    s = block.gate.scale
+    (g, u), h, x, dy = (t.double() for t in block._saved), block.down._saved[0].double(), x.double(), dy.double()
+    keep = [m.double() * ks for m in masks]
+    ud = s * dy @ Bd
+    dh = dy @ W[2] + keep[2] * (ud @ Ad)
+    sig = torch.sigmoid(g)
+    dg, du = dh * u * sig * (1 + g * (1 - sig)), dh * g * sig
+    ug, uu = s * dg @ Bg, s * du @ Bu
+    dx = dg @ W[0] + keep[0] * (ug @ Ag) + du @ W[1] + keep[1] * (uu @ Au)
+    xg, xu, hd = (keep[i] * t for i, t in enumerate((x, x, h)))
+    grads = [ug.t() @ xg, s * dg.t() @ (xg @ Ag.t()), uu.t() @ xu, s * du.t() @ (xu @ Au.t()), ud.t() @ hd, s * dy.t() @ (hd @ Ad.t())]
+    return dx, grads
+
+
+@pytest.mark.parametrize("M", [24, 187])
+@pytest.mark.parametrize("side_stream", [False, True])
+@pytest.mark.parametrize("with_bucket", [False, True])
+@pytest.mark.parametrize("out", ["new", "given", "dy", "none"])
+def test_block_backward_over_its_options(M, side_stream, with_bucket, out):
+    """dx into a new tensor, a given one, dy itself, or left out; gradients written, then added up by a second backward."""
+    H, I = 256, 512
+    x, dy = rand(M, H, seed=1).half(), rand(M, H, seed=2).half()
+    masks = [(rand(M, k, seed=3 + i) > -1.3).to(torch.uint8) for i, k in enumerate((H, H, I))]
+    bucket = GradBucket(MlpBlock.grad_numel(H, I), torch.device(DEV)) if with_bucket else None
+    block = MlpBlock(H, I, 0, DEV, bucket=bucket)
+    if side_stream:
+        block.use_grad_stream()
+    for p in block.projections:
+        p.dA.fill_(3.0)                               # overwritten by the first backward
+        p.dB.fill_(3.0)
+    for times in (1, 2):
+        block.forward(x, masks, 1.1)
+        if times == 1:
+            dx_ref, grads_ref = block_reference(block, x, masks, 1.1, dy)
+        given = {"given": torch.full_like(dy, 7.0), "dy": dy.clone()}.get(out)
+        dx = block.backward(given if out == "dy" else dy, need_dx=out != "none", accumulate_grads=times == 2, out=given)
+        assert (dx is None) == (out == "none") and (given is None or dx is given)
+        # fp16 activations on the way: a rounding (2^-12 in the 2-norm) each of dy . W_down, dg and du, dx twice
+        if dx is not None:
+            assert (dx.double() - dx_ref).norm() <= 6 * 2.0 ** -12 * dx_ref.norm()
+        for got, ref in zip((t for p in block.projections for t in (p.dA, p.dB)), grads_ref):
+            assert (got.double() - times * ref).norm() <= 6 * 2.0 ** -12 * times * ref.norm()
