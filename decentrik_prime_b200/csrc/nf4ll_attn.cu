@@ -105,9 +105,6 @@ __device__ __forceinline__ void frag_bt(uint32_t base, int k0, int n0, int lane,
   ldsm4t(tile_addr<HD>(base, k0 + (lane & 15), n0 / 8 + (lane >> 4)), b);
 }
 
-// the 128 threads of one half of a CTA
-__device__ __forceinline__ void half_sync(int half) { asm volatile("bar.sync %0, %1;" ::"r"(half + 1), "n"(kAttnThreads) : "memory"); }
-
 __device__ __forceinline__ void find_tile(const SeqTable& t, int tile, int& start, int& len, int& t0) {
   int lo = 0, hi = t.n - 1;
   while (lo < hi) {
@@ -184,7 +181,7 @@ attn_fwd_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Se
   };
   auto sync = [&] {
     if (HALVES == 1) __syncthreads();
-    else half_sync(half);
+    else named_barrier(half + 1, kAttnThreads);       // the 128 threads of this half
   };
   load(half, 0);
   load(half + HALVES, 1);
@@ -392,7 +389,7 @@ attn_dq_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Seq
   };
   auto sync = [&] {
     if (HALVES == 1) __syncthreads();
-    else half_sync(half);
+    else named_barrier(half + 1, kAttnThreads);       // the 128 threads of this half
   };
   load(half, 0);
   load(half + HALVES, 1);

@@ -40,9 +40,6 @@ __device__ __forceinline__ uint32_t down_cluster_rank() {
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
   return r;
 }
-__device__ __forceinline__ void down_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ float down_peer_load(const float* local, uint32_t rank) {
   uint32_t a = static_cast<uint32_t>(__cvta_generic_to_shared(local)), r;
   float v;
@@ -141,7 +138,7 @@ lora_down_kernel(const __half* __restrict__ act, int64_t ldact, const DownBranch
       for (int w = 0; w < NW; ++w) v += part[w][row][j];
       part[0][row][j] = v;                       // read and written by this thread only
     }
-    down_cluster_sync();
+    cluster_sync_all();
     if (down_cluster_rank() == 0) {
       for (int idx = threadIdx.x; idx < ROWS * 16; idx += NW * 32) {
         const int row = idx >> 4, j = idx & 15;
@@ -156,7 +153,7 @@ lora_down_kernel(const __half* __restrict__ act, int64_t ldact, const DownBranch
         }
       }
     }
-    down_cluster_sync();                         // peers keep their shared memory until rank 0 has read it
+    cluster_sync_all();                         // peers keep their shared memory until rank 0 has read it
   } else {
     for (int idx = threadIdx.x; idx < ROWS * 16; idx += NW * 32) {
       const int row = idx >> 4, j = idx & 15;

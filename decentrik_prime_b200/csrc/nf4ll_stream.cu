@@ -216,7 +216,7 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
     s_lv[threadIdx.x - 32] = __half_as_ushort(__float2half_rn(v));
   }
   __syncthreads();
-  if (cl > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  if (cl > 1) cluster_arrive();
 
   // Behind a rank-16 projection of the same call the weights and x may be read at once: that kernel itself went on only
   // after all earlier work on the stream had finished. Behind anything else only the tables are laid out meanwhile.
@@ -392,7 +392,7 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
     // ----------------------------------------------------------------------------- sums of the teams, of the cluster; LoRA, bias, output
     named_barrier(1, kBarThreads);
     if (p.early) pdl_wait();                        // T comes from the kernel this one was launched behind
-    if (cl > 1) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (cl > 1) cluster_wait();
     const int k = lane >> 2, q = lane & 3;          // this lane's token (of a tile of eight) and four of the sixteen rows
     const int xch_words = (cl - 1) * NT * 128;      // of a tile
     // units go round the warps, whose buffers differ; gate|up with two buffers is one warp's
@@ -510,7 +510,7 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
   }
   __syncwarp();
   if (cl > 1) {
-    if (warp < kEpiWarp) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (warp < kEpiWarp) cluster_wait();
     cluster_sync_all();                             // nobody leaves while a peer may still write to its shared memory
   }
 }
