@@ -347,7 +347,7 @@ rms_fwd_split_kernel(const float* __restrict__ x, const __half* __restrict__ del
   if (gridDim.y > 1) cluster_sync_all();           // shared memory stays until the others have read it
 }
 
-// a, b as fp16 pairs of descending weight: 33 bits, all of an fp32 value in fp16's range
+// a, b as fp16 pairs of descending weight: 33 bits of each, of which those below 2^-24 are rounded away
 __device__ __forceinline__ void split3(float a, float b, uint32_t (&p)[3]) {
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
@@ -360,7 +360,8 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t (&p)[3]) {
 
 // The expansion u . A on the tensor cores: a lane's sixteen bytes of a rank's row are four 2-column pieces, which movmatrix turns into the
 // right operand for columns 8 i + 2 w, + 1 (i = 0..3), so that over w = 0..3 lane (g, t) ends with its own columns 8 t .. + 7 of row g. u
-// goes in three fp16 parts under a power of two per row that brings its largest to [1, 2): no less than its 24 bits, whatever their size.
+// goes in three fp16 parts under a power of two per row that brings its largest rank to [2^14, 2^15): all 24 bits of every rank down to
+// 2^-15 of the largest; of smaller ones what is above 2^-40 of the largest.
 // With fp32 FMAs it was 32 loads, 256 conversions and 256 FMAs per lane and chunk, and the larger error against fp64 (9.5e-8 of the
 // result's norm at u of 1 with 1536 columns, 7.2e-8 so). us with two branches / without, one CTA and FMAs before: 1536 columns, 8 rows 13.1 / 6.0 ->
 // 4.6 / 3.0, 951 rows 22.3 / 11.1 -> 15.6 / 10.6, 2048 rows (a CTA per group) 41.4 / 20.9 -> 31.5 / 20.4; 3584 columns, 333 rows 59.8 / 20.5 ->
@@ -404,11 +405,11 @@ rms_bwd_kernel(const __half* __restrict__ dy16, int64_t lddy, float gscale, cons
     float m = fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(hi.x), fabsf(hi.y)));
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
     m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    // the exponent of the row's largest, within what two normal powers of two can undo
+    // the exponent of the row's largest, from where on 2^(14 - e) and its reciprocal are normal; a row below is exact as well
     int e = static_cast<int>(__float_as_uint(m) >> 23) - 127;
-    e = e < -126 ? -126 : e > 126 ? 126 : e;
-    const float f = __uint_as_float(static_cast<uint32_t>(127 - e) << 23);
-    back[b] = __uint_as_float(static_cast<uint32_t>(127 + e) << 23);
+    e = e < -112 ? -112 : e;
+    const float f = __uint_as_float(static_cast<uint32_t>(127 + 14 - e) << 23);
+    back[b] = __uint_as_float(static_cast<uint32_t>(127 - 14 + e) << 23);
     split3(lo.x * f, lo.y * f, ul[b]);
     split3(hi.x * f, hi.y * f, uh[b]);
   }

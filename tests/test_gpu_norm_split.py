@@ -22,8 +22,19 @@ def mask_of(M, D, seed):
 @pytest.mark.parametrize("M,D", [(1, 8), (9, 264), (8, 520), (3, 1000), (15, 1544), (300, 1544), (1100, 1544), (333, 3584), (17, 4096), (600, 4088), (1185, 1016), (2000, 72)])
 @pytest.mark.parametrize("branches", ["", "q", "v", "qv"])
 def test_split_norms(M, D, branches):
+    check_norms(M, D, branches, 0)
+
+
+# ranks of u that fall by a factor of 2 each beside rows of lora_A that rise by it: every rank counts for as much in the result
+@pytest.mark.parametrize("M,D", [(9, 264), (300, 1544), (600, 4088)])
+def test_ranks_of_unlike_size(M, D):
+    check_norms(M, D, "qv", 1)
+
+
+def check_norms(M, D, branches, fall):
     x, delta, w = rand(M, D, seed=1), rand(M, D, seed=2).half(), rand(D, seed=3)
-    A = {b: rand(16, D, seed=4 + i, scale=0.05).half() for i, b in enumerate("qv") if b in branches}
+    rank = 2.0 ** (fall * torch.arange(16, device=DEV, dtype=torch.float32))
+    A = {b: (rand(16, D, seed=4 + i, scale=0.05) * rank[:, None]).half() for i, b in enumerate("qv") if b in branches}
     m = {"q": mask_of(M, D, 6)} if "q" in branches else {}          # v without dropout
     t = {b: torch.empty(M, 16, device=DEV) for b in A}
     y, rstd, xo = torch.empty(M, D + 8, device=DEV).half(), torch.empty(M, device=DEV), torch.empty(M, D, device=DEV)
@@ -46,7 +57,7 @@ def test_split_norms(M, D, branches):
     u = {b: rand(M, 16, seed=8 + i) for i, b in enumerate(A)}
     scales = (1.0, 1e-9, 1e7)
     for i, b in enumerate(u):
-        u[b] *= torch.tensor([scales[(row + i) % 3] for row in range(M)], device=DEV)[:, None]
+        u[b] *= torch.tensor([scales[(row + i) % 3] for row in range(M)], device=DEV)[:, None] / rank
     dy, dres = rand(M, D, seed=10).half(), rand(M, D, seed=11)
     out, o16 = dres.clone(), torch.empty(M, D, device=DEV).half()
     k_norm.rms_backward(dy, 0.5, x, w, rstd, out, dres=out, uq=u.get("q"), uv=u.get("v"), aq=A.get("q"), av=A.get("v"), mq=m.get("q"), keep_scale=ks,
