@@ -555,7 +555,8 @@ static int check_grad(const nf4ll_grad& g, const char* who) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// out[M,K] = fp16(sum over branches of drop(u . A)), A [16,K] fp16, u [M,16] fp32 (two fp16 parts of it: 22 bits), under the keep-mask of
+// out[M,K] = fp16(sum over branches of drop(u . A)), A [16,K] fp16, u [M,16] fp32 (in two fp16 parts under a power of two per row: 22 bits
+// of every rank down to 2^-17 of the row's largest, of smaller ones what is above 2^-39 of it), under the keep-mask of
 // the branch's input: the LoRA terms of d(input) of projections that share an input, whose base terms one product adds to it. Two of
 // them could not share a GEMM's epilogue otherwise (two masks on one tile). A CTA takes 64 columns, whose factors its warps
 // keep in registers, and goes through blocks of sixteen rows. 2 B written and 1 B of mask read per branch and element.
@@ -606,12 +607,17 @@ lora_expand_kernel(const ExpandBranch first, const ExpandBranch second, __half* 
 #pragma unroll
     for (int n = 0; n < N; ++n) {
       const ExpandBranch& br = n ? second : first;
-      uint32_t hi[4], lo[4];                       // (row g, ranks 2t..), (row g + 8, same), (row g, ranks 2t + 8..), (row g + 8, same)
+      uint32_t part[4][2];                         // (row g, ranks 2t..), (row g + 8, same), (row g, ranks 2t + 8..), (row g + 8, same)
+      float back[2];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int64_t r = row[i & 1];
-        const float2 f = r < M ? __ldcg(reinterpret_cast<const float2*>(br.u + r * 16 + 2 * t + 8 * (i >> 1))) : make_float2(0.f, 0.f);
-        split_half2(f.x, f.y, hi[i], lo[i]);
+      for (int i = 0; i < 2; ++i) {
+        const float2 zero = make_float2(0.f, 0.f);
+        const float2* u = reinterpret_cast<const float2*>(br.u + row[i] * 16 + 2 * t);
+        const float2 a = row[i] < M ? __ldcg(u) : zero, b = row[i] < M ? __ldcg(u + 4) : zero;
+        const RowScale f = row_scale(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))));
+        split_parts(a.x * f.to, a.y * f.to, part[i]);
+        split_parts(b.x * f.to, b.y * f.to, part[i + 2]);
+        back[i] = br.mask ? f.back * br.keep_scale : f.back;
       }
       uint2 keep[kGroups][2];
 #pragma unroll
@@ -626,13 +632,13 @@ lora_expand_kernel(const ExpandBranch first, const ExpandBranch second, __half* 
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           float c[4] = {0.f, 0.f, 0.f, 0.f};
-          mma16816(c, hi[0], hi[1], hi[2], hi[3], b0[n][q][j], b1[n][q][j]);
-          mma16816(c, lo[0], lo[1], lo[2], lo[3], b0[n][q][j], b1[n][q][j]);
+#pragma unroll
+          for (int i = 0; i < 2; ++i) mma16816(c, part[0][i], part[1][i], part[2][i], part[3][i], b0[n][q][j], b1[n][q][j]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
             const int e = 2 * j + (i & 1);
             const uint32_t k = (e < 4 ? keep[q][i >> 1].x : keep[q][i >> 1].y) & 0xffu << 8 * (e & 3);
-            const float d = !br.mask ? c[i] : k ? c[i] * br.keep_scale : 0.f;
+            const float d = !br.mask || k ? c[i] * back[i >> 1] : 0.f;
             v[q][i >> 1][e] = n ? v[q][i >> 1][e] + d : d;
           }
         }

@@ -25,11 +25,36 @@ __device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
   asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
   return r;
 }
-// two values as fp16 pairs hi + lo: 22 bits of each
+// two values as fp16 pairs hi + lo: 22 bits of each, of which those below 2^-24 are rounded away; values beyond fp16's range become NaN
 __device__ __forceinline__ void split_half2(float a, float b, uint32_t& hi, uint32_t& lo) {
   hi = pack_half2_rn(a, b);
   const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&hi));
   lo = pack_half2_rn(a - f.x, b - f.y);
+}
+
+// Two values as N fp16 pairs of descending weight: 11 bits each, of which those below 2^-24 are rounded away. An infinity lies in the first.
+template <int N>
+__device__ __forceinline__ void split_parts(float a, float b, uint32_t (&p)[N]) {
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    p[i] = pack_half2_rn(a, b);
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
+    a = fabsf(f.x) <= 65504.f ? a - f.x : 0.f;
+    b = fabsf(f.y) <= 65504.f ? b - f.y : 0.f;
+  }
+}
+// For the sixteen ranks of a row, of which this lane has four and `m` is the largest of them by magnitude (the others' lie in the three
+// lanes beside it): the power of two that brings the row's largest to [2^14, 2^15), so that parts keep the bits of ranks far below it,
+// and its reciprocal. Both are normal: a row below 2^-112 is brought to less, but then all its bits lie above 2^-24.
+struct RowScale {
+  float to, back;
+};
+__device__ __forceinline__ RowScale row_scale(float m) {
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
+  m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
+  int e = static_cast<int>(__float_as_uint(m) >> 23) - 127;
+  e = e < -112 ? -112 : e;
+  return RowScale{__uint_as_float(static_cast<uint32_t>(127 + 14 - e) << 23), __uint_as_float(static_cast<uint32_t>(127 - 14 + e) << 23)};
 }
 
 struct DownBranch {

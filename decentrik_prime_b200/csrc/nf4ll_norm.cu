@@ -347,17 +347,6 @@ rms_fwd_split_kernel(const float* __restrict__ x, const __half* __restrict__ del
   if (gridDim.y > 1) cluster_sync_all();           // shared memory stays until the others have read it
 }
 
-// a, b as fp16 pairs of descending weight: 33 bits of each, of which those below 2^-24 are rounded away
-__device__ __forceinline__ void split3(float a, float b, uint32_t (&p)[3]) {
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    p[i] = pack_half2_rn(a, b);
-    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&p[i]));
-    a = fabsf(f.x) <= 65504.f ? a - f.x : 0.f;     // nothing is left of an infinity
-    b = fabsf(f.y) <= 65504.f ? b - f.y : 0.f;
-  }
-}
-
 // The expansion u . A on the tensor cores: a lane's sixteen bytes of a rank's row are four 2-column pieces, which movmatrix turns into the
 // right operand for columns 8 i + 2 w, + 1 (i = 0..3), so that over w = 0..3 lane (g, t) ends with its own columns 8 t .. + 7 of row g. u
 // goes in three fp16 parts under a power of two per row that brings its largest rank to [2^14, 2^15): all 24 bits of every rank down to
@@ -402,16 +391,10 @@ rms_bwd_kernel(const __half* __restrict__ dy16, int64_t lddy, float gscale, cons
     float2 lo = ok ? __ldg(reinterpret_cast<const float2*>(br.u + row * 16 + 2 * t)) : zero;
     float2 hi = ok ? __ldg(reinterpret_cast<const float2*>(br.u + row * 16 + 2 * t + 8)) : zero;
     lo.x *= br.keep_scale; lo.y *= br.keep_scale; hi.x *= br.keep_scale; hi.y *= br.keep_scale;
-    float m = fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(hi.x), fabsf(hi.y)));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 1));
-    m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 2));
-    // the exponent of the row's largest, from where on 2^(14 - e) and its reciprocal are normal; a row below is exact as well
-    int e = static_cast<int>(__float_as_uint(m) >> 23) - 127;
-    e = e < -112 ? -112 : e;
-    const float f = __uint_as_float(static_cast<uint32_t>(127 + 14 - e) << 23);
-    back[b] = __uint_as_float(static_cast<uint32_t>(127 - 14 + e) << 23);
-    split3(lo.x * f, lo.y * f, ul[b]);
-    split3(hi.x * f, hi.y * f, uh[b]);
+    const RowScale f = row_scale(fmaxf(fmaxf(fabsf(lo.x), fabsf(lo.y)), fmaxf(fabsf(hi.x), fabsf(hi.y))));
+    back[b] = f.back;
+    split_parts(lo.x * f.to, lo.y * f.to, ul[b]);
+    split_parts(hi.x * f.to, hi.y * f.to, uh[b]);
   }
   constexpr int KC = KEEP ? CPW : 1;               // chunks whose x and dres stay in registers
   float gv[CPW][8], xh[KC][8], dr[KC][8], cs = 0.f;

@@ -46,10 +46,14 @@ def test_gated_backward_with_lora(M, I, masked, accumulate):
 @pytest.mark.parametrize("M,K", [(1, 8), (15, 56), (16, 64), (17, 72), (65, 136), (187, 1536), (3001, 200)])
 @pytest.mark.parametrize("masked", [(), (0,), (1,), (0, 1)])
 @pytest.mark.parametrize("n", [1, 2])
-def test_expanded_lora_terms(M, K, masked, n):
+@pytest.mark.parametrize("size", [1.0, 2.0 ** -20, 2.0 ** 20])
+def test_expanded_lora_terms(M, K, masked, n, size):
+    """`size`: of u in every third row, beyond fp16's range and far below it, beside an lora_A that brings the terms back to it."""
     ldm = (K + 15) // 16 * 16
     u = [rand(M, 16, scale=0.3, seed=i) for i in range(n)]
-    A = [rand(16, K, scale=0.2, seed=5 + i).half() for i in range(n)]
+    for t in u:
+        t[::3] *= size
+    A = [(rand(16, K, scale=0.2, seed=5 + i) * size ** -0.5).half() for i in range(n)]
     masks = [(rand(M, ldm, seed=9 + i) > -1.0).to(torch.uint8)[:, :K] if i in masked else None for i in range(n)]
     out = torch.full((M, K + 8), 7.0, dtype=torch.float16, device=DEV)
     linear.lora_expand([(u[i], A[i], masks[i], 1.25) for i in range(n)], out[:, :K])
@@ -58,9 +62,20 @@ def test_expanded_lora_terms(M, K, masked, n):
         keep = 1.0 if masks[i] is None else masks[i].double() * 1.25
         ref = ref + keep * (u[i].double() @ A[i].double())
         bound = bound + 1.25 * (u[i].double().abs() @ A[i].double().abs())
-    # u in two fp16 parts (22 bits) and fp32 sums, then one rounding to fp16
+    # u in two fp16 parts (22 bits of every rank that counts) and fp32 sums, then one rounding to fp16
     assert ((out[:, :K].double() - ref).abs() <= 2.0 ** -11 * ref.abs() + 2.0 ** -20 * bound + 2.0 ** -24).all()
     assert (out[:, K:] == 7.0).all()
+
+
+def test_an_infinite_factor_reaches_its_row_only():
+    M, K = 20, 96
+    A, u = rand(16, K, seed=4).half(), rand(M, 16, seed=5)
+    u[3, 7], u[13, 0] = float("inf"), float("nan")
+    out = linear.lora_expand([(u, A, None, 1.0)], torch.empty(M, K, dtype=torch.float16, device=DEV))
+    rest = torch.ones(M, dtype=torch.bool, device=DEV)
+    rest[3] = rest[13] = False
+    assert out[rest].isfinite().all() and out[13].isnan().all()
+    assert torch.equal(out[3], torch.where(A[7] > 0, float("inf"), float("-inf")).half())
 
 
 @pytest.mark.parametrize("M", [1, 64, 187, 2048])
