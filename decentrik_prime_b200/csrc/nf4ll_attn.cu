@@ -185,7 +185,8 @@ attn_fwd_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ Se
   };
   load(half, 0);
   load(half + HALVES, 1);
-  float o[NT][4], m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  // below any finite score, and finite itself: a block whose scores are all -inf (keys that overflowed) adds nothing, wherever a chain starts
+  float o[NT][4], m[2] = {-1e30f, -1e30f}, l[2] = {0.f, 0.f};
 #pragma unroll
   for (int n = 0; n < NT; ++n)
 #pragma unroll

@@ -28,3 +28,21 @@ def test_halves_against_fp64(nh, nkv, hd, lens):
         assert rel(dqkv[:, part], dref[:, part]) <= REL
     a2, _ = att.forward(qkv, lens)
     assert torch.equal(a, a2) and torch.equal(dqkv, stack.PackedAttention.backward(state, da))
+
+
+@pytest.mark.parametrize("blocks", [(0,), (1,), (0, 1), (1, 2)])
+@pytest.mark.parametrize("n", [100, 256, 300])
+def test_keys_that_overflowed_add_nothing(n, blocks):
+    """Keys of whole blocks infinite in one coordinate, of which every query's is negative: scores of -inf, wherever a half starts."""
+    nh = nkv = 1
+    hd, theta = 64, 1.0e4
+    qkv = torch.randn(n, 3 * hd, generator=torch.Generator().manual_seed(n)).half()
+    first, second = hd // 2 - 1, hd - 1            # the pair that turns slowest: a fraction of a degree per position
+    qkv[:, [first, second]] = -1.0
+    for b in blocks:
+        # from position 1 on, where the rotated second coordinate is infinite too
+        qkv[max(1, 64 * b):64 * (b + 1), hd + first] = float("inf")
+    qkv = qkv.cuda()
+    a, _ = stack.PackedAttention(nh, nkv, hd, theta=theta).forward(qkv, [n])
+    ref, _ = reference(qkv, [n], nh, nkv, hd, theta, torch.zeros(n, hd).half().cuda())
+    assert ref.isfinite().all() and rel(a, ref) <= REL
