@@ -708,6 +708,7 @@ extern "C" int nf4ll_lora_grads_batch(const nf4ll_grad* grads, int32_t n, int64_
   bool any = false;
   for (int i = 0; i < n; ++i) {
     if (int rc = check_grad(grads[i], who)) return rc;
+    if (grads[i].dA && grads[i].mask && grads[i].ld_mask < grads[i].K) { set_detail("%s: ld_mask must be >= K", who); return NF4LL_ERR_ALIGN; }
     any |= grads[i].dA || grads[i].dB;
   }
   if (!any) return NF4LL_OK;
@@ -727,7 +728,10 @@ extern "C" int nf4ll_lora_expand(const nf4ll_expand* branches, int32_t n, int64_
   for (int i = 0; i < n; ++i) {
     const nf4ll_expand& b = branches[i];
     if (!b.u || !b.A) { set_detail("%s: a branch needs u and A", who); return NF4LL_ERR_NULL; }
-    if (off(b.u) || off(b.A) || (b.mask && (off(b.mask) || b.ld_mask % 16))) { set_detail("%s: u, A and mask 16-byte aligned, ld_mask a multiple of 16", who); return NF4LL_ERR_ALIGN; }
+    if (off(b.u) || off(b.A) || (b.mask && (off(b.mask) || b.ld_mask % 16 || b.ld_mask < K))) {
+      set_detail("%s: u, A and mask 16-byte aligned, ld_mask a multiple of 16 and >= K", who);
+      return NF4LL_ERR_ALIGN;
+    }
     br[i] = ExpandBranch{static_cast<const float*>(b.u), static_cast<const __half*>(b.A), b.mask, b.ld_mask, b.keep_scale};
   }
   if (off(out) || ldo % 8 || ldo < K) { set_detail("%s: out 16-byte aligned, its leading dimension a multiple of 8 and >= K", who); return NF4LL_ERR_ALIGN; }

@@ -401,7 +401,10 @@ extern "C" int nf4ll_gated_backward(const nf4ll_gated* q, int64_t M, int64_t I, 
       if (!s) { set_detail("%s: null pointer", who); return NF4LL_ERR_NULL; }
       if (reinterpret_cast<uintptr_t>(s) & 15) { set_detail("%s: t, u, Bt and scratch must be 16-byte aligned", who); return NF4LL_ERR_ALIGN; }
     }
-    if (q->mask && ((reinterpret_cast<uintptr_t>(q->mask) & 15) || q->ld_mask % 16)) { set_detail("%s: mask 16-byte aligned, ld_mask a multiple of 16", who); return NF4LL_ERR_ALIGN; }
+    if (q->mask && ((reinterpret_cast<uintptr_t>(q->mask) & 15) || q->ld_mask % 16 || q->ld_mask < I)) {
+      set_detail("%s: mask 16-byte aligned, ld_mask a multiple of 16 and >= I", who);
+      return NF4LL_ERR_ALIGN;
+    }
     if (scratch_bytes < nf4ll_gated_backward_bytes(M, I)) { set_detail("%s: scratch of %lld bytes", who, (long long)scratch_bytes); return NF4LL_ERR_WORKSPACE; }
   }
   if (int rc = require_sm100()) return rc;

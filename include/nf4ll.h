@@ -215,7 +215,7 @@ int nf4ll_lora_grads(const void* dy, int64_t lddy, const void* x, int64_t ldx, c
                      float scale, int32_t r, int64_t M, int64_t N, int64_t K,
                      void* dA, void* dB, int32_t accumulate, void* stream);
 
-/* The same for up to three projections over M rows each (gate, up and down of an MLP block) in one launch. */
+/* The same for up to three projections over M rows each (gate, up and down of an MLP block) in one launch; ld_mask >= K too. */
 typedef struct nf4ll_grad {
   const void* dy;           /* __half [M, lddy], N columns */
   int64_t lddy;
@@ -237,7 +237,7 @@ int nf4ll_lora_grads_batch(const nf4ll_grad* grads, int32_t n, int64_t M, int32_
  *   out[M,K] = fp16( sum_i keep_scale_i * mask_i (.) (u_i . A_i) ),   u_i fp32 [M,16] = scale_i * d(out_i) . B_i
  * (`lqx`, `lvx` of solution/fast_qwen.py:1376-1377 and the masked add of solution/k_norm.py:64-71). One accumulating
  * nf4ll_backward_dx over the stacked weight, without a LoRA branch, then completes dx: the two masks of gate and up (or q and v)
- * would not fit one GEMM's epilogue. K a multiple of 8; pointers 16-byte aligned, ldo a multiple of 8, ld_mask of 16. */
+ * would not fit one GEMM's epilogue. K a multiple of 8; pointers 16-byte aligned, ldo a multiple of 8, ld_mask of 16 and >= K. */
 typedef struct nf4ll_expand {
   const void* u;            /* fp32 [M,16] */
   const void* A;            /* __half [16,K] */
@@ -292,7 +292,8 @@ int nf4ll_swiglu_backward(const void* g, int64_t ldg, const void* u, int64_t ldu
  *   dA_down[16,I] (+)= u_down^T . drop(h),  h = fp16(silu(g) * u)                              (solution/fast_qwen.py:1369, 1371)
  * all fp32. t_gate, t_up, u_down: fp32 [M,16] of nf4ll_forward_gate_up and nf4ll_backward_dx; Bt_*: lora_B transposed, __half [16,I];
  * mask: of h. scratch: nf4ll_gated_backward_bytes(M, I) device bytes, 16-byte aligned (parts of u_gate and u_up, added up in a fixed order).
- * dg / du may alias g / u. I a multiple of 8; matrices, t, u and Bt 16-byte aligned, their leading dimensions multiples of 8, ld_mask of 16. */
+ * dg / du may alias g / u. I a multiple of 8; matrices, t, u and Bt 16-byte aligned, their leading dimensions multiples of 8,
+ * ld_mask of 16 and >= I. The mask is read 16 bytes at a time: where I % 16 is 8, eight bytes behind a row's I, which ld_mask covers. */
 typedef struct nf4ll_gated {
   const void* g;
   int64_t ldg;

@@ -94,3 +94,17 @@ def test_workspace_bytes_plan(handle):
     # few tiles: split-K partial sums
     assert handle.nf4ll_workspace_bytes(2048, 1536, 1536, 16) > 2048 * 1536 * 4
     assert handle.nf4ll_workspace_bytes(0, 1536, 1536, 16) == 0
+
+
+def test_masks_shorter_than_a_row_are_refused(handle):
+    """The pointers are never followed: every one is a well-aligned number."""
+    at, M = 1 << 20, 4
+    err = lambda: handle.nf4ll_last_error_detail().decode()  # noqa: E731
+    for ld in (0, 32, 80):
+        mask = (at, ld, 1.0)
+        grad = _lib.Grad(at, 64, at, 96, *mask, at, at, 1.0, 64, 96, at, at)
+        assert handle.nf4ll_lora_grads_batch(ctypes.byref(grad), 1, M, 0, None) == -12 and "ld_mask" in err()
+        branch = _lib.Expand(at, at, *mask)
+        assert handle.nf4ll_lora_expand(ctypes.byref(branch), 1, M, 96, at, 96, None) == -12 and "ld_mask" in err()
+        gated = _lib.Gated(*(at, 96) * 5, *mask, *(at,) * 5, 1.0, 1.0, *(at,) * 5)
+        assert handle.nf4ll_gated_backward(ctypes.byref(gated), M, 96, 0, at, 1 << 20, None) == -12 and "ld_mask" in err()
