@@ -375,7 +375,7 @@ extern "C" int nf4ll_swiglu_backward(const void* g, int64_t ldg, const void* u, 
   return NF4LL_OK;
 }
 
-// rows per pair of launches: bounds the parts of the products (128 B per row and CTA column, half of what a row of dg takes there)
+// rows per pair of launches at most: bounds the parts of the products (128 B per row and CTA column, half of what a row of dg takes there)
 constexpr int64_t kGatedSlab = 4096;
 
 extern "C" int64_t nf4ll_gated_backward_bytes(int64_t M, int64_t I) {
@@ -405,7 +405,7 @@ extern "C" int nf4ll_gated_backward(const nf4ll_gated* q, int64_t M, int64_t I, 
       set_detail("%s: mask 16-byte aligned, ld_mask a multiple of 16 and >= I", who);
       return NF4LL_ERR_ALIGN;
     }
-    if (scratch_bytes < nf4ll_gated_backward_bytes(M, I)) { set_detail("%s: scratch of %lld bytes", who, (long long)scratch_bytes); return NF4LL_ERR_WORKSPACE; }
+    if (scratch_bytes < nf4ll_gated_backward_bytes(M < kGatedRows ? M : kGatedRows, I)) { set_detail("%s: scratch of %lld bytes", who, (long long)scratch_bytes); return NF4LL_ERR_WORKSPACE; }
   }
   if (int rc = require_sm100()) return rc;
   if (!accumulate)
@@ -416,8 +416,10 @@ extern "C" int nf4ll_gated_backward(const nf4ll_gated* q, int64_t M, int64_t I, 
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   NF4LL_CUDA(cudaFuncSetAttribute(gated_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGatedSmem));
   const int64_t cols = (I + kGatedCols - 1) / kGatedCols;
-  for (int64_t m0 = 0; m0 < M; m0 += kGatedSlab) {
-    const int64_t rows = M - m0 < kGatedSlab ? M - m0 : kGatedSlab;
+  // as many rows at a time as the scratch has room for, in whole stages
+  const int64_t room = scratch_bytes / (cols * 32 * 4), slab = room >= (M < kGatedSlab ? M : kGatedSlab) ? kGatedSlab : room / kGatedRows * kGatedRows;
+  for (int64_t m0 = 0; m0 < M; m0 += slab) {
+    const int64_t rows = M - m0 < slab ? M - m0 : slab;
     // as many row ranges as one wave of four CTAs per SM holds
     const int64_t steps = (rows + kGatedRows - 1) / kGatedRows;
     int64_t ranges = 4 * static_cast<int64_t>(sms) / cols;

@@ -650,13 +650,21 @@ PyObject* py_gated_backward(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
       if (b->scalar_type() != at::kHalf || b->dim() != 2 || b->size(0) != kRank || b->size(1) != I || !b->is_contiguous() || !b->is_cuda())
         value_error("lora_B transposed shadow must be contiguous CUDA fp16 [16, %lld]", static_cast<long long>(I));
     at::Tensor ug = empty({M, kRank}, at::kFloat, g), uu = empty({M, kRank}, at::kFloat, g);
-    const int64_t bytes = nf4ll_gated_backward_bytes(M, I);
-    at::Tensor scratch = empty({std::max<int64_t>(bytes, 1)}, at::kByte, g);
+    // where the allocator does not have what all rows at once take, fewer rows at a time
+    at::Tensor scratch;
+    for (const int64_t rows : {M, std::min<int64_t>(M, 256), std::min<int64_t>(M, 16)}) {
+      try {
+        scratch = empty({std::max<int64_t>(nf4ll_gated_backward_bytes(rows, I), 1)}, at::kByte, g);
+        break;
+      } catch (const c10::OutOfMemoryError&) {
+        if (rows <= 16) throw;
+      }
+    }
     const nf4ll_gated p{g.data_ptr(), ld(g), u.data_ptr(), ld(u), dh.data_ptr(), ld(dh), dg.data_ptr(), ld(dg), du.data_ptr(), ld(du), m.c.mask, m.c.ld_mask,
                         static_cast<float>(number(a[6])), tg.data_ptr(), tu.data_ptr(), ud.data_ptr(), bg.data_ptr(), bu.data_ptr(),
                         static_cast<float>(number(a[12])), static_cast<float>(number(a[13])), ug.data_ptr(), uu.data_ptr(), dbg.data_ptr(), dbu.data_ptr(),
                         dad.data_ptr()};
-    check(nf4ll_gated_backward(&p, M, I, PyObject_IsTrue(a[17]), scratch.data_ptr(), bytes, Call(g).stream));
+    check(nf4ll_gated_backward(&p, M, I, PyObject_IsTrue(a[17]), scratch.data_ptr(), scratch.numel(), Call(g).stream));
     return pair(wrap(&ug), wrap(&uu));
   });
 }

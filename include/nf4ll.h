@@ -291,7 +291,8 @@ int nf4ll_swiglu_backward(const void* g, int64_t ldg, const void* u, int64_t ldu
  *   dB_gate[I,16] (+)= scale_gate * dg^T . t_gate    dB_up[I,16] (+)= scale_up * du^T . t_up
  *   dA_down[16,I] (+)= u_down^T . drop(h),  h = fp16(silu(g) * u)                              (solution/fast_qwen.py:1369, 1371)
  * all fp32. t_gate, t_up, u_down: fp32 [M,16] of nf4ll_forward_gate_up and nf4ll_backward_dx; Bt_*: lora_B transposed, __half [16,I];
- * mask: of h. scratch: nf4ll_gated_backward_bytes(M, I) device bytes, 16-byte aligned (parts of u_gate and u_up, added up in a fixed order).
+ * mask: of h. scratch: nf4ll_gated_backward_bytes(M, I) device bytes, 16-byte aligned (parts of u_gate and u_up, added up in a fixed order);
+ * with less, down to nf4ll_gated_backward_bytes(16, I), the rows are taken in turns of as many as it has room for.
  * dg / du may alias g / u. I a multiple of 8; matrices, t, u and Bt 16-byte aligned, their leading dimensions multiples of 8,
  * ld_mask of 16 and >= I. The mask is read 16 bytes at a time: where I % 16 is 8, eight bytes behind a row's I, which ld_mask covers. */
 typedef struct nf4ll_gated {

@@ -47,6 +47,42 @@ def test_the_smaller_route_when_memory_is_short():
         assert err <= 2e-2 and rel <= 1e-3, (name, err, rel)
 
 
+@pytest.mark.parametrize("room_for", [1000, 40])
+def test_the_gated_backward_takes_fewer_rows_at_a_time(room_for):
+    """The parts of its rank-16 products: of 8960 columns 9 KB a row. Every row's parts are added up in the same order."""
+    M, I = 2200, 8960
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *s: torch.randn(*s, device="cuda", generator=gen)  # noqa: E731
+    g, u, dh = (rand(M, I).half() for _ in range(3))
+    t, B, mask = [rand(M, 16) for _ in range(3)], [(rand(16, I) * 0.05).half() for _ in range(2)], (rand(M, I) > -1.0).to(torch.uint8)
+
+    def run(g, u, grads):
+        return linear.gated_backward(g, u, dh, mask, 1.25, *t, (B[0], 2.0), (B[1], 0.5), *grads)
+
+    inputs = [(g.clone(), u.clone(), [torch.empty(s, device="cuda") for s in ((I, 16), (I, 16), (16, I))]) for _ in range(2)]
+    want = run(*inputs[0])
+    h = _lib.lib()
+    full, part = h.nf4ll_gated_backward_bytes(M, I), h.nf4ll_gated_backward_bytes(room_for, I)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    room = torch.cuda.memory_reserved() + (4 << 20) + (part >> 21 << 21)      # the results, and large blocks in steps of 2 MB
+    try:
+        torch.cuda.set_per_process_memory_fraction(room / torch.cuda.get_device_properties(0).total_memory)
+        holes = []                                  # of segments that something else keeps
+        with pytest.raises(torch.OutOfMemoryError):
+            while True:
+                holes.append(torch.empty(full, dtype=torch.uint8, device="cuda"))
+        got = run(*inputs[1])
+        torch.cuda.synchronize()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for a, b in zip(want + inputs[0][:2], got + inputs[1][:2]):
+        assert torch.equal(a, b)
+    # fp32 sums of M terms in another order, each term an fp16 product with the side's 22 bits
+    for a, b in zip(inputs[0][2], inputs[1][2]):
+        assert (a - b).norm() <= M / 16 * 2.0 ** -22 * a.norm()
+
+
 def test_a_first_call_that_needs_no_scratch():
     """A contraction too short to be split, without LoRA: the first call on a stream, issued and captured."""
     pr = make_problem(256, 64, 130, seed=4, lora=False)
