@@ -1456,6 +1456,7 @@ static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lor
   if (g_mid.on > 0) return mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, g_mid.rb, g_mid.nt, g_mid.cl, mp);
   if (c.M > kMidMostRows) return false;
   if (c.mode == kFwd && c.M <= kStreamMaxRows) {
+    if (!stream_takes(c.M, N, K, c.gu_inter != 0)) return mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp);
     if (c.M < kMidLeastRows || (c.n_seg > 1 && !c.gu_inter) || (c.gu_inter ? N / 2 : N) * K < kMidSmallWeights) return false;
     if (!mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
     // The streaming kernel where both models put it 5 % ahead. At 16 rows, that one / this one, us: 27648 x 5120 33.9 / 35.4, 18944 x 3584
@@ -1604,7 +1605,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
   if (segments && (narrow_tiles || tune.bn == 512)) tune.bn = narrow_tiles ? 128 : 256;
   Plan pl = make_plan(mode, M, NO, KC, lora ? lora->r : 0, sms, tune);
   int kind = forward_kind(mode, M, segments != nullptr, g_tune);
-  if (kind == kStream && ((reinterpret_cast<uintptr_t>(W->qabs) & 3) || !stream_takes(W->N, W->K, false))) kind = kTiles;
+  if (kind == kStream && ((reinterpret_cast<uintptr_t>(W->qabs) & 3) || !stream_takes(M, W->N, W->K, false))) kind = kTiles;
   const int force_slices = (tune.flags & 2) ? tune.splits : 0;
   const int64_t need = kind == kTiles ? pl.total() : pl.left_bytes + pl.bt_bytes;
   if (need > 0) {
@@ -1796,7 +1797,7 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     // What the kernel for middling batches leaves of short batches and odd widths: up to 16 rows, both halves in one pass; otherwise
     // the two projections on their own, then the stand-alone gated product.
     int kind = g_tune.any() || g_tune.flags || I % 64 ? kTiles : forward_kind(kFwd, M, false, g_tune);
-    if (kind == kStream && ((reinterpret_cast<uintptr_t>(W->qabs) & 3) || !stream_takes(W->N, W->K, true))) kind = kTiles;
+    if (kind == kStream && ((reinterpret_cast<uintptr_t>(W->qabs) & 3) || !stream_takes(M, W->N, W->K, true))) kind = kTiles;
     if (kind != kTiles) {
       // both halves in one pass over the weights
       StreamCall c{};

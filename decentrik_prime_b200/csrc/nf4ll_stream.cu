@@ -55,6 +55,7 @@ constexpr int kStreamRows = 16;              // weight rows of a tile
 constexpr int kStreamProducers = 2;          // warps that copy: their lanes' bulk copies are issued one after another, some 80 clocks each
 constexpr int kStreamEpilogues = 2;          // warps that finish tiles
 constexpr int kStreamMaxStages = 8;
+constexpr int kStreamMaxCluster = 16;
 constexpr int kStreamMaxSlots = 64;          // units of a cluster that one of its CTAs finishes
 constexpr int kStreamMaxGroups = 64;         // second-level groups that a tile's blocks may touch
 constexpr int kEntryStride = 256;
@@ -394,7 +395,7 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
     if (p.early) pdl_wait();                        // T comes from the kernel this one was launched behind
     if (cl > 1) cluster_wait();
     const int k = lane >> 2, q = lane & 3;          // this lane's token (of a tile of eight) and four of the sixteen rows
-    const int xch_words = (cl - 1) * NT * 128;      // of a tile
+    const int src_words = p.M * kStreamRows, xch_words = (cl - 1) * src_words;      // a CTA's sums of a tile; all of a tile
     // units go round the warps, whose buffers differ; gate|up with two buffers is one warp's
     const int finishing = kBufs / halves < kStreamEpilogues ? 1 : kStreamEpilogues;
     for (int i = warp - kEpiWarp; ok && i < my_units && warp - kEpiWarp < finishing; i += finishing) {
@@ -442,7 +443,7 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
         if (lane == 0) mbar_arrive(smem_u32(part_empty + buf));
         if (!mine) {
           const int src = crank < owner ? crank : crank - 1;
-          const uint32_t base = map_to_cta(smem_u32(st_smem + p.off_xch) + ((slot * halves + hf) * xch_words + src * NT * 128) * 4, owner);
+          const uint32_t base = map_to_cta(smem_u32(st_smem + p.off_xch) + ((slot * halves + hf) * xch_words + src * src_words) * 4, owner);
 #pragma unroll
           for (int n = 0; n < NT; ++n)
             if (8 * n + k < p.M)
@@ -461,7 +462,7 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
               const float* from = reinterpret_cast<const float*>(st_smem + p.off_xch) + (slot * halves + hf) * xch_words + n * 128 + k * 16 + 4 * q;
               float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
               for (int r = 0; r < cl; ++r) {
-                const float4 b = r == crank ? v[n] : *reinterpret_cast<const float4*>(from + (r < crank ? r : r - 1) * NT * 128);
+                const float4 b = r == crank ? v[n] : *reinterpret_cast<const float4*>(from + (r < crank ? r : r - 1) * src_words);
                 a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
               }
               v[n] = a;
@@ -542,7 +543,7 @@ static const void* stream_kernel(int s) {
 // How many clusters of `cl` CTAs the current device holds at once, a CTA taking an SM to itself
 static int stream_clusters(int cl) {
   constexpr int kDevices = 64;
-  static int known[kDevices][9];               // 0: not asked yet; written with the same value by any thread
+  static int known[kDevices][kStreamMaxCluster + 1];      // 0: not asked yet; written with the same value by any thread
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 0;
   int n = __atomic_load_n(&known[dev][cl], __ATOMIC_RELAXED);
@@ -552,6 +553,7 @@ static int stream_clusters(int cl) {
   } else {
     const void* kernel = stream_kernel<1>(1);
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem) != cudaSuccess) return 0;
+    if (cl > 8 && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) return 0;
     PdlLaunch probe(dim3(cl), dim3(kStreamThreads), kStreamSmem, nullptr, cl, 1, false, false);
     probe.cfg.numAttrs = 1;                    // the cluster dimension only
     if (cudaOccupancyMaxActiveClusters(&n, kernel, &probe.cfg) != cudaSuccess) n = 0;
@@ -572,14 +574,20 @@ static double stream_us(int nt, int cl, int64_t tiles, int teams, int np, int s,
   return (3.5 + 0.303 * r + 0.0476 * turns * s + 0.0166 * r * static_cast<double>(blocks)) * (s == 5 ? 1.15 : 1.0);
 }
 
-// `force`: low byte warps of a team, next byte CTAs of a cluster, next byte teams (0: free)
-static bool stream_plan(int64_t N, int64_t K, int nt, bool pair, int force, StreamPlan* best) {
+// M: tokens, sixteen at most. `force`: low byte warps of a team, next byte CTAs of a cluster, next byte teams (0: free)
+static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int force, StreamPlan* best) {
+  const int nt = M > 8 ? 2 : 1;
   const int64_t bpr = K / 64, units = N / kStreamRows / (pair ? 2 : 1);
   const int warps = kStreamWarps, f_np = force & 255, f_cl = force >> 8 & 255, f_teams = force >> 16, halves = pair ? 2 : 1;
   bool found = false;
   if (units > (1 << 24)) return false;
-  for (int cl = 1; cl <= 8 && cl <= bpr; ++cl) {
+  for (int cl = 1; cl <= (nt == 1 ? kStreamMaxCluster : 8) && cl <= bpr; ++cl) {
     if (f_cl && cl != f_cl) continue;
+    // Beyond eight only for rows that eight CTAs cannot hold: such clusters leave SMs of a GPC idle. The kernel for middling batches takes
+    // what is left: rows longer still, and weights so tall that a cluster's sums leave room for one stage. us at 1 and 8 rows, here / there
+    // (and before, when all of it went to the tile kernels): 4096 x 45056 31.4, 32.0 / 48.6, 48.9 (76); 8192 x 49152 75.0, 75.7 / 94 (162);
+    // 16384 x 53248 145, 191 (with one stage 268) / 193 (330).
+    if (cl > 8 && found && best->cl <= 8) break;
     if (found && best->cl == 1) break;            // a cluster costs 2 us and more: only where one CTA cannot hold the tokens
     const int64_t blocks = (bpr + cl - 1) / cl;
     const int least = static_cast<int>((blocks + stream_blocks(nt) - 1) / stream_blocks(nt));
@@ -596,11 +604,12 @@ static bool stream_plan(int64_t N, int64_t K, int nt, bool pair, int force, Stre
     const int64_t slots = (rounds + cl - 1) / cl * halves;
     if (p.groups > kStreamMaxGroups || (cl > 1 && slots > kStreamMaxSlots)) continue;
     p.off_xch = (kStreamFixed + 127) / 128 * 128;
-    p.off_ring = static_cast<int>(p.off_xch + (cl > 1 ? slots * (cl - 1) * nt * 512 : 0));
+    p.off_ring = static_cast<int>(p.off_xch + (cl > 1 ? (slots * (cl - 1) * M * kStreamRows * 4 + 127) / 128 * 128 : 0));
     p.off_q = kStreamRows / 2 * p.pitch + kStreamScales;
     p.stage = static_cast<int>((p.off_q + kStreamRows * bpr + 16 + 127) / 128 * 128);
     const int64_t room = kStreamSmem - p.off_ring - kStreamSlack;
     const int fit = static_cast<int>(room / p.stage < kStreamMaxStages ? room / p.stage : kStreamMaxStages);
+    if (cl > 8 && fit < 2) continue;
     for (int np = least; np <= warps && np <= blocks; ++np) {
       if (f_np && np != (f_np < least ? least : f_np < warps && f_np < blocks ? f_np : warps < blocks ? warps : static_cast<int>(blocks))) continue;
       p.s = static_cast<int>((blocks + np - 1) / np);
@@ -620,15 +629,15 @@ static bool stream_plan(int64_t N, int64_t K, int nt, bool pair, int force, Stre
   return found;
 }
 
-bool stream_takes(int64_t N, int64_t K, bool gate_up) {
+bool stream_takes(int64_t M, int64_t N, int64_t K, bool gate_up) {
   if (K <= 64 * kStreamWarps * stream_blocks(1) && N <= (int64_t(1) << 28)) return true;      // one CTA holds a tile's rows
   StreamPlan p{};
-  return stream_plan(N, K, 1, gate_up, 0, &p);
+  return stream_plan(M < 8 ? M : 8, N, K, gate_up, 0, &p);
 }
 
 double stream_time_us(int64_t N, int64_t K) {
   StreamPlan p{};
-  return stream_plan(N, K, 2, false, 0, &p) ? p.us : 1e30;
+  return stream_plan(16, N, K, false, 0, &p) ? p.us : 1e30;
 }
 
 // The former kernel's time with the gated product's launch behind it, whose line against the kernel for middling batches still stands for
@@ -653,16 +662,16 @@ int stream_forward_launch(const StreamCall& c, bool early, int force, int32_t* s
     int nt = left > 8 ? 2 : 1;
     bool fused = c.h != nullptr;
     StreamPlan pl{};
-    bool found = stream_plan(W->N, W->K, nt, fused, force, &pl);
+    bool found = stream_plan(left < 16 ? left : 16, W->N, W->K, fused, force, &pl);
     if (fused && nt == 2 && (!found || pl.cl > 1)) {
       // one warp finishes both halves of a unit, which is too slow for a cluster's (55296 x 5120 at 16 rows 107 us)
       fused = false;
-      found = stream_plan(W->N, W->K, nt, false, force, &pl);
+      found = stream_plan(left < 16 ? left : 16, W->N, W->K, false, force, &pl);
     }
     if (!found) {
       nt = 1;
       fused = c.h != nullptr;
-      if (!stream_plan(W->N, W->K, 1, fused, force, &pl)) {
+      if (!stream_plan(left < 8 ? left : 8, W->N, W->K, fused, force, &pl)) {
         set_detail("weight-streaming kernel: W[%lld,%lld] is too large", static_cast<long long>(W->N), static_cast<long long>(W->K));
         return NF4LL_ERR_SHAPE;
       }
@@ -696,6 +705,7 @@ int stream_forward_launch(const StreamCall& c, bool early, int force, int32_t* s
     p.wait_ns = c.withhold ? static_cast<uint64_t>(c.wait_us) * 1000 : kWaitLimitNs;
     const void* kernel = nt == 1 ? stream_kernel<1>(pl.s) : stream_kernel<2>(pl.s);
     NF4LL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem));
+    if (pl.cl > 8) NF4LL_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     PdlLaunch lc(dim3(static_cast<unsigned>(pl.clusters * pl.cl)), dim3(kStreamThreads), pl.smem, stream, pl.cl > 1 ? pl.cl : 0, pl.cl > 1 ? 1 : 0);
     void* args[] = {&p};
     NF4LL_CUDA(cudaLaunchKernelExC(&lc.cfg, kernel, args));

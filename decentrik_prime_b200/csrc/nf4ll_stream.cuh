@@ -30,8 +30,9 @@ struct StreamCall {
 double stream_time_us(int64_t N, int64_t K);
 // Gate|up of 9 to 16 rows goes to the kernel for middling batches where its model is below this
 double stream_gate_up_line_us(int64_t N, int64_t K, int64_t M, int sms);
-// Whether the kernel takes weights of this size (rows as long as eight CTAs hold the tokens of them in registers: 43008 weights)
-bool stream_takes(int64_t N, int64_t K, bool gate_up);
+// Whether the kernel takes M tokens, eight at a time, against weights of this size: rows as long as eight CTAs hold the tokens of them in
+// registers, 43008 weights, and where a cluster of up to sixteen finds room, twice that
+bool stream_takes(int64_t M, int64_t N, int64_t K, bool gate_up);
 // `early`: the kernel launched right before on the stream is a rank-16 projection of the same call
 int stream_forward_launch(const StreamCall& c, bool early, int force, int32_t* status, cudaStream_t stream);
 

@@ -44,6 +44,29 @@ def test_forced_cuts(np, cl, teams, M):
     assert_close("y", y, reference(pr))
 
 
+# rows that eight CTAs hold and one block more, that sixteen do, and longer ones: all without scratch
+@pytest.mark.parametrize("N,K", [(128, 43008), (256, 43072), (384, 65536), (1024, 45056), (256, 86016), (256, 90112)])
+@pytest.mark.parametrize("M", [1, 5, 8, 11])
+def test_long_rows(N, K, M):
+    pr = make_problem(N, K, M, seed=N + M, lora=False, bias=True, device="cuda")
+    d = to_device(pr)
+    y = linear.forward(d.w, d.x, bias=d.bias, workspace=torch.empty(256, dtype=torch.uint8, device="cuda"))[0]
+    linear.check_status()
+    assert_close("y", y, reference(pr))
+
+
+def test_long_rows_of_gate_and_up():
+    inter, K, M = 256, 43072, 3
+    pr = make_problem(2 * inter, K, M, seed=5, lora=False, device="cuda")
+    d = to_device(pr)
+    g, u, h, _, _ = linear.forward_gate_up(d.w, d.x, workspace=torch.empty(256, dtype=torch.uint8, device="cuda"))
+    linear.check_status()
+    y = reference(pr)
+    assert_close("g", g, y[:, :inter])
+    assert_close("u", u, y[:, inter:])
+    assert torch.equal(h, linear.swiglu_forward(g, u))
+
+
 @pytest.mark.parametrize("K", [512, 5440])
 def test_absmax_codes_off_a_boundary(K):
     d = to_device(make_problem(256, K, 6, seed=K, lora=True, dropout=0.05, bias=True))
