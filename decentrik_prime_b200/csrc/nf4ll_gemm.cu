@@ -1216,7 +1216,7 @@ struct Projections {
   int64_t ldact, M, K;
   cudaStream_t stream;
   DownBranch br[2];
-  int n = 0;
+  int n = 0, last = 1;             // branches gathered; of the last launch
   bool any = false;
   int add(const nf4ll_lora* l, void* t) {
     br[n++] = {l->mask, l->ld_mask, l->keep_scale, static_cast<const __half*>(l->A), static_cast<float*>(t)};
@@ -1225,6 +1225,7 @@ struct Projections {
   int flush() {
     if (!n) return NF4LL_OK;
     const int rc = lora_down_launch(act, ldact, br, n, 1.0f, M, K, nullptr, 0, stream);
+    last = n;
     n = 0;
     any = true;
     return rc;
@@ -1643,7 +1644,8 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     counters = reinterpret_cast<int*>(ws + pl.left_bytes + pl.bt_bytes);
     counter_words = static_cast<int>(pl.counter_bytes / sizeof(int));
   }
-  bool projected = false;          // a rank-16 projection is what this call has launched last
+  bool projected = false;          // a rank-16 projection is what this call has launched last,
+  int last = 1;                    // of so many branches
   if (segments) {
     Projections t{act, ldact, M, W->K, stream};
     int64_t at = 0;
@@ -1663,6 +1665,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     }
     if (int rc = t.flush()) return rc;
     projected = t.any;
+    last = t.last;
   }
   if (lora) {
     // rank-16 projection of the activation, fp32: T = drop(x).A^T (forward) or U = s.dy.B (backward);
@@ -1707,6 +1710,7 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
       c.seg_scale[i] = segments ? p.seg_scale[i] : (lora ? lora->scale : 0.f);
     }
     c.withhold = hooks.withhold.what; c.wait_us = hooks.withhold.wait_us;
+    c.busy = projected ? lora_down_ctas(M, W->K, last, sms) : 0;
     const int rc = stream_forward_launch(c, projected && !ev0, force_slices, status, stream);
     if (rc == NF4LL_OK && ev1) { if (int rce = record_event(ev1, stream)) return rce; }
     return rc;
@@ -1820,6 +1824,7 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
       cudaEvent_t ev0 = g_ev_start, ev1 = g_ev_stop;
       g_ev_start = g_ev_stop = nullptr;
       if (ev0) { if (int rce = record_event(ev0, stream)) return rce; }
+      c.busy = t.any ? lora_down_ctas(M, W->K, t.last, sms) : 0;
       if (int rc = stream_forward_launch(c, t.any && !ev0, 0, status, stream)) return rc;
       if (ev1) { if (int rce = record_event(ev1, stream)) return rce; }
       return NF4LL_OK;

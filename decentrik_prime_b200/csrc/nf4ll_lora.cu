@@ -245,6 +245,23 @@ static int down_run(dim3 grid, unsigned cluster_y, const __half* a, int64_t ldac
 // t32 (fp32 [M,16]) = scale * (drop(act) . R^T), R [16,C] row-major, for one branch or for two over the same rows, in one launch
 // where the rows are few (q and v of a layer, gate and up: a second launch cost a decoded layer 4 us). `zero_ptr` / `zero_words`: optional 32-bit words
 // the kernel clears on the way (see the kernel).
+// How many parts of the contraction a batch that does not fill the SMs with rows is cut into, and columns of a part
+static int64_t down_parts(int64_t M, int64_t C, int n, int sms, int64_t* c_per_cta) {
+  const int64_t units = (C + kDownWarps * 32 - 1) / (kDownWarps * 32);     // 256-column units
+  int64_t ks = (2 * static_cast<int64_t>(sms)) / ((M + 31) / 32 * n);      // at most two CTAs per SM: one wave, no tail
+  if (ks > units) ks = units;
+  if (ks < 1) ks = 1;
+  // decode-sized batches are all latency: eight CTAs in one cluster (no zero-fill, no atomics) beat more CTAs + a memset
+  if (ks > 8 && M * C <= (int64_t(1) << 21)) ks = 8;
+  *c_per_cta = (units + ks - 1) / ks * (kDownWarps * 32);
+  return (C + *c_per_cta - 1) / *c_per_cta;
+}
+
+int lora_down_ctas(int64_t M, int64_t C, int n, int sms) {
+  int64_t c_per_cta = 0;
+  return static_cast<int>((M + 7) / 8 * down_parts(M, C, n, sms, &c_per_cta) * n);
+}
+
 int lora_down_launch(const void* act, int64_t ldact, const DownBranch* br, int n, float scale, int64_t M, int64_t C, int* zero_ptr, int zero_words,
                      cudaStream_t stream) {
   if (M == 0) {
@@ -268,14 +285,8 @@ int lora_down_launch(const void* act, int64_t ldact, const DownBranch* br, int n
     return down_run<2, kDownDirect, 4>(grid, 0, a, ldact, br, n, scale, M, C, C, zero_ptr, zero_words, stream);
   }
   const int64_t row_groups = (M + 31) / 32;
-  const int64_t units = (C + kDownWarps * 32 - 1) / (kDownWarps * 32);     // 256-column units
-  int64_t ks = (2 * static_cast<int64_t>(sms)) / (row_groups * n);     // at most two CTAs per SM: one wave, no tail
-  if (ks > units) ks = units;
-  if (ks < 1) ks = 1;
-  // decode-sized batches are all latency: eight CTAs in one cluster (no zero-fill, no atomics) beat more CTAs + a memset
-  if (ks > 8 && M * C <= (int64_t(1) << 21)) ks = 8;
-  const int64_t c_per_cta = (units + ks - 1) / ks * (kDownWarps * 32);
-  ks = (C + c_per_cta - 1) / c_per_cta;
+  int64_t c_per_cta = 0;
+  const int64_t ks = down_parts(M, C, n, sms, &c_per_cta);
   const dim3 grid(static_cast<unsigned>(row_groups), static_cast<unsigned>(ks));
   if (ks == 1) return down_run<4, kDownDirect, kDownWarps>(grid, 0, a, ldact, br, n, scale, M, C, c_per_cta, zero_ptr, zero_words, stream);
   if (ks <= 8) {

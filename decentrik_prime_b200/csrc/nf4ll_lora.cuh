@@ -65,6 +65,9 @@ struct DownBranch {
   float* t32;               // [M, 16]
 };
 
+// CTAs of the launch below for n branches of at most sixteen rows
+int lora_down_ctas(int64_t M, int64_t C, int n, int sms);
+
 // one or two branches over the same rows
 int lora_down_launch(const void* act, int64_t ldact, const DownBranch* br, int n, float scale, int64_t M, int64_t C, int* zero_ptr, int zero_words,
                      cudaStream_t stream);

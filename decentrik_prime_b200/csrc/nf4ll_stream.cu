@@ -71,8 +71,8 @@ constexpr int kStreamSmem = 227 * 1024;
 // the most quantisation blocks whose token rows a decoding warp keeps in registers; buffers of partial sums
 __host__ __device__ constexpr int stream_blocks(int nt) { return nt == 1 ? 7 : 5; }
 __host__ __device__ constexpr int stream_bufs(int nt) { return nt == 1 ? 4 : 2; }
-static_assert(kStreamWarps * 4 * stream_bufs(1) <= 256 && kStreamWarps * 8 * stream_bufs(2) <= 256,
-              "partial sums lie in the unused halves of the table's entries");
+constexpr int kStreamSums = kStreamWarps * 4 * stream_bufs(1);       // entries of the table in whose unused halves partial sums lie
+static_assert(kStreamSums == kStreamWarps * 8 * stream_bufs(2) && kStreamSums + 8 * kMaxSegments <= 256, "and scaled rank-16 products");
 
 enum : int { kHoldCopies = 1, kHoldClusterSums = 3 };      // nf4ll_test_mid_withhold, as it applies here
 
@@ -396,35 +396,52 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
     if (cl > 1) cluster_wait();
     const int k = lane >> 2, q = lane & 3;          // this lane's token (of a tile of eight) and four of the sixteen rows
     const int src_words = p.M * kStreamRows, xch_words = (cl - 1) * src_words;      // a CTA's sums of a tile; all of a tile
+    // The rank-16 products, scaled, go into shared memory once, behind the partial sums: a tile then waits for neither global memory nor
+    // the multiplication. Two tokens to 128 bytes, eight entries to a segment.
+    auto scaled_t = [&](int sg, int tok) { return reinterpret_cast<float*>(st_smem + (kStreamSums + 8 * sg + (tok >> 1)) * kEntryStride + 128 + 64 * (tok & 1)); };
+    {
+      static_assert(16 * 4 <= 32 * kStreamEpilogues, "sixteen bytes of a token's product to a lane");
+      const int piece = (warp - kEpiWarp) * 32 + lane;
+      float4 f[kMaxSegments];
+#pragma unroll
+      for (int sg = 0; sg < kMaxSegments; ++sg)
+        if (sg < p.n_seg && p.seg_t[sg] && piece < 4 * p.M) f[sg] = __ldcg(reinterpret_cast<const float4*>(p.seg_t[sg]) + piece);
+#pragma unroll
+      for (int sg = 0; sg < kMaxSegments; ++sg)
+        if (sg < p.n_seg && p.seg_t[sg] && piece < 4 * p.M) {
+          const float s = p.seg_scale[sg];
+          reinterpret_cast<float4*>(scaled_t(sg, piece >> 2))[piece & 3] = make_float4(f[sg].x * s, f[sg].y * s, f[sg].z * s, f[sg].w * s);
+        }
+      named_barrier(2, 32 * kStreamEpilogues);
+    }
     // units go round the warps, whose buffers differ; gate|up with two buffers is one warp's
     const int finishing = kBufs / halves < kStreamEpilogues ? 1 : kStreamEpilogues;
+    // what a tile's result is made of besides sums and products, requested before they are waited for
+    int seg = -1;                                   // its segment, where that has a rank-16 branch
+    uint2 bias;
+    uint4 br[4][2];
+    auto request = [&](int i, int hf) {
+      seg = -1;
+      bias = make_uint2(0, 0);
+      if (i >= my_units || (cl > 1 && crank != i % cl)) return;
+      const int64_t n0 = row_of(i, hf);
+      int sg = 0;
+      while (sg + 1 < p.n_seg && n0 >= p.seg_end[sg]) ++sg;
+      if (p.bias) bias = __ldg(reinterpret_cast<const uint2*>(p.bias + n0 + 4 * q));
+      if (!p.seg_t[sg]) return;
+      seg = sg;
+      const uint4* bp = reinterpret_cast<const uint4*>(p.seg_b[sg] + (n0 + 4 * q) * 16);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) { br[r][0] = __ldg(bp + 2 * r); br[r][1] = __ldg(bp + 2 * r + 1); }
+    };
     for (int i = warp - kEpiWarp; ok && i < my_units && warp - kEpiWarp < finishing; i += finishing) {
       const int owner = cl > 1 ? i % cl : 0, slot = cl > 1 ? i / cl : 0, team = p.teams > 1 ? i % p.teams : 0;
       float gate[NT][4];                            // gate|up: the first half's results as rounded
       for (int hf = 0; hf < halves; ++hf) {
         const int j = i * halves + hf, buf = j % kBufs;
         const int64_t n0 = row_of(i, hf);
-        // what the result is made of besides the sums, requested before they are waited for
-        int sg = 0;
-        while (sg + 1 < p.n_seg && n0 >= p.seg_end[sg]) ++sg;
-        const float* t32 = p.seg_t[sg];
         const bool mine = crank == owner;
-        uint4 br[4][2];
-        float tv[NT][16];
-        uint2 bias = make_uint2(0, 0);
-        if (mine && p.bias) bias = __ldg(reinterpret_cast<const uint2*>(p.bias + n0 + 4 * q));
-        if (mine && t32) {
-          const uint4* bp = reinterpret_cast<const uint4*>(p.seg_b[sg] + (n0 + 4 * q) * 16);
-#pragma unroll
-          for (int r = 0; r < 4; ++r) { br[r][0] = __ldg(bp + 2 * r); br[r][1] = __ldg(bp + 2 * r + 1); }
-#pragma unroll
-          for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) {
-              const float4 f = 8 * n + k < p.M ? __ldcg(reinterpret_cast<const float4*>(t32 + (8 * n + k) * 16) + c) : make_float4(0.f, 0.f, 0.f, 0.f);
-              tv[n][4 * c] = f.x; tv[n][4 * c + 1] = f.y; tv[n][4 * c + 2] = f.z; tv[n][4 * c + 3] = f.w;
-            }
-        }
+        request(i, hf);
         ok = stream_wait(smem_u32(part_full + buf), (j / kBufs) & 1, ab, 0x0806);
         if (!ok) break;
         float4 v[NT];
@@ -469,24 +486,40 @@ nf4_stream_kernel(const __grid_constant__ StreamParams p) {
             }
           }
         }
+        // two ranks side by side: even and odd ones add up apart
+        uint64_t l2[NT][4];
+#pragma unroll
+        for (int n = 0; n < NT; ++n) l2[n][0] = l2[n][1] = l2[n][2] = l2[n][3] = 0;
+        if (seg >= 0) {
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            uint64_t t2[NT][4];
+#pragma unroll
+            for (int n = 0; n < NT; ++n) {
+              const float4* from = reinterpret_cast<const float4*>(scaled_t(seg, 8 * n + k < p.M ? 8 * n + k : 0)) + 2 * c;
+              const float4 a = from[0], b = from[1];
+              t2[n][0] = f32x2(a.x, a.y); t2[n][1] = f32x2(a.z, a.w); t2[n][2] = f32x2(b.x, b.y); t2[n][3] = f32x2(b.z, b.w);
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              const uint32_t w[4] = {br[r][c].x, br[r][c].y, br[r][c].z, br[r][c].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const uint64_t b2 = half2_to_f32x2(w[e]);
+#pragma unroll
+                for (int n = 0; n < NT; ++n) l2[n][r] = fma2(t2[n][e], b2, l2[n][r]);
+              }
+            }
+          }
+        }
         const float2 blo = __half22float2(*reinterpret_cast<const __half2*>(&bias.x)), bhi = __half22float2(*reinterpret_cast<const __half2*>(&bias.y));
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
           const int tok = 8 * n + k;
           if (tok < p.M) {
-            float l[4] = {0.f, 0.f, 0.f, 0.f};
-            if (t32) {
-              const float scale = p.seg_scale[sg];
+            float l[4];
 #pragma unroll
-              for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                  float b[8];
-                  unpack8(br[r][c], b);
-#pragma unroll
-                  for (int e = 0; e < 8; ++e) l[r] = fmaf(tv[n][8 * c + e], b[e] * scale, l[r]);
-                }
-            }
+            for (int r = 0; r < 4; ++r) { const float2 f = f32x2_split(l2[n][r]); l[r] = f.x + f.y; }
             const uint2 out = make_uint2(pack_half2_rn((v[n].x + blo.x) + l[0], (v[n].y + blo.y) + l[1]), pack_half2_rn((v[n].z + bhi.x) + l[2], (v[n].w + bhi.y) + l[3]));
             __half* dst = p.split && n0 >= p.split ? p.y2 + tok * p.ldy2 + (n0 - p.split) : p.y + tok * p.ldy + n0;
             *reinterpret_cast<uint2*>(dst + 4 * q) = out;
@@ -574,8 +607,17 @@ static double stream_us(int nt, int cl, int64_t tiles, int teams, int np, int s,
   return (3.5 + 0.303 * r + 0.0476 * turns * s + 0.0166 * r * static_cast<double>(blocks)) * (s == 5 ? 1.15 : 1.0);
 }
 
+// With a rank-16 projection in front whose CTAs hold `busy` SMs for a while: a grid that wants more SMs than are left starts the last of its
+// CTAs that much later. What that costs a plan, against another round of tiles on the SMs that are free (and 0.1 us a tile for the
+// products where the tokens are few). Fitted to 412 calls at 1 to 16 rows of which both were timed: picking by it takes 0.2 % (from
+// nine rows on 0.3 %) longer than the faster of the two, without it 0.4 % (1.4 %). us with / without: 1536 x 8960 Q|K|V at 9 rows 12.6 / 15.2, 1024 x 8192
+// 10.0 / 11.8, 1152 x 9088 at 1 row 8.4 / 9.5.
+static double stream_beside_us(int nt, bool late, int64_t tiles, int64_t K) {
+  return (nt == 1 ? 0.1 * static_cast<double>(tiles) : 0) + (late ? fmin((nt == 1 ? 0.25 : 0.5) + 0.00015 * static_cast<double>(K), 1.9) : 0);
+}
+
 // M: tokens, sixteen at most. `force`: low byte warps of a team, next byte CTAs of a cluster, next byte teams (0: free)
-static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int force, StreamPlan* best) {
+static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int busy, int force, StreamPlan* best) {
   const int nt = M > 8 ? 2 : 1;
   const int64_t bpr = K / 64, units = N / kStreamRows / (pair ? 2 : 1);
   const int warps = kStreamWarps, f_np = force & 255, f_cl = force >> 8 & 255, f_teams = force >> 16, halves = pair ? 2 : 1;
@@ -592,37 +634,42 @@ static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int force, S
     const int64_t blocks = (bpr + cl - 1) / cl;
     const int least = static_cast<int>((blocks + stream_blocks(nt) - 1) / stream_blocks(nt));
     if (blocks > warps * stream_blocks(nt)) continue;
-    const int most = stream_clusters(cl);
-    if (most <= 0) continue;
-    StreamPlan p{};
-    p.cl = cl; p.units = units;
-    const int64_t rounds = (units + most - 1) / most;
-    p.clusters = static_cast<int>((units + rounds - 1) / rounds);
-    p.row = static_cast<int>(blocks * 32);
-    p.pitch = (2 * p.row + 95) / 128 * 128 + 32;
-    p.groups = static_cast<int>((15 * bpr + blocks + 254) / 256 + 1);
-    const int64_t slots = (rounds + cl - 1) / cl * halves;
-    if (p.groups > kStreamMaxGroups || (cl > 1 && slots > kStreamMaxSlots)) continue;
-    p.off_xch = (kStreamFixed + 127) / 128 * 128;
-    p.off_ring = static_cast<int>(p.off_xch + (cl > 1 ? (slots * (cl - 1) * M * kStreamRows * 4 + 127) / 128 * 128 : 0));
-    p.off_q = kStreamRows / 2 * p.pitch + kStreamScales;
-    p.stage = static_cast<int>((p.off_q + kStreamRows * bpr + 16 + 127) / 128 * 128);
-    const int64_t room = kStreamSmem - p.off_ring - kStreamSlack;
-    const int fit = static_cast<int>(room / p.stage < kStreamMaxStages ? room / p.stage : kStreamMaxStages);
-    if (cl > 8 && fit < 2) continue;
-    for (int np = least; np <= warps && np <= blocks; ++np) {
-      if (f_np && np != (f_np < least ? least : f_np < warps && f_np < blocks ? f_np : warps < blocks ? warps : static_cast<int>(blocks))) continue;
-      p.s = static_cast<int>((blocks + np - 1) / np);
-      p.np = np;
-      int most_teams = 0;
-      for (int t = 1; t * halves <= stream_bufs(nt) && t * np <= warps && t <= fit && (t == 1 || t <= rounds); t *= 2) most_teams = t;
-      for (int teams = 1; teams <= most_teams; teams *= 2) {
-        if (f_teams && teams != (f_teams < most_teams ? f_teams : most_teams)) continue;
-        p.teams = teams;
-        p.stages = fit / teams;
-        p.smem = p.off_ring + p.stages * teams * p.stage + kStreamSlack;
-        p.us = stream_us(nt, cl, rounds * halves, teams, np, p.s, blocks, p.stages);
-        if (!found || p.us < best->us) { *best = p; found = true; }
+    const int all = stream_clusters(cl);
+    if (all <= 0) continue;
+    const int beside = busy > 0 ? static_cast<int>((stream_clusters(1) - busy) / cl) : all;
+    for (int turn = 0; turn < (beside > 0 && beside < all ? 2 : 1); ++turn) {
+      const int most = turn ? beside : all;
+      StreamPlan p{};
+      p.cl = cl; p.units = units;
+      const int64_t rounds = (units + most - 1) / most;
+      p.clusters = static_cast<int>((units + rounds - 1) / rounds);
+      p.row = static_cast<int>(blocks * 32);
+      p.pitch = (2 * p.row + 95) / 128 * 128 + 32;
+      p.groups = static_cast<int>((15 * bpr + blocks + 254) / 256 + 1);
+      const int64_t slots = (rounds + cl - 1) / cl * halves;
+      if (p.groups > kStreamMaxGroups || (cl > 1 && slots > kStreamMaxSlots)) continue;
+      p.off_xch = (kStreamFixed + 127) / 128 * 128;
+      p.off_ring = static_cast<int>(p.off_xch + (cl > 1 ? (slots * (cl - 1) * M * kStreamRows * 4 + 127) / 128 * 128 : 0));
+      p.off_q = kStreamRows / 2 * p.pitch + kStreamScales;
+      p.stage = static_cast<int>((p.off_q + kStreamRows * bpr + 16 + 127) / 128 * 128);
+      const int64_t room = kStreamSmem - p.off_ring - kStreamSlack;
+      const int fit = static_cast<int>(room / p.stage < kStreamMaxStages ? room / p.stage : kStreamMaxStages);
+      if (cl > 8 && fit < 2) continue;
+      for (int np = least; np <= warps && np <= blocks; ++np) {
+        if (f_np && np != (f_np < least ? least : f_np < warps && f_np < blocks ? f_np : warps < blocks ? warps : static_cast<int>(blocks))) continue;
+        p.s = static_cast<int>((blocks + np - 1) / np);
+        p.np = np;
+        int most_teams = 0;
+        for (int t = 1; t * halves <= stream_bufs(nt) && t * np <= warps && t <= fit && (t == 1 || t <= rounds); t *= 2) most_teams = t;
+        for (int teams = 1; teams <= most_teams; teams *= 2) {
+          if (f_teams && teams != (f_teams < most_teams ? f_teams : most_teams)) continue;
+          p.teams = teams;
+          p.stages = fit / teams;
+          p.smem = p.off_ring + p.stages * teams * p.stage + kStreamSlack;
+          p.us = stream_us(nt, cl, rounds * halves, teams, np, p.s, blocks, p.stages);
+          if (busy > 0) p.us += stream_beside_us(nt, p.clusters > beside, rounds * halves, K);
+          if (!found || p.us < best->us) { *best = p; found = true; }
+        }
       }
     }
   }
@@ -632,12 +679,12 @@ static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int force, S
 bool stream_takes(int64_t M, int64_t N, int64_t K, bool gate_up) {
   if (K <= 64 * kStreamWarps * stream_blocks(1) && N <= (int64_t(1) << 28)) return true;      // one CTA holds a tile's rows
   StreamPlan p{};
-  return stream_plan(M < 8 ? M : 8, N, K, gate_up, 0, &p);
+  return stream_plan(M < 8 ? M : 8, N, K, gate_up, 0, 0, &p);
 }
 
 double stream_time_us(int64_t N, int64_t K) {
   StreamPlan p{};
-  return stream_plan(16, N, K, false, 0, &p) ? p.us : 1e30;
+  return stream_plan(16, N, K, false, 0, 0, &p) ? p.us : 1e30;
 }
 
 // The former kernel's time with the gated product's launch behind it, whose line against the kernel for middling batches still stands for
@@ -661,17 +708,18 @@ int stream_forward_launch(const StreamCall& c, bool early, int force, int32_t* s
     const int64_t left = c.M - m0;
     int nt = left > 8 ? 2 : 1;
     bool fused = c.h != nullptr;
+    const int busy = early && m0 == 0 ? c.busy : 0;
     StreamPlan pl{};
-    bool found = stream_plan(left < 16 ? left : 16, W->N, W->K, fused, force, &pl);
+    bool found = stream_plan(left < 16 ? left : 16, W->N, W->K, fused, busy, force, &pl);
     if (fused && nt == 2 && (!found || pl.cl > 1)) {
       // one warp finishes both halves of a unit, which is too slow for a cluster's (55296 x 5120 at 16 rows 107 us)
       fused = false;
-      found = stream_plan(left < 16 ? left : 16, W->N, W->K, false, force, &pl);
+      found = stream_plan(left < 16 ? left : 16, W->N, W->K, false, busy, force, &pl);
     }
     if (!found) {
       nt = 1;
       fused = c.h != nullptr;
-      if (!stream_plan(left < 8 ? left : 8, W->N, W->K, fused, force, &pl)) {
+      if (!stream_plan(left < 8 ? left : 8, W->N, W->K, fused, busy, force, &pl)) {
         set_detail("weight-streaming kernel: W[%lld,%lld] is too large", static_cast<long long>(W->N), static_cast<long long>(W->K));
         return NF4LL_ERR_SHAPE;
       }

@@ -22,6 +22,7 @@ struct StreamCall {
   const float* seg_t[kMaxSegments];      // [M, 16] fp32 rank-16 product of the segment, null: no LoRA
   const __half* seg_b[kMaxSegments];     // its lora_B, indexed by the row of W
   float seg_scale[kMaxSegments];
+  int busy;                              // CTAs of the rank-16 projection launched right before, each on an SM for as long as that takes
   int withhold;                          // failure-detection hook
   uint32_t wait_us;
 };

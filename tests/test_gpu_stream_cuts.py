@@ -25,7 +25,8 @@ def forward(d, w=None):
 
 
 # 84 blocks to a CTA up to 8 tokens (5376 weights), 60 beyond (3840); 9728 rows: five tiles for some CTAs, four for others
-@pytest.mark.parametrize("N,K", [(256, 64), (256, 448), (192, 5376), (256, 5440), (256, 8128), (192, 3840), (256, 3904), (9728, 512), (19456, 64)])
+@pytest.mark.parametrize("N,K", [(256, 64), (256, 448), (192, 5376), (256, 5440), (256, 8128), (192, 3840), (256, 3904), (9728, 512), (19456, 64),
+                                 (1024, 8192), (1152, 5376)])      # the last two leave SMs to the rank-16 projection
 @pytest.mark.parametrize("M", [1, 5, 8, 9, 16])
 def test_edges(N, K, M):
     pr = make_problem(N, K, M, seed=N + K + M, lora=True, dropout=0.05, bias=True, device="cuda" if N * K > 1 << 22 else "cpu")
@@ -65,6 +66,30 @@ def test_long_rows_of_gate_and_up():
     assert_close("g", g, y[:, :inter])
     assert_close("u", u, y[:, inter:])
     assert torch.equal(h, linear.swiglu_forward(g, u))
+
+
+@pytest.mark.parametrize("on", [(0, 1, 2, 3), (1, 3), (2,)])
+@pytest.mark.parametrize("M", [1, 8, 9, 16])
+def test_four_projections(M, on):
+    """As many segments as a call may have, each with a rank-16 branch of its own or none."""
+    rows, K = (256, 128, 384, 128), 1536
+    pr = make_problem(sum(rows), K, M, seed=M, lora=False, bias=True)
+    d = to_device(pr)
+    gen = torch.Generator().manual_seed(M)
+    A, B = [torch.randn(16, K, generator=gen).mul_(0.03).half() for _ in rows], [torch.randn(r, 16, generator=gen).mul_(0.05).half() for r in rows]
+    scales = (2.0, 0.5, 1.0, 3.0)
+    segments = [(r, (A[i].cuda(), B[i].cuda(), scales[i]) if i in on else None, None, 1.0) for i, r in enumerate(rows)]
+    with tiles_only():
+        y, t = linear.forward_multi(d.w, d.x, segments, bias=d.bias)
+    linear.check_status()
+    base, at = reference(pr), 0
+    for i, r in enumerate(rows):
+        ref = base[:, at:at + r]
+        if i in on:
+            ref = ref + (scales[i] * (pr.x.double() @ A[i].double().t()) @ B[i].double().t()).to(ref.dtype)
+        assert (t[i] is not None) == (i in on)
+        assert_close(f"y{i}", y[:, at:at + r], ref)
+        at += r
 
 
 @pytest.mark.parametrize("K", [512, 5440])
