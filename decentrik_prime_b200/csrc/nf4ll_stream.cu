@@ -609,9 +609,9 @@ static double stream_us(int nt, int cl, int64_t tiles, int teams, int np, int s,
 
 // With a rank-16 projection in front whose CTAs hold `busy` SMs for a while: a grid that wants more SMs than are left starts the last of its
 // CTAs that much later. What that costs a plan, against another round of tiles on the SMs that are free (and 0.1 us a tile for the
-// products where the tokens are few). Fitted to 412 calls at 1 to 16 rows of which both were timed: picking by it takes 0.2 % (from
-// nine rows on 0.3 %) longer than the faster of the two, without it 0.4 % (1.4 %). us with / without: 1536 x 8960 Q|K|V at 9 rows 12.6 / 15.2, 1024 x 8192
-// 10.0 / 11.8, 1152 x 9088 at 1 row 8.4 / 9.5.
+// products where the tokens are few). Fitted to 824 calls at 1 to 16 rows, of which both were timed: picking by it takes 0.2 % (from
+// nine rows on 0.3 %) longer than the faster of the two, without it 0.4 % (1.4 %). us with / without: Q|K|V at 9 rows 1536 x 8960 11.4 / 14.2, 1024 x 8192
+// 9.6 / 11.5; 1152 x 9088 at 1 row 8.4 / 9.3, 1024 x 27648 at 8 rows 11.9 / 13.7.
 static double stream_beside_us(int nt, bool late, int64_t tiles, int64_t K) {
   return (nt == 1 ? 0.1 * static_cast<double>(tiles) : 0) + (late ? fmin((nt == 1 ? 0.25 : 0.5) + 0.00015 * static_cast<double>(K), 1.9) : 0);
 }
@@ -636,7 +636,10 @@ static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int busy, in
     if (blocks > warps * stream_blocks(nt)) continue;
     const int all = stream_clusters(cl);
     if (all <= 0) continue;
-    const int beside = busy > 0 ? static_cast<int>((stream_clusters(1) - busy) / cl) : all;
+    // The projection's SMs, eight of a GPC at a time, leave room for two clusters less at least (one of more than eight CTAs): 44 of 45
+    // clusters of three wait for them and 43 do not, 32 of 33 of four and 31, 15 of 15 of nine and 14, whether it has 8 or 16 of them.
+    const int others = (stream_clusters(1) - busy) / cl, fewer = cl == 1 ? all : cl > 8 ? all - 1 : all - 2;
+    const int beside = busy <= 0 ? all : fewer < others ? fewer : others;
     for (int turn = 0; turn < (beside > 0 && beside < all ? 2 : 1); ++turn) {
       const int most = turn ? beside : all;
       StreamPlan p{};
