@@ -1244,18 +1244,16 @@ int launch_pair(int mode, int bm_tiles, const CUtensorMap& map, const CUtensorMa
                 const GemmParams& p, int64_t tiles_o, int64_t tiles_mp, int splits, int launch_splits, cudaStream_t stream);
 constexpr int64_t kStreamMaxRows = 16;     // most token rows of the weight-streaming kernel's own choice
 constexpr int64_t kStreamCapRows = 64;     // its limit (reachable through the tuning hook)
-// From 9 to 16 rows of one projection (or of each half of gate|up) against at least 2^24 weights, the kernel for middling batches
-// where its model (mid_plan; 5 % low there) lies below the streaming kernel's, which depends on how evenly its units go round the
-// SMs and on the tokens, and to which gate|up adds a launch. Measured, streaming / middling, us at 9 and 16 rows: 5120 x 27648
-// 55 / 41 and 63 / 41, 27648 x 5120 38 / 36 and 41 / 36, 18944 x 3584 22 / 19 and 23 / 19, 5120 x 5120 14.0 / 13.6 and 15.6 / 13.6,
-// 10240 x 2560 13.2 / 15.0 and 14.3 / 15.0, gate|up of 2 x 9472 x 3584 26 / 21 and 27 / 21; below 2^24 the streaming kernel is
-// ahead (3584 x 3584 9.2 / 10.8, 1536 x 8960 10.6 / 12.0 at 16 rows),
-// but not for gate|up of such halves, which is not asked (2 x 5504 x 2048 15.8 / 13.6). Over 51 such calls the choice takes 0.3 % longer than the
-// faster kernel, 9 % at worst (27648 x 1024). Against fp64 sums over the fp16 weights, which are the result that this path is
-// held to, the rel-L2 is 3.4e-4 in the streaming kernel and 2.1e-4 in this one; over the unrounded weights 2.8e-4 and 2.9e-4.
-// From 17 rows on the latter is ahead everywhere (1536 x 1536 at 17 rows 7.5; the streaming kernel 4.8 at 16).
+// From 9 to 16 rows the kernel for middling batches where it is the faster one by the two kernels' models (mid_plan, stream_time_us), of
+// which its own is 0.8 us low there, with gate|up 1.3, and a rank-16 projection in front costs it 2.6. Streaming / middling, us: 5120 x 27648
+// at 9 rows 40.9 / 40.1, with LoRA 49.9 / 42.9; 9344 x 11008 32.9 / 27.9; 27648 x 5120 at 16 rows 34.4 / 35.3; 18944 x 3584 18.6 / 18.7; 10240 x 5120
+// at 12 rows 16.2 / 20.2; 4096 x 4096 at 9 rows 9.0 / 11.1; gate|up of 28672 x 4096 35.0 / 32.0, with LoRA 41.2 / 34.4, of 18944 x 3584 18.6 / 21.0, of
+// 27648 x 1024 15.5 / 12.2, of 11008 x 2048 10.9 / 13.5. Over 1170 such calls (60 weights at 9, 12 and 16 rows, single, stacked and gate|up,
+// with LoRA and without) the choice takes 0.4 % longer than the faster kernel, 12 % at worst. Against fp64 sums over the fp16
+// weights, which are the result that this path is held to, the rel-L2 is 3.4e-4 in the streaming kernel and 2.1e-4 in this one; over the
+// unrounded weights 2.8e-4 and 2.9e-4. From 17 rows on the latter is ahead everywhere (1536 x 1536 at 17 rows 7.5; the streaming
+// kernel 3.8 at 16).
 constexpr int64_t kMidLeastRows = 9;       // below, the streaming kernel keeps its exact fp32 scales, and is the faster one nearly everywhere
-constexpr int64_t kMidSmallWeights = int64_t(1) << 24;
 
 // Which kernel computes a forward of M rows that neither the kernel for middling batches nor the dense GEMM takes (from 17 to 128
 // rows: only weights of 2^31 quantisation blocks and more, forced tiles, the hooks that keep the former out): the tile
@@ -1444,7 +1442,8 @@ static int run_dense(const DenseCall& c, int sms, uint8_t* ws, int32_t* status, 
 // Whether a call runs on the kernel for middling batches (nf4ll_mid.cu)
 constexpr int64_t kMidMostRows = 2560;      // beyond, the dense GEMM or the tiles without asking
 // `t`: the times of the other ways beyond kDenseNeverRows rows; `dense`: the dense GEMM is one of them
-static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lora, bool mask, int sms, const Tune& tune, MidPlan* mp) {
+// `branches`: rank-16 products that the call makes itself
+static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lora, int branches, bool mask, int sms, const Tune& tune, MidPlan* mp) {
   if (g_expire_polls != 0 || g_mid.on < 0) return false;
   const int64_t N = c.W->N, K = c.W->K, NO = c.mode == kFwd ? N : K, KC = c.mode == kFwd ? K : N;
   if (N * (K / 64) >= (int64_t(1) << 31) || c.M >= (1 << 24)) return false;      // the kernel's indices have 32 bits
@@ -1458,11 +1457,9 @@ static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lor
   if (c.M > kMidMostRows) return false;
   if (c.mode == kFwd && c.M <= kStreamMaxRows) {
     if (!stream_takes(c.M, N, K, c.gu_inter != 0)) return mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp);
-    if (c.M < kMidLeastRows || (c.n_seg > 1 && !c.gu_inter) || (c.gu_inter ? N / 2 : N) * K < kMidSmallWeights) return false;
-    if (!mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
-    // The streaming kernel where both models put it 5 % ahead. At 16 rows, that one / this one, us: 27648 x 5120 33.9 / 35.4, 18944 x 3584
-    // 17.5 / 18.7, 5120 x 27648 39.9 / 40.3; 3584 x 18944 21.2 / 24.6, 9728 x 2560 9.5 / 17.4, 4096 x 4096 9.3 / 11.3.
-    return c.gu_inter ? 1.05 * mp->us < stream_gate_up_line_us(N, K, c.M, sms) : mp->us < 1.05 * stream_time_us(N, K);
+    if (c.M < kMidLeastRows || !mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
+    const int busy = branches > 0 ? lora_down_ctas(c.M, K, branches < 2 ? 1 : 2, sms) : 0;
+    return mp->us + (c.gu_inter ? 1.3 : 0.8) + (branches > 0 ? 2.6 : 0) < stream_time_us(c.M, N, K, c.gu_inter != 0, busy);
   }
   if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
   if (c.M <= kDenseNeverRows) return true;
@@ -1599,7 +1596,9 @@ static int run_gemm(int mode, const nf4ll_mat* W, const void* act, int64_t ldact
     RowTimes t{};
     if (M > kDenseNeverRows && (dense || M <= kMidMostRows)) t = row_times(mode, M, NO, KC, 0, narrow_tiles, any_lora, sms);
     MidPlan mp;
-    if (mid_wanted(c, t, dense, any_lora, lora && lora->mask, sms, tune, &mp))
+    int branches = 0;
+    for (int i = 0; i < c.n_seg; ++i) branches += dc.lora[i] && !dc.side_ready[i];
+    if (mid_wanted(c, t, dense, any_lora, branches, lora && lora->mask, sms, tune, &mp))
       return run_mid(c, mp, dc.lora, dc.side, dc.side_ready, workspace, workspace_bytes, status, stream, who);
     if (dense && ((tune.flags & kFlagDense) || t.dense < t.decoding)) return run_dense(dc, sms, static_cast<uint8_t*>(workspace), status, stream);
   }
@@ -1793,7 +1792,7 @@ static int run_gate_up(const nf4ll_mat* W, const void* x, int64_t ldx, const nf4
     RowTimes t{};
     if (M > kDenseNeverRows && (dense || M <= kMidMostRows)) t = row_times(kFwd, M, W->N, W->K, I, false, lora_gate || lora_up, sms);
     MidPlan mp;
-    if (mid_wanted(c, t, dense, lora_gate || lora_up, false, sms, g_tune, &mp))
+    if (mid_wanted(c, t, dense, lora_gate || lora_up, (lora_gate != nullptr) + (lora_up != nullptr), false, sms, g_tune, &mp))
       return run_mid(c, mp, dc.lora, dc.side, dc.side_ready, workspace, workspace_bytes, status, stream, who);
     if (!odd && dense && ((g_tune.flags & kFlagDense) || t.dense < t.decoding)) return run_dense(dc, sms, static_cast<uint8_t*>(workspace), status, stream);
   }

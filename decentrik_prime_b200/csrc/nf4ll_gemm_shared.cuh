@@ -52,6 +52,48 @@ struct GemmParams {
   uint32_t spin_limit;     // polls of a tile counter (each followed by a short sleep) before a split gives up
 };
 
+// Plans are functions of the sizes alone; a thread keeps the last ones it used (a search takes some microseconds): 64 sets of
+// four, the least recently used of a set makes room. With one plan per set, 198 of 348 batch sizes had two of the ten plans of a
+// training layer in one set, which were then searched for on every layer of every step.
+template <typename P, int KEYS>
+class KeptPlans {
+ public:
+  // `search` fills in a plan and says whether there is one
+  template <typename F>
+  bool get(const int64_t (&key)[KEYS], P* plan, F&& search) {
+    uint64_t h = 0;
+    for (int64_t k : key) h = (h ^ static_cast<uint64_t>(k)) * 0x9e3779b97f4a7c15ull;
+    Kept* set = kept_[h >> 58];
+    Kept* e = set;
+    for (int w = 0; w < 4; ++w) {
+      bool same = set[w].used != 0;
+      for (int i = 0; i < KEYS && same; ++i) same = set[w].key[i] == key[i];
+      if (same) {
+        set[w].used = ++clock_;
+        *plan = set[w].plan;
+        return set[w].found;
+      }
+      if (set[w].used < e->used) e = set + w;
+    }
+    for (int i = 0; i < KEYS; ++i) e->key[i] = key[i];
+    e->plan = P{};
+    e->found = search(&e->plan);
+    e->used = ++clock_;
+    *plan = e->plan;
+    return e->found;
+  }
+
+ private:
+  struct Kept {
+    int64_t key[KEYS];
+    P plan;
+    bool found;
+    uint64_t used;               // 0: empty
+  };
+  Kept kept_[64][4];
+  uint64_t clock_ = 0;
+};
+
 constexpr uint32_t kCoopSpinLimit = 1u << 22;   // default for GemmParams::spin_limit
 constexpr int kFixSlots = 8;     // 16 KB slots of the split-K fix-up ring (fits every tile shape's operand rings)
 

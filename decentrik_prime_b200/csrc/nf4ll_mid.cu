@@ -952,44 +952,16 @@ static bool mid_search(int mode, int64_t M, int64_t NO, int64_t KC, bool mask, i
   return found;
 }
 
-// Plans are functions of the sizes alone; a thread keeps the last ones it used (a search takes some microseconds): 64 sets of
-// four, the least recently used of a set makes room. With one plan per set, 198 of 348 batch sizes had two of the ten plans of a
-// training layer in one set, which were then searched for on every layer of every step.
 static thread_local int64_t g_mid_searches = 0;
 bool mid_plan(int mode, int64_t M, int64_t NO, int64_t KC, bool mask, int64_t gu_inter, bool lora, int rb, int nt, int cl, MidPlan* plan) {
-  struct Kept {
-    int64_t key[6];
-    MidPlan plan;
-    bool found;
-    uint64_t used;               // 0: empty
-  };
-  constexpr int kSets = 64, kWays = 4;
-  static thread_local Kept kept[kSets][kWays];
-  static thread_local uint64_t clock = 0;
+  static thread_local KeptPlans<MidPlan, 6> kept;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) return false;
   const int64_t key[6] = {M, NO, KC, gu_inter, mode | (mask ? 2 : 0) | (lora ? 4 : 0) | (static_cast<int64_t>(dev) << 8), rb | (nt << 4) | (cl << 16)};
-  uint64_t h = 0;
-  for (int64_t k : key) h = (h ^ static_cast<uint64_t>(k)) * 0x9e3779b97f4a7c15ull;
-  Kept* set = kept[h >> 58];
-  Kept* e = set;
-  for (int w = 0; w < kWays; ++w) {
-    bool same = set[w].used != 0;
-    for (int i = 0; i < 6 && same; ++i) same = set[w].key[i] == key[i];
-    if (same) {
-      set[w].used = ++clock;
-      *plan = set[w].plan;
-      return set[w].found;
-    }
-    if (set[w].used < e->used) e = set + w;
-  }
-  ++g_mid_searches;
-  for (int i = 0; i < 6; ++i) e->key[i] = key[i];
-  e->plan = MidPlan{};
-  e->found = mid_search(mode, M, NO, KC, mask, gu_inter, lora, rb, nt, cl, &e->plan);
-  e->used = ++clock;
-  *plan = e->plan;
-  return e->found;
+  return kept.get(key, plan, [&](MidPlan* p) {
+    ++g_mid_searches;
+    return mid_search(mode, M, NO, KC, mask, gu_inter, lora, rb, nt, cl, p);
+  });
 }
 int64_t mid_searches() { return g_mid_searches; }
 static thread_local int64_t g_mid_calls = 0;

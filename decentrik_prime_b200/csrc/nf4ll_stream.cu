@@ -617,7 +617,7 @@ static double stream_beside_us(int nt, bool late, int64_t tiles, int64_t K) {
 }
 
 // M: tokens, sixteen at most. `force`: low byte warps of a team, next byte CTAs of a cluster, next byte teams (0: free)
-static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int busy, int force, StreamPlan* best) {
+static bool stream_search(int64_t M, int64_t N, int64_t K, bool pair, int busy, int force, StreamPlan* best) {
   const int nt = M > 8 ? 2 : 1;
   const int64_t bpr = K / 64, units = N / kStreamRows / (pair ? 2 : 1);
   const int warps = kStreamWarps, f_np = force & 255, f_cl = force >> 8 & 255, f_teams = force >> 16, halves = pair ? 2 : 1;
@@ -679,29 +679,38 @@ static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int busy, in
   return found;
 }
 
+static bool stream_plan(int64_t M, int64_t N, int64_t K, bool pair, int busy, int force, StreamPlan* plan) {
+  static thread_local KeptPlans<StreamPlan, 6> kept;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  const int64_t key[6] = {M, N, K, busy, force, static_cast<int64_t>(dev) << 1 | (pair ? 1 : 0)};
+  return kept.get(key, plan, [&](StreamPlan* p) { return stream_search(M, N, K, pair, busy, force, p); });
+}
+
+// The plan of a call of M <= 16 tokens. Beyond eight, gate|up forms its product in the launch only where one CTA holds a row: one warp
+// finishes both halves of a unit, which is too slow for a cluster's (55296 x 5120 at 16 rows 107 us).
+static bool stream_call_plan(int64_t M, int64_t N, int64_t K, bool gate_up, int busy, int force, bool* fused, StreamPlan* plan) {
+  *fused = gate_up;
+  if (stream_plan(M, N, K, gate_up, busy, force, plan) && !(gate_up && M > 8 && plan->cl > 1)) return true;
+  if (!gate_up || M <= 8) return false;
+  *fused = false;
+  return stream_plan(M, N, K, false, busy, force, plan);
+}
+
 bool stream_takes(int64_t M, int64_t N, int64_t K, bool gate_up) {
   if (K <= 64 * kStreamWarps * stream_blocks(1) && N <= (int64_t(1) << 28)) return true;      // one CTA holds a tile's rows
   StreamPlan p{};
   return stream_plan(M < 8 ? M : 8, N, K, gate_up, 0, 0, &p);
 }
 
-double stream_time_us(int64_t N, int64_t K) {
+// Beside the plan's own time: the gated product's launch, or what it costs the warp that forms it, of a tile; and with rank-16 products
+// made by this call, what is left of that kernel and what a tile's epilogue takes.
+double stream_time_us(int64_t M, int64_t N, int64_t K, bool gate_up, int busy) {
+  bool fused = false;
   StreamPlan p{};
-  return stream_plan(16, N, K, false, 0, 0, &p) ? p.us : 1e30;
-}
-
-// The former kernel's time with the gated product's launch behind it, whose line against the kernel for middling batches still stands for
-// gate|up of 9 to 16 rows (the present one's: 18944 x 3584 at 9 rows 18.3 us, there 21.4; 37888 x 3584 31.4 and 29.8)
-double stream_gate_up_line_us(int64_t N, int64_t K, int64_t M, int sms) {
-  const int64_t steps = (K / 64 + 3) / 4;
-  int64_t cost = 0, rt = 0;
-  for (int r = 2; r >= 1; --r)
-    for (int w : {1, 2, 3, 4, 6, 12}) {
-      const int64_t at_once = static_cast<int64_t>(sms) * (12 / w);
-      const int64_t c = (N / (16 * r) + at_once - 1) / at_once * ((steps + w - 1) / w * 4 + 3) * (r == 2 ? 10 : 6);
-      if (rt == 0 || c < cost || (c == cost && r == rt)) { cost = c; rt = r; }
-    }
-  return 0.078 * static_cast<double>(cost) + 0.0125 * static_cast<double>(M * cost) / (rt == 2 ? 10 : 6) + 4;
+  if (!stream_call_plan(M, N, K, gate_up, busy, 0, &fused, &p)) return 1e30;
+  const double tiles = static_cast<double>((p.units + p.clusters - 1) / p.clusters * (fused ? 2 : 1));
+  return p.us + (fused ? 0.35 * tiles : gate_up ? 1.3 : 0) + (busy > 0 ? 1.3 + (gate_up ? 0.25 : 0.1) * tiles : 0);
 }
 
 int stream_forward_launch(const StreamCall& c, bool early, int force, int32_t* status, cudaStream_t stream) {
@@ -709,25 +718,18 @@ int stream_forward_launch(const StreamCall& c, bool early, int force, int32_t* s
   // sixteen tokens at a time, eight where rows are too long for that; more than sixteen are asked for by the tuning hook only
   for (int64_t m0 = 0, rows = 0; m0 < c.M; m0 += rows) {
     const int64_t left = c.M - m0;
-    int nt = left > 8 ? 2 : 1;
-    bool fused = c.h != nullptr;
     const int busy = early && m0 == 0 ? c.busy : 0;
+    bool fused = false;
     StreamPlan pl{};
-    bool found = stream_plan(left < 16 ? left : 16, W->N, W->K, fused, busy, force, &pl);
-    if (fused && nt == 2 && (!found || pl.cl > 1)) {
-      // one warp finishes both halves of a unit, which is too slow for a cluster's (55296 x 5120 at 16 rows 107 us)
-      fused = false;
-      found = stream_plan(left < 16 ? left : 16, W->N, W->K, false, busy, force, &pl);
-    }
-    if (!found) {
-      nt = 1;
-      fused = c.h != nullptr;
-      if (!stream_plan(left < 8 ? left : 8, W->N, W->K, fused, busy, force, &pl)) {
+    rows = left < 16 ? left : 16;
+    if (!stream_call_plan(rows, W->N, W->K, c.h != nullptr, busy, force, &fused, &pl)) {
+      rows = left < 8 ? left : 8;
+      if (!stream_call_plan(rows, W->N, W->K, c.h != nullptr, busy, force, &fused, &pl)) {
         set_detail("weight-streaming kernel: W[%lld,%lld] is too large", static_cast<long long>(W->N), static_cast<long long>(W->K));
         return NF4LL_ERR_SHAPE;
       }
     }
-    rows = left < 8 * nt ? left : 8 * nt;
+    const int nt = rows > 8 ? 2 : 1;
     StreamParams p{};
     p.nib = W->nib; p.qabs = W->qabs; p.scale2 = W->scale2; p.offset2 = W->offset2; p.code2 = W->code2;
     p.K = W->K; p.bpr = static_cast<int>(W->K / 64); p.M = static_cast<int>(rows);

@@ -27,10 +27,9 @@ struct StreamCall {
   uint32_t wait_us;
 };
 
-// What the kernel takes for 9 to 16 tokens, behind other calls and without a rank-16 branch: a fit (nf4ll_stream.cu, stream_us)
-double stream_time_us(int64_t N, int64_t K);
-// Gate|up of 9 to 16 rows goes to the kernel for middling batches where its model is below this
-double stream_gate_up_line_us(int64_t N, int64_t K, int64_t M, int sms);
+// What the kernel takes for M <= 16 tokens, behind other calls: a fit (nf4ll_stream.cu, stream_us). `busy`: CTAs of the rank-16 projection
+// that the call launches before it, 0: none
+double stream_time_us(int64_t M, int64_t N, int64_t K, bool gate_up, int busy);
 // Whether the kernel takes M tokens, eight at a time, against weights of this size: rows as long as eight CTAs hold the tokens of them in
 // registers, 43008 weights, and where a cluster of up to sixteen finds room, twice that
 bool stream_takes(int64_t M, int64_t N, int64_t K, bool gate_up);
