@@ -668,14 +668,30 @@ static int attn_table(SeqTable* t, const int32_t* lens, int n, int at, int64_t* 
 }
 
 // Eight warps per CTA in two halves that take the key blocks in turn, each with a ring of its own, and add up at the end: half as long a
-// chain of blocks per tile. From four blocks in the longest sequence on; with fewer the second half idles and costs shared memory (sequences
-// of 130 and 129 rows, 28 heads of 128, forward 12.5 us with one half, 14.1 with two; of 190 and 150 rows 14.2 and 14.5). us, forward / backward, one half ->
-// two: 4 sequences of 951 rows, 12 heads of 128, 20.7 / 52.3 -> 18.4 / 49.0; 333 rows, 28 heads 19.6 / 53.1 -> 17.6 / 48.0; 1024 rows, 12 heads 44.0 /
-// 121 -> 32.0 / 104; 2048 rows, 28 heads 169 / 477 -> 158 / 460.
-static int attn_halves(const SeqTable& t) {
-  int longest = 0;
-  for (int i = 0; i < t.n; ++i) longest = t.tile[i + 1] - t.tile[i] > longest ? t.tile[i + 1] - t.tile[i] : longest;
-  return longest > 3 ? 2 : 1;
+// chain of blocks per tile, for twice the shared memory. From four blocks in the longest sequence on (with fewer the second half idles:
+// sequences of 130 and 129 rows, 28 heads of 128, forward 12.5 us with one half, 14.1 with two), and where the chain is what takes the time:
+// the forward while one and a half CTAs of one half per SM hold all tiles (two with heads of 64; three of 128 from 16 blocks on), dQ while the
+// SMs' share of all key blocks is less than the longest chain (and a quarter with heads of 64), or from 16 blocks on six CTAs per SM hold them
+// (three of 64). us with one half / two, forward: 12 heads of 128, 333 rows 16.3 / 11.8, 1024
+// rows 40.2 / 32.1, 10 sequences of 200 rows 22.5 / 26.2; 14 heads of 64, 600 rows 18.2 / 12.4, 10 of 200 rows 15.5 / 20.4; 28 heads of 128, 2048 rows
+// 155 / 159; backward with 12 heads of 128, 1024 rows 118 / 104, 14 of 64 and 10 sequences of 200 rows 41.7 / 45.7. Over 398 batches the choice
+// takes 0.2 % longer than the faster of the two, 7 % at worst; always two 4 % and 40 %.
+static int attn_halves(const SeqTable& t, int heads, int hd, bool backward, int* halves) {
+  int dev = 0, sms = 148;
+  NF4LL_CUDA(cudaGetDevice(&dev));
+  NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int64_t longest = 0, blocks = 0;
+  for (int i = 0; i < t.n; ++i) {
+    const int64_t n = t.tile[i + 1] - t.tile[i];
+    longest = n > longest ? n : longest;
+    blocks += n * (n + 1) / 2;
+  }
+  const int64_t ctas = static_cast<int64_t>(t.tile[t.n]) * heads;
+  const bool small = hd == 64, many = longest >= 16;
+  const bool chain = backward ? 4 * blocks * heads < (small ? 5 : 4) * longest * sms || (many && ctas < (small ? 3 : 6) * sms)
+                              : 2 * ctas < (small ? 4 : many ? 6 : 3) * sms;
+  *halves = longest > 3 && chain ? 2 : 1;
+  return NF4LL_OK;
 }
 
 template <int HD>
@@ -691,7 +707,8 @@ static int attn_forward_hd(AttnParams p, const __half* qkv, int64_t ldq, __half*
     const int64_t work = static_cast<int64_t>(t.start[t.n] - t.start[0]) * (p.heads + kv_heads) * (HD / 16);
     PdlLaunch lr(dim3(static_cast<unsigned>((work + 255) / 256 < 1184 ? (work + 255) / 256 : 1184)), dim3(256), 0, stream);
     NF4LL_CUDA(cudaLaunchKernelEx(&lr.cfg, rope_kernel, qkv, ldq, roped, p.ldr, p.trig, p.heads + kv_heads, HD, t));
-    const int halves = attn_halves(t);
+    int halves = 1;
+    if (int rc = attn_halves(t, p.heads, HD, false, &halves)) return rc;
     PdlLaunch lf(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(halves * kAttnThreads), (1 + 4 * halves) * tile, stream);
     NF4LL_CUDA(cudaLaunchKernelEx(&lf.cfg, halves == 2 ? attn_fwd_kernel<HD, 2> : attn_fwd_kernel<HD, 1>, p, t));
   }
@@ -715,7 +732,8 @@ static int attn_backward_hd(AttnParams p, const int32_t* lens, int n, int kv_hea
     const unsigned parts = static_cast<unsigned>(p.group < 8 ? p.group : 8);
     PdlLaunch lk(dim3(static_cast<unsigned>(t.tile[t.n]) * parts, static_cast<unsigned>(kv_heads)), dim3(kAttnThreads), smem_kv, stream, parts, 1);
     NF4LL_CUDA(cudaLaunchKernelEx(&lk.cfg, attn_dkv_kernel<HD>, p, t));
-    const int halves = attn_halves(t);
+    int halves = 1;
+    if (int rc = attn_halves(t, p.heads, HD, true, &halves)) return rc;
     PdlLaunch lq(dim3(static_cast<unsigned>(t.tile[t.n]), static_cast<unsigned>(p.heads)), dim3(halves * kAttnThreads), (2 + 4 * halves) * tile, stream);
     NF4LL_CUDA(cudaLaunchKernelEx(&lq.cfg, halves == 2 ? attn_dq_kernel<HD, 2> : attn_dq_kernel<HD, 1>, p, t));
   }

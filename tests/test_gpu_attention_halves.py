@@ -30,6 +30,19 @@ def test_halves_against_fp64(nh, nkv, hd, lens):
     assert torch.equal(a, a2) and torch.equal(dqkv, stack.PackedAttention.backward(state, da))
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(14, 2, 64), (12, 3, 128)])
+def test_one_half_where_the_tiles_fill_the_device(nh, nkv, hd):
+    """As many tiles as take one half again (forward and dQ), of four blocks and fewer."""
+    lens = [200] * 9 + [256, 1, 130]
+    gen = torch.Generator().manual_seed(nh)
+    qkv = torch.randn(sum(lens), (nh + 2 * nkv) * hd, generator=gen).half().cuda()
+    da = torch.randn(sum(lens), nh * hd, generator=gen).half().cuda()
+    a, state = stack.PackedAttention(nh, nkv, hd, theta=1.0e4).forward(qkv, lens)
+    dqkv = stack.PackedAttention.backward(state, da)
+    ref, dref = reference(qkv, lens, nh, nkv, hd, 1.0e4, da)
+    assert rel(a, ref) <= REL and rel(dqkv, dref) <= REL
+
+
 @pytest.mark.parametrize("blocks", [(0,), (1,), (0, 1), (1, 2)])
 @pytest.mark.parametrize("n", [100, 256, 300])
 def test_keys_that_overflowed_add_nothing(n, blocks):
