@@ -470,26 +470,46 @@ rms_bwd_kernel(const __half* __restrict__ dy16, int64_t lddy, float gscale, cons
   if (gridDim.y > 1) cluster_sync_all();
 }
 
-// CTAs per group of eight rows and 32-column chunks per CTA: as many as find room at once, each warp with a chunk at least. Two per SM
-// in powers of two; clusters of other sizes leave SMs of a GPC idle, and at two per SM some of them wait for a second wave (42 groups in
-// sevens, 2048 columns: 8.5 us against 7.7 in fours; in sixes, 1536 columns, 6.3 against 7.3 in fours). parts = 0: a second wave would be
-// needed, or a row is too long for what is free; then a CTA of sixteen warps takes the whole row (951 rows of 1536 in two waves of clusters: 23.7 us
-// against 20.3). parts = 1 is worth it in the backward only (2048 rows of 1024: 12.6 us against 15.1; forward 9.1 against 8.4).
+// How many clusters of `parts` CTAs of eight warps the current device holds at once. They lie in a GPC each, so not as many as its SMs hold
+// CTAs (two each): 74 clusters of four would, and took two waves (590 rows of 1536 backward 8.3 us, in threes 5.4).
+static int split_clusters(int parts) {
+  constexpr int kDevices = 64;
+  static int known[kDevices][9];               // 0: not asked yet; written with the same value by any thread
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) return 0;
+  int n = __atomic_load_n(&known[dev][parts], __ATOMIC_RELAXED);
+  if (n > 0) return n;
+  const void* kernel = reinterpret_cast<const void*>(rms_bwd_kernel<4, kSplitWarps, true>);
+  PdlLaunch probe(dim3(1, static_cast<unsigned>(parts)), dim3(kSplitWarps * 32), 0, nullptr, 1, static_cast<unsigned>(parts), false, false);
+  probe.cfg.numAttrs = 1;                      // the cluster dimension only
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &probe.cfg) != cudaSuccess) n = 0;
+  if (n > 0) __atomic_store_n(&known[dev][parts], n, __ATOMIC_RELAXED);
+  else (void)cudaGetLastError();
+  return n;
+}
+
+// CTAs per group of eight rows and 32-column chunks per CTA: as many CTAs as find room at once, each warp with a chunk at least. parts = 0: a
+// second wave would be needed (951 rows of 1536 in two waves of clusters: 23.7 us against 20.3), or a row is too long for what is free; then
+// a CTA of sixteen warps takes the whole row. So it does in the backward where pairs would share SMs, unevenly, without the factors' products
+// to keep them busy, or with all of a warp's registers taken: with / without two branches, us, in pairs and by whole rows, 951 rows of 896
+// columns 7.6, 5.1 and 8.8, 4.7; of 1536 13.6, 8.8 and 14.7, 8.8 (700 rows 11.1, 7.3 and 11.5, 7.0); of 2048 19.7, 13.4 and 18.3, 12.4. parts = 1 is
+// worth it in the backward only (2048 rows of 1024: 12.6 us against 15.1; forward 9.1 against 8.4).
 struct NormSplit {
   unsigned groups, parts;
   int chunks, cpw;
 };
-static int norm_split(NormSplit* s, int64_t M, int64_t D) {
+static int norm_split(NormSplit* s, int64_t M, int64_t D, bool backward, bool branches) {
   int dev = 0, sms = 148;
   NF4LL_CUDA(cudaGetDevice(&dev));
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t groups = (M + 7) / 8, all = (D + 31) / 32;
   int64_t parts = 8;
-  auto fits = [&](int64_t n) { return groups * n <= (n & (n - 1) ? 7 : 8) * static_cast<int64_t>(sms) / 4; };
+  auto fits = [&](int64_t n) { return groups <= (n > 1 ? split_clusters(static_cast<int>(n)) : 2 * static_cast<int64_t>(sms)); };
   while (parts > 1 && (!fits(parts) || all < parts * kSplitWarps)) --parts;
   *s = NormSplit{static_cast<unsigned>(groups), 0, 0, 0};
   const int64_t chunks = (all + parts - 1) / parts;
   if (!fits(parts) || chunks > 4 * kSplitWarps) return NF4LL_OK;
+  if (backward && parts == 2 && 2 * groups > sms && !(branches && chunks <= 3 * kSplitWarps)) return NF4LL_OK;
   s->chunks = static_cast<int>(chunks);
   s->parts = static_cast<unsigned>((all + chunks - 1) / chunks);
   s->cpw = static_cast<int>((chunks + kSplitWarps - 1) / kSplitWarps);
@@ -542,7 +562,7 @@ extern "C" int nf4ll_rms_forward(const float* x, const void* delta16, float* xou
   const __half* dl = static_cast<const __half*>(delta16);
   __half* y = static_cast<__half*>(y16);
   NormSplit s;
-  if (int rc = norm_split(&s, M, D)) return rc;
+  if (int rc = norm_split(&s, M, D, false, false)) return rc;
   if (s.parts > 1) {
     PdlLaunch lc(dim3(s.groups, s.parts), dim3(kSplitWarps * 32), 0, st, 1, s.parts);
     const auto kernel = s.cpw <= 1 ? rms_fwd_split_kernel<1> : s.cpw <= 2 ? rms_fwd_split_kernel<2> : s.cpw <= 3 ? rms_fwd_split_kernel<3> : rms_fwd_split_kernel<4>;
@@ -581,7 +601,7 @@ extern "C" int nf4ll_rms_backward(const void* dy16, int64_t lddy, float gscale, 
   const __half* dl = static_cast<const __half*>(delta16);
   __half* o16 = static_cast<__half*>(out16);
   NormSplit s;
-  if (int rc = norm_split(&s, M, D)) return rc;
+  if (int rc = norm_split(&s, M, D, true, ba.A || bb.A)) return rc;
   const auto kernel = !s.parts ? (D <= kNormWarps * 32 * 4 ? rms_bwd_kernel<4, kNormWarps, false> : rms_bwd_kernel<8, kNormWarps, false>)
                       : s.cpw <= 1 ? rms_bwd_kernel<1, kSplitWarps, true> : s.cpw <= 2 ? rms_bwd_kernel<2, kSplitWarps, true>
                       : s.cpw <= 3 ? rms_bwd_kernel<3, kSplitWarps, true> : rms_bwd_kernel<4, kSplitWarps, true>;
