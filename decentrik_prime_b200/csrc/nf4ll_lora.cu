@@ -380,19 +380,23 @@ struct GradProblem {
 };
 
 constexpr int kGradProblems = 6;
+template <int P>
 struct GradBatch {
-  GradProblem problem[kGradProblems];
-  int end[kGradProblems];
-  int n;
+  GradProblem problem[P];
+  int end[P];
 };
 
+// P = 2 for one projection: a CTA's fields come out of either of two constants. Read at an index that is looked up, as of six, they cost each
+// launch 0.1 us and long batches more: 17 rows of 1536 + 1536 columns 2.75 us, 2.82 so, 8192 of 3584 + 18944 126 and 130.
+template <int P>
 __global__ void __launch_bounds__(kGradThreads, 4)
-lora_grad_kernel(const __grid_constant__ GradBatch batch, int64_t M) {
+lora_grad_kernel(const __grid_constant__ GradBatch<P> batch, int64_t M) {
   pdl_wait();
   pdl_launch_dependents();
   int which = 0;
-  while (static_cast<int>(blockIdx.x) >= batch.end[which]) ++which;
-  const GradProblem& pb = batch.problem[which];
+  if (P == 2) which = static_cast<int>(blockIdx.x) >= batch.end[0] ? 1 : 0;
+  else while (static_cast<int>(blockIdx.x) >= batch.end[which]) ++which;
+  const GradProblem& pb = P == 2 ? (which ? batch.problem[1] : batch.problem[0]) : batch.problem[which];
   const __half* __restrict__ act = pb.act;
   const int64_t ldact = pb.ldact;
   const uint8_t* __restrict__ mask = pb.mask;
@@ -408,7 +412,7 @@ lora_grad_kernel(const __grid_constant__ GradBatch batch, int64_t M) {
   const uint32_t ring = smem_u32(g_smem);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
-  const int64_t c0 = static_cast<int64_t>(static_cast<int>(blockIdx.x) - (which ? batch.end[which - 1] : 0)) * kGradCols;
+  const int64_t c0 = static_cast<int64_t>(static_cast<int>(blockIdx.x) - (which == 0 ? 0 : P == 2 ? batch.end[0] : batch.end[which - 1])) * kGradCols;
   const int64_t r_begin = static_cast<int64_t>(blockIdx.y) * rows_per_cta;
   const int64_t r_end = (r_begin + rows_per_cta < M) ? r_begin + rows_per_cta : M;
   float acc[8][4];
@@ -530,21 +534,23 @@ static GradPlan grad_plan(int64_t M, int64_t C, int64_t sms, int64_t other_tiles
 
 // For each of n projections dA = u^T . drop(x) (u carries the LoRA scale, reference solution/fast_qwen.py:1370-1371) and / or
 // dB = scale * dy^T . t (fast_qwen.py:1369), all in one launch: row ranges are as long as one wave of CTAs over all of them allows.
-static int lora_grads_launch(const nf4ll_grad* grads, int n, int64_t M, cudaStream_t stream) {
+template <int P>
+static int lora_grads_run(const nf4ll_grad* grads, int n, int64_t M, cudaStream_t stream) {
   int dev = 0, sms = 148;
   NF4LL_CUDA(cudaGetDevice(&dev));
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  NF4LL_CUDA(cudaFuncSetAttribute(lora_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmemBytes));
+  NF4LL_CUDA(cudaFuncSetAttribute(lora_grad_kernel<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmemBytes));
   int64_t tiles = 0;
   for (int i = 0; i < n; ++i) tiles += (grads[i].dA ? (grads[i].K + kGradCols - 1) / kGradCols : 0) + (grads[i].dB ? (grads[i].N + kGradCols - 1) / kGradCols : 0);
-  GradBatch b{};
+  GradBatch<P> b{};
+  int used = 0;
   int64_t ranges = 1, at = 0;
   auto add = [&](GradProblem pr) {
     const GradPlan g = grad_plan(M, pr.C, sms, tiles - (pr.C + kGradCols - 1) / kGradCols);
     pr.rows_per_cta = g.rows_per;
     at += g.col_tiles;
-    b.problem[b.n] = pr;
-    b.end[b.n++] = static_cast<int>(at);
+    b.problem[used] = pr;
+    b.end[used++] = static_cast<int>(at);
     if (g.msplit > ranges) ranges = g.msplit;
   };
   for (int i = 0; i < n; ++i) {
@@ -553,8 +559,11 @@ static int lora_grads_launch(const nf4ll_grad* grads, int n, int64_t M, cudaStre
     if (g.dB) add(GradProblem{static_cast<const __half*>(g.dy), g.lddy, nullptr, 0, 1.0f, static_cast<const float*>(g.t), g.scale, g.N, 0, static_cast<float*>(g.dB), 1, 16});
   }
   PdlLaunch lc(dim3(static_cast<unsigned>(tiles), static_cast<unsigned>(ranges)), dim3(kGradThreads), kGradSmemBytes, stream);
-  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_grad_kernel, b, M));
+  NF4LL_CUDA(cudaLaunchKernelEx(&lc.cfg, lora_grad_kernel<P>, b, M));
   return NF4LL_OK;
+}
+static int lora_grads_launch(const nf4ll_grad* grads, int n, int64_t M, cudaStream_t stream) {
+  return n == 1 ? lora_grads_run<2>(grads, n, M, stream) : lora_grads_run<kGradProblems>(grads, n, M, stream);
 }
 
 static int clear_grad(const nf4ll_grad& g, cudaStream_t stream) {
