@@ -7,8 +7,8 @@
 // per sequence is the whole gain (through PyTorch: 280 launches per layer and step). The contractions use mma.sync:
 // tiles of 64 rows are too small to feed tcgen05, and at a few microseconds per launch there is nothing to win.
 // Sequence boundaries travel in the kernel parameters, so no copy to the device is needed per batch.
-// That holds for short sequences. One of 2048 rows, 28 heads, takes 618 us forward and backward (171 TFLOP/s, chained by the
-// latencies of mma.sync and ldmatrix at eight warps per SM), one of 4096 rows 2160 (196); the caller
+// That holds for short sequences. One of 2048 rows, 28 heads, takes 624 us forward and backward (169 TFLOP/s, chained by the
+// latencies of mma.sync and ldmatrix at eight warps per SM), one of 4096 rows 2158 (196); the caller
 // (stack.py) takes other kernels for such batches.
 //
 //   rope     q, k rotated once into a buffer (a key row is read by every query tile after it)

@@ -260,10 +260,11 @@ def _rows_aligned(t):
     return t if ok else t.clone(memory_format=torch.contiguous_format)      # contiguous() would hand back a packed view as it is
 
 
-# Times in us of attention forward + backward, fitted to five head layouts and eighteen batches of 128 to 8192 rows (within 15 %):
+# Times in us of attention forward + backward, the library's fitted to nine head layouts and 43 batches of 951 to 8192 rows (within 13 %; the
+# choice takes 0.3 % longer than the faster way, 11 % at worst), PyTorch's to eighteen batches of 128 to 8192 (within 15 %):
 # (start, per query head and pair of rows, per query head and row, per row of the longest sequence) of the library's kernels,
 # (start, per query head and pair of rows, per element of q, k and v, per sequence) of PyTorch's on the GPU.
-_ATTN_OWN_US = {128: (23, 3.75e-6, 1.25e-3, 0.070), 64: (18, 1.69e-6, 0.57e-3, 0.060)}
+_ATTN_OWN_US = {128: (19, 3.56e-6, 1.57e-3, 0.050), 64: (46, 2.06e-6, 0.07e-3, 0.026)}
 _ATTN_TORCH_US = {128: (48, 0.60e-6, 42.8e-6, 65), 64: (66, 0.73e-6, 24.6e-6, 60)}
 _ATTN_TORCH_HOST_US = (630, 210)        # issuing PyTorch's launches, some 70 a sequence: start, per sequence
 _ATTN_SURELY_OWN_ROWS = 1024            # up to here the library's are ahead by those figures for any heads and lengths
@@ -274,9 +275,9 @@ class PackedAttention:
     over all sequences and heads (the library's nf4ll_attention_*; reference solution/k_rope.py, k_attn.py) for fp16 rows on
     the GPU in heads of 64 or 128, PyTorch's kernels per sequence (scaled_dot_product_attention, autograd for the backward)
     for others, and for long sequences: the library's use mma.sync on tiles of 64 rows, which is faster where launches and
-    short sequences count (4 sequences of 951 rows in all, 12 heads of 128: 68 us and 1507), and slower once the products do
-    (one of 2048 rows, 28 heads: 618 us, PyTorch's 557 replayed from a graph and 840 called one by one; of 4096 rows 2160 and
-    1342; 8 of 1024 rows 1317 and 2991). Rotary embedding as in Qwen2: the two halves of a head rotate against each other,
+    short sequences count (4 sequences of 951 rows in all, 12 heads of 128: 67 us and 1507), and slower once the products do
+    (one of 2048 rows, 28 heads: 624 us, PyTorch's 561 replayed from a graph and 868 called one by one; of 4096 rows 2158 and
+    1350; 8 of 1024 rows 1270 and 2940). Rotary embedding as in Qwen2: the two halves of a head rotate against each other,
     positions restart at every sequence."""
 
     def __init__(self, n_heads, n_kv_heads, head_dim, theta=1.0e6):

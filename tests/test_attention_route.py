@@ -6,12 +6,15 @@ import pytest
 from decentrik_prime_b200 import stack
 
 MEASURED = [
-    (28, 4, 128, [1024], 234, 323, 840), (28, 4, 128, [2048], 655, 557, 840), (28, 4, 128, [3072], 1359, 860, 996), (28, 4, 128, [4096], 2257, 1215, 1342),
-    (28, 4, 128, [1024] * 8, 1317, 2578, 2992), (28, 4, 128, [512] * 16, 810, 3294, 4117), (28, 4, 128, [227, 277, 365, 82], 114, 467, 1622),
-    (12, 2, 128, [951], 161, 215, 872), (12, 2, 128, [3072], 650, 432, 928), (12, 2, 128, [6144], 2168, 892, 1028),
-    (40, 8, 128, [1024], 300, 409, 847), (40, 8, 128, [4096], 3074, 1790, 1937), (40, 8, 128, [2048] * 4, 3172, 3465, 3732),
-    (14, 2, 64, [1024], 122, 177, 853), (14, 2, 64, [4096], 647, 424, 887), (14, 2, 64, [6144], 1316, 655, 868), (14, 2, 64, [2048] * 4, 636, 797, 1480),
-    (16, 16, 64, [2048], 254, 315, 807), (16, 16, 64, [6144], 1498, 947, 1067), (16, 16, 64, [64] * 64, 60, 4000, 12477),
+    (28, 4, 128, [1024], 220, 303, 830), (28, 4, 128, [2048], 624, 561, 868), (28, 4, 128, [3072], 1294, 866, 1001),
+    (28, 4, 128, [4096], 2158, 1218, 1350), (28, 4, 128, [1024] * 8, 1270, 2518, 2940), (28, 4, 128, [512] * 16, 784, 3315, 4063),
+    (28, 4, 128, [227, 277, 365, 82], 106, 431, 1428), (12, 2, 128, [951], 126, 227, 826), (12, 2, 128, [3072], 588, 434, 807),
+    (12, 2, 128, [6144], 2057, 876, 1040), (40, 8, 128, [1024], 281, 415, 813), (40, 8, 128, [4096], 2935, 1769, 1939),
+    (40, 8, 128, [2048] * 4, 3046, 3436, 3734), (14, 2, 64, [1024], 100, 182, 801), (14, 2, 64, [4096], 625, 429, 836),
+    (14, 2, 64, [6144], 1278, 658, 839), (14, 2, 64, [2048] * 4, 620, 799, 1411), (16, 16, 64, [2048], 235, 322, 802),
+    (16, 16, 64, [6144], 1467, 945, 1075), (28, 4, 128, [1500], 398, 440, 797),
+    (12, 2, 128, [2500], 428, 389, 926), (14, 2, 64, [2048], 228, 248, 794), (14, 2, 64, [3072], 377, 340, 832),
+    (12, 2, 128, [2048] * 2, 550, 584, 1004), (28, 4, 128, [200] * 20, 317, 2264, 4429), (8, 2, 64, [2048], 178, 211, 802),
 ]
 
 
