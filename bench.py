@@ -40,9 +40,6 @@ HIDDEN, INTER, M_ROWS, P_DROP = 1536, 8960, 2048, 0.05
 WORKLOAD = "qwen2.5-1.5b-mlp-block-M2048"
 METRIC = "nf4_lora_linear_fwd_bwd_tflops_M2048"
 N_WEIGHT_SETS, N_INPUT_SETS = 8, 4
-# mean DRAM bytes (read + written) per tensor-core launch of a step, from an ncu capture of one step (not a
-# measurement of this run); reported with that label
-NCU_DRAM_BYTES_PER_LAUNCH = 53.0e6
 CPU_BUDGET_S = 100.0
 # timed steps whose tensor-core launches are bracketed by events: every 49th (49 and the 8 weight sets are coprime). Such a
 # step is issued from Python instead of replayed from its graph, which costs host time (0.5 ms here, 2 ms on a slow
@@ -491,14 +488,14 @@ def run_ours(args):
                                                             else " sustained bf16 (timed region over 1 s)"),
                              "frac_of_burst": (achieved / pk["tflops_burst"]) if achieved else None,
                              "frac_of_sustained": (achieved / pk["tflops_sustained"]) if achieved else None,
-                             "traffic": NCU_DRAM_BYTES_PER_LAUNCH,
-                             "traffic_source": "ncu capture of one step (mean DRAM bytes read + written per tensor-core launch, five of them: "
-                                               "gate and up apart in the backward), not a measurement of this run",
+                             "traffic": None,
+                             "traffic_source": "not captured for these four launches",
                              # NF4 bytes of the six weight passes of a step + every activation matrix a launch reads or
                              # writes (x, g, u, h | h, y | dy, dh | dg, du, dx read + written), over the four launches
                              "algorithmic_bytes_per_launch": (6 * INTER * HIDDEN * 0.516113
                                                               + 2 * M * (5 * HIDDEN + 7 * INTER)) / 4,
-                             "kernel": "nf4_gemm_kernel / nf4_gemm_pair_kernel (forward and backward-dX launches)",
+                             "kernel": "dense_gemm_kernel behind dequant_kernel (gate|up forward, dX of down), nf4_gemm_kernel (down forward), "
+                                       "nf4_gemm_pair_kernel (dX of gate|up)",
                              "events": events_where,
                              "launches_timed": n_kern, "avg_launch_us": kern_ms * 1e3 / max(n_kern, 1)},
                 "e2e": {"value": e2e_val, "unit": "TFLOP/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h,
