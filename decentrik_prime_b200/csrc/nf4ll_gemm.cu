@@ -1249,7 +1249,7 @@ constexpr int64_t kStreamCapRows = 64;     // its limit (reachable through the t
 // at 9 rows 40.9 / 40.1, with LoRA 49.9 / 42.9; 9344 x 11008 32.9 / 27.9; 27648 x 5120 at 16 rows 34.4 / 35.3; 18944 x 3584 18.6 / 18.7; 10240 x 5120
 // at 12 rows 16.2 / 20.2; 4096 x 4096 at 9 rows 9.0 / 11.1; gate|up of 28672 x 4096 35.0 / 32.0, with LoRA 41.2 / 34.4, of 18944 x 3584 18.6 / 21.0, of
 // 27648 x 1024 15.5 / 12.2, of 11008 x 2048 10.9 / 13.5. Over 1170 such calls (60 weights at 9, 12 and 16 rows, single, stacked and gate|up,
-// with LoRA and without) the choice takes 0.4 % longer than the faster kernel, 12 % at worst. Against fp64 sums over the fp16
+// with LoRA and without) the choice takes 0.3 % longer than the faster kernel, 11 % at worst. Against fp64 sums over the fp16
 // weights, which are the result that this path is held to, the rel-L2 is 3.4e-4 in the streaming kernel and 2.1e-4 in this one; over the
 // unrounded weights 2.8e-4 and 2.9e-4. From 17 rows on the latter is ahead everywhere (1536 x 1536 at 17 rows 7.5; the streaming
 // kernel 3.8 at 16).
@@ -1459,7 +1459,14 @@ static bool mid_wanted(const MidCall& c, const RowTimes& t, bool dense, bool lor
     if (!stream_takes(c.M, N, K, c.gu_inter != 0)) return mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp);
     if (c.M < kMidLeastRows || !mid_plan(kFwd, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
     const int busy = branches > 0 ? lora_down_ctas(c.M, K, branches < 2 ? 1 : 2, sms) : 0;
-    return mp->us + (c.gu_inter ? 1.3 : 0.8) + (branches > 0 ? 2.6 : 0) < stream_time_us(c.M, N, K, c.gu_inter != 0, busy);
+    double us = mp->us + (c.gu_inter ? 1.3 : 0.8);
+    if (branches > 0) {
+      // and more where its clusters do not all find room beside the projection (as the streaming kernel's, stream_search): 1920 x 22528
+      // Q|K|V at 9 rows 26.0 us, streaming 19.4
+      const int others = (sms - busy) / mp->cl, fewer = mp->cl == 1 ? others : mid_clusters(mp->cl) - 2;
+      us += 2.6 + (mp->clusters > (fewer < others ? fewer : others) ? (branches < 2 ? 1 : 2) * 0.00011 * static_cast<double>(K) : 0);
+    }
+    return us < stream_time_us(c.M, N, K, c.gu_inter != 0, busy);
   }
   if (!mid_plan(c.mode, c.M, NO, KC, mask, c.gu_inter, lora, 0, 0, 0, mp)) return false;
   if (c.M <= kDenseNeverRows) return true;

@@ -830,7 +830,7 @@ static int mid_encode(CUtensorMap* map, CUtensorMapDataType type, const void* ba
 }
 
 // How many clusters of `cl` CTAs the current device holds at once (148, 74, 45, 33, 26, 22, 15, 15 for 1 to 8 on the B200s at hand)
-static int mid_clusters(int cl) {
+int mid_clusters(int cl) {
   constexpr int kDevices = 64;
   static int known[kDevices][9];               // 0: not asked yet; written with the same value by any thread
   int dev = 0;

@@ -45,6 +45,7 @@ struct MidPlan {
 
 // rb / nt / cl forced where not zero (tests). False: this kernel does not take the call.
 bool mid_plan(int mode, int64_t M, int64_t NO, int64_t KC, bool mask, int64_t gu_inter, bool lora, int rb, int nt, int cl, MidPlan* plan);
+int mid_clusters(int cl);    // clusters of `cl` CTAs that the current device holds at once
 int64_t mid_searches();      // plans that the calling thread had to search for so far
 int64_t mid_calls();         // calls of the thread that this kernel has taken
 // `early`: the kernel launched right before on the stream is one of the same call that does not write act or the weight
