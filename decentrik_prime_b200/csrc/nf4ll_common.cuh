@@ -283,6 +283,10 @@ __device__ __forceinline__ void cluster_wait() {
   __syncwarp();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same right behind a barrier of the block or the warp, where the lanes are together (with the __syncwarp the kernel for middling batches
+// took 0.2 to 0.4 % longer).
+__device__ __forceinline__ void cluster_arrive_together() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait_together() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 __device__ __forceinline__ void cluster_sync_all() {
   cluster_arrive();
   asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");

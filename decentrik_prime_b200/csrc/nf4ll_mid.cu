@@ -261,7 +261,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     sLv[threadIdx.x] = v;
   }
   __syncthreads();                             // barriers and levels are there
-  if (cl > 1) cluster_arrive();
+  if (cl > 1) cluster_arrive_together();
   // the two producers go on at once; the others lay out the tables first. Nothing before pdl_wait() reads global memory.
   if (warp != 0 && warp != 2) {
     if (warp == 1) {
@@ -521,7 +521,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     // Four warps of their own finish a unit while the next one is decoded; the decoding warps help with the last one. A crew
     // is four warps, one per lane quarter of tensor memory.
     if (p.early) pdl_wait();                     // the rank-16 products come from the kernel before this one
-    if (cl > 1) cluster_wait();
+    if (cl > 1) cluster_wait_together();
     const int crew = (warp - kMidEpiWarp) >> 2;
     const int q = warp & 3, r = q * 32 + lane, tid = threadIdx.x - kMidEpiWarp * 32;
     const int last = (p.units - 1 - cluster) / n_clusters;                 // the cluster's last unit, counted from 0
@@ -794,7 +794,7 @@ nf4_mid_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
   // ------------------------------------------------------------------------------- teardown
   tc_fence_before();
   __syncwarp();
-  if (cl > 1 && warp < kMidEpiWarp) cluster_wait();
+  if (cl > 1 && warp < kMidEpiWarp) cluster_wait_together();
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
