@@ -16,8 +16,9 @@ def rand(*shape, scale=1.0, seed=0):
     return (torch.randn(*shape, generator=gen) * scale).to(DEV)
 
 
-# stages of 16 rows, row ranges of several of them, warps of 64 and CTAs of 256 columns, 16-byte pieces of the mask
-@pytest.mark.parametrize("M,I", [(1, 8), (15, 40), (16, 256), (17, 264), (33, 2056), (187, 1000), (600, 8960), (4801, 520)])
+# stages of 16 rows, row ranges of several of them, warps of 32 and CTAs of 128 columns, 16-byte pieces of the mask
+@pytest.mark.parametrize("M,I", [(1, 8), (5, 24), (9, 32), (15, 40), (20, 120), (16, 128), (33, 136), (16, 256), (17, 264), (33, 2056), (187, 1000),
+                                 (600, 8960), (4801, 520)])
 @pytest.mark.parametrize("masked,accumulate", [(True, True), (False, False)])
 def test_gated_backward_with_lora(M, I, masked, accumulate):
     gu, dh = rand(M, 2 * I, seed=1).half(), rand(M, I + 8, seed=2).half()[:, :I]

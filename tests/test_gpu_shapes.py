@@ -99,8 +99,8 @@ def test_kernel_for_middling_batches_under_the_tuning_flag(N, K, M):
 
 @pytest.mark.parametrize("M", [17, 32, 33, 64])
 def test_streaming_kernel_forced_up_to_64_rows(M):
-    """The register-level weight-streaming kernel with four and eight token tiles (17..64 rows), which the
-    default dispatch never picks: forced through the tuning hook."""
+    """The weight-streaming kernel in passes of sixteen tokens (17..64 rows), which the default dispatch never picks: forced
+    through the tuning hook."""
     for N, K in ((256, 256), (256, 384)):
         pr = make_problem(N, K, M, seed=3200 + N + K + M, lora=True, dropout=0.05, bias=True)
         ref = nf4_oracle.lora_linear_o1(oracle_weight(pr), pr.x, None, pr.bias, pr.A16, pr.B16, pr.scale, pr.mask, pr.keep_scale)
