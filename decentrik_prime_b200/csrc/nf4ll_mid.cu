@@ -1,4 +1,5 @@
-// Middling batches (17 to some hundreds of token rows, 2560 against small weights), forward and backward-dX: the WEIGHTS are the 128-row operand of
+// Middling batches (17 to some hundreds of token rows, 2560 against small weights; from 9 on where it is ahead of the
+// streaming kernel), forward and backward-dX: the WEIGHTS are the 128-row operand of
 // tcgen05.mma, the tokens its N operand (any multiple of 16 up to 240 columns, 224 with LoRA: what shared memory holds two tiles of), the contraction is cut over the CTAs of a
 // thread-block cluster. Serves the reference call sites solution/fast_qwen.py:947, 1037, 1080-1112 and, backward, 1310-1364.
 //

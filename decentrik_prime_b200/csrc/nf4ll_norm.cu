@@ -199,8 +199,8 @@ rms_fwd_kernel(const float* __restrict__ x, const __half* __restrict__ delta, fl
 // which share out the columns. The row sums meet through distributed shared memory, every CTA adding them up in rank order, and the
 // rank-16 products in the first CTA likewise. Such a batch is bound by the chain load - sum - products - store of one CTA, so what
 // counts is how little of a row a CTA has, and that the loads of the second phase are on their way before the sum: one CTA of sixteen
-// warps per 16 (D > 2048: 8) rows against this, us, with two branches / without: 1536 columns, 8 rows 9.7 / 4.9 -> 4.6 / 2.9, 333 rows 13.2 / 7.4 ->
-// 6.2 / 3.9, 951 rows 20.2 / 9.4 -> 14.1 / 7.4; 3584 columns, 8 rows 15.2 / 9.0 -> 5.7 / 3.4, 333 rows 22.1 / 9.7 -> 11.8 / 6.2.
+// warps per 16 (D > 2048: 8) rows against this, us, with two branches / without, three sets of operands in turn: 1536 columns, 8 rows 9.3 / 4.7 ->
+// 4.4 / 2.7, 333 rows 12.3 / 7.1 -> 6.0 / 3.7, 951 rows 12.5 / 7.2 -> 9.0 / 5.5; 3584 columns, 8 rows 14.3 / 8.6 -> 5.3 / 3.2, 333 rows 14.6 / 8.8 -> 8.4 / 5.1.
 // ---------------------------------------------------------------------------------------------
 constexpr int kSplitWarps = 8;
 
@@ -351,10 +351,10 @@ rms_fwd_split_kernel(const float* __restrict__ x, const __half* __restrict__ del
 // right operand for columns 8 i + 2 w, + 1 (i = 0..3), so that over w = 0..3 lane (g, t) ends with its own columns 8 t .. + 7 of row g. u
 // goes in three fp16 parts under a power of two per row that brings its largest rank to [2^14, 2^15): all 24 bits of every rank down to
 // 2^-15 of the largest; of smaller ones what is above 2^-40 of the largest.
-// With fp32 FMAs it was 32 loads, 256 conversions and 256 FMAs per lane and chunk, and the larger error against fp64 (9.5e-8 of the
-// result's norm at u of 1 with 1536 columns, 7.2e-8 so). us with two branches / without, one CTA and FMAs before: 1536 columns, 8 rows 13.1 / 6.0 ->
-// 4.6 / 3.0, 951 rows 22.3 / 11.1 -> 15.6 / 10.6, 2048 rows (a CTA per group) 41.4 / 20.9 -> 31.5 / 20.4; 3584 columns, 333 rows 59.8 / 20.5 ->
-// 14.2 / 9.6, 2048 rows 120 / 45 -> 68 / 42.
+// With fp32 FMAs it was 32 loads, 256 conversions and 256 FMAs per lane and chunk, and the larger error against fp64 (8.6e-8 of the
+// result's norm at u of 1 with 1536 columns, 6.6e-8 so). us with two branches / without, one CTA and FMAs before, three sets of operands in turn: 1536
+// columns, 8 rows 12.6 / 5.8 -> 4.4 / 2.9, 951 rows 16.7 / 8.6 -> 12.7 / 8.3, 2048 rows (a CTA per group) 39.0 / 20.6 -> 31.1 / 20.1; 3584 columns,
+// 333 rows 33.7 / 13.4 -> 10.8 / 6.9, 2048 rows 117 / 45 -> 68 / 42.
 template <int CPW, int NW, bool KEEP>
 __global__ void __launch_bounds__(NW * 32, NW == kSplitWarps ? 2 : 1)
 rms_bwd_kernel(const __half* __restrict__ dy16, int64_t lddy, float gscale, const float* __restrict__ x, const __half* __restrict__ delta,

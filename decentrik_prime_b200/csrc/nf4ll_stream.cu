@@ -12,8 +12,8 @@
 //
 // Every BYTE of codes (two 4-bit codes) becomes two fp16 levels with ONE shared-memory load from a 256-entry table of half2 pairs,
 // replicated per lane (lane l reads word l of an entry: no bank conflicts whatever the codes are) at a stride of 256 B, which makes the byte
-// permute that isolates a code byte the whole address computation; the other 128 B of an entry hold partial sums. The levels land
-// directly in the A-operand layout of mma.sync.m16n8k16; the token rows are the B operand with the same column-to-slot assignment. The
+// permute that isolates a code byte the whole address computation; the other 128 B of an entry hold partial sums and scaled rank-16
+// products. The levels land directly in the A-operand layout of mma.sync.m16n8k16; the token rows are the B operand with the same column-to-slot assignment. The
 // 64 weights of a block are accumulated on their own and folded into the running sum with that block's fp32 absmax, so the scale is
 // applied once per block:
 //     y[m,n] = sum_blocks absmax[n,b] * sum_{k in b} x[m,k] * fp16(NF4[code[n,k]])

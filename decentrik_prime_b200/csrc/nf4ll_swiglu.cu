@@ -10,8 +10,9 @@ namespace nf4ll {
 
 // Both kernels are one pass at memory speed: a thread takes several 16-byte chunks per trip, all loads of the trip issued before the
 // arithmetic, so that every SM keeps enough bytes in flight. T: how wide a chunk's number is (its row comes out of a division, which
-// took a good part of a trip in 64 bits). us at 16384 x 18944 / 2048 x 8960 / 951 x 8960 / 187 x 8960, backward: 511 / 32.2 / 16.2 / 4.6 with two
-// chunks per trip and 64-bit divisions for all, 480 / 30.8 / 15.5 / 2.9 now; forward 343 / 22.2 / 11.7 / 3.2, now 304 / 19.6 / 10.6 / 2.9.
+// took a good part of a trip in 64 bits). us at 16384 x 18944 / 2048 x 8960 / 951 x 8960 / 187 x 8960, operands
+// out of HBM, with two chunks per trip and 64-bit divisions for all and now: backward 479 / 30.9 / 15.5 / 4.6 and 480 / 30.0 / 15.1 / 4.1, forward 347 /
+// 22.8 / 11.4 / 3.3 and 305 / 19.9 / 9.8 / 3.0.
 template <typename T, int U>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __half* __restrict__ g, int64_t ldg, const __half* __restrict__ u, int64_t ldu,
