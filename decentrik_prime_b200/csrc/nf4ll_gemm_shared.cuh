@@ -58,7 +58,8 @@ struct GemmParams {
 template <typename P, int KEYS>
 class KeptPlans {
  public:
-  // `search` fills in a plan and says whether there is one
+  // `search` fills in a plan and says whether there is one; where not, the next call asks again (a query of the device may have failed for
+  // want of memory)
   template <typename F>
   bool get(const int64_t (&key)[KEYS], P* plan, F&& search) {
     uint64_t h = 0;
@@ -71,23 +72,22 @@ class KeptPlans {
       if (same) {
         set[w].used = ++clock_;
         *plan = set[w].plan;
-        return set[w].found;
+        return true;
       }
       if (set[w].used < e->used) e = set + w;
     }
     for (int i = 0; i < KEYS; ++i) e->key[i] = key[i];
     e->plan = P{};
-    e->found = search(&e->plan);
-    e->used = ++clock_;
+    const bool found = search(&e->plan);
+    e->used = found ? ++clock_ : 0;
     *plan = e->plan;
-    return e->found;
+    return found;
   }
 
  private:
   struct Kept {
     int64_t key[KEYS];
     P plan;
-    bool found;
     uint64_t used;               // 0: empty
   };
   Kept kept_[64][4];
