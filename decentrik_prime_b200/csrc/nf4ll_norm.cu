@@ -488,7 +488,10 @@ static int split_clusters(int parts) {
   return n;
 }
 
-// CTAs per group of eight rows and 32-column chunks per CTA: as many CTAs as find room at once, each warp with a chunk at least. parts = 0: a
+// CTAs per group of eight rows and 32-column chunks per CTA: as many CTAs as find room at once, behind another kernel, each warp with a chunk at
+// least. Backward in a row of calls without branches and with two, us: 54 groups of 1536 columns, two chunks to a warp either way, by fives, of which
+// the device holds 56, 5.7 and 8.8, by fours 4.9 and 7.2; 36 of 3584 columns by sevens, of which it holds 37, two chunks, 5.6 and 8.5, by sixes,
+// three chunks, 6.8 and 10.4. parts = 0: a
 // second wave would be needed (951 rows of 1536 in two waves of clusters: 23.7 us against 20.3), or a row is too long for what is free; then
 // a CTA of sixteen warps takes the whole row. So it does in the backward where pairs would share SMs, unevenly, without the factors' products
 // to keep them busy, or with all of a warp's registers taken: with / without two branches, us, in pairs and by whole rows, 951 rows of 896
@@ -504,7 +507,14 @@ static int norm_split(NormSplit* s, int64_t M, int64_t D, bool backward, bool br
   NF4LL_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int64_t groups = (M + 7) / 8, all = (D + 31) / 32;
   int64_t parts = 8;
-  auto fits = [&](int64_t n) { return groups <= (n > 1 ? split_clusters(static_cast<int>(n)) : 2 * static_cast<int64_t>(sms)); };
+  // Clusters that find no room while the kernel before this one still holds SMs come a wave later: the last two of most sizes, of fives and
+  // threes more. That costs more than a CTA less to a row would, unless its warps then had another chunk to go through (second line).
+  constexpr int kWait[2][9] = {{0, 0, 0, 3, 2, 5, 2, 2, 2}, {0, 0, 0, 1, 0, 1, 0, 0, 0}};
+  auto warp_chunks = [&](int64_t n) { return ((all + n - 1) / n + kSplitWarps - 1) / kSplitWarps; };
+  auto fits = [&](int64_t n) {
+    if (n == 1) return groups <= 2 * static_cast<int64_t>(sms);
+    return groups <= split_clusters(static_cast<int>(n)) - kWait[warp_chunks(n) < warp_chunks(n - 1)][n];
+  };
   while (parts > 1 && (!fits(parts) || all < parts * kSplitWarps)) --parts;
   *s = NormSplit{static_cast<unsigned>(groups), 0, 0, 0};
   const int64_t chunks = (all + parts - 1) / parts;
